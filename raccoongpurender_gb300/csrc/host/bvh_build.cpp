@@ -374,7 +374,7 @@ int build_bvh(rgr_scene* s, const rgr_bvh_params& params) {
             pb.c[k] = 0.5f * (pb.lo[k] + pb.hi[k]);
         }
         PrimD& r = records[t];
-        uint32_t pid = (uint32_t)t;
+        uint32_t pid = prim_word((uint32_t)t, s->tri_materials[t].type);
         for (int k = 0; k < 3; ++k) {
             r.a[k] = v[0][k];
             r.b[k] = v[1][k] - v[0][k];  // bit-identical to the kernel's v1 - v0
@@ -393,7 +393,7 @@ int build_bvh(rgr_scene* s, const rgr_bvh_params& params) {
             pb.c[k] = sp[k];
         }
         PrimD& r = records[ntri + i];
-        uint32_t pid = (uint32_t)(ntri + i), flag = 1;
+        uint32_t pid = prim_word((uint32_t)(ntri + i), s->sphere_materials[i].type), flag = 1;
         r.a[0] = sp[0];
         r.a[1] = sp[1];
         r.a[2] = sp[2];

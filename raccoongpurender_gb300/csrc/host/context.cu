@@ -153,8 +153,14 @@ RequestD request_d(const SceneView& sv, const rgr_camera& cam, const rgr_render_
 
 }  // namespace
 
-// scenes with fewer inner BVH nodes run the fused trace + logic kernel by default
-constexpr uint32_t kPersistentTraceMinNodes = 4096;
+// Pools of fewer paths run the fused trace + logic kernel by default (a bounce is then
+// bound by its launches' latency and the longest ray of each warp), larger ones the
+// persistent refilling cast and, inside a run of bounces, no logic pass (launch_inner).
+// Whole renders (4 spp, depth 6), persistent against fused, at 2^17 / 2^18 / 2^19 / 2^20 /
+// 2^22 paths: 36 triangles 0.84 / 0.98 / 1.12 / 1.24 / 1.36x, 5 K 0.80 / 1.00 / 1.17 / 1.39 /
+// 1.69x, 330 K 0.84 / 0.99 / 1.25 / 1.52 / 2.06x.  Single bounces at 2^18 / 2^20 / 2^22:
+// 36 triangles 0.87 / 1.00 / 1.07x, 5 K 0.96 / 1.22 / 1.40x.
+constexpr uint32_t kPersistentTraceMinPaths = 3u << 17;
 // rgr_trace_closest: 2^20-ray chunks in flight on their own streams, so that
 // the copies of some overlap the traversal of another (measured end to end
 // on the closest-hit workload: 2 slots 2500 Mrays/s, 3: 2647, 4: 2705-2728,
@@ -170,6 +176,8 @@ struct rgr_context {
     DeviceScene scene;
     // paths
     DevBuf slots, qid, req, queues[kNumQueues], counts, tile_new, scalars, accum, err;
+    DevBuf inner_words, inner_tiles, inner_ended;  // the bounces inside a run (launch_inner)
+    InnerView in{};
     DevBuf reqtab, done;  // request table and its per-request (done, done_ns) counters
     PathsView pv{};
     QueueView qv{};
@@ -187,8 +195,11 @@ struct rgr_context {
     bool graph_mode = true;
     int graph_steps = 1;
     int graph_steps_default = 1;
-    cudaGraphExec_t graph_exec = nullptr;
-    std::string graph_exec_key;  // graph_key() when graph_exec was captured
+    struct Graph {
+        cudaGraphExec_t exec = nullptr;
+        std::string key;  // graph_key() when it was captured
+    };
+    Graph step_graph, inner_graph;  // whole bounces; bounces inside a run (launch_inner)
     // ray-cast service buffers
     DevBuf trays[7], tprim, tt, tread, tcounter;
     // rgr_trace_closest pipeline: kTraceSlots stream slots, each with its chunk's buffers
@@ -208,7 +219,7 @@ struct rgr_context {
     // 1059.5 Mpaths/s with a warp refilled at 24 / 8 / 12 / 16 / 20 idle lanes
     // search 8: 1114.8 Mpaths/s against 1032.8 with every lane waiting for the last
     TraceShape render_trace{true, 12, 8, 0, nullptr};
-    int render_trace_mode = -1;  // 1 persistent, 0 fused, -1 by scene size at render begin
+    int render_trace_mode = -1;  // 1 persistent, 0 fused, -1 by the pool's size at render begin
     uint32_t trace_stage = 0;  // top BVH nodes staged in shared memory per CTA
     int trace_reorder = 0;     // rgr_trace_closest_device sorts the rays first
     int packed_grid = 0;       // its traversal grid (no staged nodes)
@@ -220,7 +231,7 @@ struct rgr_context {
     float scene_bounds[6] = {0, 0, 0, 0, 0, 0};
 
     ~rgr_context() {
-        if (graph_exec) cudaGraphExecDestroy(graph_exec);
+        drop_graph();
         for (cudaStream_t s : tstream)
             if (s) cudaStreamDestroy(s);
         if (stream) cudaStreamDestroy(stream);
@@ -239,6 +250,9 @@ struct rgr_context {
         AL(tile_new, 4 * (size_t)ntiles);
         AL(scalars, 8 * 8);
         AL(err, 16);
+        AL(inner_words, sizeof(uint32_t) * InnerView::kWords);
+        AL(inner_tiles, 4 * (size_t)ntiles);
+        AL(inner_ended, 2 * n);
 #undef AL
         PathsView& p = pv;
         p.set_slots(slots.p);
@@ -250,6 +264,9 @@ struct rgr_context {
         q.counts = counts.as<uint32_t>();
         q.tile_new = tile_new.as<uint32_t>();
         q.ntiles = ntiles;
+        in.words = inner_words.as<uint32_t>();
+        in.tile_first = inner_tiles.as<uint32_t>();
+        in.ended = inner_ended.as<uint16_t>();
         unsigned long long* sc = scalars.as<unsigned long long>();
         q.next_pixel = sc + 0;
         q.step_base = sc + 1;
@@ -262,15 +279,8 @@ struct rgr_context {
     int start(const RequestD* host_reqs, int nreq, unsigned long long limit, uint32_t seed_offset) {
         cudaStream_t st = stream;
         int r;
-        if (render_trace_mode < 0) {
-            // the separate persistent trace kernel pays for its launch when traversal
-            // dominates (measured: +11 % on 1.3M triangles, -30 % on 36)
-            uint32_t nodes = 0;
-            for (int k = 0; k < nreq; ++k) nodes = std::max(nodes, host_reqs[k].sc.num_nodes);
-            render_trace.persistent = nodes >= kPersistentTraceMinNodes;
-        } else {
-            render_trace.persistent = render_trace_mode != 0;
-        }
+        render_trace.persistent =
+            render_trace_mode < 0 ? npaths >= kPersistentTraceMinPaths : render_trace_mode != 0;
         if ((r = reqtab.alloc(sizeof(RequestD) * nreq)) != RGR_OK) return r;
         RGR_CUDA(cudaMemcpyAsync(reqtab.p, host_reqs, sizeof(RequestD) * nreq, cudaMemcpyHostToDevice, st));
         rp.reqs = reqtab.as<RequestD>();
@@ -357,45 +367,142 @@ struct rgr_context {
         guided = true;
         return RGR_OK;
     }
-    // run `n` bounces: replays of a graph of graph_steps bounces, then single ones
-    int run_steps(int n) {
+    // launch `g`, captured first by `launches` if there is none for the current parameters
+    template <class F>
+    int replay(Graph& g, F launches) {
         cudaStream_t st = stream;
+        const std::string key = graph_key();
+        if (g.exec && key != g.key) {
+            cudaGraphExecDestroy(g.exec);
+            g.exec = nullptr;
+        }
+        if (!g.exec) {
+            g.key = key;
+            cudaGraph_t cg = nullptr;
+            RGR_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+            const int r = launches();
+            cudaError_t e = cudaStreamEndCapture(st, &cg);
+            if (r != RGR_OK) return r;
+            RGR_CUDA(e);
+            e = cudaGraphInstantiate(&g.exec, cg, 0);
+            cudaGraphDestroy(cg);
+            RGR_CUDA(e);
+        }
+        RGR_CUDA(cudaGraphLaunch(g.exec, st));
+        return RGR_OK;
+    }
+    // run `n` bounces.  A plain render takes the bounces inside the run by
+    // launch_inner; otherwise replays of a graph of graph_steps bounces, then
+    // single ones
+    int run_steps(int n) {
+        if (n > 1 && inner()) {
+            int r = run_first();
+            if (r == RGR_OK) r = run_inner(n - 1);
+            if (r == RGR_OK) r = run_last();
+            if (r == RGR_OK) steps += n;
+            return r;
+        }
         while (n > 0) {
-            if (graph_mode) {
-                const int k = n >= graph_steps ? graph_steps : 1;
-                if (k == graph_steps || graph_steps == 1) {
-                    const std::string key = graph_key();
-                    if (graph_exec && key != graph_exec_key) drop_graph();
-                    if (!graph_exec) {
-                        graph_exec_key = key;
-                        cudaGraph_t g = nullptr;
-                        RGR_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-                        int r = RGR_OK;
-                        for (int i = 0; i < graph_steps && r == RGR_OK; ++i)
-                            r = step_launches(st, (i + 1) % train_interval() == 0);
-                        cudaError_t e = cudaStreamEndCapture(st, &g);
-                        if (r != RGR_OK) return r;
-                        RGR_CUDA(e);
-                        e = cudaGraphInstantiate(&graph_exec, g, 0);
-                        cudaGraphDestroy(g);
-                        RGR_CUDA(e);
-                    }
-                    RGR_CUDA(cudaGraphLaunch(graph_exec, st));
-                    n -= graph_steps;
-                    steps += graph_steps;
-                    continue;
-                }
+            if (graph_mode && (n >= graph_steps || graph_steps == 1)) {
+                int r = replay(step_graph, [&] {
+                    int q = RGR_OK;
+                    for (int i = 0; i < graph_steps && q == RGR_OK; ++i)
+                        q = step_launches(stream, (i + 1) % train_interval() == 0);
+                    return q;
+                });
+                if (r != RGR_OK) return r;
+                n -= graph_steps;
+                steps += graph_steps;
+                continue;
             }
-            int r = step_launches(st, (steps + 1) % (uint64_t)train_interval() == 0);
+            int r = step_launches(stream, (steps + 1) % (uint64_t)train_interval() == 0);
             if (r != RGR_OK) return r;
             n -= 1;
             steps += 1;
         }
         return RGR_OK;
     }
+    // the first bounce of a run up to its rays' cast
+    bool inner() const { return !guided && render_trace.persistent; }
+    int run_first() {
+        cudaStream_t st = stream;
+        launch_compact_new(pv, qv, st);
+        launch_shade(pv, qv, rp, shade_grid, st);
+        RGR_CUDA(launch_inner_cast(pv, qv, rp, render_trace, st));
+        launch_inner_reset(qv, in, st);
+        RGR_CUDA(cudaGetLastError());
+        return RGR_OK;
+    }
+    // `n` bounces inside the run
+    int run_inner(int n) {
+        auto one = [&]() -> int {
+            launch_inner(pv, qv, in, rp, render_trace, false, shade_grid, num_sms, stream);
+            RGR_CUDA(cudaGetLastError());
+            return RGR_OK;
+        };
+        int r = RGR_OK;
+        for (; graph_mode && n >= graph_steps && r == RGR_OK; n -= graph_steps)
+            r = replay(inner_graph, [&] {
+                int q = RGR_OK;
+                for (int i = 0; i < graph_steps && q == RGR_OK; ++i) q = one();
+                return q;
+            });
+        for (; n > 0 && r == RGR_OK; --n) r = one();
+        return r;
+    }
+    // the logic of the run's last bounce
+    int run_last() {
+        RGR_CUDA(cudaMemsetAsync(qv.tile_new, 0, sizeof(uint32_t) * ntiles, stream));
+        launch_trace_logic(pv, qv, rp, render_trace, stream);
+        if (!single_render) launch_stamp_done(rp, stream);  // batches: per-request completion times
+        RGR_CUDA(cudaGetLastError());
+        return RGR_OK;
+    }
+    // Bounces until the render is over (every path ended and the sample budget handed
+    // out), looked at after every `group` bounces, at most max_steps; `*ran`: how many.
+    int run_until_done(int group, int max_steps, int* ran, bool* over) {
+        *ran = 0;
+        *over = false;
+        while (*ran < max_steps && !*over) {
+            const int b = std::min(group, max_steps - *ran);
+            const bool last = *ran + b >= max_steps;
+            int r;
+            uint32_t words[8] = {};
+            unsigned long long np = 0;
+            if (!inner()) {
+                if ((r = run_steps(b)) != RGR_OK) return r;
+            } else {
+                if (*ran == 0 && (r = run_first()) != RGR_OK) return r;
+                if ((r = run_inner(b - 1)) != RGR_OK) return r;
+                if (last) {
+                    if ((r = run_last()) != RGR_OK) return r;
+                } else {
+                    launch_inner(pv, qv, in, rp, render_trace, true, shade_grid, num_sms, stream);
+                    RGR_CUDA(cudaGetLastError());
+                }
+                steps += b;
+            }
+            *ran += b;
+            if (!inner() || last) {
+                RGR_CUDA(cudaMemcpyAsync(words, counts.p, 32, cudaMemcpyDeviceToHost, stream));
+                RGR_CUDA(cudaMemcpyAsync(&np, scalars.p, 8, cudaMemcpyDeviceToHost, stream));
+                RGR_CUDA(cudaStreamSynchronize(stream));
+                uint64_t live = 0;
+                for (int k = 1; k < kNumQueues; ++k) live += words[k];
+                *over = np >= rp.sample_limit && live == 0;
+            } else {
+                RGR_CUDA(cudaMemcpyAsync(words, in.words + InnerView::kStop, 4, cudaMemcpyDeviceToHost, stream));
+                RGR_CUDA(cudaStreamSynchronize(stream));
+                *over = words[0] != 0u;
+            }
+        }
+        return RGR_OK;
+    }
     void drop_graph() {
-        if (graph_exec) cudaGraphExecDestroy(graph_exec);
-        graph_exec = nullptr;
+        for (Graph* g : {&step_graph, &inner_graph}) {
+            if (g->exec) cudaGraphExecDestroy(g->exec);
+            g->exec = nullptr;
+        }
     }
     // Everything a captured bounce graph bakes in: the kernels' parameter
     // structs and launch shapes.  A new render whose key is unchanged (same
@@ -407,6 +514,7 @@ struct rgr_context {
         auto add = [&k](const void* p, size_t n) { k.append(static_cast<const char*>(p), n); };
         add(&pv, sizeof(pv));
         add(&qv, sizeof(qv));
+        add(&in, sizeof(in));
         add(&rp, sizeof(rp));
         add(&shade_grid, sizeof(shade_grid));
         add(&render_trace, sizeof(render_trace));
@@ -584,21 +692,11 @@ int rgr_render_until_done(rgr_context* c, int32_t max_steps, int32_t* steps_done
     RGR_NVTX_RANGE("rgr_render_until_done");
     if (!c || max_steps < 0) return RGR_E_INVALID;
     if (!c->begun || c->rp.sample_limit == 0) return RGR_E_STATE;
-    int32_t done = 0;
-    while (done < max_steps) {
-        int batch = std::min<int32_t>(8, max_steps - done);
-        int r = rgr_render_step(c, batch);
-        if (r != RGR_OK) return r;
-        done += batch;
-        uint32_t counts[8];
-        unsigned long long np = 0;
-        RGR_CUDA(cudaMemcpyAsync(counts, c->counts.p, 32, cudaMemcpyDeviceToHost, c->stream));
-        RGR_CUDA(cudaMemcpyAsync(&np, c->scalars.p, 8, cudaMemcpyDeviceToHost, c->stream));
-        RGR_CUDA(cudaStreamSynchronize(c->stream));
-        uint64_t live = 0;
-        for (int k = 1; k < kNumQueues; ++k) live += counts[k];
-        if (np >= c->rp.sample_limit && live == 0) break;
-    }
+    RGR_CUDA(cudaSetDevice(c->device));
+    int done = 0;
+    bool over = false;
+    int r = c->run_until_done(8, max_steps, &done, &over);
+    if (r != RGR_OK) return r;
     if (steps_done) *steps_done = done;
     return rgr_synchronize(c);
 }
@@ -1152,20 +1250,19 @@ int rgr_batch_run(rgr_batch* b, int32_t order_policy, int32_t steps_per_launch, 
     c->npix = 0;
     r = c->start(table.data(), n, begin, b->reqs[order[0]]->cfg.seed_offset);
     if (r != RGR_OK) return r;
-    c->graph_steps = steps_per_launch;
+    // a replayed graph: the bounces of a group before the one whose outcome is looked at
+    c->graph_steps = std::max(1, steps_per_launch - 1);
     k_stamp<<<1, 1, 0, st>>>(b->stamp.as<unsigned long long>());
     std::vector<unsigned long long> done(2 * n);
-    int32_t ran = 0;
-    bool all = false;
-    while (ran < max_steps && !all) {
-        r = c->run_steps(steps_per_launch);
-        if (r != RGR_OK) return r;
-        ran += steps_per_launch;
-        RGR_CUDA(cudaMemcpyAsync(done.data(), c->done.p, 16 * (size_t)n, cudaMemcpyDeviceToHost, st));
-        RGR_CUDA(cudaStreamSynchronize(st));
-        all = true;
-        for (int k = 0; k < n; ++k) all = all && done[2 * k] == table[k].sample_end - table[k].sample_begin;
-    }
+    int ran = 0;
+    bool over = false;
+    // whole groups, as many as reach max_steps
+    const int64_t most = ((int64_t)max_steps + steps_per_launch - 1) / steps_per_launch * steps_per_launch;
+    if ((r = c->run_until_done(steps_per_launch, (int)std::min<int64_t>(most, INT32_MAX), &ran, &over)) != RGR_OK) return r;
+    RGR_CUDA(cudaMemcpyAsync(done.data(), c->done.p, 16 * (size_t)n, cudaMemcpyDeviceToHost, st));
+    RGR_CUDA(cudaStreamSynchronize(st));
+    bool all = true;
+    for (int k = 0; k < n; ++k) all = all && done[2 * k] == table[k].sample_end - table[k].sample_begin;
     c->graph_steps = c->graph_steps_default;
     c->drop_graph();
     unsigned long long t0 = 0;

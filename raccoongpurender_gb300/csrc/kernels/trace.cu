@@ -114,10 +114,11 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
         trace_warp_round<kCount, kStaged, kSmemStack>(sc, s, ray != ~0ull && s.link != kDone, b.search, &cnt, err, pol,
                                                       stn);
         if (ray != ~0ull && s.link == kDone) {
-            __stcs(b.prim + ray, s.prim);
+            const int32_t prim = hit_id(s.prim);
+            __stcs(b.prim + ray, prim);
             __stcs(b.t + ray, s.tmin);
             if (b.ng) {
-                f3 n = s.prim >= 0 ? hit_normal(sc, s.prim, s.ro, s.rd, s.tmin) : mk(0.0f, 0.0f, 0.0f);
+                f3 n = prim >= 0 ? hit_normal(sc, prim, s.ro, s.rd, s.tmin) : mk(0.0f, 0.0f, 0.0f);
                 b.ng[3 * ray + 0] = n.x;
                 b.ng[3 * ray + 1] = n.y;
                 b.ng[3 * ray + 2] = n.z;

@@ -153,7 +153,7 @@ struct TraceCounters {
 struct TraceState {
     f3 ro, rd, inv;
     float tmin;       // ExtensionResult.tmin: far clip in, hit distance out
-    int32_t prim;     // -1 until a primitive is hit
+    int32_t prim;     // -1 until a primitive is hit, then its record's word (hit_id, hit_type)
     uint32_t link;    // next node link; kDone when the ray is finished
     int sp;           // pending far links; the newest is in `top`, older ones in stack[0..sp-2]
     uint32_t top;
@@ -161,6 +161,10 @@ struct TraceState {
     uint32_t* sstk;   // this thread's shared-memory entries (stride kStackThreads), with kSm > 0
     uint32_t stack[kStackSize];
 };
+
+// the primitive id (-1: none) and material type in a record's word
+RGR_DEV int32_t hit_id(int32_t word) { return word < 0 ? -1 : (word & 0x0fffffff); }
+RGR_DEV int hit_type(int32_t word) { return word >> 28; }
 
 template <int kSm>
 RGR_DEV void stack_put(TraceState& s, int i, uint32_t v) {
@@ -336,7 +340,7 @@ RGR_DEV int32_t trace_closest(const SceneView& sc, f3 ro, f3 rd, float& tmin, Tr
     const uint64_t pol = l2_evict_last_policy();
     while (s.link != kDone) trace_round<kCount>(sc, s, cnt, err, pol);
     tmin = s.tmin;
-    return s.prim;
+    return hit_id(s.prim);
 }
 
 // geometric normal of a hit (extension_ray_cast_stackless.cl:224-239), from

@@ -1,7 +1,7 @@
 // wavefront.cu — the per-bounce kernels of the wavefront path tracer (sm_103a).
 //
 // One reference step() (common/wavefront_path_tracing.hpp:591-939) is about
-// twenty launches of 2^22 work items.  Here it is three kernels and a memset:
+// twenty launches of 2^22 work items.  Here a bounce by itself is:
 //   1. compact_new  — ordered compaction of the slots logic marked "new path"
 //      (slot order, so pixels are assigned exactly as a sequential run of
 //      new_path.cl:41-43 over that queue would);
@@ -10,15 +10,23 @@
 //      order, new_path / strategy_selection / envmap sample / BSDF sample or
 //      pdf / envmap pdf / material stage / homogeneous_volume_through, keeping
 //      IncidentSample and ShadingResult in registers;
-//   3. trace_logic  — logic.cl after the bounce's closest hits (cast by the
-//      persistent trace kernel, or fused for small scenes): throughput update,
-//      envmap on miss, Russian roulette, FP64 per-pixel accumulation, and the
-//      appends to the next step's material queues, aggregated per warp
-//      (match_any) and per block (shared-memory counts, one global atomic per
-//      queue per block).
+//   3. trace_paths  — the closest hits, by persistent refilling warps (large pools);
+//   4. trace_logic  — logic.cl (after casting the rays itself in small pools):
+//      throughput update, envmap on miss, Russian roulette, FP64 per-pixel
+//      accumulation, and the appends to the next step's material queues, aggregated
+//      per warp (match_any) and per block (shared-memory counts, one global atomic
+//      per queue per block).
+// Inside a run of several bounces the logic is not a pass of its own: the cast
+// finds where each path goes next, k_classify builds the queues from a byte per
+// slot, k_new_paths finishes the ended paths and starts the new ones, k_shade_inner
+// does the logic's share of the others (launch_inner in wavefront.cuh).  At 2^24 paths of
+// the mixed 1080p render a bounce was 1.15 ms shading, 2.25 cast and 1.15 logic; it is
+// 0.06 classification, 0.48 new paths, 0.81 shading and 2.3 cast: 91.5 to 73.3 ms.
 // Every slot's arithmetic is the reference kernels' arithmetic (see the
 // file:line notes); the translation unit is built with --fmad=false.
 #include <cuda_fp16.h>
+
+#include <algorithm>
 
 #include "wavefront.cuh"
 #include "traverse.cuh"
@@ -219,54 +227,45 @@ RGR_DEV float incident_pdf(const Incident& is) {  // types.cl:65-71
     return pdf;
 }
 
-// One slot's share of a step, from new_path to homogeneous_volume_through.
-// k: the queue the slot came from (0 = new path, else its material type).
+// A slot's path state in registers, as the shading stages see it.
+struct SlotState {
+    f3 ro, rd, T, L, Ng;
+    float tmin;
+    int32_t hv, hs;      // volume hit (negative: none), surface hit
+    uint32_t pixel;
+    uint32_t logic_i;    // segments so far
+    int vcount;          // volumes the path is inside; their ids in va, vb.xyz
+    int4 va, vb;
+    Rng rng;
+};
+
+// One slot's share of a step, from new_path to homogeneous_volume_through, on
+// its state in registers.  k: the queue the slot came from (0 = new path, else
+// its material type); a new path replaces everything but the RNG state and the
+// volume list and reads the ended path's volume hit.
 // Guided renders: gi is the slot's index among this bounce's guided items
 // (its mixture in gd.lobes), ~0u when the vertex is not guided.
+// Returns whether the stage changed L.
 template <bool kGuided>
-RGR_DEV void shade_slot(const RequestD& rq, const PathsView& P, int k, uint32_t slot, unsigned long long gpix,
-                        const GuideRenderD& gd, uint32_t gi) {
+RGR_DEV bool shade_state(const RequestD& rq, int k, uint32_t slot, unsigned long long gpix, const GuideRenderD& gd,
+                         uint32_t gi, SlotState& st) {
     const SceneView& sc = rq.sc;
-    // Path state moves by 32-byte sector of the slot record and only where this
-    // item uses it (a material queue is a sparse subset of the slots, so each
-    // sector touched costs a DRAM sector): a new path (k = 0) replaces everything
-    // but its RNG state and the volume hit of the ended path, so it skips the
-    // (T, L) sector and the volume list; L is stored only when the stage changes
-    // it; the first half of the volume list is loaded only when the list is used.
     const bool fresh = k == 0;
-    float4 ro4, rd4, ng4, rng4, T4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), L4 = T4;
-    int4 va = make_int4(0, 0, 0, 0), vb = va;
-    // the ray's sector and the (ng, rng) sector, each in one access; (T, L) likewise
-    ld_sector<0>(P, slot, ro4, rd4);
-    ld_sector<2>(P, slot, ng4, rng4);
-    int vcount = 0;
-    if (!fresh) {
-        ld_sector<1>(P, slot, T4, L4);
-        vcount = vcount_of(__float_as_uint(L4.w));
-        if (k == kMatVolume || vcount > 0) {
-            float4 a, b;
-            ld_sector<3>(P, slot, a, b);
-            va = make_int4(__float_as_int(a.x), __float_as_int(a.y), __float_as_int(a.z), __float_as_int(a.w));
-            vb = make_int4(__float_as_int(b.x), __float_as_int(b.y), __float_as_int(b.z), __float_as_int(b.w));
-        }
-    } else {
-        ro4 = ng4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-    Rng rng = rng_of_bits(rng4);
-    f3 ro = xyz(ro4), rd = xyz(rd4), T = xyz(T4), L = mk(0, 0, 0), Ng = xyz(ng4);
-    float tmin = ro4.w;
-    int32_t hv = __float_as_int(rd4.w);
-    int32_t hs = __float_as_int(ng4.w);
-    uint32_t pixel = __float_as_uint(T4.w);
-    uint32_t logic_i = 0;
+    f3 &ro = st.ro, &rd = st.rd, &T = st.T, &L = st.L, &Ng = st.Ng;
+    float& tmin = st.tmin;
+    int32_t &hv = st.hv, &hs = st.hs;
+    int& vcount = st.vcount;
+    int4 &va = st.va, &vb = st.vb;
+    Rng& rng = st.rng;
 
     if (k == 0) {  // new_path (new_path.cl:17-83)
         const CameraD& cam = rq.cam;
         T = mk(1, 1, 1);
         L = mk(0, 0, 0);
-        logic_i = 0;
+        st.logic_i = 0;
         uint32_t npix = cam.w * cam.h;
-        pixel = (uint32_t)(gpix % (unsigned long long)npix);
+        const uint32_t pixel = (uint32_t)(gpix % (unsigned long long)npix);
+        st.pixel = pixel;
         uint32_t x = pixel % cam.w, y = pixel / cam.w;
         float ux = rng.uniform();
         float uy = rng.uniform();
@@ -502,7 +501,7 @@ RGR_DEV void shade_slot(const RequestD& rq, const PathsView& P, int k, uint32_t 
             vcount++;
         }
         va = make_int4(vols[0], vols[1], vols[2], vols[3]);
-        vb = make_int4(vols[4], vols[5], vols[6], vcount);
+        vb = make_int4(vols[4], vols[5], vols[6], 0);
         ro = ro + rd * (tmin + 1.0e-5f);
     } else if (k == kMatVolumeInside) {  // homogeneous_volume_inside_stage (homogeneous_volume.cl:90-129)
         int2 mi = __ldg(sc.materials + hv);
@@ -545,16 +544,10 @@ RGR_DEV void shade_slot(const RequestD& rq, const PathsView& P, int k, uint32_t 
     }
     // logic.cl:31-33, applied here: the stage that made the shading result consumes it.
     // L + T * shLe leaves L's bits unchanged when shLe is zero and T finite (L is
-    // never -0), so L is read and written only otherwise, for new paths and in
+    // never -0), so L counts as changed only otherwise, for new paths and in
     // guided renders (the training records carry it).
     const bool touch_L = fresh || kGuided || shLe.x != 0.0f || shLe.y != 0.0f || shLe.z != 0.0f ||
                          !is_finite(T.x) || !is_finite(T.y) || !is_finite(T.z);
-    // the volume stage changes the volume count, which L.w carries
-    const bool store_L = touch_L || k == kMatVolume;
-    if (store_L && !fresh) {
-        L = xyz(L4);
-        logic_i = depth_of(__float_as_uint(L4.w));
-    }
     L = L + T * shLe;
     T = T * shT;
     if (kGuided && is.sel2 != 0.0f && gd.record && guide_training_open(gd.train)) {
@@ -590,18 +583,113 @@ RGR_DEV void shade_slot(const RequestD& rq, const PathsView& P, int k, uint32_t 
         float u = rng.uniform();
         tmin = -1.0f / vol.w * log_(u);
     }
-    st_sector<0>(P, slot, f4(ro, tmin), f4(rd, __int_as_float(hv)));
-    if (store_L)  // a new path's count is 0; its list keeps the stale ids
-        st_sector<1>(P, slot, f4(T, __uint_as_float(pixel)), f4(L, __uint_as_float(depth_word(logic_i, vcount))));
-    else  // the sector was read above: this half store finds it in L2
-        P.T[slot] = f4(T, __uint_as_float(pixel));
-    if (k == kMatVolume) {
-        vb.w = vcount;
-        st_sector<3>(P, slot,
-                     make_float4(__int_as_float(va.x), __int_as_float(va.y), __int_as_float(va.z), __int_as_float(va.w)),
-                     make_float4(__int_as_float(vb.x), __int_as_float(vb.y), __int_as_float(vb.z), __int_as_float(vb.w)));
+    return touch_L;
+}
+
+// The hit that k_trace_paths left in a slot's ray sector (primitive -2 - hv):
+// its surface, normal and, where the per-triangle table gives it, material type
+// (else mtype stays -1).
+RGR_DEV void resolve_hit(const SceneView& sc, const float4& ro4, const float4& rd4, int32_t& hv, int32_t& hs,
+                         float4& ng4, int& mtype) {
+    if (hv > -2) return;
+    hs = -2 - hv;
+    hv = -1;
+    if (sc.tri_normals && hs < sc.sphere_begin) {
+        const float4 tn = __ldg(sc.tri_normals + hs);
+        ng4 = f4(xyz(tn), __int_as_float(hs));
+        mtype = __float_as_int(tn.w);
+    } else {
+        ng4 = f4(hit_normal(sc, hs, xyz(ro4), xyz(rd4), ro4.w), __int_as_float(hs));
     }
-    st_sector<2>(P, slot, f4(Ng, __int_as_float(hs)), rng_bits(rng));
+}
+
+// What the logic does to a path that goes on (logic.cl:27-190): the Russian
+// roulette's draw and T / cp (exactly T where the roulette is off: cp is 1).
+RGR_DEV void logic_advance(const RequestD& rq, uint32_t logic_i, f3& T, Rng& rng) {
+    float cp = 1.0f;
+    if ((long long)rq.rr_depth < (long long)logic_i) cp = fmin_(0.2126f * T.x + 0.7152f * T.y + 0.0722f * T.z, 1.0f);
+    rng.uniform();
+    T = T / cp;
+}
+
+// Whether the logic ends a path whatever its ray meets: Russian roulette, a black
+// throughput, or the depth limit (logic_decide without the miss).
+RGR_DEV bool logic_ends(const RequestD& rq, const PathsView& P, uint32_t slot, f3 T, uint32_t logic_i) {
+    const float lum = 0.2126f * T.x + 0.7152f * T.y + 0.0722f * T.z;
+    bool ends = lum < 1.0e-5f || (rq.max_depth > 0 && (long long)logic_i >= (long long)rq.max_depth);
+    if ((long long)rq.rr_depth < (long long)logic_i) {
+        Rng rng = rng_load(P.rng, slot);
+        ends = ends || !(rng.uniform() < fmin_(lum, 1.0f));
+    }
+    return ends;
+}
+
+// The volume list of a slot (its record's last sector).
+RGR_DEV void load_volumes(const PathsView& P, uint32_t slot, SlotState& st) {
+    float4 a, b;
+    ld_sector<3>(P, slot, a, b);
+    st.va = make_int4(__float_as_int(a.x), __float_as_int(a.y), __float_as_int(a.z), __float_as_int(a.w));
+    st.vb = make_int4(__float_as_int(b.x), __float_as_int(b.y), __float_as_int(b.z), __float_as_int(b.w));
+}
+RGR_DEV void store_volumes(const PathsView& P, uint32_t slot, const SlotState& st) {
+    const int4 va = st.va, vb = st.vb;
+    st_sector<3>(P, slot,
+                 make_float4(__int_as_float(va.x), __int_as_float(va.y), __int_as_float(va.z), __int_as_float(va.w)),
+                 make_float4(__int_as_float(vb.x), __int_as_float(vb.y), __int_as_float(vb.z),
+                             __int_as_float(st.vcount)));
+}
+
+// shade_state on a slot's record in memory.  kInner: the bounce before was a bounce
+// inside a run, whose logic left the state of a path that goes on as the trace
+// kernel did: its share (the hit, the draw, T / cp, the segment count) comes first.
+template <bool kGuided, bool kInner = false>
+RGR_DEV void shade_slot(const RequestD& rq, const PathsView& P, int k, uint32_t slot, unsigned long long gpix,
+                        const GuideRenderD& gd, uint32_t gi) {
+    // Path state moves by 32-byte sector of the slot record and only where this
+    // item uses it (a material queue is a sparse subset of the slots, so each
+    // sector touched costs a DRAM sector): a new path (k = 0) replaces everything
+    // but its RNG state and the volume hit of the ended path, so it skips the
+    // (T, L) sector and the volume list; L is stored only when the stage changes
+    // it; the first half of the volume list is loaded only when the list is used.
+    const bool fresh = k == 0;
+    float4 ro4, rd4, ng4, rng4, T4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), L4 = T4;
+    SlotState st;
+    st.va = make_int4(0, 0, 0, 0), st.vb = st.va;
+    // the ray's sector and the (ng, rng) sector, each in one access; (T, L) likewise
+    ld_sector<0>(P, slot, ro4, rd4);
+    ld_sector<2>(P, slot, ng4, rng4);
+    st.vcount = 0;
+    if (!fresh) {
+        ld_sector<1>(P, slot, T4, L4);
+        st.vcount = vcount_of(__float_as_uint(L4.w));
+        if (k == kMatVolume || st.vcount > 0) load_volumes(P, slot, st);
+    } else {
+        ro4 = ng4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    st.rng = rng_of_bits(rng4);
+    st.ro = xyz(ro4), st.rd = xyz(rd4), st.T = xyz(T4), st.L = xyz(L4), st.Ng = xyz(ng4);
+    st.tmin = ro4.w;
+    st.hv = __float_as_int(rd4.w);
+    st.hs = __float_as_int(ng4.w);
+    st.pixel = __float_as_uint(T4.w);
+    st.logic_i = depth_of(__float_as_uint(L4.w));
+    if (kInner) {
+        int mtype;
+        resolve_hit(rq.sc, ro4, rd4, st.hv, st.hs, ng4, mtype);
+        st.Ng = xyz(ng4);
+        logic_advance(rq, st.logic_i, st.T, st.rng);
+        st.logic_i += 1;
+    }
+    // the volume stage changes the volume count, which L.w carries
+    const bool store_L = shade_state<kGuided>(rq, k, slot, gpix, gd, gi, st) || k == kMatVolume || kInner;
+    st_sector<0>(P, slot, f4(st.ro, st.tmin), f4(st.rd, __int_as_float(st.hv)));
+    if (store_L)  // a new path's count is 0; its list keeps the stale ids
+        st_sector<1>(P, slot, f4(st.T, __uint_as_float(st.pixel)),
+                     f4(st.L, __uint_as_float(depth_word(st.logic_i, st.vcount))));
+    else  // the sector was read above: this half store finds it in L2
+        P.T[slot] = f4(st.T, __uint_as_float(st.pixel));
+    if (k == kMatVolume) store_volumes(P, slot, st);
+    st_sector<2>(P, slot, f4(st.Ng, __int_as_float(st.hs)), rng_bits(st.rng));
 }
 
 // ------------------------------------------------------------ kernels
@@ -627,14 +715,11 @@ __global__ void k_init(PathsView P, QueueView Q, uint32_t seed_offset) {
     }
     uint4 s = make_uint4((uint32_t)r[0], (uint32_t)(r[0] >> 32), (uint32_t)r[1], (uint32_t)(r[1] >> 32));
     if ((s.x | s.y | s.z | s.w) == 0u) s.x = 1u;
-    P.rng[i] = s;
-    P.ro[i] = make_float4(0, 0, 0, kFltMax);
-    P.rd[i] = make_float4(0, 0, 0, __int_as_float(-1));
-    P.T[i] = make_float4(0, 0, 0, 0);
-    P.L[i] = make_float4(0, 0, 0, 0);
-    P.ng[i] = make_float4(0, 0, 0, __int_as_float(-1));
-    P.va[i] = make_int4(0, 0, 0, 0);
-    P.vb[i] = make_int4(0, 0, 0, 0);
+    const float4 zero = make_float4(0, 0, 0, 0);
+    st_sector<0>(P, i, make_float4(0, 0, 0, kFltMax), make_float4(0, 0, 0, __int_as_float(-1)));
+    st_sector<1>(P, i, zero, zero);
+    st_sector<2>(P, i, make_float4(0, 0, 0, __int_as_float(-1)), rng_bits(Rng{s.x, s.y, s.z, s.w}));
+    st_sector<3>(P, i, zero, zero);
     P.qid[i] = 0;  // initialize_all_as_new_path (new_path.cl:9-15)
     P.req[i] = 0;
 }
@@ -742,6 +827,24 @@ __device__ __forceinline__ void shade_items(const PathsView& P, const QueueView&
     }
 }
 
+// The completion time of each request whose paths have all finished, stamped
+// once by the bounce in which its last path ended (after that bounce's logic
+// kernel, when its accumulation is complete).  The logic kernel only counts
+// finished paths: an atomic with a returned value per warp, to find the last
+// one, queued the warps on the requests' counters.  Requests i, i + stride, ...
+RGR_DEV void stamp_done(const RenderParams& rp, int i, int stride) {
+    for (int r = i; r < rp.nreq; r += stride) {
+        const RequestD& q = rp.reqs[r];
+        if (q.done == nullptr || *q.done_ns != 0ull || *q.done != q.sample_end - q.sample_begin) continue;
+        unsigned long long t;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        *q.done_ns = t;
+    }
+}
+__global__ void k_stamp_done(RenderParams rp) {
+    stamp_done(rp, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
 // The plain and guided shading kernels: one queue item per thread, all
 // queues in one launch, held to 4 resident 256-thread blocks per SM (64
 // registers, a few spilled: the mixed 1080p render 1370 against 1347 Mpaths/s
@@ -755,6 +858,24 @@ __device__ __forceinline__ void shade_items(const PathsView& P, const QueueView&
 #endif
 __global__ void __launch_bounds__(256, RGR_SHADE_MIN_BLOCKS) k_shade(PathsView P, QueueView Q, RenderParams rp) {
     shade_items<false>(P, Q, rp);
+}
+// the material queues of a bounce inside a run (k_new_paths has taken the new paths)
+__global__ void __launch_bounds__(256, RGR_SHADE_MIN_BLOCKS) k_shade_inner(PathsView P, QueueView Q, RenderParams rp) {
+    // the ended paths of the bounce before are finished and counted
+    if (blockIdx.x == 0) stamp_done(rp, (int)threadIdx.x, (int)blockDim.x);
+    uint32_t off[kNumQueues];  // off[k]: the first item of queue k + 1
+    off[0] = 0;
+#pragma unroll
+    for (int k = 1; k < kNumQueues; ++k) off[k] = off[k - 1] + Q.counts[k];
+    const uint32_t total = off[kNumQueues - 1];
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+        int k = 1;
+#pragma unroll
+        for (int j = 1; j < kNumQueues - 1; ++j) k += (i >= off[j]) ? 1 : 0;
+        const uint32_t slot = queue_items(Q, k)[i - pick(off, k - 1)];
+        shade_slot<false, true>(rp.reqs[P.req[slot]], P, k, slot, 0ull, rp.gd, ~0u);
+    }
 }
 __global__ void __launch_bounds__(256, RGR_SHADE_GUIDED_MIN_BLOCKS) k_shade_guided(PathsView P, QueueView Q,
                                                                                   RenderParams rp) {
@@ -871,9 +992,14 @@ RGR_DEV float guide_write(const GuideRenderD& gd, uint32_t slot, const GuideOffe
 // field P.rd.w (its readers take a negative id as none); the logic kernel computes
 // Ng into P.ng.  A miss leaves P.ng.w at the -1 the shading stage wrote.  Each slot may belong
 // to another request (scene).
+// kInner: a bounce inside a run (launch_inner).  The cast also decides where the path
+// goes next and writes it as the slot's queue id: what ends a path whatever its ray
+// meets (logic_ends) is found as the ray is taken, from the sector beside the
+// ray's in the same line, and kept in the slot word's top bit (slots are below 2^28).
 #ifndef RGR_TRACE_PATHS_MIN_BLOCKS  // 4 / 5 / 6 (64 / 48 / 40 registers, 6 spilling): 1428 / 1473 / 1442 Mpaths/s
 #define RGR_TRACE_PATHS_MIN_BLOCKS 5
 #endif
+template <bool kInner>
 __global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS) k_trace_paths(PathsView P, QueueView Q, RenderParams rp,
                                                          unsigned long long* next, int refill, int search) {
     const unsigned full = 0xffffffffu;
@@ -890,6 +1016,8 @@ __global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS) k_trace_paths
     s.sstk = s_stack + threadIdx.x;
     const SceneView* scp = &rp.reqs[0].sc;  // a valid scene on idle lanes too
     uint32_t slot = ~0u;  // ~0: idle
+    constexpr uint32_t kEnds = 0x80000000u;
+    bool vol = false;  // kInner: the path is in a volume that ends its ray
     bool exhausted = false;
     uint32_t err = 0;
     for (;;) {
@@ -911,9 +1039,16 @@ __global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS) k_trace_paths
                     // the shading kernel): material-queue items skip the check
                     if (k != 0 || P.qid[r] != kQueueIdle) {
                         slot = r;
-                        scp = &rp.reqs[P.req[r]].sc;
+                        const RequestD* rq = &rp.reqs[P.req[r]];
+                        scp = &rq->sc;
                         float4 ro4, rd4;
                         ld_sector<0>(P, r, ro4, rd4);
+                        if (kInner) {
+                            float4 T4, L4;
+                            ld_sector<1>(P, r, T4, L4);
+                            if (logic_ends(*rq, P, r, xyz(T4), depth_of(__float_as_uint(L4.w)))) slot |= kEnds;
+                            vol = __float_as_int(rd4.w) >= 0;
+                        }
                         trace_begin(*scp, s, xyz(ro4), xyz(rd4), ro4.w);
                     }
                 }
@@ -926,13 +1061,18 @@ __global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS) k_trace_paths
         trace_warp_round<false, false, kSmemStack>(*scp, s, slot != ~0u && s.link != kDone, search, nullptr, err,
                                                    pol);
         if (slot != ~0u && s.link == kDone) {
+            const uint32_t id = kInner ? slot & ~kEnds : slot;
+            if (kInner) {
+                const int q = s.prim >= 0 ? hit_type(s.prim) : (vol ? (int)kMatVolumeInside : 0);
+                P.qid[id] = (uint8_t)((slot & kEnds) ? 0 : q);
+            }
             if (s.prim >= 0) {
                 // the ray's whole sector in one store (a partial store to a line that is
                 // not in L2 costs a read of the sector from DRAM); the hit primitive
                 // rides where the volume-hit id goes (none after a surface hit: every
                 // reader takes a negative id as none), and the logic kernel, which
                 // writes the (ng, rng) sector anyway, computes the normal
-                st_sector<0>(P, slot, f4(s.ro, s.tmin), f4(s.rd, __int_as_float(-2 - s.prim)));
+                st_sector<0>(P, id, f4(s.ro, s.tmin), f4(s.rd, __int_as_float(-2 - hit_id(s.prim))));
             }
             slot = ~0u;
         }
@@ -940,10 +1080,63 @@ __global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS) k_trace_paths
     if (err) atomicOr(rp.err, err);
 }
 
+// logic.cl:27-190 up to the accumulation, without the envmap's radiance: throughput,
+// Russian roulette, depth limit.  Returns whether the path ends; a path that
+// left the scene (hs < 0 and hv < 0) ends and is still owed T * envmap.
+RGR_DEV bool logic_decide(const RequestD& rq, int32_t hs, int32_t hv, uint32_t logic_i, f3& T, f3& L, Rng& rng) {
+    bool newPath = hs < 0 && hv < 0;
+    float lum = 0.2126f * T.x + 0.7152f * T.y + 0.0722f * T.z;
+    float cp = 1.0f;
+    if ((long long)rq.rr_depth < (long long)logic_i) cp = fmin_(lum, 1.0f);
+    float u = rng.uniform();
+    if (u < cp) {
+        T = T / cp;
+    } else {
+        newPath = true;
+    }
+    if (lum < 1.0e-5f) newPath = true;
+    // depth limit: end after segment max_depth, adding the emission that the
+    // next material stage would add (lambertian.cl:395)
+    if (rq.max_depth > 0 && !newPath && (long long)logic_i >= (long long)rq.max_depth) {
+        if (0 <= hs) {
+            const SceneView& sc = rq.sc;
+            int2 m = __ldg(sc.materials + hs);
+            f3 Le = mk(0, 0, 0);
+            if (m.x == kMatLambertian) Le = xyz(__ldg(sc.lambertians + 2 * (size_t)m.y));
+            L = L + T * Le;
+        }
+        newPath = true;
+    }
+    return newPath;
+}
+
+// an ended path's radiance into its pixel's FP64 sums, unless it is discarded
+// (not finite, or at the clamp); returns whether it was kept
+RGR_DEV bool accumulate(const RequestD& rq, uint32_t pixel, f3 L) {
+    const float cl = rq.radiance_clamp;
+    if (!(is_finite(L.x) && is_finite(L.y) && is_finite(L.z) && L.x < cl && L.y < cl && L.z < cl)) return false;
+    double* a = rq.accum + 4 * (size_t)pixel;
+    atomicAdd(a + 0, (double)L.x);
+    atomicAdd(a + 1, (double)L.y);
+    atomicAdd(a + 2, (double)L.z);
+    atomicAdd(a + 3, 1.0);
+    return true;
+}
+
+// finished paths per request (stamp_done takes the completion times); called by
+// the lanes `active` of a warp, `ended` on those whose path of request req ended
+RGR_DEV void count_done(const RequestD& rq, int req, bool ended, unsigned active) {
+    const unsigned donemask = __ballot_sync(active, ended);
+    if (ended && rq.done != nullptr) {
+        const unsigned peers = __match_any_sync(donemask, req);
+        if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(rq.done, (unsigned long long)__popc(peers));
+    }
+}
+
 // The logic of one live slot (logic.cl:27-190) after its extension ray;
-// returns the queue of its next step (0: a new path, counted per tile here;
-// a material queue: appended by the caller).  kPreTraced: k_trace_paths has
-// cast the extension rays of this bounce; otherwise the thread traces first.
+// returns the queue of its next step (0: a new path; the caller counts and
+// appends).  kPreTraced: k_trace_paths has cast the extension rays of this
+// bounce; otherwise the thread traces first.
 template <bool kGuided, bool kPreTraced>
 RGR_DEV int logic_slot(const PathsView& P, const QueueView& Q, const RenderParams& rp, uint32_t slot,
                        unsigned active, GuideOffer& go) {
@@ -959,85 +1152,34 @@ RGR_DEV int logic_slot(const PathsView& P, const QueueView& Q, const RenderParam
     f3 rd = xyz(rd4);
     int32_t hv = __float_as_int(rd4.w);
     uint32_t err = 0;
-    int32_t hs;
-    int mtype = -1;  // the hit triangle's material type, where the triangle table gave it
-    if (kPreTraced) {
-        hs = __float_as_int(ng4.w);
-        if (hv <= -2) {  // k_trace_paths found primitive -2 - hv
-            hs = -2 - hv;
-            hv = -1;
-            if (sc.tri_normals && hs < sc.sphere_begin) {
-                const float4 tn = __ldg(sc.tri_normals + hs);
-                ng4 = f4(xyz(tn), __int_as_float(hs));
-                mtype = __float_as_int(tn.w);
-            } else {
-                ng4 = f4(hit_normal(sc, hs, xyz(ro4), rd, ro4.w), __int_as_float(hs));
-            }
-        }
-    } else {
+    if (!kPreTraced) {
         // extension_ray_cast (extension_ray_cast_stackless.cl:202-246)
         f3 ro = xyz(ro4);
-        float tmin = ro4.w;
-        hs = trace_closest<false>(sc, ro, rd, tmin, nullptr, err);
+        const int32_t prim = trace_closest<false>(sc, ro, rd, ro4.w, nullptr, err);
         ld_sector<1>(P, slot, T4, L4);
         ld_sector<2>(P, slot, ng4, rng4);
-        if (hs >= 0) {
-            ng4 = f4(hit_normal(sc, hs, ro, rd, tmin), __int_as_float(hs));
-            hv = -1;
-            st_sector<0>(P, slot, f4(ro, tmin), f4(rd, __int_as_float(-1)));
+        if (prim >= 0) {
+            hv = -2 - prim;
+            st_sector<0>(P, slot, ro4, f4(rd, __int_as_float(-1)));
         }
     }
+    int32_t hs = __float_as_int(ng4.w);
+    int mtype = -1;  // the hit triangle's material type, where the triangle table gave it
+    resolve_hit(sc, ro4, rd4, hv, hs, ng4, mtype);
     // logic (logic.cl:27-190)
     f3 T = xyz(T4), L = xyz(L4);
     const uint32_t lw = __float_as_uint(L4.w);  // segment count and volume count
-    uint32_t logic_i = depth_of(lw);
+    const uint32_t logic_i = depth_of(lw);
     Rng rng = rng_of_bits(rng4);
-    bool evalEnv = false, newPath = false;
-    if (hs < 0 && hv < 0) {
-        newPath = true;
-        evalEnv = true;
-    }
-    float lum = 0.2126f * T.x + 0.7152f * T.y + 0.0722f * T.z;
-    float cp = 1.0f;
-    if ((long long)rq.rr_depth < (long long)logic_i) cp = fmin_(lum, 1.0f);
-    float u = rng.uniform();
-    if (u < cp) {
-        T = T / cp;
-    } else {
-        newPath = true;
-    }
-    if (lum < 1.0e-5f) newPath = true;
-    if (evalEnv && sc.has_env) L = L + T * envmap_value(sc, rd, logic_i == 0);
-    // depth limit: end after segment max_depth, adding the emission that the
-    // next material stage would add (lambertian.cl:395)
-    if (rq.max_depth > 0 && !newPath && (long long)logic_i >= (long long)rq.max_depth) {
-        if (0 <= hs) {
-            int2 m = __ldg(sc.materials + hs);
-            f3 Le = mk(0, 0, 0);
-            if (m.x == kMatLambertian) Le = xyz(__ldg(sc.lambertians + 2 * (size_t)m.y));
-            L = L + T * Le;
-        }
-        newPath = true;
-    }
-    if (newPath) {
-        const float cl = rq.radiance_clamp;
-        if (is_finite(L.x) && is_finite(L.y) && is_finite(L.z) && L.x < cl && L.y < cl && L.z < cl) {
-            double* a = rq.accum + 4 * (size_t)__float_as_uint(T4.w);
-            atomicAdd(a + 0, (double)L.x);
-            atomicAdd(a + 1, (double)L.y);
-            atomicAdd(a + 2, (double)L.z);
-            atomicAdd(a + 3, 1.0);
-        }
-    }
+    const bool newPath = logic_decide(rq, hs, hv, logic_i, T, L, rng);
+    if (hs < 0 && hv < 0 && sc.has_env) L = L + T * envmap_value(sc, rd, logic_i == 0);
+    const bool kept = newPath && accumulate(rq, __float_as_uint(T4.w), L);
     // No samples once the sample budget is handed out: the paths still in
     // flight are the long ones, and a few iterations on that subset alone
     // undo much of what the guide learned (the same for every thread).
     if (kGuided && rp.gd.record && guide_training_open(rp.gd.train) &&
-        !(rp.sample_limit != 0ull && *Q.next_pixel >= rp.sample_limit)) {
-        const float cl = rq.radiance_clamp;
-        const bool kept = is_finite(L.x) && is_finite(L.y) && is_finite(L.z) && L.x < cl && L.y < cl && L.z < cl;
-        guide_offer(rp.gd, slot, L, newPath && kept, go);
-    }
+        !(rp.sample_limit != 0ull && *Q.next_pixel >= rp.sample_limit))
+        guide_offer(rp.gd, slot, L, kept, go);
     st_sector<1>(P, slot, f4(T, T4.w), f4(L, __uint_as_float(depth_word(logic_i + 1, vcount_of(lw)))));
     st_sector<2>(P, slot, ng4, rng_bits(rng));
     int q;
@@ -1049,27 +1191,8 @@ RGR_DEV int logic_slot(const PathsView& P, const QueueView& Q, const RenderParam
         q = kMatVolumeInside;
     }
     P.qid[slot] = (uint8_t)q;
-    {
-        // new paths: count per tile for the ordered compaction
-        const unsigned newmask = __ballot_sync(active, q == 0);
-        if (q == 0) {
-            unsigned tp = __match_any_sync(newmask, (int)(slot / kTile));
-            int leader = __ffs(tp) - 1;
-            if ((int)(threadIdx.x & 31) == leader) atomicAdd(Q.tile_new + slot / kTile, (uint32_t)__popc(tp));
-        }
-    }
-    {
-        int lane = threadIdx.x & 31;
-        if (err) atomicOr(rp.err, err);
-        // finished paths per request (k_stamp_done stamps the completion times)
-        const unsigned donemask = __ballot_sync(active, newPath);
-        if (newPath && rq.done != nullptr) {
-            unsigned peers = __match_any_sync(donemask, req);
-            if (lane == __ffs(peers) - 1) {
-                atomicAdd(rq.done, (unsigned long long)__popc(peers));
-            }
-        }
-    }
+    if (err) atomicOr(rp.err, err);
+    count_done(rq, req, newPath, active);
     return q;
 }
 
@@ -1099,12 +1222,10 @@ __global__ void __launch_bounds__(kLogicThreads, kPreTraced ? (kGuided ? 5 : RGR
     int q = 0;
     GuideOffer go;
     if (live) q = logic_slot<kGuided, kPreTraced>(P, Q, rp, slot, active, go);
-    const bool mat = live && q != 0;
-    const unsigned matmask = __ballot_sync(full, mat);
     __syncthreads();  // s_q, s_samples, s_offered cleared
     uint32_t off = 0;
-    if (mat) {
-        const unsigned peers = __match_any_sync(matmask, q);
+    if (live) {
+        const unsigned peers = __match_any_sync(active, q);
         const int leader = __ffs(peers) - 1;
         uint32_t base = 0;
         if (lane == leader) base = atomicAdd(&s_q[q], (uint32_t)__popc(peers));
@@ -1125,7 +1246,9 @@ __global__ void __launch_bounds__(kLogicThreads, kPreTraced ? (kGuided ? 5 : RGR
     const int nlive = __syncthreads_count(live);
     if (threadIdx.x < kNumQueues) {
         const uint32_t n = s_q[threadIdx.x];
-        if (n) s_q[threadIdx.x] = atomicAdd(Q.counts + threadIdx.x, n);
+        // queue 0: new paths per tile, for the ordered compaction (a block's slots lie in one tile)
+        if (n && threadIdx.x == 0) atomicAdd(Q.tile_new + slot / kTile, n);
+        else if (n) s_q[threadIdx.x] = atomicAdd(Q.counts + threadIdx.x, n);
     }
     if (kGuided && threadIdx.x == 32) {
         if (s_samples) s_samples = atomicAdd(rp.gd.train.count, s_samples);
@@ -1133,7 +1256,7 @@ __global__ void __launch_bounds__(kLogicThreads, kPreTraced ? (kGuided ? 5 : RGR
     }
     if (threadIdx.x == 0 && nlive) atomicAdd(rp.rays, (unsigned long long)nlive);
     __syncthreads();
-    if (mat) queue_items(Q, q)[s_q[q] + off] = slot;
+    if (live && q != 0) queue_items(Q, q)[s_q[q] + off] = slot;
     if (kGuided && __any_sync(full, go.take != 0u)) {
         float ws = go.take ? guide_write(rp.gd, slot, go, s_samples + sidx) : 0.0f;
         for (int o = 16; o > 0; o >>= 1) ws += __shfl_xor_sync(full, ws, o);
@@ -1141,19 +1264,223 @@ __global__ void __launch_bounds__(kLogicThreads, kPreTraced ? (kGuided ? 5 : RGR
     }
 }
 
-// The completion time of each request whose paths have all finished, stamped
-// once by the bounce in which its last path ended (after that bounce's logic
-// kernel, when its accumulation is complete).  The logic kernel only counts
-// finished paths: an atomic with a returned value per warp, to find the last
-// one, queued the warps on the requests' counters.
-__global__ void k_stamp_done(RenderParams rp) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rp.nreq) return;
-    const RequestD& q = rp.reqs[r];
-    if (q.done == nullptr || *q.done_ns != 0ull || *q.done != q.sample_end - q.sample_begin) return;
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    *q.done_ns = t;
+// The queues of a bounce inside a run, from the queue ids that the cast left: block t
+// takes the tile [t*4096, (t+1)*4096), 16 consecutive slots a thread.  Counts per
+// class as 16-bit fields of two words (a tile's fit), scanned over the block; the
+// tile's slots go to shared memory in class order and from there to the queues, one
+// atomic per queue per block: 16 MB of ids for 2^24 slots instead of a pass over
+// their records.  The ended paths' slots go to the tile's own stretch of I.ended, in
+// slot order.  The last block to finish scans the tiles' counts of them, so that
+// k_new_paths can number them (pixels are assigned as new_path.cl:41-43 would over
+// the slots in order), hands the bounce's counts to the kernels that follow,
+// advances the sample counter (finalize_new_path, new_path.cl:85-88) and clears what
+// the next bounce counts in, so that a bounce needs no memset.
+__global__ void __launch_bounds__(256) k_classify(PathsView P, QueueView Q, InnerView I, RenderParams rp,
+                                                  unsigned long long* trace_next, int boundary) {
+    const unsigned full = 0xffffffffu;
+    __shared__ unsigned long long s_lo[8], s_hi[8];
+    __shared__ uint32_t s_off[kNumQueues + 1], s_base[kNumQueues], s_last;
+    __shared__ uint16_t s_list[kTile];
+    const uint32_t t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint4 q4 = *reinterpret_cast<const uint4*>(P.qid + t * kTile + tid * 16);
+    const uint32_t words[4] = {q4.x, q4.y, q4.z, q4.w};
+    // fields: queues 0..3 in lo, 4..6 in hi; idle slots in none
+    unsigned long long lo = 0ull, hi = 0ull;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const uint32_t q = (words[k >> 2] >> (8 * (k & 3))) & 0xffu;
+        if (q < 4u) lo += 1ull << (16 * q);
+        else if (q < (uint32_t)kNumQueues) hi += 1ull << (16 * (q - 4u));
+    }
+    unsigned long long ilo = lo, ihi = hi;  // inclusive over the warp
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long a = __shfl_up_sync(full, ilo, o), b = __shfl_up_sync(full, ihi, o);
+        if ((int)lane >= o) ilo += a, ihi += b;
+    }
+    if (lane == 31) s_lo[warp] = ilo, s_hi[warp] = ihi;
+    __syncthreads();
+    unsigned long long plo = ilo - lo, phi = ihi - hi, tlo = 0ull, thi = 0ull;
+#pragma unroll
+    for (uint32_t w = 0; w < 8; ++w) {
+        if (w < warp) plo += s_lo[w], phi += s_hi[w];
+        tlo += s_lo[w], thi += s_hi[w];
+    }
+    uint32_t off[kNumQueues + 1];
+    off[0] = 0;
+#pragma unroll
+    for (int k = 0; k < kNumQueues; ++k)
+        off[k + 1] = off[k] + (uint32_t)((k < 4 ? tlo >> (16 * k) : thi >> (16 * (k - 4))) & 0xffffull);
+    if (tid < (uint32_t)kNumQueues) {
+        const uint32_t n = pick(off, (int)tid + 1) - pick(off, (int)tid);
+        s_off[tid] = pick(off, (int)tid);
+        if (tid == 0) {
+            Q.tile_new[t] = n;
+            if (off[kNumQueues]) atomicAdd(rp.rays, (unsigned long long)off[kNumQueues]);
+        } else if (n) {
+            s_base[tid] = atomicAdd(Q.counts + tid, n);
+        }
+    }
+    if (off[kNumQueues] != 0u) {  // not an idle tile (the same in every thread)
+        // the thread's slots into class order
+        plo += (unsigned long long)off[0] | (unsigned long long)off[1] << 16 | (unsigned long long)off[2] << 32 |
+               (unsigned long long)off[3] << 48;
+        phi += (unsigned long long)off[4] | (unsigned long long)off[5] << 16 | (unsigned long long)off[6] << 32;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const uint32_t q = (words[k >> 2] >> (8 * (k & 3))) & 0xffu;
+            if (q < 4u) {
+                s_list[(plo >> (16 * q)) & 0xffffull] = (uint16_t)(tid * 16 + k);
+                plo += 1ull << (16 * q);
+            } else if (q < (uint32_t)kNumQueues) {
+                s_list[(phi >> (16 * (q - 4u))) & 0xffffull] = (uint16_t)(tid * 16 + k);
+                phi += 1ull << (16 * (q - 4u));
+            }
+        }
+        __syncthreads();
+        for (uint32_t j = tid; j < off[1]; j += 256) I.ended[t * kTile + j] = s_list[j];
+        for (uint32_t j = off[1] + tid; j < off[kNumQueues]; j += 256) {
+            int q = 1;
+#pragma unroll
+            for (int k = 2; k < kNumQueues; ++k) q += j >= off[k] ? 1 : 0;
+            queue_items(Q, q)[s_base[q] + j - s_off[q]] = t * kTile + s_list[j];
+        }
+    }
+    // the last block: every block's counts are in
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(I.words + InnerView::kTicket, 1u) + 1u == gridDim.x ? 1u : 0u;
+    __syncthreads();
+    if (!s_last) return;
+    uint32_t run = 0;
+    __shared__ uint32_t s_sum[8];
+    for (uint32_t b0 = 0; b0 < Q.ntiles; b0 += 1024) {  // four tiles a thread
+        uint32_t v[4], x = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t i = b0 + 4 * tid + k;
+            v[k] = i < Q.ntiles ? __ldcg(Q.tile_new + i) : 0u;
+            x += v[k];
+        }
+        uint32_t inc = x;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(full, inc, o);
+            if ((int)lane >= o) inc += y;
+        }
+        if (lane == 31) s_sum[warp] = inc;
+        __syncthreads();
+        uint32_t e = run + inc - x;
+#pragma unroll
+        for (uint32_t w = 0; w < 8; ++w) {
+            if (w < warp) e += s_sum[w];
+            run += s_sum[w];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t i = b0 + 4 * tid + k;
+            if (i < Q.ntiles) I.tile_first[i] = e;
+            e += v[k];
+        }
+        __syncthreads();  // s_sum is read
+    }
+    if (tid == 0) {
+        uint32_t went_on = 0;
+        for (int k = 1; k < kNumQueues; ++k) went_on |= I.words[k] = __ldcg(Q.counts + k);
+        for (int k = 1; k < kNumQueues; ++k) Q.counts[k] = 0u;
+        const unsigned long long np = *Q.next_pixel;
+        const bool over = boundary && went_on == 0u && np >= rp.sample_limit;
+        I.words[InnerView::kEnded] = run;
+        I.words[InnerView::kStop] = over ? 1u : 0u;
+        I.words[InnerView::kTicket] = 0u;
+        I.words[0] = over ? 0u : run;
+        if (!over) {
+            Q.counts[0] = run;
+            *Q.step_base = np;
+            *Q.next_pixel = np + run;
+        }
+        *trace_next = 0ull;
+    }
+}
+
+// The paths that ended in a bounce inside a run, and the new ones in their slots: the
+// logic of the ended path (its envmap radiance and accumulation; the cast has
+// only found that it ends), then the new path's first ray.  One ended path per
+// thread, numbered in slot order, so that every lane has work; the slots go to queue 0
+// for the cast.
+// Bound by the records' DRAM traffic (a 128-byte line read, 96 bytes written per slot)
+// and, where paths leave the scene, the envmap look-up's arithmetic.
+// When the render is over (launch_inner's boundary) the paths are only finished.
+constexpr int kNewPathsBlocks = 8;  // per SM
+__global__ void __launch_bounds__(256) k_new_paths(PathsView P, QueueView Q, InnerView I, RenderParams rp) {
+    const unsigned full = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t total = I.words[InnerView::kEnded];
+    const bool over = I.words[InnerView::kStop] != 0u;
+    const unsigned long long np = *Q.step_base;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t j0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); j0 < total; j0 += stride) {
+        // the tile of the warp's first path: the last one whose first number is <= j0
+        // (a 32-way search of the scanned counts), then each lane's own
+        uint32_t lo = 0, n = Q.ntiles;
+        while (n > 1u) {
+            const uint32_t step = (n + 31u) / 32u, i = lo + lane * step;
+            const unsigned m = __ballot_sync(full, lane * step < n && I.tile_first[i] <= j0);
+            const uint32_t k = 31u - __clz(m);  // lane 0's is always
+            lo += k * step;
+            n = min(step, n - k * step);
+        }
+        const uint32_t j = j0 + lane;
+        const unsigned have = __ballot_sync(full, j < total);
+        if (j >= total) continue;
+        uint32_t t = lo, tf = I.tile_first[lo];
+        while (t + 1u < Q.ntiles) {
+            const uint32_t next = I.tile_first[t + 1u];
+            if (next > j) break;
+            ++t;
+            tf = next;
+        }
+        const uint32_t slot = t * kTile + I.ended[t * kTile + (j - tf)];
+        // the ended path
+        const int req = P.req[slot];
+        const RequestD& old = rp.reqs[req];
+        float4 ro4, rd4, T4, L4, ng4, rng4;
+        ld_sector<0>(P, slot, ro4, rd4);
+        ld_sector<1>(P, slot, T4, L4);
+        ld_sector<2>(P, slot, ng4, rng4);
+        SlotState st;
+        const int32_t word = __float_as_int(rd4.w);  // the hit, or the volume hit
+        st.hv = word <= -2 ? -1 : word;
+        const int32_t hs = word <= -2 ? -2 - word : -1;
+        const uint32_t lw = __float_as_uint(L4.w);
+        st.T = xyz(T4), st.L = xyz(L4);
+        st.rng = rng_of_bits(rng4);
+        logic_decide(old, hs, st.hv, depth_of(lw), st.T, st.L, st.rng);
+        if (hs < 0 && st.hv < 0 && old.sc.has_env)
+            st.L = st.L + st.T * envmap_value(old.sc, xyz(rd4), depth_of(lw) == 0);
+        accumulate(old, __float_as_uint(T4.w), st.L);
+        count_done(old, req, true, have);
+        unsigned long long gpix = np + j;
+        const bool retire = rp.sample_limit != 0ull && gpix >= rp.sample_limit;
+        if (!over) Q.items[0][j] = slot;
+        if (over || retire) {  // the state as the plain logic leaves it
+            int32_t h2 = __float_as_int(ng4.w), v2 = word;
+            int mtype;
+            resolve_hit(old.sc, ro4, rd4, v2, h2, ng4, mtype);
+            st_sector<1>(P, slot, f4(st.T, T4.w),
+                         f4(st.L, __uint_as_float(depth_word(depth_of(lw) + 1, vcount_of(lw)))));
+            st_sector<2>(P, slot, ng4, rng_bits(st.rng));
+            if (!over) P.qid[slot] = kQueueIdle;  // sample budget reached: the slot retires
+            continue;
+        }
+        int r = 0;  // the request whose sample range holds this global sample index
+        while (r + 1 < rp.nreq && gpix >= rp.reqs[r].sample_end) ++r;
+        P.req[slot] = (uint16_t)r;
+        gpix -= rp.reqs[r].sample_begin;
+        st.va = make_int4(0, 0, 0, 0), st.vb = st.va;
+        shade_state<false>(rp.reqs[r], 0, slot, gpix, rp.gd, ~0u, st);
+        st_sector<0>(P, slot, f4(st.ro, st.tmin), f4(st.rd, __int_as_float(st.hv)));
+        st_sector<1>(P, slot, f4(st.T, __uint_as_float(st.pixel)), f4(st.L, __uint_as_float(depth_word(0u, 0))));
+        st_sector<2>(P, slot, f4(st.Ng, __int_as_float(st.hs)), rng_bits(st.rng));
+    }
 }
 
 // RGB16 intermediate (accumlation.cl:6-25) from FP64 sums: mean in double,
@@ -1280,7 +1607,7 @@ cudaError_t launch_trace_paths(const PathsView& p, const QueueView& q, const Ren
     if (!ts.persistent) return cudaSuccess;
     const cudaError_t e = cudaMemsetAsync(ts.counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
-    k_trace_paths<<<ts.grid, kStackThreads, 0, st>>>(p, q, rp, ts.counter, ts.refill, ts.search);
+    k_trace_paths<false><<<ts.grid, kStackThreads, 0, st>>>(p, q, rp, ts.counter, ts.refill, ts.search);
     return cudaSuccess;
 }
 
@@ -1302,13 +1629,38 @@ void launch_trace_logic(const PathsView& p, const QueueView& q, const RenderPara
     }
 }
 
+// what a bounce inside a run counts in
+void launch_inner_reset(const QueueView& q, const InnerView& in, cudaStream_t st) {
+    cudaMemsetAsync(in.words, 0, sizeof(uint32_t) * InnerView::kWords, st);
+    cudaMemsetAsync(q.counts + 1, 0, sizeof(uint32_t) * (kNumQueues - 1), st);
+}
+
+cudaError_t launch_inner_cast(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
+                              cudaStream_t st) {
+    const cudaError_t e = cudaMemsetAsync(ts.counter, 0, sizeof(unsigned long long), st);
+    if (e != cudaSuccess) return e;
+    k_trace_paths<true><<<ts.grid, kStackThreads, 0, st>>>(p, q, rp, ts.counter, ts.refill, ts.search);
+    return cudaSuccess;
+}
+
+void launch_inner(const PathsView& p, const QueueView& q, const InnerView& in, const RenderParams& rp,
+                  const TraceShape& ts, bool boundary, int shade_grid, int num_sms, cudaStream_t st) {
+    k_classify<<<q.ntiles, 256, 0, st>>>(p, q, in, rp, ts.counter, boundary ? 1 : 0);
+    const int blocks = std::min((int)((p.n + 255) / 256), num_sms * kNewPathsBlocks);
+    k_new_paths<<<blocks, 256, 0, st>>>(p, q, in, rp);
+    QueueView u = q;
+    u.counts = in.words;
+    k_shade_inner<<<shade_grid, 256, 0, st>>>(p, u, rp);
+    k_trace_paths<true><<<ts.grid, kStackThreads, 0, st>>>(p, u, rp, ts.counter, ts.refill, ts.search);
+}
+
 void launch_stamp_done(const RenderParams& rp, cudaStream_t st) {
     if (rp.nreq > 0) k_stamp_done<<<(rp.nreq + 127) / 128, 128, 0, st>>>(rp);
 }
 
 int trace_paths_max_blocks_per_sm() {
     int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_paths, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_paths<false>, 256, 0);
     return nb;
 }
 void launch_readback(int fmt, const double* accum, uint32_t npix, void* out, cudaStream_t st) {

@@ -270,6 +270,33 @@ cudaError_t launch_trace_paths(const PathsView& p, const QueueView& q, const Ren
                                cudaStream_t st);
 void launch_trace_logic(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
                         cudaStream_t st);
+// One bounce inside a run of several (plain renders).  Between two bounces of a
+// run nobody looks at the state, so there is no logic pass over it: the cast decides
+// each path's next queue as its ray ends (the hit's material type is in the
+// primitive's record) and writes it as the slot's queue id, a byte; then
+//   1. k_classify builds the queues and the new-path counts from those bytes;
+//   2. k_new_paths finishes the paths that ended (logic, envmap, accumulation) and
+//      starts the new ones in their slots;
+//   3. k_shade_inner shades the material queues, with the logic's share of a path
+//      that goes on first;
+//   4. the cast of the bounce's rays.
+// A run of n bounces is compaction, shading and cast (launch_compact_new,
+// launch_shade, launch_inner_cast, launch_inner_reset), n - 1 of these, and the plain
+// logic kernel, which leaves the state and the queues as a bounce alone does.
+// boundary: if no path went on and the sample budget is handed out, the render is
+// over: the ended paths are finished, the state is what the plain logic leaves, and
+// word kStop of InnerView is 1 (0 otherwise).
+struct InnerView {
+    enum { kTicket = 8, kStop = 9, kEnded = 10, kWords = 16 };
+    uint32_t* words;       // 0..6 the counts of the bounce's queues; the words above
+    uint32_t* tile_first;  // per tile: the ended paths of the tiles before it
+    uint16_t* ended;       // per tile kTile entries: its ended paths' slots, less the tile's first
+};
+void launch_inner_reset(const QueueView& q, const InnerView& in, cudaStream_t st);
+cudaError_t launch_inner_cast(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
+                              cudaStream_t st);
+void launch_inner(const PathsView& p, const QueueView& q, const InnerView& in, const RenderParams& rp,
+                  const TraceShape& ts, bool boundary, int shade_grid, int num_sms, cudaStream_t st);
 int trace_paths_max_blocks_per_sm();
 // per-request completion stamps of a batch (after the logic kernel of a bounce)
 void launch_stamp_done(const RenderParams& rp, cudaStream_t st);

@@ -53,8 +53,12 @@ inline uint32_t make_leaf_link(uint32_t first, uint32_t count) {
     return kLeafFlag | ((count - 1u) << 28) | first;
 }
 // Primitive record, 48 bytes, in leaf order (= the reference primitive_ids order).
-//   triangle: (v0.xyz, id) (v1-v0, 0) (v2-v0, 0)
-//   sphere:   (center.xyz, id) (radius, 0, 0, flag 1) (0)
+//   triangle: (v0.xyz, word) (v1-v0, 0) (v2-v0, 0)
+//   sphere:   (center.xyz, word) (radius, 0, 0, flag 1) (0)
+// word: the primitive id (below 2^28), and in bits 28..30 its material type (1..5),
+// so that a render's cast knows the queue of a hit without another gather
+constexpr uint32_t kPrimIdMask = 0x0fffffffu;
+inline uint32_t prim_word(uint32_t id, int32_t type) { return id | (uint32_t)type << 28; }
 struct alignas(16) PrimD {
     float a[4];
     float b[4];
