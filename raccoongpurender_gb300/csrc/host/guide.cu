@@ -158,24 +158,27 @@ void rgr_guide::infer_paths(const PathsView& p, const QueueView& q, const GuideR
         launch_guide_infer_paths(view, p, q, gd, guide_infer_grid(num_sms), st);
 }
 
-void rgr_guide::gradient_launches(const float* smp, const uint32_t* count, uint32_t cap, uint32_t min_count,
-                                  const float* wsum, float weight_scale, int grid, cudaStream_t st) {
-    if (cfg.training_kernel == RGR_GUIDE_TCGEN05) {
-        launch_guide_train_tc(view, smp, count, cap, min_count, wsum, weight_scale, grid, gpart.as<float>(),
-                              error_word(), st);
-        launch_guide_grad_reduce(view, gpart.as<float>(), (uint32_t)grid, count, min_count, st);
-    } else {
-        launch_guide_train(view, smp, count, cap, min_count, wsum, weight_scale, grid, st);
-    }
+GuideAdam rgr_guide::adam() const { return GuideAdam{cfg.learning_rate, cfg.beta1, cfg.beta2, cfg.epsilon}; }
+
+void rgr_guide::iteration_launches(const float* smp, const uint32_t* count, uint32_t n, const GuideTrainD& t,
+                                   const float* wsum, float weight_scale, int grid, bool step, float* grads,
+                                   cudaStream_t st) {
+    launch_guide_train_tc(view, smp, count, n, t.min_count, wsum, weight_scale, grid, gpart.as<float>(), error_word(),
+                          st);
+    launch_guide_update_tc(view, gpart.as<float>(), (uint32_t)grid, count, n, grads, step, adam(), t, st);
 }
 
 int rgr_guide::train_launches(cudaStream_t st) {
-    if (cfg.train) {
-        gradient_launches(train.samples, train.count, train.cap, train.min_count, train.wsum, 1.0f, num_sms, st);
-        launch_guide_adam(view, train.count, train.min_count, train.iter, cfg.learning_rate, cfg.beta1, cfg.beta2,
-                          cfg.epsilon, st);
+    if (cfg.train && cfg.training_kernel == RGR_GUIDE_TCGEN05) {
+        iteration_launches(train.samples, train.count, train.cap, train, train.wsum, 1.0f, num_sms, true, nullptr, st);
+    } else {
+        if (cfg.train) {
+            launch_guide_train(view, train.samples, train.count, train.cap, train.min_count, train.wsum, 1.0f, num_sms,
+                               st);
+            launch_guide_adam(view, train.count, train.min_count, train.iter, adam(), st);
+        }
+        launch_guide_finish(view, train, st);
     }
-    launch_guide_finish(view, train, st);
     RGR_CUDA(cudaGetLastError());
     return RGR_OK;
 }
@@ -345,19 +348,28 @@ int rgr_guide_train_device(rgr_guide* g, const float* samples, uint32_t n, float
     if (!g || (n && !samples) || !std::isfinite(weight_scale)) return RGR_E_INVALID;
     RGR_CUDA(cudaSetDevice(g->device));
     cudaStream_t st = (cudaStream_t)stream;
+    float hl = 0.0f;
+    if (n > 0 && g->cfg.training_kernel == RGR_GUIDE_TCGEN05) {
+        g->iteration_launches(samples, nullptr, n, g->test, nullptr, weight_scale, train_grid(*g, n), apply_adam != 0,
+                              grads, st);
+        RGR_CUDA(cudaGetLastError());
+        RGR_CUDA(cudaMemcpyAsync(&hl, g->loss.as<float>() + 1, 4, cudaMemcpyDeviceToHost, st));
+        RGR_CUDA(cudaStreamSynchronize(st));
+        if (loss) *loss = hl;
+        return RGR_OK;
+    }
     RGR_CUDA(cudaMemcpyAsync(g->test.count, &n, 4, cudaMemcpyHostToDevice, st));
     RGR_CUDA(cudaMemsetAsync(g->loss.p, 0, 4, st));
-    g->gradient_launches(samples, g->test.count, n, 0u, nullptr, weight_scale, train_grid(*g, n), st);
+    if (n > 0)
+        launch_guide_train(g->view, samples, g->test.count, n, 0u, nullptr, weight_scale, train_grid(*g, n), st);
     RGR_CUDA(cudaGetLastError());
     if (grads) {
         RGR_CUDA(cudaMemcpyAsync(grads, g->gW.p, 4 * kGuideWeights, cudaMemcpyDeviceToDevice, st));
         RGR_CUDA(cudaMemcpyAsync(grads + kGuideWeights, g->gb.p, 4 * kGuideBiases, cudaMemcpyDeviceToDevice, st));
     }
-    float hl = 0.0f;
     RGR_CUDA(cudaMemcpyAsync(&hl, g->loss.p, 4, cudaMemcpyDeviceToHost, st));
     if (apply_adam) {
-        launch_guide_adam(g->view, g->test.count, 0u, g->test.iter, g->cfg.learning_rate, g->cfg.beta1, g->cfg.beta2,
-                          g->cfg.epsilon, st);
+        launch_guide_adam(g->view, g->test.count, 0u, g->test.iter, g->adam(), st);
         launch_guide_finish(g->view, g->test, st);
         RGR_CUDA(cudaGetLastError());
     } else {
@@ -376,12 +388,16 @@ int rgr_guide_train_device_async(rgr_guide* g, const float* samples, uint32_t n,
     if (n == 0) return RGR_OK;
     RGR_CUDA(cudaSetDevice(g->device));
     cudaStream_t st = (cudaStream_t)stream;
+    if (g->cfg.training_kernel == RGR_GUIDE_TCGEN05) {
+        g->iteration_launches(samples, nullptr, n, g->test, nullptr, weight_scale, train_grid(*g, n), true, nullptr, st);
+        RGR_CUDA(cudaGetLastError());
+        return RGR_OK;
+    }
     // n reaches the test stream's count word by a kernel, in stream order
     RGR_CUDA(cudaMemsetAsync(g->loss.p, 0, 4, st));
     launch_guide_set_count(g->test.count, n, st);
-    g->gradient_launches(samples, g->test.count, n, 0u, nullptr, weight_scale, train_grid(*g, n), st);
-    launch_guide_adam(g->view, g->test.count, 0u, g->test.iter, g->cfg.learning_rate, g->cfg.beta1, g->cfg.beta2,
-                      g->cfg.epsilon, st);
+    launch_guide_train(g->view, samples, g->test.count, n, 0u, nullptr, weight_scale, train_grid(*g, n), st);
+    launch_guide_adam(g->view, g->test.count, 0u, g->test.iter, g->adam(), st);
     launch_guide_finish(g->view, g->test, st);
     RGR_CUDA(cudaGetLastError());
     return RGR_OK;

@@ -28,8 +28,9 @@ struct rgr_guide {
     // the launches that follow the trace/logic kernel of a guided render on the
     // bounces that end a training interval: train, Adam, reset the stream
     int train_launches(cudaStream_t st);
-    // one iteration's gradient launches (the configured training kernel) over
-    // min(*count, cap) samples, into gW, gb and the loss; `grid` CTAs
-    void gradient_launches(const float* samples, const uint32_t* count, uint32_t cap, uint32_t min_count,
-                           const float* wsum, float weight_scale, int grid, cudaStream_t st);
+    rgr::dev::GuideAdam adam() const;
+    // one iteration with the tcgen05 kernels over min(*count, n) samples (n with count null):
+    // gradients to `grads` if given; with `step`, Adam and the bookkeeping of t; `grid` CTAs
+    void iteration_launches(const float* samples, const uint32_t* count, uint32_t n, const rgr::dev::GuideTrainD& t,
+                            const float* wsum, float weight_scale, int grid, bool step, float* grads, cudaStream_t st);
 };

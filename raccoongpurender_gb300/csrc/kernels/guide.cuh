@@ -56,7 +56,8 @@ struct GuideView {
     float* gb;
     float* m;              // Adam moments, kGuideParams each (weights then biases)
     float* v;
-    float* loss;           // sum of sample losses of the last batch
+    float* loss;           // [0] sum of sample losses of the current batch, [1] of the last one
+                           // (tcgen05 training); [2] the update kernel's block ticket
     GuideParams params;
     uint32_t stall_mma;    // failure-detection tests: the tcgen05 inference kernel's MMA warps
                            // issue nothing, so its row threads' bounded waits run out
@@ -258,6 +259,58 @@ __device__ __forceinline__ void mixture_sample(const uint4* p, float u0, float u
     d[2] = z * n;
 }
 
+// ------------------------------------------------------------ Adam
+struct GuideAdam {
+    float lr, beta1, beta2, eps;
+};
+// Adam on parameter i (weights, then biases) with gradient gr, iteration number t: FP32
+// master, moments, and the BF16 copies that the inference and training kernels read
+__device__ __forceinline__ void adam_update(const GuideView& g, uint32_t i, float gr, float t, const GuideAdam& a) {
+    const float bc1 = 1.0f - powf(a.beta1, t), bc2 = 1.0f - powf(a.beta2, t);
+    const bool is_w = i < (uint32_t)kGuideWeights;
+    float* p = is_w ? g.w + i : g.b + (i - kGuideWeights);
+    const float mm = a.beta1 * g.m[i] + (1.0f - a.beta1) * gr;
+    const float vv = a.beta2 * g.v[i] + (1.0f - a.beta2) * gr * gr;
+    g.m[i] = mm;
+    g.v[i] = vv;
+    // a parameter whose gradient was always zero (the padding) keeps m = v = 0 and does not move
+    const float nv = *p - a.lr * (mm / bc1) / (sqrtf(vv / bc2) + a.eps);
+    *p = nv;
+    if (is_w) {
+        const __nv_bfloat16 h = __float2bfloat16_rn(nv);
+        g.wbf[i] = h;
+        const uint32_t l = i / 4096u, in = (i / 64u) % 64u, out = i % 64u;
+        if (!wt_is_bias_slot(l, in)) *reinterpret_cast<__nv_bfloat16*>(g.wt_sw + wt_sw_offset(l, in, out)) = h;
+    } else {
+        const uint32_t j = i - kGuideWeights, l = j / 64u, out = j % 64u;
+        const __nv_bfloat16 hi = __float2bfloat16_rn(nv);
+        const __nv_bfloat16 lo = __float2bfloat16_rn(nv - __bfloat162float(hi));
+        *reinterpret_cast<__nv_bfloat16*>(g.wt_sw + wt_bias_offset(l, out, 0)) = hi;
+        *reinterpret_cast<__nv_bfloat16*>(g.wt_sw + wt_bias_offset(l, out, 1)) = lo;
+    }
+}
+// after an iteration over c samples (one thread): advance *iter, log the loss, retune the
+// acceptance, reset the counters; fewer than min_count samples carry over
+__device__ __forceinline__ void finish_iteration(const GuideView& g, const GuideTrainD& t, uint32_t c) {
+    const unsigned long long cand = *t.candidates;
+    // aim the next iteration at `cap` accepted records
+    if (cand > 0ull) *t.accept = fminf(1.0f, (float)t.cap / (float)cand);
+    // no step this bounce: the samples stay for the next one.  Few paths end at the
+    // tail of a render, and Adam's normalised step would turn a handful of samples
+    // into a full-size, noisy update.
+    if (c < t.min_count) return;
+    if (c > 0u) {
+        const uint32_t it = *t.iter;
+        t.loss_hist[it % kLossHist] = g.loss[0];
+        *t.iter = it + 1u;
+    }
+    *t.last = min(c, t.cap);
+    *t.count = 0u;
+    *t.wsum = 0.0f;
+    *t.candidates = 0ull;
+    g.loss[0] = 0.0f;
+}
+
 // ------------------------------------------------------------ launchers (guide_mlp.cu)
 size_t guide_infer_smem();
 size_t guide_train_smem();
@@ -277,23 +330,27 @@ void launch_guide_train(const GuideView& g, const float* samples, const uint32_t
                         uint32_t min_count, const float* wsum, float weight_scale, int grid, cudaStream_t st);
 // Adam on the accumulated gradients when *count > 0 and >= min_count; iteration number from *iter + 1
 void launch_guide_adam(const GuideView& g, const uint32_t* count, uint32_t min_count, const uint32_t* iter,
-                       float lr, float beta1, float beta2, float eps, cudaStream_t st);
+                       const GuideAdam& adam, cudaStream_t st);
 // *count = n, in stream order (the sample count of an iteration enqueued from the host)
 void launch_guide_set_count(uint32_t* count, uint32_t n, cudaStream_t st);
 // after an iteration: advance *iter, log the loss, retune the acceptance, reset counters
 void launch_guide_finish(const GuideView& g, const GuideTrainD& t, cudaStream_t st);
 
 // tcgen05 / TMEM training (guide_train_tc.cu): one iteration over min(*count, cap)
-// samples into the CTAs' slots of `part` (grid x kGuidePartStride floats), nothing
-// while fewer than min_count samples are in; then launch_guide_grad_reduce sums
-// the grid's slots into gW, gb and the loss.  A timed-out wait sets bit 1 of *err.
+// samples (cap of them with count null) into the CTAs' slots of `part` (grid x
+// kGuidePartStride floats), nothing while fewer than min_count samples are in.  A
+// timed-out wait sets bit 1 of *err.
 size_t guide_train_tc_smem();
 int guide_train_tc_attributes();  // cudaError_t of opting the kernel into its shared memory
 void launch_guide_train_tc(const GuideView& g, const float* samples, const uint32_t* count, uint32_t cap,
                            uint32_t min_count, const float* wsum, float weight_scale, int grid, float* part,
                            uint32_t* err, cudaStream_t st);
-void launch_guide_grad_reduce(const GuideView& g, const float* part, uint32_t nparts, const uint32_t* count,
-                              uint32_t min_count, cudaStream_t st);
+// What follows it: the sum of the grid's slots, in a fixed order, as the gradients (to
+// `grads`, kGuideParams floats, if given) and the loss (g.loss[1]); with `step` also Adam
+// (iteration number *t.iter + 1) and the iteration's bookkeeping in t.
+void launch_guide_update_tc(const GuideView& g, const float* part, uint32_t nparts, const uint32_t* count,
+                            uint32_t cap, float* grads, bool step, const GuideAdam& adam, const GuideTrainD& t,
+                            cudaStream_t st);
 
 // tcgen05 / TMEM inference (guide_tc.cu): same results as the mma.sync kernels up
 // to FP32 accumulation order; a timed-out tensor-core wait sets bit 0 of *err

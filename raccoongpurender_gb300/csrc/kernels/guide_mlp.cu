@@ -514,63 +514,16 @@ __global__ void __launch_bounds__(32 * kTrainWarps) k_guide_train(GuideView gv, 
 }
 
 // ---------------------------------------------------------------- Adam
-__global__ void k_guide_adam(GuideView g, const uint32_t* count, uint32_t min_count, const uint32_t* iter, float lr,
-                             float beta1, float beta2, float eps) {
+__global__ void k_guide_adam(GuideView g, const uint32_t* count, uint32_t min_count, const uint32_t* iter, GuideAdam a) {
     if (*count == 0u || *count < min_count) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kGuideParams) return;
-    const float t = (float)(*iter + 1u);
-    const float bc1 = 1.0f - powf(beta1, t), bc2 = 1.0f - powf(beta2, t);
-    const bool is_w = i < kGuideWeights;
-    float* p = is_w ? g.w + i : g.b + (i - kGuideWeights);
-    float* grad = is_w ? g.gW + i : g.gb + (i - kGuideWeights);
-    const float gr = *grad;
-    const float mm = beta1 * g.m[i] + (1.0f - beta1) * gr;
-    const float vv = beta2 * g.v[i] + (1.0f - beta2) * gr * gr;
-    g.m[i] = mm;
-    g.v[i] = vv;
-    // a parameter whose gradient was always zero (the padding) keeps m = v = 0 and does not move
-    const float nv = *p - lr * (mm / bc1) / (sqrtf(vv / bc2) + eps);
-    *p = nv;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (uint32_t)kGuideParams) return;
+    float* grad = i < (uint32_t)kGuideWeights ? g.gW + i : g.gb + (i - kGuideWeights);
+    adam_update(g, i, *grad, (float)(*iter + 1u), a);
     *grad = 0.0f;
-    if (is_w) {
-        const __nv_bfloat16 h = __float2bfloat16_rn(nv);
-        g.wbf[i] = h;
-        const uint32_t l = (uint32_t)i / 4096u, in = ((uint32_t)i / 64u) % 64u, out = (uint32_t)i % 64u;
-        if (!wt_is_bias_slot(l, in)) *reinterpret_cast<__nv_bfloat16*>(g.wt_sw + wt_sw_offset(l, in, out)) = h;
-    } else {
-        const uint32_t j = (uint32_t)(i - kGuideWeights), l = j / 64u, out = j % 64u;
-        const __nv_bfloat16 hi = __float2bfloat16_rn(nv);
-        const __nv_bfloat16 lo = __float2bfloat16_rn(nv - __bfloat162float(hi));
-        *reinterpret_cast<__nv_bfloat16*>(g.wt_sw + wt_bias_offset(l, out, 0)) = hi;
-        *reinterpret_cast<__nv_bfloat16*>(g.wt_sw + wt_bias_offset(l, out, 1)) = lo;
-    }
 }
 
-__global__ void k_guide_finish(GuideView g, GuideTrainD t) {
-    const uint32_t c = *t.count;
-    if (c < t.min_count) {
-        // no step this bounce: the samples stay for the next one.  Few paths
-        // end at the tail of a render, and Adam's normalised step would turn
-        // a handful of samples into a full-size, noisy update.
-        const unsigned long long cand = *t.candidates;
-        if (cand > 0ull) *t.accept = fminf(1.0f, (float)t.cap / (float)cand);
-        return;
-    }
-    if (c > 0u) {
-        const uint32_t it = *t.iter;
-        t.loss_hist[it % kLossHist] = *g.loss;
-        *t.iter = it + 1u;
-    }
-    *t.last = min(c, t.cap);
-    // aim the next iteration at `cap` accepted records
-    const unsigned long long cand = *t.candidates;
-    if (cand > 0ull) *t.accept = fminf(1.0f, (float)t.cap / (float)cand);
-    *t.count = 0u;
-    *t.wsum = 0.0f;
-    *t.candidates = 0ull;
-    *g.loss = 0.0f;
-}
+__global__ void k_guide_finish(GuideView g, GuideTrainD t) { finish_iteration(g, t, *t.count); }
 
 __global__ void k_guide_set_count(uint32_t* count, uint32_t n) { *count = n; }
 
@@ -605,8 +558,8 @@ void launch_guide_train(const GuideView& g, const float* samples, const uint32_t
 }
 
 void launch_guide_adam(const GuideView& g, const uint32_t* count, uint32_t min_count, const uint32_t* iter,
-                       float lr, float beta1, float beta2, float eps, cudaStream_t st) {
-    k_guide_adam<<<(kGuideParams + 255) / 256, 256, 0, st>>>(g, count, min_count, iter, lr, beta1, beta2, eps);
+                       const GuideAdam& adam, cudaStream_t st) {
+    k_guide_adam<<<(kGuideParams + 255) / 256, 256, 0, st>>>(g, count, min_count, iter, adam);
 }
 
 void launch_guide_finish(const GuideView& g, const GuideTrainD& t, cudaStream_t st) {
