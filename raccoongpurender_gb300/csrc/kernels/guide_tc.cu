@@ -3,33 +3,40 @@
 // tensor memory (TMEM) and the weights in shared memory.
 //
 // A CTA (one per SM) holds kTcGroups groups of 128 row threads and kMmaWarps
-// warps that only issue MMAs.  A group works on tiles of 128 rows, kBufs tiles
-// in flight (buffers); thread t of the group owns row t of each from the input
+// warps that only issue MMAs.  A group works on one tile of 128 rows at a time;
+// thread t of the group owns row t of it from the input
 // encoding to the result.  Per tile in flight TMEM holds the
 // 128 x 64 FP32 accumulator and the layer's input as 64 bf16 a row (lane =
-// row).  Per layer and buffer:
+// row).  Per layer:
 //  * the row threads write the layer's input into TMEM (tcgen05.st): the
 //    encoding for the first layer, else the ReLU of the previous layer's
 //    accumulators, packed to bf16 in the same conversion (cvt.rn.relu.bf16x2);
-//    then they arrive on the buffer's a_full mbarrier;
-//  * an MMA warp, polling its buffers' a_full barriers, issues the layer
+//    then each warp arrives on the tile's a_full mbarrier;
+//  * an MMA warp, polling its tiles' a_full barriers, issues the layer
 //    (M 128, N 64, K 16, BF16 x BF16 -> FP32, A from TMEM, B = the layer's W^T
 //    from shared memory, 128-byte swizzle): for a hidden or the output layer
 //    one MMA that starts the accumulator at the bias (a TMEM chunk of ones
 //    times a B chunk holding each bias as the sum of two bf16 values), then
 //    one per 16 inputs; the first layer's 3 MMAs cover the encoding's 36
 //    inputs and two inputs fixed at 1.0 that carry its bias.  It commits them
-//    to the buffer's d_full mbarrier;
+//    to the tile's d_full mbarrier;
 //  * the row threads wait on d_full (a bounded wait) and read the
 //    accumulators back (tcgen05.ld).
 // While the tensor core runs one tile's layer, the row threads of the other
-// tiles (other groups, or the group's other buffers) run their epilogues.  After the last layer each thread has its row's 40
-// outputs in registers and computes the mixture (or keeps the raw outputs)
-// without any exchange; the tile's results (80-byte FP16 mixture records, or
-// 192 bytes of raw outputs) are staged in shared memory and leave in one bulk
-// copy.  Weights and bias chunks are staged once
-// per CTA by one bulk copy.  Every wait is bounded: on a timeout the CTA
-// records an error, stops issuing and frees its TMEM.
+// groups run their epilogues.  A group's next tile is encoded while the last
+// layer of the current one runs, and its first layer starts as soon as the
+// current outputs are in registers: the thread then has its row's 41
+// outputs and computes the mixture, or stores the raw outputs, while the tensor core
+// works; a warp's 32 rows (80-byte mixture records, or 192 bytes) are staged in shared
+// memory and leave in one bulk copy.  Weights and bias chunks are staged once per CTA
+// by one bulk copy, which only the MMA warps wait for.  Every wait is bounded: on a
+// timeout the CTA records an error, stops issuing and frees its TMEM.
+//
+// Bound by a row thread's chain: of 32k cycles for three tiles 3.2k pass before the
+// tensor memory is allocated, 7k waiting for the twelve hidden layers, 5k in their
+// epilogues, 3.4k in the encodings, 3.4k staging the outputs.  2^18 rows, launches in a row:
+// 22.6 us with the outputs staged (four-way bank conflicts, two group barriers) and the
+// next tile encoded before its first layer could start; 20.5 us.
 #include <cuda_bf16.h>
 
 #include "guide.cuh"
@@ -38,37 +45,26 @@ namespace rgr {
 namespace dev {
 namespace {
 
-// 128-row groups of row threads per CTA, and tiles in flight per group.  Five
-// groups of one tile each (2^18 rows: 19.0 us) beat two of two tiles (21.1 us)
-// and one of four or five (27 us): the row threads' encoding, epilogues and
-// mixtures, more than the MMAs, need the parallelism.  Five tiles of 96 TMEM
-// columns and the ones chunk fill the SM's 512 columns.
-#ifndef RGR_GUIDE_TC_GROUPS
-#define RGR_GUIDE_TC_GROUPS 5
-#endif
-constexpr int kTcGroups = RGR_GUIDE_TC_GROUPS;
-#ifndef RGR_GUIDE_TC_BUFS
-#define RGR_GUIDE_TC_BUFS 1
-#endif
-constexpr int kBufs = RGR_GUIDE_TC_BUFS;              // tiles in flight per group
+// 128-row groups of row threads per CTA, one tile each.  Five groups (2^18 rows:
+// 19.0 us) beat two groups of two tiles in flight (21.1 us) and one of four or
+// five (27 us): the row threads' encoding, epilogues and mixtures, more than the MMAs,
+// need the parallelism.  Five tiles of 96 TMEM columns and the ones chunk fill the SM's
+// 512 columns.
+constexpr int kTcGroups = 5;
 constexpr int kGroupThreads = 128;                    // rows per tile, one per thread
-// warps that issue the MMAs: warp kMmaWarp + m serves the buffers b = i kBufs + j
-// (group i, buffer j) with b % kMmaWarps == m (an issuing thread waits out
-// most of each MMA's issue latency, so buffers that share a warp share it)
-#ifndef RGR_GUIDE_TC_MMA_WARPS
-#define RGR_GUIDE_TC_MMA_WARPS 3
-#endif
-constexpr int kMmaWarps = RGR_GUIDE_TC_MMA_WARPS;
+// warps that issue the MMAs: warp kMmaWarp + m serves the groups i with i % kMmaWarps == m
+// (an issuing thread waits out most of each MMA's issue latency, so groups that share
+// a warp share it)
+constexpr int kMmaWarps = 3;
 constexpr int kMmaWarp = kTcGroups * 4;               // the first MMA warp
 constexpr int kTcThreads = kTcGroups * kGroupThreads + 32 * kMmaWarps;
 constexpr uint32_t kCtaRows = kTcGroups * 128u;       // rows of one tile per group
-constexpr int kAccs = kTcGroups * kBufs;              // tiles in flight per CTA
 // TMEM per tile in flight: the 128 x 64 FP32 accumulator (columns 0..63) and
 // the layer's input, 64 bf16 a row packed in pairs (columns 64..95); then the
 // ones chunk of the bias MMAs (row elements 0 and 1 are 1.0; 8 columns read,
 // 32 written)
 constexpr uint32_t kAccCols = 96;
-constexpr uint32_t kOnesCol = kAccs * kAccCols;
+constexpr uint32_t kOnesCol = kTcGroups * kAccCols;
 constexpr int kTcCols = 512;                          // TMEM columns allocated (a power of two)
 static_assert(kOnesCol + 32 <= (uint32_t)kTcCols, "TMEM columns");
 constexpr uint32_t kWaitNs = 1000000000u;             // a wait gives up after 1 s (%globaltimer)
@@ -77,10 +73,11 @@ constexpr uint32_t kErrTimeout = 1u;
 
 struct __align__(1024) SmemTc {
     unsigned char wt[kGuideWtBytes];                // the staged weights and bias chunks (50 x 1024 B)
-    unsigned char out[kTcGroups][128 * 4 * kGuideRowOutputs];  // a tile's output rows (80 or 192 bytes), one bulk copy
+    unsigned char out[kTcGroups * 4][32 * 4 * kGuideRowOutputs];  // a warp's rows (80 or 192 bytes), one bulk copy
     unsigned long long wbar;                        // the weights' bulk copy
-    unsigned long long a_full[kTcGroups][kBufs];    // the A tile of the next layer is written (128 arrivals)
-    unsigned long long d_full[kTcGroups][kBufs];    // the layer's MMAs are done (one commit)
+    unsigned long long obar;                        // the ones chunk is written (4 arrivals)
+    unsigned long long a_full[kTcGroups];           // the A tile of the next layer is written (one arrival per warp)
+    unsigned long long d_full[kTcGroups];           // the layer's MMAs are done (one commit)
     uint32_t tmem_base;
     uint32_t error;
 };
@@ -143,14 +140,22 @@ __device__ __forceinline__ uint32_t global_ns() {
     return t;
 }
 // bounded wait for the phase with the given parity: false after kWaitNs (or
-// kWaitPolls polls)
+// kWaitPolls polls); the timer, a slow register to read, is not read by a short wait
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-    const uint32_t t0 = global_ns();
+    uint32_t t0 = 0u;
     for (uint32_t i = 0; i < kWaitPolls; ++i) {
         if (mbar_try_wait(mbar, parity)) return true;
-        if ((i & 63u) == 63u && global_ns() - t0 > kWaitNs) return false;
+        if ((i & 63u) == 63u) {
+            const uint32_t now = global_ns();
+            if (i == 63u) t0 = now;
+            else if (now - t0 > kWaitNs) return false;
+        }
     }
     return false;
+}
+// the same by a whole (converged) warp, the same answer in every lane
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t mbar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait(mbar, parity));
 }
 // true in one lane of the (converged) warp
 __device__ __forceinline__ bool elect_one() {
@@ -179,21 +184,6 @@ __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
-
-// barrier of group g's 128 threads (named barrier g + 1) that also returns
-// whether any of them passed `mine` = true, the same answer in every thread
-__device__ __forceinline__ bool group_sync_any(uint32_t g, bool mine) {
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.u32 q, %1, 0;\n\t"
-        "bar.red.or.pred p, %2, %3, q;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(r)
-        : "r"((uint32_t)mine), "r"(g + 1u), "r"((uint32_t)kGroupThreads)
-        : "memory");
-    return r != 0u;
-}
 
 // FP32 accumulators of this thread's TMEM lane: 32 columns / 8 columns from taddr
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
@@ -248,7 +238,8 @@ __device__ __forceinline__ uint32_t relu_pack2(uint32_t lo, uint32_t hi) {
 // follows).  The row's 48 inputs as the first layer's A: 24 TMEM columns of
 // bf16 pairs (features 2c, 2c + 1 in column c, the lower one in the low
 // half); inputs 36 and 37 are 1.0 and carry the layer's bias, 38..47 zero.
-__device__ __forceinline__ void encode_store(uint32_t taddr, const float* x9, const GuideParams& gp) {
+// encode_row computes the 18 words of the features, store_input writes the input.
+__device__ __forceinline__ void encode_row(const float* x9, const GuideParams& gp, uint32_t* w) {
     float v[9];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -256,7 +247,6 @@ __device__ __forceinline__ void encode_store(uint32_t taddr, const float* x9, co
         v[3 + c] = 0.5f * (x9[3 + c] + 1.0f);
         v[6 + c] = 0.5f * (x9[6 + c] + 1.0f);
     }
-    uint32_t w[32];
 #pragma unroll
     for (int i = 0; i < 9; ++i) {
         float s, c;
@@ -264,10 +254,17 @@ __device__ __forceinline__ void encode_store(uint32_t taddr, const float* x9, co
         w[2 * i] = pack2(s, c);
         w[2 * i + 1] = pack2(2.0f * s * c, (c - s) * (c + s));
     }
-    w[18] = 0x3f803f80u;
-#pragma unroll
-    for (int i = 19; i < 32; ++i) w[i] = 0u;
-    tmem_st32(taddr, w);
+}
+__device__ __forceinline__ void store_input(uint32_t taddr, const uint32_t* w) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(taddr),
+        "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]), "r"(w[9]),
+        "r"(w[10]), "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15])
+        : "memory");
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%4,%4,%4,%4};\n" ::"r"(taddr + 16u),
+                 "r"(w[16]), "r"(w[17]), "r"(0x3f803f80u), "r"(0u)
+                 : "memory");
 }
 
 // ReLU of this row's 64 accumulators, as the next layer's A (32 columns at a_taddr)
@@ -317,6 +314,39 @@ __device__ __forceinline__ void row_mixture(const float* o, float alpha, uint4* 
     dst[4] = make_uint4(half2_bits(w[0] * r, w[1] * r), half2_bits(w[2] * r, w[3] * r), half2_bits(w[4] * r, w[5] * r),
                         half2_bits(w[6] * r, w[7] * r));
 }
+
+// The raw outputs of a row (48 words) into its 192 bytes of the warp's staging rows.  At a
+// stride of 192 bytes the 16-byte chunks of eight consecutive rows meet in two of the
+// eight bank groups; each row takes the chunks of a group of four in an order rotated
+// by (row / 2) % 4, so that the eight lie in eight.  (Stored unrotated, or as sectors straight
+// to global memory, a tile's rows took 3.2k cycles: 32 rows are 32 lines either way.)
+__device__ __forceinline__ void stage_row(unsigned char* row, uint32_t lane, const uint32_t* o) {
+    const bool r1 = (lane & 2u) != 0u, r2 = (lane & 4u) != 0u;
+    const uint32_t s = (lane >> 1) & 3u;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+        uint4 v[4], u[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const uint32_t* x = o + 16 * b + 4 * c;
+            v[c] = make_uint4(x[0], x[1], x[2], x[3]);
+        }
+        auto pick4 = [](bool p, const uint4& a, const uint4& c) {
+            return make_uint4(p ? a.x : c.x, p ? a.y : c.y, p ? a.z : c.z, p ? a.w : c.w);
+        };
+#pragma unroll
+        for (int c = 0; c < 4; ++c) u[c] = pick4(r1, v[(c + 1) & 3], v[c]);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) v[c] = pick4(r2, u[(c + 2) & 3], u[c]);
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; ++q)
+            *reinterpret_cast<uint4*>(row + 64 * b + 16u * ((q + s) & 3u)) = v[q];
+    }
+}
+
+// the line at p on its way to L1 (a row's 48 bytes lie in one): held there, not in registers,
+// while the layers run
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 // The 48 bytes a row's input comes from: the slot's (ro, rd, ng) for a
 // path vertex, the first 12 floats of a 16-float row otherwise.
@@ -375,12 +405,7 @@ __device__ __forceinline__ void issue_layer(uint32_t l, uint32_t tm, uint32_t ta
 // kPaths: rows are this bounce's guided queue items, output their mixtures;
 // otherwise rows of 16 floats in `rows`, output 40 raw floats per row.
 //
-// Tile k of group g is tile (blockIdx.x + k gridDim.x) kTcGroups + g of the
-// rows; the group runs its tiles kBufs at a time, tile k in buffer k % kBufs.
-// Per layer and buffer the group's threads write the layer's input and arrive
-// on a_full; the MMA warp serving the buffer, polling its a_full barriers,
-// issues that buffer's next layer and commits it to d_full; the threads wait
-// on d_full and run the epilogue.
+// Tile k of group g is tile (blockIdx.x + k gridDim.x) kTcGroups + g of the rows.
 template <bool kPaths>
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_guide_infer_tc(GuideView gv, const float* __restrict__ rows, uint32_t nrows, float* __restrict__ out,
@@ -393,16 +418,16 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     // warp and group indices the compiler knows to be warp-uniform, so that the
     // MMA operands derived from them live in uniform registers
     const uint32_t warp = __shfl_sync(0xffffffffu, t >> 5, 0), g = warp >> 2;
-    if (t == 0) {
+    if (t == 32u * kMmaWarp) {  // beside warp 0's allocation
         S.error = 0u;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&S.wbar)) : "memory");
-        for (int i = 0; i < kTcGroups; ++i)
-            for (int j = 0; j < kBufs; ++j) {
-                asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&S.a_full[i][j])),
-                             "r"(kGroupThreads)
-                             : "memory");
-                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&S.d_full[i][j])) : "memory");
-            }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;\n" ::"r"(smem_u32(&S.obar)) : "memory");
+        for (int i = 0; i < kTcGroups; ++i) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&S.a_full[i])),
+                         "r"(kGroupThreads / 32)
+                         : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&S.d_full[i])) : "memory");
+        }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         // the weights and bias chunks, already in the staged layout (wt_sw), by
         // one bulk copy completing on wbar's first phase
@@ -421,188 +446,172 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
-    fence_before();
-    __syncthreads();
-    fence_after();
-    const uint32_t tmem = S.tmem_base;
-    const uint32_t ones = tmem + kOnesCol, wt_addr = smem_u32(S.wt);
-    if (warp < 4) {  // the ones chunk, one row per lane of the first four warps
-        uint32_t r32[32] = {0x3f803f80u};
-        tmem_st32(ones + ((32u * warp) << 16), r32);
-        tmem_wait_st();
-    }
-    fence_before();
-    __syncthreads();
-    fence_after();
-    const bool failed0 = __syncthreads_or(!mbar_wait(smem_u32(&S.wbar), 0u)) != 0;  // the weights have landed
-    if (failed0 && t == 0) S.error = kErrTimeout;
     const uint32_t ntiles = (n + 127u) / 128u, stride = gridDim.x * kTcGroups;
     // tiles of group gg: tile k is base + k stride while below ntiles
     auto tiles_of = [&](uint32_t gg) -> uint32_t {
         const uint32_t base = blockIdx.x * kTcGroups + gg;
         return base < ntiles ? (ntiles - base + stride - 1u) / stride : 0u;
     };
+    // the first tile's rows, on their way while the tensor memory is allocated
+    RowIn in = {};
+    if (warp < (uint32_t)kMmaWarp) {
+        const uint32_t r = (blockIdx.x * kTcGroups + g) * 128u + lt;
+        if (r < n) in = load_row<kPaths>(P, rows, r, kPaths ? guide_row_slot(Q, gd, r) : 0u);
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = S.tmem_base;
+    const uint32_t ones = tmem + kOnesCol, wt_addr = smem_u32(S.wt);
 
     if (warp >= (uint32_t)kMmaWarp) {
         const uint32_t mw = warp - (uint32_t)kMmaWarp;
         // ---------------------------------------------------- MMA warp
-        uint32_t left[kTcGroups][kBufs], lay[kTcGroups][kBufs], ph[kTcGroups][kBufs];
+        uint32_t left[kTcGroups], lay[kTcGroups], ph[kTcGroups];
 #pragma unroll
         for (int i = 0; i < kTcGroups; ++i) {
-            const uint32_t k = (failed0 || gv.stall_mma) ? 0u : tiles_of(i);  // a stalled warp issues nothing
-#pragma unroll
-            for (int j = 0; j < kBufs; ++j) {
-                const bool mine = (uint32_t)((i * kBufs + j) % kMmaWarps) == mw;
-                left[i][j] = mine ? kGuideLayers * ((k + (uint32_t)(kBufs - 1 - j)) / kBufs) : 0u;  // layers to issue
-                lay[i][j] = 0u;
-                ph[i][j] = 0u;
-            }
+            const uint32_t k = gv.stall_mma ? 0u : tiles_of(i);  // a stalled warp issues nothing
+            left[i] = (uint32_t)(i % kMmaWarps) == mw ? kGuideLayers * k : 0u;  // layers to issue
+            lay[i] = 0u;
+            ph[i] = 0u;
         }
-        uint32_t last = global_ns();  // when the warp last issued
-        uint32_t idle = 0;
-        for (;;) {
+        uint32_t last = 0u, idle = 0u;  // when the warp fell idle, polls since
+        // the weights have landed, and the ones chunk is written
+        bool ok = gv.stall_mma || (mbar_wait_warp(smem_u32(&S.wbar), 0u) && mbar_wait_warp(smem_u32(&S.obar), 0u));
+        if (!ok && elect_one()) S.error = kErrTimeout;
+        fence_after();
+        while (ok) {
             bool any = false, progressed = false;
 #pragma unroll
             for (int i = 0; i < kTcGroups; ++i) {
-#pragma unroll
-                for (int j = 0; j < kBufs; ++j) {
-                    if (left[i][j] == 0u) continue;
-                    any = true;
-                    const bool ready = __shfl_sync(0xffffffffu, (uint32_t)mbar_test(smem_u32(&S.a_full[i][j]), ph[i][j]), 0) != 0u;
-                    if (!ready) continue;
-                    ph[i][j] ^= 1u;
-                    fence_after();
-                    if (elect_one()) {
-                        const uint32_t acc = tmem + kAccCols * (kBufs * i + j);
-                        issue_layer(lay[i][j], acc, acc + 64u, ones, wt_addr, smem_u32(&S.d_full[i][j]));
-                    }
-                    __syncwarp();
-                    lay[i][j] = lay[i][j] + 1u == (uint32_t)kGuideLayers ? 0u : lay[i][j] + 1u;
-                    --left[i][j];
-                    progressed = true;
+                if (left[i] == 0u) continue;
+                any = true;
+                const bool ready = __shfl_sync(0xffffffffu, (uint32_t)mbar_test(smem_u32(&S.a_full[i]), ph[i]), 0) != 0u;
+                if (!ready) continue;
+                ph[i] ^= 1u;
+                fence_after();
+                if (elect_one()) {
+                    const uint32_t acc = tmem + kAccCols * i;
+                    issue_layer(lay[i], acc, acc + 64u, ones, wt_addr, smem_u32(&S.d_full[i]));
                 }
+                __syncwarp();
+                lay[i] = lay[i] + 1u == (uint32_t)kGuideLayers ? 0u : lay[i] + 1u;
+                --left[i];
+                progressed = true;
             }
             if (!any) break;
             idle = progressed ? 0u : idle + 1u;
-            if (progressed) last = global_ns();
-            if (idle >= kWaitPolls || ((idle & 63u) == 63u && global_ns() - last > kWaitNs)) {
-                if (elect_one()) S.error = kErrTimeout;  // no buffer became ready within the limit
-                break;
+            if ((idle & 63u) == 63u) {
+                const uint32_t now = global_ns();
+                if (idle == 63u) last = now;
+                if (idle >= kWaitPolls || now - last > kWaitNs) {
+                    if (elect_one()) S.error = kErrTimeout;  // no buffer became ready within the limit
+                    break;
+                }
             }
         }
     } else {
         // ---------------------------------------------------- epilogue groups
         const uint32_t lane_off = (32u * (warp & 3u)) << 16;  // this warp's 32 TMEM lanes
-        const uint32_t kt = failed0 ? 0u : tiles_of(g);
+        const uint32_t lane = t & 31u, kt = tiles_of(g);
         const uint32_t base = blockIdx.x * kTcGroups + g;
-        uint32_t pd[kBufs] = {};
+        const uint32_t tm = tmem + kAccCols * g + lane_off;  // this thread's accumulator; its input above
+        const uint32_t af = smem_u32(&S.a_full[g]), df = smem_u32(&S.d_full[g]);
+        uint32_t pd = 0u, w[18];
         bool timed_out = false;
-        // inputs of the next pair, loaded while the current pair runs its layers
-        RowIn in[kBufs] = {};
-#pragma unroll
-        for (int j = 0; j < kBufs; ++j) {
-            const uint32_t r = (base + j * stride) * 128u + lt;
-            if ((uint32_t)j < kt && r < n) in[j] = load_row<kPaths>(P, rows, r, kPaths ? guide_row_slot(Q, gd, r) : 0u);
+        // a warp's rows of the layer's input are in TMEM: one arrival for the 32 of them
+        auto arrive = [&](uint32_t bar) {
+            tmem_wait_st();
+            fence_before();
+            __syncwarp();
+            if (lane == 0u) mbar_arrive(bar);
+        };
+        if (warp < 4) {  // the ones chunk, one row per lane of the first four warps
+            uint32_t r32[32] = {0x3f803f80u};
+            tmem_st32(ones + lane_off, r32);
+            arrive(smem_u32(&S.obar));
         }
-        for (uint32_t k = 0; k < kt; k += kBufs) {
-            const uint32_t nb = min((uint32_t)kBufs, kt - k);
-#pragma unroll
-            for (int j = 0; j < kBufs; ++j) {
-                if ((uint32_t)j >= nb) break;
-                const uint32_t r = (base + (k + j) * stride) * 128u + lt;
-                float x9[9];
-                row_x9<kPaths>(in[j], x9);
-                if (r >= n) x9[0] = x9[1] = x9[2] = x9[3] = x9[4] = x9[5] = x9[6] = x9[7] = x9[8] = 0.0f;
-                encode_store(tmem + kAccCols * (kBufs * g + j) + 64u + lane_off, x9, gv.params);
-                tmem_wait_st();  // this thread's A row is in TMEM before the MMA warp learns of it
-                fence_before();
-                mbar_arrive(smem_u32(&S.a_full[g][j]));
-            }
-            uint32_t next_slot[kBufs];
-#pragma unroll
-            for (int j = 0; j < kBufs; ++j) {
-                const uint32_t r = (base + (k + kBufs + j) * stride) * 128u + lt;
-                next_slot[j] = (kPaths && k + kBufs + j < kt && r < n) ? guide_row_slot(Q, gd, r) : 0u;
-            }
-            for (int l = 0; l < kGuideLayers; ++l) {
-#pragma unroll
-                for (int j = 0; j < kBufs; ++j) {
-                    if ((uint32_t)j >= nb) break;
-                    const uint32_t tile = base + (k + j) * stride, r = tile * 128u + lt;
-                    if (timed_out || !mbar_wait(smem_u32(&S.d_full[g][j]), pd[j])) {  // after one timeout, no more waits
-                        timed_out = true;
-                        S.error = kErrTimeout;
-                    }
-                    pd[j] ^= 1u;
-                    fence_after();
-                    const uint32_t tm = tmem + kAccCols * (kBufs * g + j) + lane_off;
-                    if (l + 1 < kGuideLayers) {
-                        relu_store(tm, tm + 64u);
-                        tmem_wait_st();
-                        fence_before();
-                        mbar_arrive(smem_u32(&S.a_full[g][j]));
-                        continue;
-                    }
-                    uint32_t o[kGuideRowOutputs];
-                    tmem_ld32(tm, o);
-                    tmem_ld8(tm + 32u, o + 32);
-                    if (kPaths) {
-                        tmem_ld1(tm + 40u, o + 40);  // the selection logit only
-                    } else {
-                        tmem_ld8(tm + 40u, o + 40);
-                    }
-                    tmem_wait_ld();
-                    fence_before();
-                    // the staging rows are free once the previous bulk copy has read them
-                    if (lt == 0u) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
-                    if (group_sync_any(g, timed_out)) {
-                        timed_out = true;
-                        break;
-                    }
-                    // the row's result (the 80-byte FP16 mixture record, or the 192
-                    // bytes of raw outputs), then the tile's rows to global memory
-                    // in one bulk copy
-                    constexpr uint32_t kRowBytes = kPaths ? 16u * kGuideMixVecs : 4u * kGuideRowOutputs;
-                    unsigned char* row_out = S.out[g] + kRowBytes * lt;
-                    if (r < n) {
-                        if (kPaths) {
-                            float of[kGuideOutputs];
-#pragma unroll
-                            for (int q = 0; q < kGuideOutputs; ++q) of[q] = __uint_as_float(o[q]);
-                            const float alpha =
-                                gd.learn_frac ? alpha_of(__uint_as_float(o[kGuideSelOutput])) : gd.guide_frac;
-                            row_mixture(of, alpha, reinterpret_cast<uint4*>(row_out));
-                        } else {
-#pragma unroll
-                            for (int q = 0; q < kGuideRowOutputs / 4; ++q)
-                                reinterpret_cast<uint4*>(row_out)[q] = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2],
-                                                                                  o[4 * q + 3]);
-                        }
-                    }
-                    fence_async_smem();
-                    asm volatile("bar.sync %0, %1;\n" ::"r"(g + 1u), "r"((uint32_t)kGroupThreads) : "memory");
-                    if (lt == 0u) {
-                        unsigned char* dst =
-                            kPaths ? reinterpret_cast<unsigned char*>(gd.lobes) : reinterpret_cast<unsigned char*>(out);
-                        asm volatile(
-                            "cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n"
-                            "cp.async.bulk.commit_group;\n" ::"l"(dst + (size_t)kRowBytes * tile * 128u),
-                            "r"(smem_u32(S.out[g])), "r"(kRowBytes * min(128u, n - tile * 128u))
-                            : "memory");
-                    }
+        // the row's encoding into w (zeros past the end: some row of the tile is below n)
+        auto encode = [&](uint32_t r) {
+            float x9[9];
+            row_x9<kPaths>(in, x9);
+            if (r >= n) x9[0] = x9[1] = x9[2] = x9[3] = x9[4] = x9[5] = x9[6] = x9[7] = x9[8] = 0.0f;
+            encode_row(x9, gv.params, w);
+        };
+        if (kt > 0u) {
+            encode(base * 128u + lt);
+            store_input(tm + 64u, w);
+            arrive(af);
+        }
+        // the warp's staging rows and where they go
+        constexpr uint32_t kRowBytes = kPaths ? 16u * kGuideMixVecs : 4u * kGuideRowOutputs;
+        unsigned char* stage = S.out[warp];
+        unsigned char* dst = kPaths ? reinterpret_cast<unsigned char*>(gd.lobes) : reinterpret_cast<unsigned char*>(out);
+        for (uint32_t k = 0; k < kt; ++k) {
+            const uint32_t tile = base + k * stride, r = tile * 128u + lt, rn = r + stride * 128u;
+            const bool more = k + 1u < kt;
+            const uint32_t next_slot = (kPaths && more && rn < n) ? guide_row_slot(Q, gd, rn) : 0u;
+#pragma unroll 1
+            for (int l = 0; l + 1 < kGuideLayers; ++l) {
+                if (l == 1 && more && rn < n)
+                    prefetch_l1(kPaths ? (const void*)&P.ro[next_slot] : (const void*)(rows + 16 * (size_t)rn));
+                if (!mbar_wait_warp(df, pd)) {
+                    timed_out = true;
+                    break;
                 }
-                if (timed_out) break;
-                if (l == 1) {
+                pd ^= 1u;
+                fence_after();
+                relu_store(tm, tm + 64u);
+                arrive(af);
+            }
+            if (!timed_out && more) {  // while the last layer runs
+                if (rn < n) in = load_row<kPaths>(P, rows, rn, next_slot);
+                encode(rn);
+            }
+            if (timed_out || !mbar_wait_warp(df, pd)) {  // after one timeout, no more waits
+                timed_out = true;
+                S.error = kErrTimeout;
+                break;
+            }
+            pd ^= 1u;
+            fence_after();
+            if (more) store_input(tm + 64u, w);
+            uint32_t o[kGuideRowOutputs];
+            tmem_ld32(tm, o);
+            tmem_ld8(tm + 32u, o + 32);
+            if (kPaths) {
+                tmem_ld1(tm + 40u, o + 40);  // the selection logit only
+            } else {
+                tmem_ld8(tm + 40u, o + 40);
+            }
+            tmem_wait_ld();
+            if (more) arrive(af);  // the next tile's first layer may overwrite the accumulator
+            // the staging rows are free once the previous bulk copy has read them
+            if (lane == 0u) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+            __syncwarp();
+            if (r < n) {
+                if (kPaths) {  // the row's 80-byte FP16 mixture record
+                    float of[kGuideOutputs];
 #pragma unroll
-                    for (int j = 0; j < kBufs; ++j) {
-                        const uint32_t r = (base + (k + kBufs + j) * stride) * 128u + lt;
-                        if (k + kBufs + j < kt && r < n) in[j] = load_row<kPaths>(P, rows, r, next_slot[j]);
-                    }
+                    for (int q = 0; q < kGuideOutputs; ++q) of[q] = __uint_as_float(o[q]);
+                    const float alpha = gd.learn_frac ? alpha_of(__uint_as_float(o[kGuideSelOutput])) : gd.guide_frac;
+                    row_mixture(of, alpha, reinterpret_cast<uint4*>(stage + kRowBytes * lane));
+                } else {
+                    stage_row(stage + kRowBytes * lane, lane, o);
                 }
             }
-            if (timed_out) break;
+            fence_async_smem();
+            __syncwarp();
+            const uint32_t first = r - lane;  // the warp's first row
+            if (lane == 0u && first < n) {
+                asm volatile(
+                    "cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n"
+                    "cp.async.bulk.commit_group;\n" ::"l"(dst + (size_t)kRowBytes * first),
+                    "r"(smem_u32(stage)), "r"(kRowBytes * min(32u, n - first))
+                    : "memory");
+            }
         }
-        if (lt == 0u) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");  // this group's stores are done
+        if (lane == 0u) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");  // this warp's stores are done
     }
     fence_before();
     __syncthreads();
