@@ -165,6 +165,11 @@ constexpr uint32_t kPersistentTraceMinPaths = 3u << 17;
 // the copies of some overlap the traversal of another (measured end to end
 // on the closest-hit workload: 2 slots 2500 Mrays/s, 3: 2647, 4: 2705-2728,
 // 6: 2682, 8: 2627; 8 slots of 2^19 rays: 2749)
+// rgr_trace_closest_device sorts the rays, where asked to, from this many on: the
+// sort's launches cost 21 us, and a call of fewer is bound by its longest rays.  Random rays
+// in 1.31M triangles, sorted / unsorted: 1 K 104 / 60 us, 20 K 160 / 123, 60 K 241 / 222,
+// 400 K 332 / 309, 1M 467 / 464, 4M 1178 / 1241 (from 2^16 to 1M the caller's choice stands).
+constexpr uint64_t kReorderMinRays = 1ull << 16;
 constexpr int kZeroCopyRefill = 32;  // refill threshold of the zero-copy closest-hit launch
 constexpr int kTraceSlots = 4;
 
@@ -218,7 +223,7 @@ struct rgr_context {
     // refill 12: the mixed 1080p render at 2^24 paths runs 1047.7 / 1066.6 / 1067.6 / 1066.5 /
     // 1059.5 Mpaths/s with a warp refilled at 24 / 8 / 12 / 16 / 20 idle lanes
     // search 8: 1114.8 Mpaths/s against 1032.8 with every lane waiting for the last
-    TraceShape render_trace{true, 12, 8, 0, nullptr};
+    TraceShape render_trace{true, 12, 8, 0, nullptr, nullptr};
     int render_trace_mode = -1;  // 1 persistent, 0 fused, -1 by the pool's size at render begin
     uint32_t trace_stage = 0;  // top BVH nodes staged in shared memory per CTA
     int trace_reorder = 0;     // rgr_trace_closest_device sorts the rays first
@@ -517,7 +522,9 @@ struct rgr_context {
         add(&in, sizeof(in));
         add(&rp, sizeof(rp));
         add(&shade_grid, sizeof(shade_grid));
-        add(&render_trace, sizeof(render_trace));
+        add(&render_trace.persistent, sizeof(render_trace.persistent));
+        for (const int v : {render_trace.refill, render_trace.search, render_trace.grid}) add(&v, sizeof(v));
+        if (render_trace.one) add(render_trace.one, sizeof(SceneView));  // the cast's kernel argument
         add(&graph_steps, sizeof(graph_steps));
         add(&guided, sizeof(guided));
         add(&single_render, sizeof(single_render));  // batches add the completion stamps
@@ -643,6 +650,7 @@ int rgr_render_begin(rgr_context* c, const rgr_camera* cam, const rgr_render_con
     // no completion counter: nothing reads a single render's completion time, and
     // the counter cost every warp of the logic kernel an atomic on one address
     RequestD q = request_d(c->scene.sv, *cam, k, c->accum.as<double>(), 0ull, limit ? limit : ~0ull, nullptr);
+    c->render_trace.one = &c->scene.sv;
     if ((r = c->setup_guiding()) != RGR_OK) return r;
     if (c->guided) q.flags |= kFlagFixBacksideEnvPdf | kFlagTwoSidedLambertian;
     if ((r = c->start(&q, 1, limit, k.seed_offset)) != RGR_OK) return r;
@@ -872,7 +880,7 @@ int rgr_trace_closest_device(rgr_context* c, const rgr_ray_soa* rays, uint64_t n
     int r = c->err.alloc(16);
     if (r != RGR_OK) return r;
     if ((r = c->tcounter.alloc(8)) != RGR_OK) return r;
-    if (c->trace_reorder && n < (1ull << 32)) {
+    if (c->trace_reorder && n >= kReorderMinRays && n < (1ull << 32)) {
         if ((r = c->tbins.alloc(2 * sizeof(uint32_t) * kRayBins)) != RGR_OK) return r;
         if ((r = c->tpacked.alloc(32 * (size_t)n)) != RGR_OK) return r;
         if ((r = c->trank.alloc(4 * (size_t)n)) != RGR_OK) return r;
@@ -1248,6 +1256,7 @@ int rgr_batch_run(rgr_batch* b, int32_t order_policy, int32_t steps_per_launch, 
         begin += q.samples;
     }
     c->npix = 0;
+    c->render_trace.one = nullptr;  // scenes by request
     r = c->start(table.data(), n, begin, b->reqs[order[0]]->cfg.seed_offset);
     if (r != RGR_OK) return r;
     // a replayed graph: the bounces of a group before the one whose outcome is looked at

@@ -71,9 +71,10 @@ RGR_DEV void ld_keep8(const float4* ptr, uint64_t pol, float4& a, float4& b) {
 // slabs_with_hit (extension_ray_cast_stackless.cl:35-50).  fminf/fmaxf have
 // the reference's NaN behaviour; their results only feed comparisons, so the
 // sign of a zero result cannot change a decision.  kNanCheck = false is the
-// same function for rays whose products (lo - ro) * inv cannot be NaN (see
-// ray_is_nan_free); the reference's select(t, -t', isnan(t)) is then the
-// identity.
+// same function for rays whose products (lo - ro) * inv cannot be NaN and whose far
+// clip is a number >= 0 (see ray_is_nan_free); the reference's
+// select(t, -t', isnan(t)) is then the identity, and its three comparisons are
+// one: max(0, rmin) <= min(rmax, farclip).
 template <bool kNanCheck>
 RGR_DEV bool slab(float lox, float loy, float loz, float hix, float hiy, float hiz, f3 ro, f3 inv, float farclip,
                   float& h0, float& h1) {
@@ -91,6 +92,7 @@ RGR_DEV bool slab(float lox, float loy, float loz, float hix, float hiy, float h
     float rmax = fminf(fminf(fmaxf(t0x, t1x), fmaxf(t0y, t1y)), fmaxf(t0z, t1z));
     h0 = fmaxf(0.0f, rmin);
     h1 = fminf(rmax, farclip);
+    if (!kNanCheck) return h0 <= h1;
     return rmin <= rmax && 0.0f <= rmax && rmin <= farclip;
 }
 
@@ -98,9 +100,9 @@ RGR_DEV bool slab(float lox, float loy, float loz, float hix, float hiy, float h
 // component is finite and non-zero, and the scene box is small (checked on
 // the host): the difference is finite and the product of two finite non-zero
 // numbers is a number or an infinity.
-RGR_DEV bool ray_is_nan_free(f3 ro, f3 inv, bool scene_small) {
+RGR_DEV bool ray_is_nan_free(f3 ro, f3 inv, float tmax, bool scene_small) {
     const float kBig = 1.0e30f;
-    return scene_small && fabsf(ro.x) <= kBig && fabsf(ro.y) <= kBig && fabsf(ro.z) <= kBig &&
+    return scene_small && tmax >= 0.0f && fabsf(ro.x) <= kBig && fabsf(ro.y) <= kBig && fabsf(ro.z) <= kBig &&
            is_finite_nonzero(inv.x) && is_finite_nonzero(inv.y) && is_finite_nonzero(inv.z);
 }
 
@@ -186,7 +188,7 @@ RGR_DEV void trace_begin(const SceneView& sc, TraceState& s, f3 ro, f3 rd, float
     s.prim = -1;
     s.link = sc.num_prims == 0 ? kDone : sc.root_link;
     s.sp = 0;
-    s.nan_free = ray_is_nan_free(ro, s.inv, sc.small_coords != 0);
+    s.nan_free = ray_is_nan_free(ro, s.inv, tmax, sc.small_coords != 0);
 }
 
 // the newest pending far link, or kDone; the next one is fetched from the

@@ -996,12 +996,16 @@ RGR_DEV float guide_write(const GuideRenderD& gd, uint32_t slot, const GuideOffe
 // goes next and writes it as the slot's queue id: what ends a path whatever its ray
 // meets (logic_ends) is found as the ray is taken, from the sector beside the
 // ray's in the same line, and kept in the slot word's top bit (slots are below 2^28).
+// kOne: a render of one request; its scene `one` is a kernel argument (constant bank).
+// Read through the request table, a lane's node pointer was loaded again at every
+// step (mixed 1080p render at 2^22 paths 24.35 ms, 23.85 with the argument).
 #ifndef RGR_TRACE_PATHS_MIN_BLOCKS  // 4 / 5 / 6 (64 / 48 / 40 registers, 6 spilling): 1428 / 1473 / 1442 Mpaths/s
 #define RGR_TRACE_PATHS_MIN_BLOCKS 5
 #endif
-template <bool kInner>
-__global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS) k_trace_paths(PathsView P, QueueView Q, RenderParams rp,
-                                                         unsigned long long* next, int refill, int search) {
+template <bool kInner, bool kOne>
+__global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS)
+    k_trace_paths(PathsView P, QueueView Q, RenderParams rp, unsigned long long* next, int refill, int search,
+                  SceneView one) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
@@ -1014,7 +1018,7 @@ __global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS) k_trace_paths
     __shared__ uint32_t s_stack[kSmemStack > 0 ? kSmemStack * kStackThreads : 1];
     TraceState s;
     s.sstk = s_stack + threadIdx.x;
-    const SceneView* scp = &rp.reqs[0].sc;  // a valid scene on idle lanes too
+    const SceneView* scp = kOne ? &one : &rp.reqs[0].sc;  // a valid scene on idle lanes too
     uint32_t slot = ~0u;  // ~0: idle
     constexpr uint32_t kEnds = 0x80000000u;
     bool vol = false;  // kInner: the path is in a volume that ends its ray
@@ -1039,8 +1043,8 @@ __global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS) k_trace_paths
                     // the shading kernel): material-queue items skip the check
                     if (k != 0 || P.qid[r] != kQueueIdle) {
                         slot = r;
-                        const RequestD* rq = &rp.reqs[P.req[r]];
-                        scp = &rq->sc;
+                        const RequestD* rq = kOne ? rp.reqs : rp.reqs + P.req[r];
+                        if (!kOne) scp = &rq->sc;
                         float4 ro4, rd4;
                         ld_sector<0>(P, r, ro4, rd4);
                         if (kInner) {
@@ -1049,7 +1053,7 @@ __global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS) k_trace_paths
                             if (logic_ends(*rq, P, r, xyz(T4), depth_of(__float_as_uint(L4.w)))) slot |= kEnds;
                             vol = __float_as_int(rd4.w) >= 0;
                         }
-                        trace_begin(*scp, s, xyz(ro4), xyz(rd4), ro4.w);
+                        trace_begin(kOne ? one : *scp, s, xyz(ro4), xyz(rd4), ro4.w);
                     }
                 }
             }
@@ -1058,8 +1062,8 @@ __global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS) k_trace_paths
             if (exhausted) break;
             continue;
         }
-        trace_warp_round<false, false, kSmemStack>(*scp, s, slot != ~0u && s.link != kDone, search, nullptr, err,
-                                                   pol);
+        trace_warp_round<false, false, kSmemStack>(kOne ? one : *scp, s, slot != ~0u && s.link != kDone, search,
+                                                   nullptr, err, pol);
         if (slot != ~0u && s.link == kDone) {
             const uint32_t id = kInner ? slot & ~kEnds : slot;
             if (kInner) {
@@ -1602,12 +1606,22 @@ void launch_shade(const PathsView& p, const QueueView& q, const RenderParams& rp
     else
         k_shade<<<grid, 256, 0, st>>>(p, q, rp);
 }
+template <bool kInner>
+static void cast_paths(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
+                       cudaStream_t st) {
+    if (ts.one && rp.nreq == 1)
+        k_trace_paths<kInner, true><<<ts.grid, kStackThreads, 0, st>>>(p, q, rp, ts.counter, ts.refill, ts.search, *ts.one);
+    else
+        k_trace_paths<kInner, false>
+            <<<ts.grid, kStackThreads, 0, st>>>(p, q, rp, ts.counter, ts.refill, ts.search, SceneView{});
+}
+
 cudaError_t launch_trace_paths(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
                                cudaStream_t st) {
     if (!ts.persistent) return cudaSuccess;
     const cudaError_t e = cudaMemsetAsync(ts.counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
-    k_trace_paths<false><<<ts.grid, kStackThreads, 0, st>>>(p, q, rp, ts.counter, ts.refill, ts.search);
+    cast_paths<false>(p, q, rp, ts, st);
     return cudaSuccess;
 }
 
@@ -1639,7 +1653,7 @@ cudaError_t launch_inner_cast(const PathsView& p, const QueueView& q, const Rend
                               cudaStream_t st) {
     const cudaError_t e = cudaMemsetAsync(ts.counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
-    k_trace_paths<true><<<ts.grid, kStackThreads, 0, st>>>(p, q, rp, ts.counter, ts.refill, ts.search);
+    cast_paths<true>(p, q, rp, ts, st);
     return cudaSuccess;
 }
 
@@ -1651,7 +1665,7 @@ void launch_inner(const PathsView& p, const QueueView& q, const InnerView& in, c
     QueueView u = q;
     u.counts = in.words;
     k_shade_inner<<<shade_grid, 256, 0, st>>>(p, u, rp);
-    k_trace_paths<true><<<ts.grid, kStackThreads, 0, st>>>(p, u, rp, ts.counter, ts.refill, ts.search);
+    cast_paths<true>(p, u, rp, ts, st);
 }
 
 void launch_stamp_done(const RenderParams& rp, cudaStream_t st) {
@@ -1660,7 +1674,7 @@ void launch_stamp_done(const RenderParams& rp, cudaStream_t st) {
 
 int trace_paths_max_blocks_per_sm() {
     int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_paths<false>, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_paths<true, false>, 256, 0);
     return nb;
 }
 void launch_readback(int fmt, const double* accum, uint32_t npix, void* out, cudaStream_t st) {

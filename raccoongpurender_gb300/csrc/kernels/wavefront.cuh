@@ -257,13 +257,14 @@ void launch_guide_select(const PathsView& p, const QueueView& q, const GuideRend
 // `grid` CTAs, `counter` a device word it may use; launch_trace_paths, between
 // the shading kernel and the queue resets), then the logic kernel; otherwise
 // one kernel traces and runs the logic per slot (launch_trace_paths does
-// nothing).
+// nothing).  `one`: the scene of a render of a single request, or null.
 struct TraceShape {
     bool persistent;
     int refill;
     int search;
     int grid;
     unsigned long long* counter;
+    const SceneView* one = nullptr;
 };
 // returns the status of its counter reset (launch errors: cudaGetLastError)
 cudaError_t launch_trace_paths(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
