@@ -7,9 +7,10 @@
 //
 // Persistent warps: each warp keeps 32 rays in flight and, between traversal
 // rounds, hands finished lanes new rays from a global counter (one atomic per
-// refill per warp); a call of few rays is spread over the warps instead.  Within a round the lanes take node steps while at least
+// refill per warp).  Within a round the lanes take node steps while at least
 // `search` of them still search for their next leaf; the others wait at
-// theirs.  Rays are read and results written with streaming (evict-first)
+// theirs.  A warp left with a few rays, and a call of few rays, which is spread over
+// the warps instead, go on lane by lane (kTailLanes, spread).  Rays are read and results written with streaming (evict-first)
 // cache hints; the tree is read with an L2 evict-last policy.
 // Each ray's traversal is unchanged, so results do not depend on the
 // schedule.
@@ -62,7 +63,8 @@ RGR_DEV void ld_record(const float4* ptr, float4& a, float4& b) {
         : "l"(ptr));
 }
 
-template <bool kCount, bool kStaged, bool kPacked = false>
+// kFew: each lane takes one ray of its warp's share, without the rounds
+template <bool kCount, bool kStaged, bool kPacked, bool kFew>
 __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneView sc, RayBatch b) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -75,7 +77,7 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
         for (uint32_t i = threadIdx.x; i < 4u * stn.n; i += blockDim.x) s_nodes[i] = __ldg(sc.nodes + i);
         __syncthreads();
     }
-    __shared__ uint32_t s_stack[kSmemStack > 0 ? kSmemStack * kStackThreads : 1];
+    __shared__ uint32_t s_stack[(kSmemStack + 1) * kStackThreads];  // the last row: see touch
     TraceState s;
     s.sstk = s_stack + threadIdx.x;
     TraceCounters cnt;
@@ -96,13 +98,29 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
         }
         if (kCount) cnt = TraceCounters();
     };
-    if (b.share) {  // few rays: the warp's share of them, and no more
+    auto put = [&]() {
+        const int32_t prim = hit_id(s.prim);
+        __stcs(b.prim + ray, prim);
+        __stcs(b.t + ray, s.tmin);
+        if (b.ng) {
+            f3 n = prim >= 0 ? hit_normal(sc, prim, s.ro, s.rd, s.tmin) : mk(0.0f, 0.0f, 0.0f);
+            b.ng[3 * ray + 0] = n.x;
+            b.ng[3 * ray + 1] = n.y;
+            b.ng[3 * ray + 2] = n.z;
+        }
+        if (kCount) {
+            b.nodes[ray] = cnt.nodes;
+            b.prims[ray] = cnt.prims;
+        }
+        ray = ~0ull;
+    };
+    uint32_t err = 0;
+    if (kFew) {
         const uint64_t r = ((uint64_t)blockIdx.x * (kStackThreads / 32) + (threadIdx.x >> 5)) * b.share + lane;
         if ((uint32_t)lane < b.share && r < b.n) take(r);
     }
-    bool exhausted = b.share != 0u;
-    uint32_t err = 0;
-    for (;;) {
+    bool exhausted = false;
+    while (!kFew) {
         const unsigned idle = __ballot_sync(full, ray == ~0ull);
         if (!exhausted && (int)__popc(idle) >= b.refill) {
             const uint32_t need = __popc(idle);
@@ -115,28 +133,17 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
                 if (r < b.n) take(r);
             }
         }
-        if (__ballot_sync(full, ray != ~0ull) == 0u) {
-            if (exhausted) break;
-            continue;
-        }
+        const unsigned held = __ballot_sync(full, ray != ~0ull);
+        if (exhausted && __popc(held) <= kTailLanes) break;
+        if (held == 0u) continue;
         trace_warp_round<kCount, kStaged, kSmemStack>(sc, s, ray != ~0ull && s.link != kDone, b.search, &cnt, err, pol,
                                                       stn);
-        if (ray != ~0ull && s.link == kDone) {
-            const int32_t prim = hit_id(s.prim);
-            __stcs(b.prim + ray, prim);
-            __stcs(b.t + ray, s.tmin);
-            if (b.ng) {
-                f3 n = prim >= 0 ? hit_normal(sc, prim, s.ro, s.rd, s.tmin) : mk(0.0f, 0.0f, 0.0f);
-                b.ng[3 * ray + 0] = n.x;
-                b.ng[3 * ray + 1] = n.y;
-                b.ng[3 * ray + 2] = n.z;
-            }
-            if (kCount) {
-                b.nodes[ray] = cnt.nodes;
-                b.prims[ray] = cnt.prims;
-            }
-            ray = ~0ull;
-        }
+        if (ray != ~0ull && s.link == kDone) put();
+    }
+    if (ray != ~0ull) {
+        while (s.link != kDone) trace_round<kCount, kStaged, kSmemStack, true>(sc, s, &cnt, err, pol, stn);
+        put();
+        touch_done();
     }
     if (err) atomicOr(b.err, err);
 }
@@ -325,9 +332,11 @@ __global__ void __launch_bounds__(256) k_ray_scatter(RaySoA r, uint64_t n, RayKe
 namespace {
 // A call of few rays (at most kFewRays a warp of the grid) is bound by the latency of its
 // longest ray's steps, so its rays are spread over the warps, ceil(n / warps) each,
-// without the counter and its reset: 1000 / 6000 / 20000 random rays in a 20 K-triangle
-// scene, calls in a row, 57.5 / 69.2 / 70.7 us in whole warps, 35.1 / 43.3 / 60.0 spread.
-// From there on whole warps win (60,000: 79 us, 91 spread ten a warp).  Returns the rays a warp, 0 for the counter, which it resets; *blocks: at most `grid`.
+// without the counter and its reset, and go on lane by lane: 1000 / 6000 / 20000 random
+// rays in a 20 K-triangle scene, calls in a row, 57.5 / 69.2 / 70.7 us in whole warps,
+// 35.1 / 43.3 / 60.0 spread, 24.9 / 34.9 / 53.7 with the next links brought into L1 (touch).
+// From there on whole warps win (60,000: 79 us, 91 spread ten a warp).  Returns the rays
+// a warp, 0 for the counter, which it resets; *blocks: at most `grid`.
 constexpr uint64_t kFewRays = 4;
 uint32_t spread(uint64_t n, int grid, int* blocks, unsigned long long* counter, cudaStream_t st) {
     const uint64_t per = kStackThreads / 32, warps = (uint64_t)grid * per;
@@ -351,10 +360,12 @@ void launch_trace_rays(const SceneView& sc, const float* ox, const float* oy, co
     const uint32_t share = spread(n, grid, &blocks, counter, st);
     RayBatch b{ox, oy, oz, dx, dy, dz, tmax, nullptr, n, prim, t, ng, nullptr, nullptr, err, counter, share, refill,
                search, stage};
-    if (stage > 0)
-        k_trace_rays<false, true><<<blocks, kStackThreads, 64 * (size_t)stage, st>>>(sc, b);
+    if (share)
+        k_trace_rays<false, false, false, true><<<blocks, kStackThreads, 0, st>>>(sc, b);
+    else if (stage > 0)
+        k_trace_rays<false, true, false, false><<<blocks, kStackThreads, 64 * (size_t)stage, st>>>(sc, b);
     else
-        k_trace_rays<false, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
+        k_trace_rays<false, false, false, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
 }
 
 void launch_trace_rays_counts(const SceneView& sc, const float* ox, const float* oy, const float* oz, const float* dx,
@@ -365,7 +376,10 @@ void launch_trace_rays_counts(const SceneView& sc, const float* ox, const float*
     int blocks;
     const uint32_t share = spread(n, grid, &blocks, counter, st);
     RayBatch b{ox, oy, oz, dx, dy, dz, tmax, nullptr, n, prim, t, nullptr, nodes, prims, err, counter, share, 16, 1, 0u};
-    k_trace_rays<true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
+    if (share)
+        k_trace_rays<true, false, false, true><<<blocks, kStackThreads, 0, st>>>(sc, b);
+    else
+        k_trace_rays<true, false, false, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
 }
 
 // the per-triangle table of a scene (its tri_normals still null): the normal,
@@ -406,17 +420,20 @@ void launch_trace_packed(const SceneView& sc, const float4* packed, uint64_t n, 
     const uint32_t share = spread(n, grid, &blocks, counter, st);
     RayBatch b{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, packed, n, prim, t, ng, nullptr,
                nullptr, err, counter, share, refill, search, 0u};
-    k_trace_rays<false, false, true><<<blocks, kStackThreads, 0, st>>>(sc, b);
+    if (share)
+        k_trace_rays<false, false, true, true><<<blocks, kStackThreads, 0, st>>>(sc, b);
+    else
+        k_trace_rays<false, false, true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
 }
 
 int trace_rays_max_blocks_per_sm(uint32_t stage) {
     int nb = 0;
     if (stage > 0) {
-        cudaFuncSetAttribute(k_trace_rays<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(k_trace_rays<false, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(64 * kMaxStagedNodes));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_rays<false, true>, 256, 64 * (size_t)stage);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_rays<false, true, false, false>, 256, 64 * (size_t)stage);
     } else {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_rays<false, false>, 256, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_rays<false, false, false, false>, 256, 0);
     }
     return nb;
 }

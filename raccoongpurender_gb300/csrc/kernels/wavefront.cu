@@ -1015,7 +1015,7 @@ __global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS)
 #pragma unroll
     for (int k = 0; k < kNumQueues; ++k) off[k + 1] = off[k] + Q.counts[k];
     const uint32_t total = off[kNumQueues];
-    __shared__ uint32_t s_stack[kSmemStack > 0 ? kSmemStack * kStackThreads : 1];
+    __shared__ uint32_t s_stack[(kSmemStack + 1) * kStackThreads];  // the last row: see touch
     TraceState s;
     s.sstk = s_stack + threadIdx.x;
     const SceneView* scp = kOne ? &one : &rp.reqs[0].sc;  // a valid scene on idle lanes too
@@ -1024,6 +1024,22 @@ __global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS)
     bool vol = false;  // kInner: the path is in a volume that ends its ray
     bool exhausted = false;
     uint32_t err = 0;
+    auto put = [&]() {
+        const uint32_t id = kInner ? slot & ~kEnds : slot;
+        if (kInner) {
+            const int q = s.prim >= 0 ? hit_type(s.prim) : (vol ? (int)kMatVolumeInside : 0);
+            P.qid[id] = (uint8_t)((slot & kEnds) ? 0 : q);
+        }
+        if (s.prim >= 0) {
+            // the ray's whole sector in one store (a partial store to a line that is
+            // not in L2 costs a read of the sector from DRAM); the hit primitive
+            // rides where the volume-hit id goes (none after a surface hit: every
+            // reader takes a negative id as none), and the logic kernel, which
+            // writes the (ng, rng) sector anyway, computes the normal
+            st_sector<0>(P, id, f4(s.ro, s.tmin), f4(s.rd, __int_as_float(-2 - hit_id(s.prim))));
+        }
+        slot = ~0u;
+    };
     for (;;) {
         const unsigned idle = __ballot_sync(full, slot == ~0u);
         if (!exhausted && (int)__popc(idle) >= refill) {
@@ -1058,28 +1074,17 @@ __global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS)
                 }
             }
         }
-        if (__ballot_sync(full, slot != ~0u) == 0u) {
-            if (exhausted) break;
-            continue;
-        }
+        const unsigned held = __ballot_sync(full, slot != ~0u);
+        if (exhausted && __popc(held) <= kTailLanes) break;
+        if (held == 0u) continue;
         trace_warp_round<false, false, kSmemStack>(kOne ? one : *scp, s, slot != ~0u && s.link != kDone, search,
                                                    nullptr, err, pol);
-        if (slot != ~0u && s.link == kDone) {
-            const uint32_t id = kInner ? slot & ~kEnds : slot;
-            if (kInner) {
-                const int q = s.prim >= 0 ? hit_type(s.prim) : (vol ? (int)kMatVolumeInside : 0);
-                P.qid[id] = (uint8_t)((slot & kEnds) ? 0 : q);
-            }
-            if (s.prim >= 0) {
-                // the ray's whole sector in one store (a partial store to a line that is
-                // not in L2 costs a read of the sector from DRAM); the hit primitive
-                // rides where the volume-hit id goes (none after a surface hit: every
-                // reader takes a negative id as none), and the logic kernel, which
-                // writes the (ng, rng) sector anyway, computes the normal
-                st_sector<0>(P, id, f4(s.ro, s.tmin), f4(s.rd, __int_as_float(-2 - hit_id(s.prim))));
-            }
-            slot = ~0u;
-        }
+        if (slot != ~0u && s.link == kDone) put();
+    }
+    if (slot != ~0u) {  // the last few paths of the warp, lane by lane
+        while (s.link != kDone) trace_round<false, false, kSmemStack, true>(kOne ? one : *scp, s, nullptr, err, pol);
+        put();
+        touch_done();
     }
     if (err) atomicOr(rp.err, err);
 }

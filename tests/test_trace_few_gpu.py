@@ -4,7 +4,7 @@ far clip is not a positive number.  All against the oracle, bit for bit."""
 import numpy as np
 import pytest
 
-from raccoongpurender_gb300 import scenes
+from raccoongpurender_gb300 import materials, scenes
 from tests.conftest import bits
 from tests.helpers import build
 
@@ -63,3 +63,32 @@ def test_far_clip(rg, po, tmax, n):
     prim, t, _ = _hits(lane, rays)
     assert (prim == oprim).all()
     assert ((bits(t) == bits(ot)) | (np.isnan(t) & np.isnan(ot))).all()
+
+
+@pytest.mark.parametrize("leaf", [1, 4, 8])
+@pytest.mark.parametrize("n", [5, 4 * WARPS, 5 * WARPS])
+def test_deep_tree(rg, po, n, leaf):
+    """Triangles at distances that double from one to the next, whose boxes the rays pass
+    from the smallest on: more pending links than the stack's entries in shared memory, in
+    the lanes that go alone (few rays; the last ones of a warp) and in whole warps."""
+    k = np.repeat(np.exp2(np.arange(-20, 20, dtype=np.float64)), 3)
+    size = k * 0.3
+    p = np.stack([k, np.zeros_like(k), np.zeros_like(k)], 1)
+    p[0::3, 1:] = np.stack([-size[0::3], -size[0::3]], 1)
+    p[1::3, 1:] = np.stack([size[1::3], -size[1::3]], 1)
+    p[2::3, 1:] = np.stack([-size[2::3], size[2::3]], 1)
+    tris = np.arange(len(p), dtype=np.uint32).reshape(-1, 3)
+    mesh = scenes.Mesh(p.astype(np.float32), tris, [materials.lambertian()] * len(tris))
+    sm, osc = build(mesh, leaf=leaf)
+    lane = rg.WavefrontLane(0, 1024)
+    lane.setup(sm)
+    rays = scenes.random_rays(n, (-1e-6, -1e-6, -1e-6), (1e-6, 1e-6, 1e-6), seed=n)
+    rng = np.random.default_rng(n)
+    yz = rng.uniform(-0.2, 0.31, (n, 2))  # with y + z > 0 past every triangle
+    d = np.concatenate([np.ones((n, 1)), yz], 1)
+    rays.d[:] = (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+    rays.d[::7] *= -1.0
+    oprim, ot, _ = osc.trace(rays.packed8(), threads=16)
+    assert n < 100 or 0.1 < (oprim >= 0).mean() < 0.9
+    prim, t, _ = _hits(lane, rays)
+    assert (prim == oprim).all() and (bits(t) == bits(ot)).all()
