@@ -316,7 +316,7 @@ struct rgr_context {
         RGR_CUDA(launch_trace_paths(pv, qv, rp, render_trace, st));
         RGR_CUDA(cudaMemsetAsync(qv.counts + 1, 0, sizeof(uint32_t) * (kNumQueues - 1), st));
         RGR_CUDA(cudaMemsetAsync(qv.tile_new, 0, sizeof(uint32_t) * ntiles, st));
-        launch_trace_logic(pv, qv, rp, render_trace, st);
+        launch_trace_logic(pv, qv, rp, render_trace, num_sms, st);
         if (!single_render) launch_stamp_done(rp, st);  // batches: per-request completion times
         RGR_CUDA(cudaGetLastError());
         if (guided && train_now) return guide->train_launches(st);
@@ -458,7 +458,7 @@ struct rgr_context {
     // the logic of the run's last bounce
     int run_last() {
         RGR_CUDA(cudaMemsetAsync(qv.tile_new, 0, sizeof(uint32_t) * ntiles, stream));
-        launch_trace_logic(pv, qv, rp, render_trace, stream);
+        launch_trace_logic(pv, qv, rp, render_trace, num_sms, stream);
         if (!single_render) launch_stamp_done(rp, stream);  // batches: per-request completion times
         RGR_CUDA(cudaGetLastError());
         return RGR_OK;

@@ -197,7 +197,7 @@ extern "C" int rgr_render_noalloc(rgr_context* c, const rgr_camera* cam, const r
             !ok(cudaMemsetAsync(q.counts + 1, 0, sizeof(uint32_t) * (kNumQueues - 1), st), "cudaMemsetAsync") ||
             !ok(cudaMemsetAsync(q.tile_new, 0, sizeof(uint32_t) * ntiles, st), "cudaMemsetAsync"))
             return RGR_E_CUDA;
-        launch_trace_logic(p, q, rp, ts, st);
+        launch_trace_logic(p, q, rp, ts, sms, st);
         // a failed launch stops the call at the bounce it happened in
         if (!ok(cudaGetLastError(), "kernel launch")) return RGR_E_CUDA;
     }

@@ -377,18 +377,6 @@ RGR_DEV void trace_warp_round(const SceneView& sc, TraceState& s, bool active, i
     if (active) s.link = link;
 }
 
-// Closest hit of one ray.  tmin in: the ray's far clip (ExtensionResult.tmin);
-// out: the hit distance (unchanged on a miss).  Returns the primitive id or -1.
-template <bool kCount>
-RGR_DEV int32_t trace_closest(const SceneView& sc, f3 ro, f3 rd, float& tmin, TraceCounters* cnt, uint32_t& err) {
-    TraceState s;
-    trace_begin(sc, s, ro, rd, tmin);
-    const uint64_t pol = l2_evict_last_policy();
-    while (s.link != kDone) trace_round<kCount>(sc, s, cnt, err, pol);
-    tmin = s.tmin;
-    return hit_id(s.prim);
-}
-
 // geometric normal of a hit (extension_ray_cast_stackless.cl:224-239), from
 // the original vertices so the subtractions match the reference exactly
 RGR_DEV f3 triangle_normal(const SceneView& sc, int32_t prim) {

@@ -1145,32 +1145,23 @@ RGR_DEV void count_done(const RequestD& rq, int req, bool ended, unsigned active
 // The logic of one live slot (logic.cl:27-190) after its extension ray;
 // returns the queue of its next step (0: a new path; the caller counts and
 // appends).  kPreTraced: k_trace_paths has cast the extension rays of this
-// bounce; otherwise the thread traces first.
+// bounce and written the hit; otherwise it is the primitive `prim` (-1: none) at t.
 template <bool kGuided, bool kPreTraced>
 RGR_DEV int logic_slot(const PathsView& P, const QueueView& Q, const RenderParams& rp, uint32_t slot,
-                       unsigned active, GuideOffer& go) {
+                       unsigned active, GuideOffer& go, int32_t prim = -1, float t = 0.0f) {
     const int req = P.req[slot];
     const RequestD& rq = rp.reqs[req];
     const SceneView& sc = rq.sc;
     float4 ro4, rd4, ng4, rng4, T4, L4;
     ld_sector<0>(P, slot, ro4, rd4);
-    if (kPreTraced) {  // the trace kernel wrote the hit; else loaded after the traversal
-        ld_sector<1>(P, slot, T4, L4);
-        ld_sector<2>(P, slot, ng4, rng4);
-    }
+    ld_sector<1>(P, slot, T4, L4);
+    ld_sector<2>(P, slot, ng4, rng4);
     f3 rd = xyz(rd4);
     int32_t hv = __float_as_int(rd4.w);
-    uint32_t err = 0;
-    if (!kPreTraced) {
-        // extension_ray_cast (extension_ray_cast_stackless.cl:202-246)
-        f3 ro = xyz(ro4);
-        const int32_t prim = trace_closest<false>(sc, ro, rd, ro4.w, nullptr, err);
-        ld_sector<1>(P, slot, T4, L4);
-        ld_sector<2>(P, slot, ng4, rng4);
-        if (prim >= 0) {
-            hv = -2 - prim;
-            st_sector<0>(P, slot, ro4, f4(rd, __int_as_float(-1)));
-        }
+    if (!kPreTraced && prim >= 0) {
+        ro4.w = t;
+        hv = -2 - prim;
+        st_sector<0>(P, slot, ro4, f4(rd, __int_as_float(-1)));
     }
     int32_t hs = __float_as_int(ng4.w);
     int mtype = -1;  // the hit triangle's material type, where the triangle table gave it
@@ -1200,24 +1191,19 @@ RGR_DEV int logic_slot(const PathsView& P, const QueueView& Q, const RenderParam
         q = kMatVolumeInside;
     }
     P.qid[slot] = (uint8_t)q;
-    if (err) atomicOr(rp.err, err);
     count_done(rq, req, newPath, active);
     return q;
 }
 
-// The logic kernel, one thread per slot.  Material-queue appends are gathered
+// The logic of a block's slots, all of tile `tile`, one a thread (`live` where it has
+// one); logic(active, go) runs a live slot's.  Material-queue appends are gathered
 // per block (shared-memory counts, then one global atomic per queue), and so
 // is the ray count: with one atomic per warp all warps of the launch queued on
 // the same few counters.
 constexpr int kLogicThreads = 256;
-template <bool kGuided, bool kPreTraced>
-// latency-bound: 6 resident blocks per SM for the logic alone (40 registers; the
-// render 0.6 % faster than at 5), 5 while it records guide samples, 4 with the
-// traversal fused in
-#ifndef RGR_LOGIC_MIN_BLOCKS  // the plain pre-traced logic: 5 / 6 / 7 give 1464 / 1472 / 1436 Mpaths/s
-#define RGR_LOGIC_MIN_BLOCKS 6
-#endif
-__global__ void __launch_bounds__(kLogicThreads, kPreTraced ? (kGuided ? 5 : RGR_LOGIC_MIN_BLOCKS) : 4) k_trace_logic(PathsView P, QueueView Q, RenderParams rp) {
+template <bool kGuided, typename Logic>
+RGR_DEV void logic_block(const QueueView& Q, const RenderParams& rp, uint32_t slot, uint32_t tile, bool live,
+                         Logic logic) {
     const unsigned full = 0xffffffffu;
     __shared__ uint32_t s_q[kNumQueues];  // items per queue, then the block's base in it
     __shared__ uint32_t s_samples, s_offered;  // guided recording: accepted samples (then their base), offered
@@ -1225,12 +1211,10 @@ __global__ void __launch_bounds__(kLogicThreads, kPreTraced ? (kGuided ? 5 : RGR
     if (kGuided && threadIdx.x == 32) s_samples = s_offered = 0u;
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
-    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = slot < P.n && P.qid[slot] != kQueueIdle;
     const unsigned active = __ballot_sync(full, live);
     int q = 0;
     GuideOffer go;
-    if (live) q = logic_slot<kGuided, kPreTraced>(P, Q, rp, slot, active, go);
+    if (live) q = logic(active, go);
     __syncthreads();  // s_q, s_samples, s_offered cleared
     uint32_t off = 0;
     if (live) {
@@ -1256,7 +1240,7 @@ __global__ void __launch_bounds__(kLogicThreads, kPreTraced ? (kGuided ? 5 : RGR
     if (threadIdx.x < kNumQueues) {
         const uint32_t n = s_q[threadIdx.x];
         // queue 0: new paths per tile, for the ordered compaction (a block's slots lie in one tile)
-        if (n && threadIdx.x == 0) atomicAdd(Q.tile_new + slot / kTile, n);
+        if (n && threadIdx.x == 0) atomicAdd(Q.tile_new + tile, n);
         else if (n) s_q[threadIdx.x] = atomicAdd(Q.counts + threadIdx.x, n);
     }
     if (kGuided && threadIdx.x == 32) {
@@ -1270,6 +1254,115 @@ __global__ void __launch_bounds__(kLogicThreads, kPreTraced ? (kGuided ? 5 : RGR
         float ws = go.take ? guide_write(rp.gd, slot, go, s_samples + sidx) : 0.0f;
         for (int o = 16; o > 0; o >>= 1) ws += __shfl_xor_sync(full, ws, o);
         if (lane == 0 && ws > 0.0f) atomicAdd(rp.gd.train.wsum, ws);
+    }
+}
+
+// The logic kernel of a cast made before, one thread per slot.
+// latency-bound: 6 resident blocks per SM for the logic alone (40 registers; the
+// render 0.6 % faster than at 5), 5 while it records guide samples
+#ifndef RGR_LOGIC_MIN_BLOCKS  // the plain pre-traced logic: 5 / 6 / 7 give 1464 / 1472 / 1436 Mpaths/s
+#define RGR_LOGIC_MIN_BLOCKS 6
+#endif
+template <bool kGuided>
+__global__ void __launch_bounds__(kLogicThreads, kGuided ? 5 : RGR_LOGIC_MIN_BLOCKS)
+    k_logic(PathsView P, QueueView Q, RenderParams rp) {
+    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = slot < P.n && P.qid[slot] != kQueueIdle;
+    logic_block<kGuided>(Q, rp, slot, slot / kTile, live, [&](unsigned active, GuideOffer& go) {
+        return logic_slot<kGuided, true>(P, Q, rp, slot, active, go);
+    });
+}
+
+// Cast and logic of a bounce in one launch, for small pools.  A block takes the live ones
+// of `span` consecutive slots of one tile: it lists them in shared memory, its warps cast
+// their rays (a warp takes the next rays of the list as its lanes fall idle, and
+// ends lane by lane, as in k_trace_paths), the hits stay in shared memory, and the logic
+// goes over the list.  Bound by instruction issue at few lanes and by the longest rays: with
+// one thread a slot, from its ray to its queue, 6 to 8 of a warp's lanes were in use,
+// now 12 to 15.  Whole renders (4 spp, depth 6) at 2^15 / 2^17 / 2^18 paths, one thread a slot
+// and now: 5 K triangles 2028 / 2643 / 3794 us and 1963 / 2596 / 3400, 80 K triangles
+// 1536 / 1954 / 2699 and 1414 / 1775 / 2243; 36 triangles 883 / 1264 / 1808 and
+// 939 / 1283 / 1783 (a ray is over before the list pays).
+// 4 blocks an SM: 5 the same to 2 % slower.  `span`: 256 while the blocks are one wave,
+// else 512 (256 against 512 at 2^17: 2596 / 2646 us in 5 K triangles, 1775 / 1851 in
+// 80 K; at 2^18 3807 / 3400 and 2538 / 2243).
+constexpr int kCastLogicBlocks = 4;
+constexpr uint32_t kCastSpan = 512;
+template <bool kGuided, bool kOne>
+__global__ void __launch_bounds__(kLogicThreads, kCastLogicBlocks)
+    k_cast_logic(PathsView P, QueueView Q, RenderParams rp, uint32_t span, int refill, int search, SceneView one) {
+    const unsigned full = 0xffffffffu;
+    __shared__ uint32_t s_stack[(kSmemStack + 1) * kStackThreads];  // the last row: see touch
+    __shared__ uint32_t s_slot[kCastSpan];
+    __shared__ int32_t s_prim[kCastSpan];
+    __shared__ float s_t[kCastSpan];
+    __shared__ uint32_t s_n, s_next;
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    const uint32_t first = blockIdx.x * span;
+    if (threadIdx.x == 0) s_n = s_next = 0u;
+    __syncthreads();
+    for (uint32_t o = threadIdx.x; o < span; o += kLogicThreads) {
+        const uint32_t slot = first + o;
+        const bool live = slot < P.n && P.qid[slot] != kQueueIdle;
+        const unsigned m = __ballot_sync(full, live);
+        uint32_t base = 0;
+        if (lane == 0 && m) base = atomicAdd(&s_n, (uint32_t)__popc(m));
+        base = __shfl_sync(full, base, 0);
+        if (live) s_slot[base + __popc(m & lt)] = slot;
+    }
+    __syncthreads();
+    const uint32_t n = s_n;
+    // extension_ray_cast (extension_ray_cast_stackless.cl:202-246)
+    const uint64_t pol = l2_evict_last_policy();
+    TraceState s;
+    s.sstk = s_stack + threadIdx.x;
+    const SceneView* scp = kOne ? &one : &rp.reqs[0].sc;  // a valid scene on idle lanes too
+    uint32_t item = ~0u, err = 0;
+    bool exhausted = false;
+    auto put = [&]() {
+        s_t[item] = s.tmin;
+        s_prim[item] = hit_id(s.prim);
+        item = ~0u;
+    };
+    for (;;) {
+        const unsigned idle = __ballot_sync(full, item == ~0u);
+        if (!exhausted && (int)__popc(idle) >= refill) {
+            const uint32_t need = __popc(idle);
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(&s_next, need);
+            base = __shfl_sync(full, base, 0);
+            if (base + need >= n) exhausted = true;
+            const uint32_t i = base + __popc(idle & lt);
+            if (item == ~0u && i < n) {
+                item = i;
+                float4 ro4, rd4;
+                ld_sector<0>(P, s_slot[i], ro4, rd4);
+                if (!kOne) scp = &rp.reqs[P.req[s_slot[i]]].sc;
+                trace_begin(kOne ? one : *scp, s, xyz(ro4), xyz(rd4), ro4.w);
+            }
+        }
+        const unsigned held = __ballot_sync(full, item != ~0u);
+        if (exhausted && __popc(held) <= kTailLanes) break;
+        if (held == 0u) continue;
+        trace_warp_round<false, false, kSmemStack>(kOne ? one : *scp, s, item != ~0u && s.link != kDone, search,
+                                                   nullptr, err, pol);
+        if (item != ~0u && s.link == kDone) put();
+    }
+    if (item != ~0u) {  // the last few paths of the warp, lane by lane
+        while (s.link != kDone) trace_round<false, false, kSmemStack, true>(kOne ? one : *scp, s, nullptr, err, pol);
+        put();
+        touch_done();
+    }
+    if (err) atomicOr(rp.err, err);
+    __syncthreads();
+    for (uint32_t o = 0; o < n; o += kLogicThreads) {
+        const uint32_t i = o + threadIdx.x;
+        const uint32_t slot = i < n ? s_slot[i] : 0u;
+        logic_block<kGuided>(Q, rp, slot, first / kTile, i < n, [&](unsigned active, GuideOffer& go) {
+            return logic_slot<kGuided, false>(P, Q, rp, slot, active, go, s_prim[i], s_t[i]);
+        });
+        __syncthreads();  // before the counts are cleared again
     }
 }
 
@@ -1630,22 +1723,29 @@ cudaError_t launch_trace_paths(const PathsView& p, const QueueView& q, const Ren
     return cudaSuccess;
 }
 
+template <bool kGuided>
+static void trace_logic(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
+                        int num_sms, cudaStream_t st) {
+    if (ts.persistent) {
+        k_logic<kGuided><<<(p.n + kLogicThreads - 1) / kLogicThreads, kLogicThreads, 0, st>>>(p, q, rp);
+        return;
+    }
+    const uint32_t span = p.n <= kCastSpan / 2 * (uint32_t)(num_sms * kCastLogicBlocks) ? kCastSpan / 2 : kCastSpan;
+    const unsigned nb = (p.n + span - 1) / span;
+    if (ts.one && rp.nreq == 1)
+        k_cast_logic<kGuided, true><<<nb, kLogicThreads, 0, st>>>(p, q, rp, span, ts.refill, ts.search, *ts.one);
+    else
+        k_cast_logic<kGuided, false><<<nb, kLogicThreads, 0, st>>>(p, q, rp, span, ts.refill, ts.search, SceneView{});
+}
+
 void launch_trace_logic(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
-                        cudaStream_t st) {
-    const unsigned nb = (p.n + kLogicThreads - 1) / kLogicThreads;
+                        int num_sms, cudaStream_t st) {
     // the guided variant differs only in recording training samples: a render
     // with a frozen guide runs the plain one (fewer registers)
-    const bool recording = rp.gd.lobes && rp.gd.record;
-    if (ts.persistent) {
-        if (recording)
-            k_trace_logic<true, true><<<nb, kLogicThreads, 0, st>>>(p, q, rp);
-        else
-            k_trace_logic<false, true><<<nb, kLogicThreads, 0, st>>>(p, q, rp);
-    } else if (recording) {
-        k_trace_logic<true, false><<<nb, kLogicThreads, 0, st>>>(p, q, rp);
-    } else {
-        k_trace_logic<false, false><<<nb, kLogicThreads, 0, st>>>(p, q, rp);
-    }
+    if (rp.gd.lobes && rp.gd.record)
+        trace_logic<true>(p, q, rp, ts, num_sms, st);
+    else
+        trace_logic<false>(p, q, rp, ts, num_sms, st);
 }
 
 // what a bounce inside a run counts in

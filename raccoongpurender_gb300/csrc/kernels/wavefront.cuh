@@ -256,8 +256,7 @@ void launch_guide_select(const PathsView& p, const QueueView& q, const GuideRend
 // lanes are idle, node steps while `search` lanes still search for a leaf,
 // `grid` CTAs, `counter` a device word it may use; launch_trace_paths, between
 // the shading kernel and the queue resets), then the logic kernel; otherwise
-// one kernel traces and runs the logic per slot (launch_trace_paths does
-// nothing).  `one`: the scene of a render of a single request, or null.
+// one kernel casts and runs the logic (launch_trace_paths does nothing).  `one`: the scene of a render of a single request, or null.
 struct TraceShape {
     bool persistent;
     int refill;
@@ -270,7 +269,7 @@ struct TraceShape {
 cudaError_t launch_trace_paths(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
                                cudaStream_t st);
 void launch_trace_logic(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
-                        cudaStream_t st);
+                        int num_sms, cudaStream_t st);
 // One bounce inside a run of several (plain renders).  Between two bounces of a
 // run nobody looks at the state, so there is no logic pass over it: the cast decides
 // each path's next queue as its ray ends (the hit's material type is in the
