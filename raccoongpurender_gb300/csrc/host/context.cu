@@ -251,7 +251,7 @@ struct rgr_context {
         AL(qid, n);
         AL(req, 2 * n);
         for (int q = 0; q < kNumQueues; ++q) AL(queues[q], 4 * n);
-        AL(counts, 4 * 8);
+        AL(counts, 4 * 16);
         AL(tile_new, 4 * (size_t)ntiles);
         AL(scalars, 8 * 8);
         AL(err, 16);
@@ -267,6 +267,7 @@ struct rgr_context {
         QueueView& q = qv;
         for (int i = 0; i < kNumQueues; ++i) q.items[i] = queues[i].as<uint32_t>();
         q.counts = counts.as<uint32_t>();
+        q.taken = q.counts + 8;
         q.tile_new = tile_new.as<uint32_t>();
         q.ntiles = ntiles;
         in.words = inner_words.as<uint32_t>();
@@ -291,7 +292,7 @@ struct rgr_context {
         rp.reqs = reqtab.as<RequestD>();
         rp.nreq = nreq;
         rp.sample_limit = limit;
-        RGR_CUDA(cudaMemsetAsync(counts.p, 0, 32, st));
+        RGR_CUDA(cudaMemsetAsync(counts.p, 0, 64, st));
         RGR_CUDA(cudaMemsetAsync(scalars.p, 0, 64, st));
         RGR_CUDA(cudaMemsetAsync(err.p, 0, 16, st));
         launch_init(pv, qv, seed_offset, st);
@@ -309,13 +310,11 @@ struct rgr_context {
     }
     // train_now: a guided render ends a training interval with this bounce
     int step_launches(cudaStream_t st, bool train_now = true) {
-        launch_compact_new(pv, qv, st);
+        launch_compact_new(pv, qv, render_trace.counter, st);
         if (guided && rp.gd.max_depth) launch_guide_select(pv, qv, rp.gd, shade_grid, st);
         if (guided) guide->infer_paths(pv, qv, rp.gd, st);
         launch_shade(pv, qv, rp, shade_grid, st);
-        RGR_CUDA(launch_trace_paths(pv, qv, rp, render_trace, st));
-        RGR_CUDA(cudaMemsetAsync(qv.counts + 1, 0, sizeof(uint32_t) * (kNumQueues - 1), st));
-        RGR_CUDA(cudaMemsetAsync(qv.tile_new, 0, sizeof(uint32_t) * ntiles, st));
+        launch_trace_paths(pv, qv, rp, render_trace, st);
         launch_trace_logic(pv, qv, rp, render_trace, num_sms, st);
         if (!single_render) launch_stamp_done(rp, st);  // batches: per-request completion times
         RGR_CUDA(cudaGetLastError());
@@ -431,10 +430,10 @@ struct rgr_context {
     bool inner() const { return !guided && render_trace.persistent; }
     int run_first() {
         cudaStream_t st = stream;
-        launch_compact_new(pv, qv, st);
+        launch_compact_new(pv, qv, render_trace.counter, st);
         launch_shade(pv, qv, rp, shade_grid, st);
-        RGR_CUDA(launch_inner_cast(pv, qv, rp, render_trace, st));
-        launch_inner_reset(qv, in, st);
+        launch_inner_cast(pv, qv, rp, render_trace, st);
+        launch_inner_reset(in, st);
         RGR_CUDA(cudaGetLastError());
         return RGR_OK;
     }

@@ -140,6 +140,7 @@ extern "C" int rgr_render_noalloc(rgr_context* c, const rgr_camera* cam, const r
     QueueView q;
     for (int i = 0; i < kNumQueues; ++i) q.items[i] = reinterpret_cast<uint32_t*>(base + kOffQueues + align256(4 * kN) * i);
     q.counts = reinterpret_cast<uint32_t*>(base + kOffCounts);
+    q.taken = q.counts + 8;
     q.tile_new = reinterpret_cast<uint32_t*>(base + kOffTiles);
     q.ntiles = ntiles;
     unsigned long long* scal = reinterpret_cast<unsigned long long*>(base + kOffScalars);
@@ -191,12 +192,9 @@ extern "C" int rgr_render_noalloc(rgr_context* c, const rgr_camera* cam, const r
     const TraceShape ts{true, 24, 8,
                         sms * (trace_paths_max_blocks_per_sm() > 0 ? trace_paths_max_blocks_per_sm() : 1), scal + 3};
     for (int32_t i = 0; i < steps; ++i) {
-        launch_compact_new(p, q, st);
+        launch_compact_new(p, q, ts.counter, st);
         launch_shade(p, q, rp, sms * 8, st);
-        if (!ok(launch_trace_paths(p, q, rp, ts, st), "cudaMemsetAsync") ||
-            !ok(cudaMemsetAsync(q.counts + 1, 0, sizeof(uint32_t) * (kNumQueues - 1), st), "cudaMemsetAsync") ||
-            !ok(cudaMemsetAsync(q.tile_new, 0, sizeof(uint32_t) * ntiles, st), "cudaMemsetAsync"))
-            return RGR_E_CUDA;
+        launch_trace_paths(p, q, rp, ts, st);
         launch_trace_logic(p, q, rp, ts, sms, st);
         // a failed launch stops the call at the bounce it happened in
         if (!ok(cudaGetLastError(), "kernel launch")) return RGR_E_CUDA;

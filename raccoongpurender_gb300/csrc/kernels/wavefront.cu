@@ -724,8 +724,13 @@ __global__ void k_init(PathsView P, QueueView Q, uint32_t seed_offset) {
     P.req[i] = 0;
 }
 
-// Ordered compaction of new-path slots: block t owns slots [t*4096, (t+1)*4096).
-__global__ void __launch_bounds__(256) k_compact_new(PathsView P, QueueView Q) {
+// Ordered compaction of new-path slots: block t owns slots [t*4096, (t+1)*4096).  The last
+// block starts the bounce: it takes the queues' counts for the kernels up to the cast, and
+// clears them for the logic, and the cast's counter; the shading kernel clears the tile
+// counts.  Two memsets between a small pool's kernels cost 5 to 10 % of its renders: at 2^15 /
+// 2^17 / 2^18 paths 939 / 1283 / 1783 us with them and 884 / 1160 / 1705 without (36
+// triangles), 1963 / 2596 / 3400 and 1838 / 2460 / 3280 (5 K triangles).
+__global__ void __launch_bounds__(256) k_compact_new(PathsView P, QueueView Q, unsigned long long* cast_counter) {
     __shared__ uint32_t s_warp[8];
     __shared__ uint32_t s_prefix;
     const uint32_t t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -776,7 +781,13 @@ __global__ void __launch_bounds__(256) k_compact_new(PathsView P, QueueView Q) {
     }
     if (t == Q.ntiles - 1 && tid == 0) {
         uint32_t all = prefix + total;
-        Q.counts[0] = all;
+        Q.counts[0] = Q.taken[0] = all;
+#pragma unroll
+        for (int k = 1; k < kNumQueues; ++k) {
+            Q.taken[k] = Q.counts[k];
+            Q.counts[k] = 0u;
+        }
+        *cast_counter = 0ull;
         unsigned long long np = *Q.next_pixel;
         *Q.step_base = np;
         *Q.next_pixel = np + all;  // finalize_new_path (new_path.cl:85-88)
@@ -788,13 +799,14 @@ __device__ __forceinline__ void shade_items(const PathsView& P, const QueueView&
     uint32_t off[kNumQueues + 1];
     off[0] = 0;
 #pragma unroll
-    for (int k = 0; k < kNumQueues; ++k) off[k + 1] = off[k] + Q.counts[k];
+    for (int k = 0; k < kNumQueues; ++k) off[k + 1] = off[k] + Q.taken[k];
     const uint32_t total = off[kNumQueues];
     // guided items are numbered Lambertian, Ward, in-volume (as the inference kernel does)
     const uint32_t g4 = off[kMatLambertian + 1] - off[kMatLambertian];
     const uint32_t g6 = g4 + (off[kMatWard + 1] - off[kMatWard]);
     const unsigned long long base_pixel = *Q.step_base;
     const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < Q.ntiles; i += stride) Q.tile_new[i] = 0u;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         int k = 0;
 #pragma unroll
@@ -866,7 +878,7 @@ __global__ void __launch_bounds__(256, RGR_SHADE_MIN_BLOCKS) k_shade_inner(Paths
     uint32_t off[kNumQueues];  // off[k]: the first item of queue k + 1
     off[0] = 0;
 #pragma unroll
-    for (int k = 1; k < kNumQueues; ++k) off[k] = off[k - 1] + Q.counts[k];
+    for (int k = 1; k < kNumQueues; ++k) off[k] = off[k - 1] + Q.taken[k];
     const uint32_t total = off[kNumQueues - 1];
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -1013,7 +1025,7 @@ __global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS)
     uint32_t off[kNumQueues + 1];
     off[0] = 0;
 #pragma unroll
-    for (int k = 0; k < kNumQueues; ++k) off[k + 1] = off[k] + Q.counts[k];
+    for (int k = 0; k < kNumQueues; ++k) off[k + 1] = off[k] + Q.taken[k];
     const uint32_t total = off[kNumQueues];
     __shared__ uint32_t s_stack[(kSmemStack + 1) * kStackThreads];  // the last row: see touch
     TraceState s;
@@ -1690,8 +1702,8 @@ void launch_init(const PathsView& p, const QueueView& q, uint32_t seed_offset, c
     uint32_t n = q.ntiles * kTile;
     k_init<<<(n + 255) / 256, 256, 0, st>>>(p, q, seed_offset);
 }
-void launch_compact_new(const PathsView& p, const QueueView& q, cudaStream_t st) {
-    k_compact_new<<<q.ntiles, 256, 0, st>>>(p, q);
+void launch_compact_new(const PathsView& p, const QueueView& q, unsigned long long* cast_counter, cudaStream_t st) {
+    k_compact_new<<<q.ntiles, 256, 0, st>>>(p, q, cast_counter);
 }
 void launch_guide_select(const PathsView& p, const QueueView& q, const GuideRenderD& gd, int grid, cudaStream_t st) {
     cudaMemsetAsync(gd.nsel, 0, sizeof(uint32_t), st);
@@ -1714,13 +1726,9 @@ static void cast_paths(const PathsView& p, const QueueView& q, const RenderParam
             <<<ts.grid, kStackThreads, 0, st>>>(p, q, rp, ts.counter, ts.refill, ts.search, SceneView{});
 }
 
-cudaError_t launch_trace_paths(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
-                               cudaStream_t st) {
-    if (!ts.persistent) return cudaSuccess;
-    const cudaError_t e = cudaMemsetAsync(ts.counter, 0, sizeof(unsigned long long), st);
-    if (e != cudaSuccess) return e;
-    cast_paths<false>(p, q, rp, ts, st);
-    return cudaSuccess;
+void launch_trace_paths(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
+                        cudaStream_t st) {
+    if (ts.persistent) cast_paths<false>(p, q, rp, ts, st);
 }
 
 template <bool kGuided>
@@ -1749,17 +1757,13 @@ void launch_trace_logic(const PathsView& p, const QueueView& q, const RenderPara
 }
 
 // what a bounce inside a run counts in
-void launch_inner_reset(const QueueView& q, const InnerView& in, cudaStream_t st) {
+void launch_inner_reset(const InnerView& in, cudaStream_t st) {
     cudaMemsetAsync(in.words, 0, sizeof(uint32_t) * InnerView::kWords, st);
-    cudaMemsetAsync(q.counts + 1, 0, sizeof(uint32_t) * (kNumQueues - 1), st);
 }
 
-cudaError_t launch_inner_cast(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
-                              cudaStream_t st) {
-    const cudaError_t e = cudaMemsetAsync(ts.counter, 0, sizeof(unsigned long long), st);
-    if (e != cudaSuccess) return e;
+void launch_inner_cast(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
+                       cudaStream_t st) {
     cast_paths<true>(p, q, rp, ts, st);
-    return cudaSuccess;
 }
 
 void launch_inner(const PathsView& p, const QueueView& q, const InnerView& in, const RenderParams& rp,
@@ -1768,7 +1772,7 @@ void launch_inner(const PathsView& p, const QueueView& q, const InnerView& in, c
     const int blocks = std::min((int)((p.n + 255) / 256), num_sms * kNewPathsBlocks);
     k_new_paths<<<blocks, 256, 0, st>>>(p, q, in, rp);
     QueueView u = q;
-    u.counts = in.words;
+    u.taken = in.words;
     k_shade_inner<<<shade_grid, 256, 0, st>>>(p, u, rp);
     cast_paths<true>(p, u, rp, ts, st);
 }

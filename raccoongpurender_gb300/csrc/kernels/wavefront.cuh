@@ -106,7 +106,8 @@ __device__ __forceinline__ Rng rng_of_bits(const float4& v) {
 
 struct QueueView {
     uint32_t* items[kNumQueues];
-    uint32_t* counts;               // [kNumQueues]
+    uint32_t* counts;               // [kNumQueues]: what the logic appends
+    uint32_t* taken;                // [kNumQueues]: the items of the bounce being shaded
     uint32_t* tile_new;             // new paths per tile, for the ordered compaction
     uint32_t ntiles;
     unsigned long long* next_pixel; // new_path.cl next_pixel_index
@@ -220,10 +221,10 @@ struct GuideRenderD {
 // queue 1 (Lambertian), queue 4 (Ward), then queue 6 (in-volume) when
 // volumes are guided.
 __device__ __forceinline__ uint32_t guided_items(const QueueView& Q, const GuideRenderD& gd) {
-    return Q.counts[kMatLambertian] + Q.counts[kMatWard] + (gd.volumes ? Q.counts[kMatVolumeInside] : 0u);
+    return Q.taken[kMatLambertian] + Q.taken[kMatWard] + (gd.volumes ? Q.taken[kMatVolumeInside] : 0u);
 }
 __device__ __forceinline__ uint32_t guided_item_slot(const QueueView& Q, uint32_t gi) {
-    const uint32_t c1 = Q.counts[kMatLambertian], c4 = Q.counts[kMatWard];
+    const uint32_t c1 = Q.taken[kMatLambertian], c4 = Q.taken[kMatWard];
     if (gi < c1) return Q.items[kMatLambertian][gi];
     if (gi < c1 + c4) return Q.items[kMatWard][gi - c1];
     return Q.items[kMatVolumeInside][gi - c1 - c4];
@@ -247,7 +248,8 @@ struct RenderParams {
 
 // launchers (wavefront.cu)
 void launch_init(const PathsView& p, const QueueView& q, uint32_t seed_offset, cudaStream_t st);
-void launch_compact_new(const PathsView& p, const QueueView& q, cudaStream_t st);
+// starts a bounce; cast_counter: the cast's (TraceShape::counter)
+void launch_compact_new(const PathsView& p, const QueueView& q, unsigned long long* cast_counter, cudaStream_t st);
 void launch_shade(const PathsView& p, const QueueView& q, const RenderParams& rp, int grid, cudaStream_t st);
 // the guided items at vertices 1..gd.max_depth of their paths (gd.sel / remap / nsel; *nsel zeroed first)
 void launch_guide_select(const PathsView& p, const QueueView& q, const GuideRenderD& gd, int grid, cudaStream_t st);
@@ -265,8 +267,7 @@ struct TraceShape {
     unsigned long long* counter;
     const SceneView* one = nullptr;
 };
-// returns the status of its counter reset (launch errors: cudaGetLastError)
-cudaError_t launch_trace_paths(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
+void launch_trace_paths(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
                                cudaStream_t st);
 void launch_trace_logic(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
                         int num_sms, cudaStream_t st);
@@ -292,9 +293,9 @@ struct InnerView {
     uint32_t* tile_first;  // per tile: the ended paths of the tiles before it
     uint16_t* ended;       // per tile kTile entries: its ended paths' slots, less the tile's first
 };
-void launch_inner_reset(const QueueView& q, const InnerView& in, cudaStream_t st);
-cudaError_t launch_inner_cast(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
-                              cudaStream_t st);
+void launch_inner_reset(const InnerView& in, cudaStream_t st);
+void launch_inner_cast(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
+                       cudaStream_t st);
 void launch_inner(const PathsView& p, const QueueView& q, const InnerView& in, const RenderParams& rp,
                   const TraceShape& ts, bool boundary, int shade_grid, int num_sms, cudaStream_t st);
 int trace_paths_max_blocks_per_sm();
