@@ -724,6 +724,16 @@ __global__ void k_init(PathsView P, QueueView Q, uint32_t seed_offset) {
     P.req[i] = 0;
 }
 
+// The kernels of a bounce follow one another as programmatic dependent launches: the next
+// kernel's blocks are brought up as the last of this one's end, and wait, here, until it
+// has finished and its stores are visible.  Every thread of each kernel calls it first,
+// so that a kernel's end is also that of all before it.  Only the scene's tables are read
+// through the read-only path.  Whole renders at 2^15 / 2^18 paths 884 / 1705 us without,
+// 866 / 1680 with (36 triangles), eight requests 3654 and 3590; with griddepcontrol.launch_dependents
+// right after the wait 1068 / 1741 and 3610 (the waiting blocks crowd onto the SMs that happen to have
+// room).
+RGR_DEV void follow() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Ordered compaction of new-path slots: block t owns slots [t*4096, (t+1)*4096).  The last
 // block starts the bounce: it takes the queues' counts for the kernels up to the cast, and
 // clears them for the logic, and the cast's counter; the shading kernel clears the tile
@@ -731,6 +741,7 @@ __global__ void k_init(PathsView P, QueueView Q, uint32_t seed_offset) {
 // 2^17 / 2^18 paths 939 / 1283 / 1783 us with them and 884 / 1160 / 1705 without (36
 // triangles), 1963 / 2596 / 3400 and 1838 / 2460 / 3280 (5 K triangles).
 __global__ void __launch_bounds__(256) k_compact_new(PathsView P, QueueView Q, unsigned long long* cast_counter) {
+    follow();
     __shared__ uint32_t s_warp[8];
     __shared__ uint32_t s_prefix;
     const uint32_t t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -854,6 +865,7 @@ RGR_DEV void stamp_done(const RenderParams& rp, int i, int stride) {
     }
 }
 __global__ void k_stamp_done(RenderParams rp) {
+    follow();
     stamp_done(rp, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
@@ -869,10 +881,12 @@ __global__ void k_stamp_done(RenderParams rp) {
 #define RGR_SHADE_GUIDED_MIN_BLOCKS 4
 #endif
 __global__ void __launch_bounds__(256, RGR_SHADE_MIN_BLOCKS) k_shade(PathsView P, QueueView Q, RenderParams rp) {
+    follow();
     shade_items<false>(P, Q, rp);
 }
 // the material queues of a bounce inside a run (k_new_paths has taken the new paths)
 __global__ void __launch_bounds__(256, RGR_SHADE_MIN_BLOCKS) k_shade_inner(PathsView P, QueueView Q, RenderParams rp) {
+    follow();
     // the ended paths of the bounce before are finished and counted
     if (blockIdx.x == 0) stamp_done(rp, (int)threadIdx.x, (int)blockDim.x);
     uint32_t off[kNumQueues];  // off[k]: the first item of queue k + 1
@@ -891,6 +905,7 @@ __global__ void __launch_bounds__(256, RGR_SHADE_MIN_BLOCKS) k_shade_inner(Paths
 }
 __global__ void __launch_bounds__(256, RGR_SHADE_GUIDED_MIN_BLOCKS) k_shade_guided(PathsView P, QueueView Q,
                                                                                   RenderParams rp) {
+    follow();
     shade_items<true>(P, Q, rp);
 }
 
@@ -1018,6 +1033,7 @@ template <bool kInner, bool kOne>
 __global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS)
     k_trace_paths(PathsView P, QueueView Q, RenderParams rp, unsigned long long* next, int refill, int search,
                   SceneView one) {
+    follow();
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
@@ -1278,6 +1294,7 @@ RGR_DEV void logic_block(const QueueView& Q, const RenderParams& rp, uint32_t sl
 template <bool kGuided>
 __global__ void __launch_bounds__(kLogicThreads, kGuided ? 5 : RGR_LOGIC_MIN_BLOCKS)
     k_logic(PathsView P, QueueView Q, RenderParams rp) {
+    follow();
     const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = slot < P.n && P.qid[slot] != kQueueIdle;
     logic_block<kGuided>(Q, rp, slot, slot / kTile, live, [&](unsigned active, GuideOffer& go) {
@@ -1303,6 +1320,7 @@ constexpr uint32_t kCastSpan = 512;
 template <bool kGuided, bool kOne>
 __global__ void __launch_bounds__(kLogicThreads, kCastLogicBlocks)
     k_cast_logic(PathsView P, QueueView Q, RenderParams rp, uint32_t span, int refill, int search, SceneView one) {
+    follow();
     const unsigned full = 0xffffffffu;
     __shared__ uint32_t s_stack[(kSmemStack + 1) * kStackThreads];  // the last row: see touch
     __shared__ uint32_t s_slot[kCastSpan];
@@ -1391,6 +1409,7 @@ __global__ void __launch_bounds__(kLogicThreads, kCastLogicBlocks)
 // the next bounce counts in, so that a bounce needs no memset.
 __global__ void __launch_bounds__(256) k_classify(PathsView P, QueueView Q, InnerView I, RenderParams rp,
                                                   unsigned long long* trace_next, int boundary) {
+    follow();
     const unsigned full = 0xffffffffu;
     __shared__ unsigned long long s_lo[8], s_hi[8];
     __shared__ uint32_t s_off[kNumQueues + 1], s_base[kNumQueues], s_last;
@@ -1525,6 +1544,7 @@ __global__ void __launch_bounds__(256) k_classify(PathsView P, QueueView Q, Inne
 // When the render is over (launch_inner's boundary) the paths are only finished.
 constexpr int kNewPathsBlocks = 8;  // per SM
 __global__ void __launch_bounds__(256) k_new_paths(PathsView P, QueueView Q, InnerView I, RenderParams rp) {
+    follow();
     const unsigned full = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t total = I.words[InnerView::kEnded];
@@ -1698,12 +1718,27 @@ __global__ void k_debug_slots(PathsView P, uint32_t* out) {
 
 }  // namespace
 
+// launches a kernel that begins with follow()
+template <class... P, class... A>
+static void chain(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, const A&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 void launch_init(const PathsView& p, const QueueView& q, uint32_t seed_offset, cudaStream_t st) {
     uint32_t n = q.ntiles * kTile;
     k_init<<<(n + 255) / 256, 256, 0, st>>>(p, q, seed_offset);
 }
 void launch_compact_new(const PathsView& p, const QueueView& q, unsigned long long* cast_counter, cudaStream_t st) {
-    k_compact_new<<<q.ntiles, 256, 0, st>>>(p, q, cast_counter);
+    chain(k_compact_new, q.ntiles, 256, st, p, q, cast_counter);
 }
 void launch_guide_select(const PathsView& p, const QueueView& q, const GuideRenderD& gd, int grid, cudaStream_t st) {
     cudaMemsetAsync(gd.nsel, 0, sizeof(uint32_t), st);
@@ -1712,18 +1747,19 @@ void launch_guide_select(const PathsView& p, const QueueView& q, const GuideRend
 
 void launch_shade(const PathsView& p, const QueueView& q, const RenderParams& rp, int grid, cudaStream_t st) {
     if (rp.gd.lobes)
-        k_shade_guided<<<grid, 256, 0, st>>>(p, q, rp);
+        chain(k_shade_guided, grid, 256, st, p, q, rp);
     else
-        k_shade<<<grid, 256, 0, st>>>(p, q, rp);
+        chain(k_shade, grid, 256, st, p, q, rp);
 }
 template <bool kInner>
 static void cast_paths(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
                        cudaStream_t st) {
     if (ts.one && rp.nreq == 1)
-        k_trace_paths<kInner, true><<<ts.grid, kStackThreads, 0, st>>>(p, q, rp, ts.counter, ts.refill, ts.search, *ts.one);
+        chain(k_trace_paths<kInner, true>, ts.grid, kStackThreads, st, p, q, rp, ts.counter, ts.refill, ts.search,
+              *ts.one);
     else
-        k_trace_paths<kInner, false>
-            <<<ts.grid, kStackThreads, 0, st>>>(p, q, rp, ts.counter, ts.refill, ts.search, SceneView{});
+        chain(k_trace_paths<kInner, false>, ts.grid, kStackThreads, st, p, q, rp, ts.counter, ts.refill, ts.search,
+              SceneView{});
 }
 
 void launch_trace_paths(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
@@ -1735,15 +1771,15 @@ template <bool kGuided>
 static void trace_logic(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
                         int num_sms, cudaStream_t st) {
     if (ts.persistent) {
-        k_logic<kGuided><<<(p.n + kLogicThreads - 1) / kLogicThreads, kLogicThreads, 0, st>>>(p, q, rp);
+        chain(k_logic<kGuided>, (p.n + kLogicThreads - 1) / kLogicThreads, kLogicThreads, st, p, q, rp);
         return;
     }
     const uint32_t span = p.n <= kCastSpan / 2 * (uint32_t)(num_sms * kCastLogicBlocks) ? kCastSpan / 2 : kCastSpan;
     const unsigned nb = (p.n + span - 1) / span;
     if (ts.one && rp.nreq == 1)
-        k_cast_logic<kGuided, true><<<nb, kLogicThreads, 0, st>>>(p, q, rp, span, ts.refill, ts.search, *ts.one);
+        chain(k_cast_logic<kGuided, true>, nb, kLogicThreads, st, p, q, rp, span, ts.refill, ts.search, *ts.one);
     else
-        k_cast_logic<kGuided, false><<<nb, kLogicThreads, 0, st>>>(p, q, rp, span, ts.refill, ts.search, SceneView{});
+        chain(k_cast_logic<kGuided, false>, nb, kLogicThreads, st, p, q, rp, span, ts.refill, ts.search, SceneView{});
 }
 
 void launch_trace_logic(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
@@ -1768,17 +1804,17 @@ void launch_inner_cast(const PathsView& p, const QueueView& q, const RenderParam
 
 void launch_inner(const PathsView& p, const QueueView& q, const InnerView& in, const RenderParams& rp,
                   const TraceShape& ts, bool boundary, int shade_grid, int num_sms, cudaStream_t st) {
-    k_classify<<<q.ntiles, 256, 0, st>>>(p, q, in, rp, ts.counter, boundary ? 1 : 0);
+    chain(k_classify, q.ntiles, 256, st, p, q, in, rp, ts.counter, boundary ? 1 : 0);
     const int blocks = std::min((int)((p.n + 255) / 256), num_sms * kNewPathsBlocks);
-    k_new_paths<<<blocks, 256, 0, st>>>(p, q, in, rp);
+    chain(k_new_paths, blocks, 256, st, p, q, in, rp);
     QueueView u = q;
     u.taken = in.words;
-    k_shade_inner<<<shade_grid, 256, 0, st>>>(p, u, rp);
+    chain(k_shade_inner, shade_grid, 256, st, p, u, rp);
     cast_paths<true>(p, u, rp, ts, st);
 }
 
 void launch_stamp_done(const RenderParams& rp, cudaStream_t st) {
-    if (rp.nreq > 0) k_stamp_done<<<(rp.nreq + 127) / 128, 128, 0, st>>>(rp);
+    if (rp.nreq > 0) chain(k_stamp_done, (rp.nreq + 127) / 128, 128, st, rp);
 }
 
 int trace_paths_max_blocks_per_sm() {
