@@ -4,6 +4,8 @@
 // launch sequence is captured once into a CUDA graph and replayed, instead of
 // the reference's ~24 enqueued NDRange launches per bounce.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cmath>
@@ -170,7 +172,6 @@ constexpr uint32_t kPersistentTraceMinPaths = 3u << 17;
 // in 1.31M triangles, sorted / unsorted: 1 K 104 / 60 us, 20 K 160 / 123, 60 K 241 / 222,
 // 400 K 332 / 309, 1M 467 / 464, 4M 1178 / 1241 (from 2^16 to 1M the caller's choice stands).
 constexpr uint64_t kReorderMinRays = 1ull << 16;
-constexpr int kZeroCopyRefill = 32;  // refill threshold of the zero-copy closest-hit launch
 constexpr int kTraceSlots = 4;
 
 struct rgr_context {
@@ -212,6 +213,7 @@ struct rgr_context {
         DevBuf rays[7], prim, t, counter, err;
     } tslot[kTraceSlots];
     cudaStream_t tstream[kTraceSlots] = {};  // [0] unused: slot 0 runs on `stream`
+    uint32_t* link_err = nullptr;  // the zero-copy path's error word (pinned host memory)
     int trace_host_mode = RGR_TRACE_HOST_AUTO;  // rgr_trace_closest: zero copy where it can, or staged copies
     int trace_grid = 0;      // persistent traversal grid (SMs x resident blocks)
     int trace_refill = 24;   // refill a warp when this many lanes are idle (measured best of 1..32)
@@ -240,6 +242,7 @@ struct rgr_context {
         for (cudaStream_t s : tstream)
             if (s) cudaStreamDestroy(s);
         if (stream) cudaStreamDestroy(stream);
+        if (link_err) cudaFreeHost(link_err);
     }
     // the resident path pool: state, queues, counters (WavefrontLane::setup, :451-522)
     int alloc_pool() {
@@ -1022,6 +1025,23 @@ void* device_view(const void* p, bool pageable_ok) {
         return a.devicePointer;
     return pageable_ok ? const_cast<void*>(p) : nullptr;
 }
+
+// Brings in the pages of two result arrays, `bytes` each, contents unchanged.  The pages of a
+// fresh allocation would fault one by one under the GPU's stores, which take a 64 KB page at a
+// time far slower than the CPU does.  It runs beside the kernel, both arrays from the front, as
+// the kernel takes the rays: 1M rays into new arrays 2950 us without, 670 with it before
+// the launch, 426 beside the kernel (256 KB at a time; 1 MB: 495); into old ones 400 / 413 / 400.
+void populate(void* a, void* b, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const size_t chunk = 256u << 10;
+    for (size_t o = 0; o < bytes; o += chunk)
+        for (void* p : {a, b}) {
+            const uintptr_t from = ((uintptr_t)p + o) / page * page, to = (uintptr_t)p + std::min(o + chunk, bytes);
+            madvise((void*)from, to - from, MADV_POPULATE_WRITE);  // where it cannot, the pages still fault
+        }
+#endif
+}
 }  // namespace
 
 int rgr_trace_closest(rgr_context* c, const rgr_ray_soa* rays, uint64_t n, int32_t* prim, float* t) {
@@ -1047,20 +1067,16 @@ int rgr_trace_closest(rgr_context* c, const rgr_ray_soa* rays, uint64_t n, int32
         float* dt = direct ? (float*)device_view(t, pageable) : nullptr;
         if (direct && dprim && dt) {
             rgr_context::TraceSlot& ts = c->tslot[0];
-            if ((r = ts.counter.alloc(8)) != RGR_OK || (r = ts.err.alloc(16)) != RGR_OK) return r;
+            if ((r = ts.counter.alloc(8)) != RGR_OK) return r;
+            if (!c->link_err) RGR_CUDA(cudaMallocHost(&c->link_err, sizeof(uint32_t)));
+            *c->link_err = 0u;
             cudaStream_t st = c->stream;
-            RGR_CUDA(cudaMemsetAsync(ts.err.p, 0, 4, st));
-            // a warp refills only when all its lanes are idle: each refill's reads across
-            // the link then serve 32 rays (measured: 3030 Mrays/s end to end, against
-            // 2905 with the threshold tuned for rays in device memory)
-            launch_trace_rays(c->scene.sv, dsrc[0], dsrc[1], dsrc[2], dsrc[3], dsrc[4], dsrc[5], dsrc[6], n, dprim, dt,
-                              nullptr, ts.err.as<uint32_t>(), ts.counter.as<unsigned long long>(), kZeroCopyRefill,
-                              c->trace_search, c->trace_grid, c->trace_stage, st);
+            launch_trace_rays_link(c->scene.sv, dsrc, n, dprim, dt, c->link_err, ts.counter.as<unsigned long long>(),
+                                   c->trace_refill, c->trace_search, c->trace_grid, st);
             RGR_CUDA(cudaGetLastError());
-            uint32_t err = 0;
-            RGR_CUDA(cudaMemcpyAsync(&err, ts.err.p, 4, cudaMemcpyDeviceToHost, st));
+            populate(prim, t, 4 * n);
             RGR_CUDA(cudaStreamSynchronize(st));
-            if (err) {
+            if (*c->link_err) {
                 set_error("traversal stack overflow");
                 return RGR_E_OVERFLOW;
             }

@@ -63,8 +63,23 @@ RGR_DEV void ld_record(const float4* ptr, float4& a, float4& b) {
         : "l"(ptr));
 }
 
+// Results in host memory (kLink) cross the link in runs: the rays of one refill are
+// consecutive, and their hits wait in shared memory until the last of them is known.
+// Single 4-byte stores keep the link busy: 1M random rays in 330 K triangles took 400 us with
+// only the results across it, 342 with only the rays (320 with neither), the whole call
+// 502 and now 400 us; 2M rays in 1.31M triangles 957 and 787.  (The rays' reads hide behind the
+// traversal: copying them to shared memory a batch ahead was slower, 549, as every
+// warp's first rays then share the link with the others' second.)  A warp keeps up to
+// kRuns runs open; to begin another it writes what the oldest has, and that one's missing
+// rays write their own.
+constexpr int kRuns = 4;
+struct LinkRuns {
+    int32_t prim[kRuns][32];
+    float t[kRuns][32];
+};
+
 // kFew: each lane takes one ray of its warp's share, without the rounds
-template <bool kCount, bool kStaged, bool kPacked, bool kFew>
+template <bool kCount, bool kStaged, bool kPacked, bool kFew, bool kLink>
 __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneView sc, RayBatch b) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -82,6 +97,23 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
     s.sstk = s_stack + threadIdx.x;
     TraceCounters cnt;
     uint64_t ray = ~0ull;  // ~0: idle
+    __shared__ LinkRuns s_runs[kLink ? kStackThreads / 32 : 1];
+    LinkRuns& runs = s_runs[kLink ? threadIdx.x >> 5 : 0];
+    uint64_t run_base = 0;                // lane k < kRuns: run k's first ray,
+    unsigned run_rays = 0, run_done = 0;  // its rays and the finished ones of them (none: free)
+    int run = -1, place = 0;              // this lane's ray's run, and its place there
+    int oldest = 0;
+    // writes the finished rays of run k, which is free then
+    auto flush = [&](int k) {
+        const uint64_t base = __shfl_sync(full, run_base, k);
+        const unsigned done = __shfl_sync(full, run_done, k);
+        if ((done >> lane) & 1u) {
+            __stcs(b.prim + base + lane, runs.prim[k][lane]);
+            __stcs(b.t + base + lane, runs.t[k][lane]);
+        }
+        __syncwarp();
+        if (lane == k) run_rays = run_done = 0u;
+    };
     auto take = [&](uint64_t r) {
         if (kPacked) {
             float4 o4, d4;
@@ -100,8 +132,13 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
     };
     auto put = [&]() {
         const int32_t prim = hit_id(s.prim);
-        __stcs(b.prim + ray, prim);
-        __stcs(b.t + ray, s.tmin);
+        if (kLink && run >= 0) {
+            runs.prim[run][place] = prim;
+            runs.t[run][place] = s.tmin;
+        } else {
+            __stcs(b.prim + ray, prim);
+            __stcs(b.t + ray, s.tmin);
+        }
         if (b.ng) {
             f3 n = prim >= 0 ? hit_normal(sc, prim, s.ro, s.rd, s.tmin) : mk(0.0f, 0.0f, 0.0f);
             b.ng[3 * ray + 0] = n.x;
@@ -128,6 +165,22 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
             if (lane == 0) base = atomicAdd(b.next, (unsigned long long)need);
             base = __shfl_sync(full, base, 0);
             if (base + need >= b.n) exhausted = true;
+            if (kLink && base < b.n) {  // a run of the new rays
+                const int k = oldest;
+                oldest = (oldest + 1) % kRuns;
+                if (__shfl_sync(full, run_rays, k)) {
+                    flush(k);
+                    if (run == k) run = -1;
+                }
+                if (lane == k) {
+                    run_base = base;
+                    run_rays = b.n - base >= need ? (need < 32u ? (1u << need) - 1u : full) : (1u << (b.n - base)) - 1u;
+                }
+                if (ray == ~0ull) {
+                    run = k;
+                    place = __popc(idle & lt);
+                }
+            }
             if (ray == ~0ull) {
                 const uint64_t r = base + __popc(idle & lt);
                 if (r < b.n) take(r);
@@ -138,7 +191,22 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
         if (held == 0u) continue;
         trace_warp_round<kCount, kStaged, kSmemStack>(sc, s, ray != ~0ull && s.link != kDone, b.search, &cnt, err, pol,
                                                       stn);
-        if (ray != ~0ull && s.link == kDone) put();
+        const bool ended = ray != ~0ull && s.link == kDone;
+        if (ended) put();
+        if (kLink) {
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < kRuns; ++k) {
+                const unsigned places = __reduce_or_sync(full, ended && run == k ? 1u << place : 0u);
+                if (lane == k) run_done |= places;
+                if (places && __shfl_sync(full, run_done == run_rays, k)) flush(k);
+            }
+        }
+    }
+    if (kLink) {  // the last rays write their own
+#pragma unroll
+        for (int k = 0; k < kRuns; ++k) flush(k);
+        run = -1;
     }
     if (ray != ~0ull) {
         while (s.link != kDone) trace_round<kCount, kStaged, kSmemStack, true>(sc, s, &cnt, err, pol, stn);
@@ -361,11 +429,26 @@ void launch_trace_rays(const SceneView& sc, const float* ox, const float* oy, co
     RayBatch b{ox, oy, oz, dx, dy, dz, tmax, nullptr, n, prim, t, ng, nullptr, nullptr, err, counter, share, refill,
                search, stage};
     if (share)
-        k_trace_rays<false, false, false, true><<<blocks, kStackThreads, 0, st>>>(sc, b);
+        k_trace_rays<false, false, false, true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
     else if (stage > 0)
-        k_trace_rays<false, true, false, false><<<blocks, kStackThreads, 64 * (size_t)stage, st>>>(sc, b);
+        k_trace_rays<false, true, false, false, false><<<blocks, kStackThreads, 64 * (size_t)stage, st>>>(sc, b);
     else
-        k_trace_rays<false, false, false, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
+        k_trace_rays<false, false, false, false, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
+}
+
+// rays and results in host memory
+void launch_trace_rays_link(const SceneView& sc, const float* const* rays, uint64_t n, int32_t* prim, float* t,
+                            uint32_t* err, unsigned long long* counter, int refill, int search, int grid,
+                            cudaStream_t st) {
+    if (n == 0) return;
+    int blocks;
+    const uint32_t share = spread(n, grid, &blocks, counter, st);
+    RayBatch b{rays[0], rays[1], rays[2], rays[3], rays[4], rays[5], rays[6], nullptr, n, prim, t, nullptr,
+               nullptr, nullptr, err, counter, share, refill, search, 0u};
+    if (share)
+        k_trace_rays<false, false, false, true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
+    else
+        k_trace_rays<false, false, false, false, true><<<blocks, kStackThreads, 0, st>>>(sc, b);
 }
 
 void launch_trace_rays_counts(const SceneView& sc, const float* ox, const float* oy, const float* oz, const float* dx,
@@ -377,9 +460,9 @@ void launch_trace_rays_counts(const SceneView& sc, const float* ox, const float*
     const uint32_t share = spread(n, grid, &blocks, counter, st);
     RayBatch b{ox, oy, oz, dx, dy, dz, tmax, nullptr, n, prim, t, nullptr, nodes, prims, err, counter, share, 16, 1, 0u};
     if (share)
-        k_trace_rays<true, false, false, true><<<blocks, kStackThreads, 0, st>>>(sc, b);
+        k_trace_rays<true, false, false, true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
     else
-        k_trace_rays<true, false, false, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
+        k_trace_rays<true, false, false, false, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
 }
 
 // the per-triangle table of a scene (its tri_normals still null): the normal,
@@ -421,19 +504,19 @@ void launch_trace_packed(const SceneView& sc, const float4* packed, uint64_t n, 
     RayBatch b{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, packed, n, prim, t, ng, nullptr,
                nullptr, err, counter, share, refill, search, 0u};
     if (share)
-        k_trace_rays<false, false, true, true><<<blocks, kStackThreads, 0, st>>>(sc, b);
+        k_trace_rays<false, false, true, true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
     else
-        k_trace_rays<false, false, true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
+        k_trace_rays<false, false, true, false, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
 }
 
 int trace_rays_max_blocks_per_sm(uint32_t stage) {
     int nb = 0;
     if (stage > 0) {
-        cudaFuncSetAttribute(k_trace_rays<false, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(k_trace_rays<false, true, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(64 * kMaxStagedNodes));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_rays<false, true, false, false>, 256, 64 * (size_t)stage);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_rays<false, true, false, false, false>, 256, 64 * (size_t)stage);
     } else {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_rays<false, false, false, false>, 256, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_rays<false, false, false, false, false>, 256, 0);
     }
     return nb;
 }

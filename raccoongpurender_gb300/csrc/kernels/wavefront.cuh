@@ -314,6 +314,10 @@ void launch_trace_rays(const SceneView& sc, const float* ox, const float* oy, co
                        const float* dy, const float* dz, const float* tmax, uint64_t n, int32_t* prim, float* t,
                        float* ng, uint32_t* err, unsigned long long* counter, int refill, int search, int grid,
                        uint32_t stage, cudaStream_t st);
+// the same for rays and results in host memory that the GPU reads and writes across a coherent link
+void launch_trace_rays_link(const SceneView& sc, const float* const* rays, uint64_t n, int32_t* prim, float* t,
+                            uint32_t* err, unsigned long long* counter, int refill, int search, int grid,
+                            cudaStream_t st);
 void launch_trace_rays_counts(const SceneView& sc, const float* ox, const float* oy, const float* oz, const float* dx,
                               const float* dy, const float* dz, const float* tmax, uint64_t n, int32_t* prim,
                               float* t, uint32_t* nodes, uint32_t* prims, uint32_t* err, unsigned long long* counter,

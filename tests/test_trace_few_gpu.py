@@ -92,3 +92,20 @@ def test_deep_tree(rg, po, n, leaf):
     assert n < 100 or 0.1 < (oprim >= 0).mean() < 0.9
     prim, t, _ = _hits(lane, rays)
     assert (prim == oprim).all() and (bits(t) == bits(ot)).all()
+
+
+@pytest.mark.parametrize("refill", [1, 7, 16, 32])
+@pytest.mark.parametrize("n", [4 * 152 * 8 + 1, 100001])
+def test_host_runs(rg, po, refill, n):
+    """Hits written across the link in runs: short runs and whole ones, more open than a warp
+    keeps, a last run cut by the end."""
+    mesh = scenes.displaced_icosphere(4, seed=7)
+    sm, osc = build(mesh)
+    lane = rg.WavefrontLane(0, 1024)
+    lane.setup(sm)
+    lane.set_trace_tuning(refill, 1)  # one block an SM: many refills a warp
+    rays = scenes.random_rays(n, (-1.3, -1.3, -1.3), (1.3, 1.3, 1.3), seed=n + refill)
+    rays.tmax[::3] = 0.05  # over at once, beside long ones
+    oprim, ot, _ = osc.trace(rays.packed8(), threads=16)
+    prim, t = lane.trace_closest(rays)
+    assert (prim == oprim).all() and (bits(t) == bits(ot)).all()
