@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -151,6 +152,24 @@ RequestD request_d(const SceneView& sv, const rgr_camera& cam, const rgr_render_
     q.done = done;
     q.done_ns = done ? done + 1 : nullptr;
     return q;
+}
+
+// Brings in the pages of arrays that the host will get `bytes` of results in each, contents
+// unchanged.  The pages of a fresh allocation would fault one by one under the GPU's stores, which
+// take a 64 KB page at a time far slower than the CPU does, or under the copy's.  It runs
+// beside the GPU's work, all arrays from the front, as closest hits arrive: 1M hits into
+// new arrays 2950 us without, 670 with it before the launch, 426 beside the kernel (256 KB
+// at a time; 1 MB: 495); into old ones 400 / 413 / 400.
+void populate(std::initializer_list<void*> arrays, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const size_t chunk = 256u << 10;
+    for (size_t o = 0; o < bytes; o += chunk)
+        for (void* p : arrays) {
+            const uintptr_t from = ((uintptr_t)p + o) / page * page, to = (uintptr_t)p + std::min(o + chunk, bytes);
+            madvise((void*)from, to - from, MADV_POPULATE_WRITE);  // where it cannot, the pages still fault
+        }
+#endif
 }
 
 }  // namespace
@@ -1026,22 +1045,6 @@ void* device_view(const void* p, bool pageable_ok) {
     return pageable_ok ? const_cast<void*>(p) : nullptr;
 }
 
-// Brings in the pages of two result arrays, `bytes` each, contents unchanged.  The pages of a
-// fresh allocation would fault one by one under the GPU's stores, which take a 64 KB page at a
-// time far slower than the CPU does.  It runs beside the kernel, both arrays from the front, as
-// the kernel takes the rays: 1M rays into new arrays 2950 us without, 670 with it before
-// the launch, 426 beside the kernel (256 KB at a time; 1 MB: 495); into old ones 400 / 413 / 400.
-void populate(void* a, void* b, size_t bytes) {
-#ifdef MADV_POPULATE_WRITE
-    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
-    const size_t chunk = 256u << 10;
-    for (size_t o = 0; o < bytes; o += chunk)
-        for (void* p : {a, b}) {
-            const uintptr_t from = ((uintptr_t)p + o) / page * page, to = (uintptr_t)p + std::min(o + chunk, bytes);
-            madvise((void*)from, to - from, MADV_POPULATE_WRITE);  // where it cannot, the pages still fault
-        }
-#endif
-}
 }  // namespace
 
 int rgr_trace_closest(rgr_context* c, const rgr_ray_soa* rays, uint64_t n, int32_t* prim, float* t) {
@@ -1074,7 +1077,7 @@ int rgr_trace_closest(rgr_context* c, const rgr_ray_soa* rays, uint64_t n, int32
             launch_trace_rays_link(c->scene.sv, dsrc, n, dprim, dt, c->link_err, ts.counter.as<unsigned long long>(),
                                    c->trace_refill, c->trace_search, c->trace_grid, st);
             RGR_CUDA(cudaGetLastError());
-            populate(prim, t, 4 * n);
+            populate({prim, t}, 4 * n);
             RGR_CUDA(cudaStreamSynchronize(st));
             if (*c->link_err) {
                 set_error("traversal stack overflow");
