@@ -239,7 +239,8 @@ int rgr_render_restore(rgr_context* c, const void* src, uint64_t src_bytes);
 /* merge_from (:963-991): add src's accumulation into dst (replicas on several GPUs) */
 int rgr_accum_merge(rgr_context* dst, rgr_context* src);
 int rgr_synchronize(rgr_context* c);
-/* capture the bounce loop in a CUDA graph (1) or launch stage by stage (0; default 1) */
+/* capture the bounce loop in a CUDA graph (1) or launch stage by stage (0); by default guided
+   renders replay a graph and plain ones, whose launches overlap, do not.  Results are identical. */
 int rgr_set_graph_mode(rgr_context* c, int32_t enabled);
 
 /* merge_intermediate (accumlation.cl:27-49): a <- count-weighted merge of two
@@ -266,7 +267,7 @@ void rgr_batch_destroy(rgr_batch* b);
 /* the scene is uploaded once per distinct scene; cfg->spp must be > 0 */
 int rgr_batch_add(rgr_batch* b, const rgr_scene* scene, const rgr_camera* cam, const rgr_render_config* cfg,
                   int32_t* request_id);
-/* render every request to completion, replaying a CUDA graph of steps_per_launch bounces */
+/* render every request to completion, looking whether it is over every steps_per_launch bounces */
 int rgr_batch_run(rgr_batch* b, int32_t order_policy, int32_t steps_per_launch, int32_t max_steps,
                   int32_t* steps_done);
 int rgr_batch_readback(rgr_batch* b, int32_t request_id, int32_t fmt, void* dst, uint64_t dst_bytes);
@@ -321,7 +322,7 @@ int rgr_render_noalloc(rgr_context* c, const rgr_camera* cam, const rgr_render_c
                        int32_t steps, double* accum_out, void* stream);
 
 /* Launch shape of the bounce loop: resident 256-thread shade blocks per SM
-   (1..64) and bounces per replayed CUDA graph (1..256).  Chosen by the
+   (1..64) and bounces per CUDA graph, where one is replayed (1..256).  Chosen by the
    autotuner (raccoongpurender_gb300/autotune.py). */
 int rgr_set_render_tuning(rgr_context* c, int32_t shade_blocks_per_sm, int32_t graph_steps);
 
@@ -333,8 +334,8 @@ int rgr_set_trace_tuning(rgr_context* c, int32_t refill, int32_t blocks_per_sm);
 /* How a bounce casts its extension rays: persistent = 1 runs a persistent
    closest-hit kernel over the slots just shaded whose warps take new slots
    when at least `refill` (1..32, default 12) lanes are idle, then the logic
-   kernel; persistent = 0 traces and runs the logic in one kernel, one thread
-   per slot; persistent = -1 (default) picks 1 for pools of at least 3 * 2^17
+   kernel; persistent = 0 casts and runs the logic in one kernel, a block
+   per 256 or 512 slots; persistent = -1 (default) picks 1 for pools of at least 3 * 2^17
    paths.  Results are identical.  Takes effect at the next
    rgr_render_begin. */
 int rgr_set_render_trace(rgr_context* c, int32_t persistent, int32_t refill);
@@ -359,7 +360,8 @@ int rgr_set_trace_staging(rgr_context* c, uint32_t staged_nodes);
 /* Ray reordering of rgr_trace_closest_device (no counterpart in the
    reference): reorder = 1 sorts the rays by a 16-bit key of their origin and
    direction before the traversal (a counting sort on the device, 36 bytes of
-   scratch per ray; calls of 2^32 rays or more are traced unsorted), so that a
+   scratch per ray; calls of fewer than 2^16 rays, whose longest rays take longer
+   than sorting could save, and of 2^32 or more are traced unsorted), so that a
    warp's rays walk similar paths through the tree; it pays for incoherent rays
    and costs more than it saves on coherent ones (camera rays).  0 = off
    (default).  Results are identical either way; the order only changes the

@@ -620,8 +620,8 @@ class WavefrontLane:
 
     def set_trace_reorder(self, reorder: int) -> None:
         """trace_closest_device sorts the rays by origin and direction before the
-        traversal (1) or takes them in the given order (0, default).  Results are
-        identical; sorting pays for incoherent rays."""
+        traversal (1; calls of at least 65,536 rays) or takes them in the given order
+        (0, default).  Results are identical; sorting pays for incoherent rays."""
         _check(self._lib.rgr_set_trace_reorder(self._h, reorder), "rgr_set_trace_reorder")
 
     def trace_closest_counts_device(self, soa_ptrs, n: int, prim_ptr: int, t_ptr: int, nodes_ptr: int,
@@ -776,7 +776,7 @@ ORDER_FIFO, ORDER_SHORTEST_FIRST = 0, 1
 
 class Batch:
     """Many render requests of uneven size sharing one path pool and one
-    graph-replayed bounce loop."""
+    bounce loop."""
 
     def __init__(self, device: int = 0, path_count: int = 1 << 22):
         self._lib = load_library()

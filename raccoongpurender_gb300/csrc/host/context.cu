@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstring>
 #include <initializer_list>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -172,6 +173,45 @@ void populate(std::initializer_list<void*> arrays, size_t bytes) {
 #endif
 }
 
+// Pinned host memory for the words that a context's calls wait for: copied to in its stream's
+// order, read after one wait for the stream.
+struct Mail {
+    unsigned long long next_pixel;
+    uint32_t counts[8], stop, err;
+    uint32_t link_err;  // the zero-copy path's error word, written by its kernel
+    uint32_t pad;
+};
+// Pinning a page takes some 120 us and a context 15 to create, so the first 64 contexts of
+// the process share one allocation; a further one has its own.
+constexpr int kSharedMails = 64;
+std::mutex mail_mutex;
+Mail* shared_mails = nullptr;
+uint64_t shared_taken = 0;  // a bit each
+
+Mail* take_mail() {
+    std::lock_guard<std::mutex> lock(mail_mutex);
+    Mail* m = nullptr;
+    if (!shared_mails && !cuda_ok(cudaHostAlloc(&shared_mails, sizeof(Mail) * kSharedMails, cudaHostAllocPortable),
+                                  "cudaHostAlloc")) {
+        shared_mails = nullptr;
+        return nullptr;
+    }
+    for (int k = 0; k < kSharedMails; ++k)
+        if (!((shared_taken >> k) & 1u)) {
+            shared_taken |= 1ull << k;
+            return shared_mails + k;
+        }
+    return cuda_ok(cudaHostAlloc(&m, sizeof(Mail), cudaHostAllocPortable), "cudaHostAlloc") ? m : nullptr;
+}
+void give_mail(Mail* m) {  // its context's stream is idle
+    if (!m) return;
+    std::lock_guard<std::mutex> lock(mail_mutex);
+    if (m >= shared_mails && m < shared_mails + kSharedMails)
+        shared_taken &= ~(1ull << (m - shared_mails));
+    else
+        cudaFreeHost(m);
+}
+
 }  // namespace
 
 // Pools of fewer paths run the fused trace + logic kernel by default (a bounce is then
@@ -203,6 +243,7 @@ struct rgr_context {
     DevBuf slots, qid, req, queues[kNumQueues], counts, tile_new, scalars, accum, err;
     DevBuf inner_words, inner_tiles, inner_ended;  // the bounces inside a run (launch_inner)
     InnerView in{};
+    Mail* mail = nullptr;
     DevBuf reqtab, done;  // request table and its per-request (done, done_ns) counters
     PathsView pv{};
     QueueView qv{};
@@ -217,7 +258,7 @@ struct rgr_context {
     int shade_grid = 0;
     int shade_blocks_per_sm = 8;
     // CUDA graph of `graph_steps` bounces
-    bool graph_mode = true;
+    int graph_mode = -1;  // replay captured bounces: 0 no, 1 yes, -1 where that is the faster (graphs)
     int graph_steps = 1;
     int graph_steps_default = 1;
     struct Graph {
@@ -232,7 +273,6 @@ struct rgr_context {
         DevBuf rays[7], prim, t, counter, err;
     } tslot[kTraceSlots];
     cudaStream_t tstream[kTraceSlots] = {};  // [0] unused: slot 0 runs on `stream`
-    uint32_t* link_err = nullptr;  // the zero-copy path's error word (pinned host memory)
     int trace_host_mode = RGR_TRACE_HOST_AUTO;  // rgr_trace_closest: zero copy where it can, or staged copies
     int trace_grid = 0;      // persistent traversal grid (SMs x resident blocks)
     int trace_refill = 24;   // refill a warp when this many lanes are idle (measured best of 1..32)
@@ -261,7 +301,7 @@ struct rgr_context {
         for (cudaStream_t s : tstream)
             if (s) cudaStreamDestroy(s);
         if (stream) cudaStreamDestroy(stream);
-        if (link_err) cudaFreeHost(link_err);
+        give_mail(mail);
     }
     // the resident path pool: state, queues, counters (WavefrontLane::setup, :451-522)
     int alloc_pool() {
@@ -310,16 +350,18 @@ struct rgr_context {
         render_trace.persistent =
             render_trace_mode < 0 ? npaths >= kPersistentTraceMinPaths : render_trace_mode != 0;
         if ((r = reqtab.alloc(sizeof(RequestD) * nreq)) != RGR_OK) return r;
-        RGR_CUDA(cudaMemcpyAsync(reqtab.p, host_reqs, sizeof(RequestD) * nreq, cudaMemcpyHostToDevice, st));
         rp.reqs = reqtab.as<RequestD>();
         rp.nreq = nreq;
         rp.sample_limit = limit;
-        RGR_CUDA(cudaMemsetAsync(counts.p, 0, 64, st));
-        RGR_CUDA(cudaMemsetAsync(scalars.p, 0, 64, st));
-        RGR_CUDA(cudaMemsetAsync(err.p, 0, 16, st));
-        launch_init(pv, qv, seed_offset, st);
+        const InitView w{scalars.as<unsigned long long>(), err.as<uint32_t>(),
+                         nreq == 1 ? done.as<unsigned long long>() : nullptr,
+                         nreq == 1 ? reqtab.as<RequestD>() : nullptr};
+        launch_init(pv, qv, seed_offset, w, host_reqs[0], st);
         RGR_CUDA(cudaGetLastError());
-        RGR_CUDA(cudaStreamSynchronize(st));  // host_reqs may be a temporary
+        if (nreq > 1) {
+            RGR_CUDA(cudaMemcpyAsync(reqtab.p, host_reqs, sizeof(RequestD) * nreq, cudaMemcpyHostToDevice, st));
+            RGR_CUDA(cudaStreamSynchronize(st));  // host_reqs may be a temporary
+        }
         shade_grid = num_sms * shade_blocks_per_sm;
         graph_steps = graph_steps_default;
         // a replayed graph holds whole training intervals
@@ -429,7 +471,7 @@ struct rgr_context {
             return r;
         }
         while (n > 0) {
-            if (graph_mode && (n >= graph_steps || graph_steps == 1)) {
+            if (graphs() && (n >= graph_steps || graph_steps == 1)) {
                 int r = replay(step_graph, [&] {
                     int q = RGR_OK;
                     for (int i = 0; i < graph_steps && q == RGR_OK; ++i)
@@ -448,6 +490,11 @@ struct rgr_context {
         }
         return RGR_OK;
     }
+    // Plain bounces are launched one by one by default: their launches overlap (follow), which
+    // a replay ends with, and a render's first pass need not capture.  A preview frame of 12 bounces
+    // 2708 us replayed, 2671 launched, a 65,536-pixel render 558 and 548 (its first 4300
+    // and 2613); a guided render, of more launches a bounce, 6929 and 6974.
+    bool graphs() const { return graph_mode < 0 ? guided : graph_mode != 0; }
     // the first bounce of a run up to its rays' cast
     bool inner() const { return !guided && render_trace.persistent; }
     int run_first() {
@@ -467,7 +514,7 @@ struct rgr_context {
             return RGR_OK;
         };
         int r = RGR_OK;
-        for (; graph_mode && n >= graph_steps && r == RGR_OK; n -= graph_steps)
+        for (; graphs() && n >= graph_steps && r == RGR_OK; n -= graph_steps)
             r = replay(inner_graph, [&] {
                 int q = RGR_OK;
                 for (int i = 0; i < graph_steps && q == RGR_OK; ++i) q = one();
@@ -493,8 +540,6 @@ struct rgr_context {
             const int b = std::min(group, max_steps - *ran);
             const bool last = *ran + b >= max_steps;
             int r;
-            uint32_t words[8] = {};
-            unsigned long long np = 0;
             if (!inner()) {
                 if ((r = run_steps(b)) != RGR_OK) return r;
             } else {
@@ -510,17 +555,27 @@ struct rgr_context {
             }
             *ran += b;
             if (!inner() || last) {
-                RGR_CUDA(cudaMemcpyAsync(words, counts.p, 32, cudaMemcpyDeviceToHost, stream));
-                RGR_CUDA(cudaMemcpyAsync(&np, scalars.p, 8, cudaMemcpyDeviceToHost, stream));
-                RGR_CUDA(cudaStreamSynchronize(stream));
+                RGR_CUDA(cudaMemcpyAsync(mail->counts, counts.p, 32, cudaMemcpyDeviceToHost, stream));
+                RGR_CUDA(cudaMemcpyAsync(&mail->next_pixel, scalars.p, 8, cudaMemcpyDeviceToHost, stream));
+                if ((r = wait()) != RGR_OK) return r;
                 uint64_t live = 0;
-                for (int k = 1; k < kNumQueues; ++k) live += words[k];
-                *over = np >= rp.sample_limit && live == 0;
+                for (int k = 1; k < kNumQueues; ++k) live += mail->counts[k];
+                *over = mail->next_pixel >= rp.sample_limit && live == 0;
             } else {
-                RGR_CUDA(cudaMemcpyAsync(words, in.words + InnerView::kStop, 4, cudaMemcpyDeviceToHost, stream));
-                RGR_CUDA(cudaStreamSynchronize(stream));
-                *over = words[0] != 0u;
+                RGR_CUDA(cudaMemcpyAsync(&mail->stop, in.words + InnerView::kStop, 4, cudaMemcpyDeviceToHost, stream));
+                if ((r = wait()) != RGR_OK) return r;
+                *over = mail->stop != 0u;
             }
+        }
+        return RGR_OK;
+    }
+    // waits for the stream; reports what the render's capacity checks found
+    int wait() {
+        if (begun) RGR_CUDA(cudaMemcpyAsync(&mail->err, err.p, 4, cudaMemcpyDeviceToHost, stream));
+        RGR_CUDA(cudaStreamSynchronize(stream));
+        if (begun && mail->err) {
+            set_error("device capacity check fired (flags " + std::to_string(mail->err) + ")");
+            return RGR_E_OVERFLOW;
         }
         return RGR_OK;
     }
@@ -607,7 +662,8 @@ int rgr_context_create(rgr_context** out, int32_t device, uint32_t path_count) {
     if (!c) return RGR_E_OOM;
     c->device = device;
     if (!cuda_ok(cudaSetDevice(device), "cudaSetDevice") ||
-        !cuda_ok(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "cudaStreamCreate")) {
+        !cuda_ok(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "cudaStreamCreate") ||
+        !(c->mail = take_mail())) {
         delete c;
         return RGR_E_CUDA;
     }
@@ -630,7 +686,7 @@ void rgr_context_destroy(rgr_context* c) {
 
 int rgr_set_graph_mode(rgr_context* c, int32_t enabled) {
     if (!c) return RGR_E_INVALID;
-    c->graph_mode = enabled != 0;
+    c->graph_mode = enabled != 0 ? 1 : 0;
     c->drop_graph();
     return RGR_OK;
 }
@@ -666,7 +722,6 @@ int rgr_render_begin(rgr_context* c, const rgr_camera* cam, const rgr_render_con
     if ((r = c->accum.alloc(32 * (size_t)c->npix)) != RGR_OK) return r;
     if ((r = c->done.alloc(16)) != RGR_OK) return r;
     RGR_CUDA(cudaMemsetAsync(c->accum.p, 0, 32 * (size_t)c->npix, c->stream));
-    RGR_CUDA(cudaMemsetAsync(c->done.p, 0, 16, c->stream));
     const unsigned long long limit = k.spp ? (unsigned long long)k.spp * c->npix : 0ull;
     // no completion counter: nothing reads a single render's completion time, and
     // the counter cost every warp of the logic kernel an atomic on one address
@@ -705,16 +760,7 @@ int rgr_render_step(rgr_context* c, int32_t steps) {
 int rgr_synchronize(rgr_context* c) {
     if (!c) return RGR_E_INVALID;
     RGR_CUDA(cudaSetDevice(c->device));
-    RGR_CUDA(cudaStreamSynchronize(c->stream));
-    uint32_t err = 0;
-    if (c->begun) {
-        RGR_CUDA(cudaMemcpy(&err, c->err.p, 4, cudaMemcpyDeviceToHost));
-        if (err) {
-            set_error("device capacity check fired (flags " + std::to_string(err) + ")");
-            return RGR_E_OVERFLOW;
-        }
-    }
-    return RGR_OK;
+    return c->wait();
 }
 
 int rgr_render_until_done(rgr_context* c, int32_t max_steps, int32_t* steps_done) {
@@ -727,7 +773,7 @@ int rgr_render_until_done(rgr_context* c, int32_t max_steps, int32_t* steps_done
     int r = c->run_until_done(8, max_steps, &done, &over);
     if (r != RGR_OK) return r;
     if (steps_done) *steps_done = done;
-    return rgr_synchronize(c);
+    return done ? RGR_OK : c->wait();  // each group of bounces ends with a wait
 }
 
 namespace {
@@ -1071,15 +1117,14 @@ int rgr_trace_closest(rgr_context* c, const rgr_ray_soa* rays, uint64_t n, int32
         if (direct && dprim && dt) {
             rgr_context::TraceSlot& ts = c->tslot[0];
             if ((r = ts.counter.alloc(8)) != RGR_OK) return r;
-            if (!c->link_err) RGR_CUDA(cudaMallocHost(&c->link_err, sizeof(uint32_t)));
-            *c->link_err = 0u;
+            c->mail->link_err = 0u;
             cudaStream_t st = c->stream;
-            launch_trace_rays_link(c->scene.sv, dsrc, n, dprim, dt, c->link_err, ts.counter.as<unsigned long long>(),
+            launch_trace_rays_link(c->scene.sv, dsrc, n, dprim, dt, &c->mail->link_err, ts.counter.as<unsigned long long>(),
                                    c->trace_refill, c->trace_search, c->trace_grid, st);
             RGR_CUDA(cudaGetLastError());
             populate({prim, t}, 4 * n);
             RGR_CUDA(cudaStreamSynchronize(st));
-            if (*c->link_err) {
+            if (c->mail->link_err) {
                 set_error("traversal stack overflow");
                 return RGR_E_OVERFLOW;
             }
@@ -1262,7 +1307,7 @@ int rgr_batch_run(rgr_batch* b, int32_t order_policy, int32_t steps_per_launch, 
     if (r != RGR_OK) return r;
     if ((r = c->done.alloc(16 * (size_t)n)) != RGR_OK) return r;
     if ((r = b->stamp.alloc(8)) != RGR_OK) return r;
-    RGR_CUDA(cudaMemsetAsync(c->done.p, 0, 16 * (size_t)n, st));
+    if (n > 1) RGR_CUDA(cudaMemsetAsync(c->done.p, 0, 16 * (size_t)n, st));
     std::vector<RequestD> table(n);
     unsigned long long begin = 0;
     for (int k = 0; k < n; ++k) {

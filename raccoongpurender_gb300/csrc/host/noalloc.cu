@@ -181,13 +181,9 @@ extern "C" int rgr_render_noalloc(rgr_context* c, const rgr_camera* cam, const r
     rp.rays = scal + 2;
 
     // the array keeps the previous call's contents: reset counters and output
-    if (!ok(cudaMemsetAsync(base + kOffCounts, 0, 256, st), "cudaMemsetAsync") ||
-        !ok(cudaMemsetAsync(base + kOffScalars, 0, 256, st), "cudaMemsetAsync") ||
-        !ok(cudaMemsetAsync(base + kOffErr, 0, 256, st), "cudaMemsetAsync") ||
-        !ok(cudaMemsetAsync(accum_out, 0, sizeof(double) * 4 * (size_t)npix, st), "cudaMemsetAsync") ||
-        !ok(cudaMemcpyAsync(base + kOffRequest, &rq, sizeof(rq), cudaMemcpyHostToDevice, st), "cudaMemcpyAsync"))
-        return RGR_E_CUDA;
-    launch_init(p, q, k.seed_offset, st);
+    if (!ok(cudaMemsetAsync(accum_out, 0, sizeof(double) * 4 * (size_t)npix, st), "cudaMemsetAsync")) return RGR_E_CUDA;
+    launch_init(p, q, k.seed_offset, InitView{scal, rp.err, nullptr, reinterpret_cast<RequestD*>(base + kOffRequest)}, rq,
+                st);
     if (!ok(cudaGetLastError(), "kernel launch")) return RGR_E_CUDA;
     const TraceShape ts{true, 24, 8,
                         sms * (trace_paths_max_blocks_per_sm() > 0 ? trace_paths_max_blocks_per_sm() : 1), scal + 3};

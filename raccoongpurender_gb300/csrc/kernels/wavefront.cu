@@ -693,8 +693,18 @@ RGR_DEV void shade_slot(const RequestD& rq, const PathsView& P, int k, uint32_t 
 }
 
 // ------------------------------------------------------------ kernels
-__global__ void k_init(PathsView P, QueueView Q, uint32_t seed_offset) {
+// The pool of a new render: its counters, error word and, of a render of one request
+// (table set), the request table.  (As three memsets, a copy and a wait for it they were
+// 25 of the 43 us that a render of 65,536 pixels took to begin.)
+__global__ void k_init(PathsView P, QueueView Q, uint32_t seed_offset, InitView w, RequestD one) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 8u) {
+        Q.counts[i] = Q.taken[i] = 0u;
+        w.scalars[i] = 0ull;
+        if (i < 4u) w.err[i] = 0u;
+        if (i < 2u && w.done) w.done[i] = 0ull;
+        if (i == 0u && w.table) *w.table = one;
+    }
     if (i < Q.ntiles) {
         uint32_t beg = i * kTile;
         Q.tile_new[i] = min(kTile, P.n - beg);
@@ -1745,9 +1755,10 @@ static void chain(void (*kernel)(P...), unsigned grid, unsigned block, cudaStrea
     cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
-void launch_init(const PathsView& p, const QueueView& q, uint32_t seed_offset, cudaStream_t st) {
+void launch_init(const PathsView& p, const QueueView& q, uint32_t seed_offset, const InitView& w, const RequestD& one,
+                 cudaStream_t st) {
     uint32_t n = q.ntiles * kTile;
-    k_init<<<(n + 255) / 256, 256, 0, st>>>(p, q, seed_offset);
+    k_init<<<(n + 255) / 256, 256, 0, st>>>(p, q, seed_offset, w, one);
 }
 void launch_compact_new(const PathsView& p, const QueueView& q, unsigned long long* cast_counter, cudaStream_t st) {
     chain(k_compact_new, q.ntiles, 256, st, p, q, cast_counter);

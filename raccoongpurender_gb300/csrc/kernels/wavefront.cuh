@@ -247,7 +247,15 @@ struct RenderParams {
 };
 
 // launchers (wavefront.cu)
-void launch_init(const PathsView& p, const QueueView& q, uint32_t seed_offset, cudaStream_t st);
+// cleared with the pool: a render's words, beside the 8 each of QueueView's counts and taken
+struct InitView {
+    unsigned long long* scalars;  // 8: next pixel, step base, rays cast, the cast's counter
+    uint32_t* err;                // 4
+    unsigned long long* done;     // 2, or null
+    RequestD* table;              // gets the one request, or null
+};
+void launch_init(const PathsView& p, const QueueView& q, uint32_t seed_offset, const InitView& w, const RequestD& one,
+                 cudaStream_t st);
 // starts a bounce; cast_counter: the cast's (TraceShape::counter)
 void launch_compact_new(const PathsView& p, const QueueView& q, unsigned long long* cast_counter, cudaStream_t st);
 void launch_shade(const PathsView& p, const QueueView& q, const RenderParams& rp, int grid, cudaStream_t st);
