@@ -239,8 +239,9 @@ int rgr_render_restore(rgr_context* c, const void* src, uint64_t src_bytes);
 /* merge_from (:963-991): add src's accumulation into dst (replicas on several GPUs) */
 int rgr_accum_merge(rgr_context* dst, rgr_context* src);
 int rgr_synchronize(rgr_context* c);
-/* capture the bounce loop in a CUDA graph (1) or launch stage by stage (0); by default guided
-   renders replay a graph and plain ones, whose launches overlap, do not.  Results are identical. */
+/* capture the bounce loop in a CUDA graph (1) or launch stage by stage (0); by default
+   renders that train a guide replay a graph and others, whose launches overlap, do not.
+   Results are identical. */
 int rgr_set_graph_mode(rgr_context* c, int32_t enabled);
 
 /* merge_intermediate (accumlation.cl:27-49): a <- count-weighted merge of two

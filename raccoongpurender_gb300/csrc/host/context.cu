@@ -216,7 +216,7 @@ void give_mail(Mail* m) {  // its context's stream is idle
 
 // Pools of fewer paths run the fused trace + logic kernel by default (a bounce is then
 // bound by its launches' latency and the longest ray of each warp), larger ones the
-// persistent refilling cast and, inside a run of bounces, no logic pass (launch_inner).
+// persistent refilling cast and, inside a run of bounces, no logic pass (launch_inner_queues).
 // Whole renders (4 spp, depth 6), persistent against fused, at 2^17 / 2^18 / 2^19 / 2^20 /
 // 2^22 paths: 36 triangles 0.84 / 0.98 / 1.12 / 1.24 / 1.36x, 5 K 0.80 / 1.00 / 1.17 / 1.39 /
 // 1.69x, 330 K 0.84 / 0.99 / 1.25 / 1.52 / 2.06x.  Single bounces at 2^18 / 2^20 / 2^22:
@@ -241,7 +241,7 @@ struct rgr_context {
     DeviceScene scene;
     // paths
     DevBuf slots, qid, req, queues[kNumQueues], counts, tile_new, scalars, accum, err;
-    DevBuf inner_words, inner_tiles, inner_ended;  // the bounces inside a run (launch_inner)
+    DevBuf inner_words, inner_tiles, inner_ended;  // the bounces inside a run (launch_inner_queues)
     InnerView in{};
     Mail* mail = nullptr;
     DevBuf reqtab, done;  // request table and its per-request (done, done_ns) counters
@@ -265,7 +265,7 @@ struct rgr_context {
         cudaGraphExec_t exec = nullptr;
         std::string key;  // graph_key() when it was captured
     };
-    Graph step_graph, inner_graph;  // whole bounces; bounces inside a run (launch_inner)
+    Graph step_graph, inner_graph;  // whole bounces; bounces inside a run (launch_inner_queues)
     // ray-cast service buffers
     DevBuf trays[7], tprim, tt, tread, tcounter;
     // rgr_trace_closest pipeline: kTraceSlots stream slots, each with its chunk's buffers
@@ -372,11 +372,15 @@ struct rgr_context {
         single_render = false;
         return RGR_OK;
     }
+    // the mixtures of a guided bounce's items
+    void infer(const QueueView& q, bool inside, cudaStream_t st) {
+        if (rp.gd.max_depth) launch_guide_select(pv, q, rp.gd, inside, shade_grid, st);
+        guide->infer_paths(pv, q, rp.gd, inside ? rp.reqs : nullptr, st);
+    }
     // train_now: a guided render ends a training interval with this bounce
     int step_launches(cudaStream_t st, bool train_now = true) {
         launch_compact_new(pv, qv, render_trace.counter, st);
-        if (guided && rp.gd.max_depth) launch_guide_select(pv, qv, rp.gd, shade_grid, st);
-        if (guided) guide->infer_paths(pv, qv, rp.gd, st);
+        if (guided) infer(qv, false, st);
         launch_shade(pv, qv, rp, shade_grid, st);
         launch_trace_paths(pv, qv, rp, render_trace, st);
         launch_trace_logic(pv, qv, rp, render_trace, num_sms, st);
@@ -459,14 +463,15 @@ struct rgr_context {
         RGR_CUDA(cudaGraphLaunch(g.exec, st));
         return RGR_OK;
     }
-    // run `n` bounces.  A plain render takes the bounces inside the run by
-    // launch_inner; otherwise replays of a graph of graph_steps bounces, then
+    // run `n` bounces.  A render that records nothing takes the bounces inside the run by
+    // run_bounce; otherwise replays of a graph of graph_steps bounces, then
     // single ones
     int run_steps(int n) {
         if (n > 1 && inner()) {
             int r = run_first();
             if (r == RGR_OK) r = run_inner(n - 1);
             if (r == RGR_OK) r = run_last();
+            if (r == RGR_OK) r = run_trained(n);
             if (r == RGR_OK) steps += n;
             return r;
         }
@@ -490,29 +495,39 @@ struct rgr_context {
         }
         return RGR_OK;
     }
-    // Plain bounces are launched one by one by default: their launches overlap (follow), which
+    // Bounces are launched one by one by default: their launches overlap (follow), which
     // a replay ends with, and a render's first pass need not capture.  A preview frame of 12 bounces
     // 2708 us replayed, 2671 launched, a 65,536-pixel render 558 and 548 (its first 4300
-    // and 2613); a guided render, of more launches a bounce, 6929 and 6974.
-    bool graphs() const { return graph_mode < 0 ? guided : graph_mode != 0; }
+    // and 2613), a guided one with a frozen guide 6299 and 6314 (its first 8752 and 7199); where the
+    // guide trains, with more launches a bounce, a replay is the faster.
+    bool graphs() const { return graph_mode < 0 ? guided && !inner() : graph_mode != 0; }
     // the first bounce of a run up to its rays' cast
-    bool inner() const { return !guided && render_trace.persistent; }
+    bool inner() const {
+        return render_trace.persistent && (!guided || (!rp.gd.record && guide->frozen()));
+    }
     int run_first() {
         cudaStream_t st = stream;
         launch_compact_new(pv, qv, render_trace.counter, st);
+        if (guided) infer(qv, false, st);
         launch_shade(pv, qv, rp, shade_grid, st);
         launch_inner_cast(pv, qv, rp, render_trace, st);
         launch_inner_reset(in, st);
         RGR_CUDA(cudaGetLastError());
         return RGR_OK;
     }
+    // a bounce inside the run
+    int run_bounce(bool boundary) {
+        launch_inner_queues(pv, qv, in, rp, render_trace, boundary, num_sms, stream);
+        QueueView u = qv;
+        u.taken = in.words;
+        if (guided) infer(u, true, stream);
+        launch_inner_shade(pv, u, rp, render_trace, shade_grid, stream);
+        RGR_CUDA(cudaGetLastError());
+        return RGR_OK;
+    }
     // `n` bounces inside the run
     int run_inner(int n) {
-        auto one = [&]() -> int {
-            launch_inner(pv, qv, in, rp, render_trace, false, shade_grid, num_sms, stream);
-            RGR_CUDA(cudaGetLastError());
-            return RGR_OK;
-        };
+        auto one = [&] { return run_bounce(false); };
         int r = RGR_OK;
         for (; graphs() && n >= graph_steps && r == RGR_OK; n -= graph_steps)
             r = replay(inner_graph, [&] {
@@ -531,6 +546,12 @@ struct rgr_context {
         RGR_CUDA(cudaGetLastError());
         return RGR_OK;
     }
+    // `b` bounces with a frozen guide: the end of their training intervals is bookkeeping that nothing
+    // between them reads and that leaves the same however often it is done
+    int run_trained(int b) {
+        const uint64_t ti = (uint64_t)train_interval();
+        return guided && (steps + b) / ti > steps / ti ? guide->train_launches(stream) : RGR_OK;
+    }
     // Bounces until the render is over (every path ended and the sample budget handed
     // out), looked at after every `group` bounces, at most max_steps; `*ran`: how many.
     int run_until_done(int group, int max_steps, int* ran, bool* over) {
@@ -548,9 +569,9 @@ struct rgr_context {
                 if (last) {
                     if ((r = run_last()) != RGR_OK) return r;
                 } else {
-                    launch_inner(pv, qv, in, rp, render_trace, true, shade_grid, num_sms, stream);
-                    RGR_CUDA(cudaGetLastError());
+                    if ((r = run_bounce(true)) != RGR_OK) return r;
                 }
+                if ((r = run_trained(b)) != RGR_OK) return r;
                 steps += b;
             }
             *ran += b;

@@ -151,9 +151,10 @@ int rgr_guide::set_bounds(const float lo[3], const float hi[3]) {
 
 uint32_t* rgr_guide::error_word() const { return reinterpret_cast<uint32_t*>(counters.as<unsigned char>() + kCtrErr); }
 
-void rgr_guide::infer_paths(const PathsView& p, const QueueView& q, const GuideRenderD& gd, cudaStream_t st) {
+void rgr_guide::infer_paths(const PathsView& p, const QueueView& q, const GuideRenderD& gd, const RequestD* inner,
+                            cudaStream_t st) {
     if (cfg.inference_kernel == RGR_GUIDE_TCGEN05)
-        launch_guide_infer_paths_tc(view, p, q, gd, guide_tc_grid(num_sms), error_word(), st);
+        launch_guide_infer_paths_tc(view, p, q, gd, inner, guide_tc_grid(num_sms), error_word(), st);
     else
         launch_guide_infer_paths(view, p, q, gd, guide_infer_grid(num_sms), st);
 }

@@ -22,8 +22,11 @@ struct rgr_guide {
     int init(const rgr_guide_config& c);
     int set_bounds(const float lo[3], const float hi[3]);
     // the bounce's inference launch (tcgen05 or mma.sync kernel, per cfg)
+    // inner: the render's request, for a bounce inside a run (launch_inner_queues); else null
     void infer_paths(const rgr::dev::PathsView& p, const rgr::dev::QueueView& q, const rgr::dev::GuideRenderD& gd,
-                     cudaStream_t st);
+                     const rgr::dev::RequestD* inner, cudaStream_t st);
+    // renders with the weights as they are: such a render's bounces need no logic pass of their own
+    bool frozen() const { return !cfg.train && cfg.inference_kernel == RGR_GUIDE_TCGEN05; }
     uint32_t* error_word() const;
     // the launches that follow the trace/logic kernel of a guided render on the
     // bounces that end a training interval: train, Adam, reset the stream

@@ -360,7 +360,7 @@ int guide_tc_grid(int num_sms);
 void launch_guide_infer_tc(const GuideView& g, const float* rows, uint32_t n, float* out, int grid, uint32_t* err,
                            cudaStream_t st);
 void launch_guide_infer_paths_tc(const GuideView& g, const PathsView& p, const QueueView& q, const GuideRenderD& gd,
-                                 int grid, uint32_t* err, cudaStream_t st);
+                                 const RequestD* inner, int grid, uint32_t* err, cudaStream_t st);
 
 }  // namespace dev
 }  // namespace rgr

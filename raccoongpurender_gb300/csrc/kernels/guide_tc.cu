@@ -40,6 +40,7 @@
 #include <cuda_bf16.h>
 
 #include "guide.cuh"
+#include "traverse.cuh"
 
 namespace rgr {
 namespace dev {
@@ -353,8 +354,20 @@ __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefe
 struct RowIn {
     float4 a, b, c;
 };
-template <bool kPaths>
-__device__ __forceinline__ RowIn load_row(const PathsView& P, const float* rows, uint32_t r, uint32_t slot) {
+// kInner: inside a run the record still holds the hit as the cast left it (resolve_hit); a
+// volume vertex has no surface.
+template <bool kPaths, bool kInner>
+__device__ __forceinline__ RowIn load_row(const PathsView& P, const float* rows, uint32_t r, uint32_t slot,
+                                          const RequestD* inner) {
+    if (kInner) {
+        RowIn in;
+        ld_sector<0>(P, slot, in.a, in.b);
+        in.c = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
+        int32_t hv = __float_as_int(in.b.w), hs = -1;
+        int mtype;
+        resolve_hit(inner->sc, in.a, in.b, hv, hs, in.c, mtype);
+        return in;
+    }
     if (kPaths) return RowIn{P.ro[slot], P.rd[slot], P.ng[slot]};
     const float4* p = reinterpret_cast<const float4*>(rows + 16 * (size_t)r);
     return RowIn{p[0], p[1], p[2]};
@@ -406,10 +419,10 @@ __device__ __forceinline__ void issue_layer(uint32_t l, uint32_t tm, uint32_t ta
 // otherwise rows of 16 floats in `rows`, output 40 raw floats per row.
 //
 // Tile k of group g is tile (blockIdx.x + k gridDim.x) kTcGroups + g of the rows.
-template <bool kPaths>
+template <bool kPaths, bool kInner>
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_guide_infer_tc(GuideView gv, const float* __restrict__ rows, uint32_t nrows, float* __restrict__ out,
-                     PathsView P, QueueView Q, GuideRenderD gd, uint32_t* err) {
+                     PathsView P, QueueView Q, GuideRenderD gd, const RequestD* inner, uint32_t* err) {
     extern __shared__ unsigned char smem_raw[];
     SmemTc& S = *reinterpret_cast<SmemTc*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t n = kPaths ? guide_rows(Q, gd) : nrows;
@@ -456,7 +469,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     RowIn in = {};
     if (warp < (uint32_t)kMmaWarp) {
         const uint32_t r = (blockIdx.x * kTcGroups + g) * 128u + lt;
-        if (r < n) in = load_row<kPaths>(P, rows, r, kPaths ? guide_row_slot(Q, gd, r) : 0u);
+        if (r < n) in = load_row<kPaths, kInner>(P, rows, r, kPaths ? guide_row_slot(Q, gd, r) : 0u, inner);
     }
     fence_before();
     __syncthreads();
@@ -565,7 +578,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 arrive(af);
             }
             if (!timed_out && more) {  // while the last layer runs
-                if (rn < n) in = load_row<kPaths>(P, rows, rn, next_slot);
+                if (rn < n) in = load_row<kPaths, kInner>(P, rows, rn, next_slot, inner);
                 encode(rn);
             }
             if (timed_out || !mbar_wait_warp(df, pd)) {  // after one timeout, no more waits
@@ -627,11 +640,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 size_t guide_tc_smem() { return sizeof(SmemTc) + 1024; }
 
 int guide_tc_attributes() {
-    cudaError_t e = cudaFuncSetAttribute(k_guide_infer_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)guide_tc_smem());
+    const int bytes = (int)guide_tc_smem();
+    cudaError_t e = cudaFuncSetAttribute(k_guide_infer_tc<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_guide_infer_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)guide_tc_smem());
+        e = cudaFuncSetAttribute(k_guide_infer_tc<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_guide_infer_tc<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     return (int)e;
 }
 
@@ -644,13 +658,18 @@ void launch_guide_infer_tc(const GuideView& g, const float* rows, uint32_t n, fl
     if (n == 0) return;
     const uint32_t need = (n + kCtaRows - 1u) / kCtaRows;
     if ((uint32_t)grid > need) grid = (int)need;
-    k_guide_infer_tc<false><<<grid, kTcThreads, guide_tc_smem(), st>>>(g, rows, n, out, PathsView{}, QueueView{},
-                                                                      GuideRenderD{}, err);
+    k_guide_infer_tc<false, false>
+        <<<grid, kTcThreads, guide_tc_smem(), st>>>(g, rows, n, out, PathsView{}, QueueView{}, GuideRenderD{}, nullptr, err);
 }
 
 void launch_guide_infer_paths_tc(const GuideView& g, const PathsView& p, const QueueView& q, const GuideRenderD& gd,
-                                 int grid, uint32_t* err, cudaStream_t st) {
-    k_guide_infer_tc<true><<<grid, kTcThreads, guide_tc_smem(), st>>>(g, nullptr, 0, nullptr, p, q, gd, err);
+                                 const RequestD* inner, int grid, uint32_t* err, cudaStream_t st) {
+    if (inner)
+        k_guide_infer_tc<true, true>
+            <<<grid, kTcThreads, guide_tc_smem(), st>>>(g, nullptr, 0, nullptr, p, q, gd, inner, err);
+    else
+        k_guide_infer_tc<true, false>
+            <<<grid, kTcThreads, guide_tc_smem(), st>>>(g, nullptr, 0, nullptr, p, q, gd, nullptr, err);
 }
 
 }  // namespace dev

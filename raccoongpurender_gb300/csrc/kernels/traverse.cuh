@@ -393,5 +393,22 @@ RGR_DEV f3 hit_normal(const SceneView& sc, int32_t prim, f3 ro, f3 rd, float t) 
     return normalize((ro + rd * t) - xyz(s));
 }
 
+// The hit that k_trace_paths left in a slot's ray sector (primitive -2 - hv):
+// its surface, normal and, where the per-triangle table gives it, material type
+// (else mtype stays -1).
+RGR_DEV void resolve_hit(const SceneView& sc, const float4& ro4, const float4& rd4, int32_t& hv, int32_t& hs,
+                         float4& ng4, int& mtype) {
+    if (hv > -2) return;
+    hs = -2 - hv;
+    hv = -1;
+    if (sc.tri_normals && hs < sc.sphere_begin) {
+        const float4 tn = __ldg(sc.tri_normals + hs);
+        ng4 = f4(xyz(tn), __int_as_float(hs));
+        mtype = __float_as_int(tn.w);
+    } else {
+        ng4 = f4(hit_normal(sc, hs, xyz(ro4), xyz(rd4), ro4.w), __int_as_float(hs));
+    }
+}
+
 }  // namespace dev
 }  // namespace rgr

@@ -19,7 +19,7 @@
 // Inside a run of several bounces the logic is not a pass of its own: the cast
 // finds where each path goes next, k_classify builds the queues from a byte per
 // slot, k_new_paths finishes the ended paths and starts the new ones, k_shade_inner
-// does the logic's share of the others (launch_inner in wavefront.cuh).  At 2^24 paths of
+// does the logic's share of the others (launch_inner_queues in wavefront.cuh).  At 2^24 paths of
 // the mixed 1080p render a bounce was 1.15 ms shading, 2.25 cast and 1.15 logic; it is
 // 0.06 classification, 0.48 new paths, 0.81 shading and 2.3 cast: 91.5 to 73.3 ms.
 // Every slot's arithmetic is the reference kernels' arithmetic (see the
@@ -586,23 +586,6 @@ RGR_DEV bool shade_state(const RequestD& rq, int k, uint32_t slot, unsigned long
     return touch_L;
 }
 
-// The hit that k_trace_paths left in a slot's ray sector (primitive -2 - hv):
-// its surface, normal and, where the per-triangle table gives it, material type
-// (else mtype stays -1).
-RGR_DEV void resolve_hit(const SceneView& sc, const float4& ro4, const float4& rd4, int32_t& hv, int32_t& hs,
-                         float4& ng4, int& mtype) {
-    if (hv > -2) return;
-    hs = -2 - hv;
-    hv = -1;
-    if (sc.tri_normals && hs < sc.sphere_begin) {
-        const float4 tn = __ldg(sc.tri_normals + hs);
-        ng4 = f4(xyz(tn), __int_as_float(hs));
-        mtype = __float_as_int(tn.w);
-    } else {
-        ng4 = f4(hit_normal(sc, hs, xyz(ro4), xyz(rd4), ro4.w), __int_as_float(hs));
-    }
-}
-
 // What the logic does to a path that goes on (logic.cl:27-190): the Russian
 // roulette's draw and T / cp (exactly T where the roulette is off: cp is 1).
 RGR_DEV void logic_advance(const RequestD& rq, uint32_t logic_i, f3& T, Rng& rng) {
@@ -895,7 +878,9 @@ __global__ void __launch_bounds__(256, RGR_SHADE_MIN_BLOCKS) k_shade(PathsView P
     shade_items<false>(P, Q, rp);
 }
 // the material queues of a bounce inside a run (k_new_paths has taken the new paths)
-__global__ void __launch_bounds__(256, RGR_SHADE_MIN_BLOCKS) k_shade_inner(PathsView P, QueueView Q, RenderParams rp) {
+template <bool kGuided>
+__global__ void __launch_bounds__(256, kGuided ? RGR_SHADE_GUIDED_MIN_BLOCKS : RGR_SHADE_MIN_BLOCKS)
+    k_shade_inner(PathsView P, QueueView Q, RenderParams rp) {
     follow();
     // the ended paths of the bounce before are finished and counted
     if (blockIdx.x == 0) stamp_done(rp, (int)threadIdx.x, (int)blockDim.x);
@@ -904,13 +889,24 @@ __global__ void __launch_bounds__(256, RGR_SHADE_MIN_BLOCKS) k_shade_inner(Paths
 #pragma unroll
     for (int k = 1; k < kNumQueues; ++k) off[k] = off[k - 1] + Q.taken[k];
     const uint32_t total = off[kNumQueues - 1];
+    // guided items are numbered as in shade_items
+    const uint32_t g4 = off[kMatLambertian] - off[kMatLambertian - 1];
+    const uint32_t g6 = g4 + (off[kMatWard] - off[kMatWard - 1]);
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         int k = 1;
 #pragma unroll
         for (int j = 1; j < kNumQueues - 1; ++j) k += (i >= off[j]) ? 1 : 0;
         const uint32_t slot = queue_items(Q, k)[i - pick(off, k - 1)];
-        shade_slot<false, true>(rp.reqs[P.req[slot]], P, k, slot, 0ull, rp.gd, ~0u);
+        uint32_t gi = ~0u;
+        if (kGuided) {
+            const uint32_t o = i - pick(off, k - 1);  // its place in the queue
+            if (k == kMatLambertian) gi = o;
+            else if (k == kMatWard) gi = g4 + o;
+            else if (k == kMatVolumeInside && rp.gd.volumes) gi = g6 + o;
+            if (gi != ~0u && rp.gd.max_depth) gi = rp.gd.remap[gi];  // its inference row, or unguided
+        }
+        shade_slot<kGuided, true>(rp.reqs[P.req[slot]], P, k, slot, 0ull, rp.gd, gi);
     }
 }
 __global__ void __launch_bounds__(256, RGR_SHADE_GUIDED_MIN_BLOCKS) k_shade_guided(PathsView P, QueueView Q,
@@ -923,8 +919,9 @@ __global__ void __launch_bounds__(256, RGR_SHADE_GUIDED_MIN_BLOCKS) k_shade_guid
 // max_depth of its path (logic_i counts the path's segments so far) become
 // the inference rows, appended with one atomic per warp; the others keep
 // BSDF and envmap sampling.  The row order does not matter: a row's mixture
-// depends on that row alone.
-__global__ void __launch_bounds__(256) k_guide_select(PathsView P, QueueView Q, GuideRenderD gd) {
+// depends on that row alone.  ahead: 1 inside a run, whose logic has not counted the last
+// segment yet.
+__global__ void __launch_bounds__(256) k_guide_select(PathsView P, QueueView Q, GuideRenderD gd, uint32_t ahead) {
     const uint32_t n = guided_items(Q, gd);
     const int lane = threadIdx.x & 31;
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -934,7 +931,7 @@ __global__ void __launch_bounds__(256) k_guide_select(PathsView P, QueueView Q, 
         bool take = false;
         if (gi < n) {
             slot = guided_item_slot(Q, gi);
-            take = depth_of(__float_as_uint(P.L[slot].w)) <= gd.max_depth;
+            take = depth_of(__float_as_uint(P.L[slot].w)) + ahead <= gd.max_depth;
         }
         const unsigned m = __ballot_sync(0xffffffffu, take);
         uint32_t first = 0;
@@ -1029,7 +1026,7 @@ RGR_DEV float guide_write(const GuideRenderD& gd, uint32_t slot, const GuideOffe
 // field P.rd.w (its readers take a negative id as none); the logic kernel computes
 // Ng into P.ng.  A miss leaves P.ng.w at the -1 the shading stage wrote.  Each slot may belong
 // to another request (scene).
-// kInner: a bounce inside a run (launch_inner).  The cast also decides where the path
+// kInner: a bounce inside a run (launch_inner_queues).  The cast also decides where the path
 // goes next and writes it as the slot's queue id: what ends a path whatever its ray
 // meets (logic_ends) is found as the ray is taken, from the sector beside the
 // ray's in the same line, and kept in the slot word's top bit (slots are below 2^28).
@@ -1551,7 +1548,7 @@ __global__ void __launch_bounds__(256) k_classify(PathsView P, QueueView Q, Inne
 // for the cast.
 // Bound by the records' DRAM traffic (a 128-byte line read, 96 bytes written per slot)
 // and, where paths leave the scene, the envmap look-up's arithmetic.
-// When the render is over (launch_inner's boundary) the paths are only finished.
+// When the render is over (launch_inner_queues' boundary) the paths are only finished.
 constexpr int kNewPathsBlocks = 8;  // per SM
 __global__ void __launch_bounds__(256) k_new_paths(PathsView P, QueueView Q, InnerView I, RenderParams rp) {
     follow();
@@ -1763,9 +1760,10 @@ void launch_init(const PathsView& p, const QueueView& q, uint32_t seed_offset, c
 void launch_compact_new(const PathsView& p, const QueueView& q, unsigned long long* cast_counter, cudaStream_t st) {
     chain(k_compact_new, q.ntiles, 256, st, p, q, cast_counter);
 }
-void launch_guide_select(const PathsView& p, const QueueView& q, const GuideRenderD& gd, int grid, cudaStream_t st) {
+void launch_guide_select(const PathsView& p, const QueueView& q, const GuideRenderD& gd, bool inner, int grid,
+                         cudaStream_t st) {
     cudaMemsetAsync(gd.nsel, 0, sizeof(uint32_t), st);
-    k_guide_select<<<grid, 256, 0, st>>>(p, q, gd);
+    k_guide_select<<<grid, 256, 0, st>>>(p, q, gd, inner ? 1u : 0u);
 }
 
 void launch_shade(const PathsView& p, const QueueView& q, const RenderParams& rp, int grid, cudaStream_t st) {
@@ -1825,14 +1823,19 @@ void launch_inner_cast(const PathsView& p, const QueueView& q, const RenderParam
     cast_paths<true>(p, q, rp, ts, st);
 }
 
-void launch_inner(const PathsView& p, const QueueView& q, const InnerView& in, const RenderParams& rp,
-                  const TraceShape& ts, bool boundary, int shade_grid, int num_sms, cudaStream_t st) {
+void launch_inner_queues(const PathsView& p, const QueueView& q, const InnerView& in, const RenderParams& rp,
+                         const TraceShape& ts, bool boundary, int num_sms, cudaStream_t st) {
     chain(k_classify, q.ntiles, 256, st, p, q, in, rp, ts.counter, boundary ? 1 : 0);
     const int blocks = std::min((int)((p.n + 255) / 256), num_sms * kNewPathsBlocks);
     chain(k_new_paths, blocks, 256, st, p, q, in, rp);
-    QueueView u = q;
-    u.taken = in.words;
-    chain(k_shade_inner, shade_grid, 256, st, p, u, rp);
+}
+
+void launch_inner_shade(const PathsView& p, const QueueView& u, const RenderParams& rp, const TraceShape& ts,
+                        int shade_grid, cudaStream_t st) {
+    if (rp.gd.lobes)
+        chain(k_shade_inner<true>, shade_grid, 256, st, p, u, rp);
+    else
+        chain(k_shade_inner<false>, shade_grid, 256, st, p, u, rp);
     cast_paths<true>(p, u, rp, ts, st);
 }
 

@@ -260,7 +260,8 @@ void launch_init(const PathsView& p, const QueueView& q, uint32_t seed_offset, c
 void launch_compact_new(const PathsView& p, const QueueView& q, unsigned long long* cast_counter, cudaStream_t st);
 void launch_shade(const PathsView& p, const QueueView& q, const RenderParams& rp, int grid, cudaStream_t st);
 // the guided items at vertices 1..gd.max_depth of their paths (gd.sel / remap / nsel; *nsel zeroed first)
-void launch_guide_select(const PathsView& p, const QueueView& q, const GuideRenderD& gd, int grid, cudaStream_t st);
+void launch_guide_select(const PathsView& p, const QueueView& q, const GuideRenderD& gd, bool inner, int grid,
+                         cudaStream_t st);
 // How a bounce casts its extension rays: persistent = a separate persistent
 // closest-hit kernel over the slots just shaded (warps refilled when `refill`
 // lanes are idle, node steps while `search` lanes still search for a leaf,
@@ -279,13 +280,14 @@ void launch_trace_paths(const PathsView& p, const QueueView& q, const RenderPara
                                cudaStream_t st);
 void launch_trace_logic(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
                         int num_sms, cudaStream_t st);
-// One bounce inside a run of several (plain renders).  Between two bounces of a
+// One bounce inside a run of several (plain renders, and guided ones that record nothing).  Between two bounces of a
 // run nobody looks at the state, so there is no logic pass over it: the cast decides
 // each path's next queue as its ray ends (the hit's material type is in the
 // primitive's record) and writes it as the slot's queue id, a byte; then
 //   1. k_classify builds the queues and the new-path counts from those bytes;
 //   2. k_new_paths finishes the paths that ended (logic, envmap, accumulation) and
 //      starts the new ones in their slots;
+//   (guided: the inference, over the hits as the cast left them)
 //   3. k_shade_inner shades the material queues, with the logic's share of a path
 //      that goes on first;
 //   4. the cast of the bounce's rays.
@@ -304,8 +306,12 @@ struct InnerView {
 void launch_inner_reset(const InnerView& in, cudaStream_t st);
 void launch_inner_cast(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
                        cudaStream_t st);
-void launch_inner(const PathsView& p, const QueueView& q, const InnerView& in, const RenderParams& rp,
-                  const TraceShape& ts, bool boundary, int shade_grid, int num_sms, cudaStream_t st);
+// 1 and 2
+void launch_inner_queues(const PathsView& p, const QueueView& q, const InnerView& in, const RenderParams& rp,
+                         const TraceShape& ts, bool boundary, int num_sms, cudaStream_t st);
+// 3 and 4; u: the queues with `taken` at InnerView::words
+void launch_inner_shade(const PathsView& p, const QueueView& u, const RenderParams& rp, const TraceShape& ts,
+                        int shade_grid, cudaStream_t st);
 int trace_paths_max_blocks_per_sm();
 // per-request completion stamps of a batch (after the logic kernel of a bounce)
 void launch_stamp_done(const RenderParams& rp, cudaStream_t st);
