@@ -1404,9 +1404,9 @@ __global__ void __launch_bounds__(kLogicThreads, kCastLogicBlocks)
 }
 
 // The queues of a bounce inside a run, from the queue ids that the cast left: block t
-// takes the tile [t*4096, (t+1)*4096), 16 consecutive slots a thread.  Counts per
-// class as 16-bit fields of two words (a tile's fit), scanned over the block; the
-// tile's slots go to shared memory in class order and from there to the queues, one
+// takes the tile [t*4096, (t+1)*4096), 8 consecutive slots a thread.  Counts per class as
+// 9-bit fields of one word (a warp's 256 fit) are scanned over the warp, then warp k
+// scans class k's over the warps; the tile's slots go to shared memory in class order and from there to the queues, one
 // atomic per queue per block: 16 MB of ids for 2^24 slots instead of a pass over
 // their records.  The ended paths' slots go to the tile's own stretch of I.ended, in
 // slot order.  The last block to finish scans the tiles' counts of them, so that
@@ -1414,71 +1414,78 @@ __global__ void __launch_bounds__(kLogicThreads, kCastLogicBlocks)
 // the slots in order), hands the bounce's counts to the kernels that follow,
 // advances the sample counter (finalize_new_path, new_path.cl:85-88) and clears what
 // the next bounce counts in, so that a bounce needs no memset.
-__global__ void __launch_bounds__(256) k_classify(PathsView P, QueueView Q, InnerView I, RenderParams rp,
-                                                  unsigned long long* trace_next, int boundary) {
+// Bound by its chain of steps (256 tiles 12.4 us with 16 slots a thread, 11.0 so).
+constexpr uint32_t kClassifyThreads = 512, kClassifyWarps = kClassifyThreads / 32;
+__global__ void __launch_bounds__(kClassifyThreads) k_classify(PathsView P, QueueView Q, InnerView I, RenderParams rp,
+                                                               unsigned long long* trace_next, int boundary) {
     follow();
     const unsigned full = 0xffffffffu;
-    __shared__ unsigned long long s_lo[8], s_hi[8];
+    __shared__ unsigned long long s_warp[kClassifyWarps];
+    __shared__ uint32_t s_pos[kNumQueues][kClassifyWarps];  // where a warp's slots of a class go in s_list
     __shared__ uint32_t s_off[kNumQueues + 1], s_base[kNumQueues], s_last;
     __shared__ uint16_t s_list[kTile];
+    constexpr uint32_t kEach = kTile / kClassifyThreads;
     const uint32_t t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint4 q4 = *reinterpret_cast<const uint4*>(P.qid + t * kTile + tid * 16);
-    const uint32_t words[4] = {q4.x, q4.y, q4.z, q4.w};
-    // fields: queues 0..3 in lo, 4..6 in hi; idle slots in none
-    unsigned long long lo = 0ull, hi = 0ull;
+    const uint2 q8 = *reinterpret_cast<const uint2*>(P.qid + t * kTile + tid * kEach);
+    // the queue of the thread's slot k; idle ones are above
+    auto queue = [&](uint32_t k) { return ((k < 4u ? q8.x : q8.y) >> (8 * (k & 3u))) & 0xffu; };
+    unsigned long long f = 0ull;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-        const uint32_t q = (words[k >> 2] >> (8 * (k & 3))) & 0xffu;
-        if (q < 4u) lo += 1ull << (16 * q);
-        else if (q < (uint32_t)kNumQueues) hi += 1ull << (16 * (q - 4u));
-    }
-    unsigned long long ilo = lo, ihi = hi;  // inclusive over the warp
+    for (uint32_t k = 0; k < kEach; ++k)
+        if (queue(k) < (uint32_t)kNumQueues) f += 1ull << (9 * queue(k));
+    unsigned long long inc = f;  // inclusive over the warp
     for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long a = __shfl_up_sync(full, ilo, o), b = __shfl_up_sync(full, ihi, o);
-        if ((int)lane >= o) ilo += a, ihi += b;
+        const unsigned long long a = __shfl_up_sync(full, inc, o);
+        if ((int)lane >= o) inc += a;
     }
-    if (lane == 31) s_lo[warp] = ilo, s_hi[warp] = ihi;
+    if (lane == 31) s_warp[warp] = inc;
     __syncthreads();
-    unsigned long long plo = ilo - lo, phi = ihi - hi, tlo = 0ull, thi = 0ull;
+    uint32_t base = 0;
+    if (warp < (uint32_t)kNumQueues) {
+        const unsigned long long w = lane < kClassifyWarps ? s_warp[lane] : 0ull;
+        uint32_t below = 0, n = (uint32_t)(w >> (9 * warp)) & 511u, sum = n;
 #pragma unroll
-    for (uint32_t w = 0; w < 8; ++w) {
-        if (w < warp) plo += s_lo[w], phi += s_hi[w];
-        tlo += s_lo[w], thi += s_hi[w];
-    }
-    uint32_t off[kNumQueues + 1];
-    off[0] = 0;
-#pragma unroll
-    for (int k = 0; k < kNumQueues; ++k)
-        off[k + 1] = off[k] + (uint32_t)((k < 4 ? tlo >> (16 * k) : thi >> (16 * (k - 4))) & 0xffffull);
-    if (tid < (uint32_t)kNumQueues) {
-        const uint32_t n = pick(off, (int)tid + 1) - pick(off, (int)tid);
-        s_off[tid] = pick(off, (int)tid);
-        if (tid == 0) {
-            Q.tile_new[t] = n;
-            if (off[kNumQueues]) atomicAdd(rp.rays, (unsigned long long)off[kNumQueues]);
-        } else if (n) {
-            s_base[tid] = atomicAdd(Q.counts + tid, n);
+        for (uint32_t k = 0; k + 1 < (uint32_t)kNumQueues; ++k)
+            if (k < warp) below += (uint32_t)(w >> (9 * k)) & 511u;
+        below = __reduce_add_sync(full, below);
+        for (int o = 1; o < (int)kClassifyWarps; o <<= 1) {
+            const uint32_t a = __shfl_up_sync(full, sum, o);
+            if ((int)lane >= o) sum += a;
         }
-    }
-    if (off[kNumQueues] != 0u) {  // not an idle tile (the same in every thread)
-        // the thread's slots into class order
-        plo += (unsigned long long)off[0] | (unsigned long long)off[1] << 16 | (unsigned long long)off[2] << 32 |
-               (unsigned long long)off[3] << 48;
-        phi += (unsigned long long)off[4] | (unsigned long long)off[5] << 16 | (unsigned long long)off[6] << 32;
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            const uint32_t q = (words[k >> 2] >> (8 * (k & 3))) & 0xffu;
-            if (q < 4u) {
-                s_list[(plo >> (16 * q)) & 0xffffull] = (uint16_t)(tid * 16 + k);
-                plo += 1ull << (16 * q);
-            } else if (q < (uint32_t)kNumQueues) {
-                s_list[(phi >> (16 * (q - 4u))) & 0xffffull] = (uint16_t)(tid * 16 + k);
-                phi += 1ull << (16 * (q - 4u));
+        if (lane < kClassifyWarps) s_pos[warp][lane] = below + sum - n;
+        const uint32_t total = __shfl_sync(full, sum, kClassifyWarps - 1);
+        if (lane == 0) {
+            s_off[warp] = below;
+            if (warp == 0) {
+                Q.tile_new[t] = total;
+            } else if (total) {
+                base = atomicAdd(Q.counts + warp, total);
+            }
+            if (warp + 1 == (uint32_t)kNumQueues) {
+                s_off[kNumQueues] = below + total;
+                if (below + total) atomicAdd(rp.rays, (unsigned long long)(below + total));
             }
         }
+    }
+    __syncthreads();
+    uint32_t off[kNumQueues + 1];
+#pragma unroll
+    for (int k = 0; k <= kNumQueues; ++k) off[k] = s_off[k];
+    if (off[kNumQueues] != 0u) {  // not an idle tile (the same in every thread)
+        // the thread's slots into class order
+        unsigned long long e = inc - f;
+#pragma unroll
+        for (uint32_t k = 0; k < kEach; ++k) {
+            const uint32_t q = queue(k);
+            if (q < (uint32_t)kNumQueues) {
+                s_list[s_pos[q][warp] + ((uint32_t)(e >> (9 * q)) & 511u)] = (uint16_t)(tid * kEach + k);
+                e += 1ull << (9 * q);
+            }
+        }
+        if (lane == 0 && warp < (uint32_t)kNumQueues) s_base[warp] = base;
         __syncthreads();
-        for (uint32_t j = tid; j < off[1]; j += 256) I.ended[t * kTile + j] = s_list[j];
-        for (uint32_t j = off[1] + tid; j < off[kNumQueues]; j += 256) {
+        for (uint32_t j = tid; j < off[1]; j += kClassifyThreads) I.ended[t * kTile + j] = s_list[j];
+        for (uint32_t j = off[1] + tid; j < off[kNumQueues]; j += kClassifyThreads) {
             int q = 1;
 #pragma unroll
             for (int k = 2; k < kNumQueues; ++k) q += j >= off[k] ? 1 : 0;
@@ -1491,9 +1498,19 @@ __global__ void __launch_bounds__(256) k_classify(PathsView P, QueueView Q, Inne
     if (tid == 0) s_last = atomicAdd(I.words + InnerView::kTicket, 1u) + 1u == gridDim.x ? 1u : 0u;
     __syncthreads();
     if (!s_last) return;
+    uint32_t went_on = 0;
+    unsigned long long np = 0;
+    if (tid == 0) {  // on their way while the block scans
+        np = *Q.next_pixel;
+#pragma unroll
+        for (int k = 1; k < kNumQueues; ++k) {
+            went_on |= I.words[k] = __ldcg(Q.counts + k);
+            Q.counts[k] = 0u;
+        }
+    }
     uint32_t run = 0;
-    __shared__ uint32_t s_sum[8];
-    for (uint32_t b0 = 0; b0 < Q.ntiles; b0 += 1024) {  // four tiles a thread
+    __shared__ uint32_t s_sum[kClassifyWarps];
+    for (uint32_t b0 = 0; b0 < Q.ntiles; b0 += 4 * kClassifyThreads) {  // four tiles a thread
         uint32_t v[4], x = 0;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -1510,7 +1527,7 @@ __global__ void __launch_bounds__(256) k_classify(PathsView P, QueueView Q, Inne
         __syncthreads();
         uint32_t e = run + inc - x;
 #pragma unroll
-        for (uint32_t w = 0; w < 8; ++w) {
+        for (uint32_t w = 0; w < kClassifyWarps; ++w) {
             if (w < warp) e += s_sum[w];
             run += s_sum[w];
         }
@@ -1523,10 +1540,6 @@ __global__ void __launch_bounds__(256) k_classify(PathsView P, QueueView Q, Inne
         __syncthreads();  // s_sum is read
     }
     if (tid == 0) {
-        uint32_t went_on = 0;
-        for (int k = 1; k < kNumQueues; ++k) went_on |= I.words[k] = __ldcg(Q.counts + k);
-        for (int k = 1; k < kNumQueues; ++k) Q.counts[k] = 0u;
-        const unsigned long long np = *Q.next_pixel;
         const bool over = boundary && went_on == 0u && np >= rp.sample_limit;
         I.words[InnerView::kEnded] = run;
         I.words[InnerView::kStop] = over ? 1u : 0u;
@@ -1825,7 +1838,7 @@ void launch_inner_cast(const PathsView& p, const QueueView& q, const RenderParam
 
 void launch_inner_queues(const PathsView& p, const QueueView& q, const InnerView& in, const RenderParams& rp,
                          const TraceShape& ts, bool boundary, int num_sms, cudaStream_t st) {
-    chain(k_classify, q.ntiles, 256, st, p, q, in, rp, ts.counter, boundary ? 1 : 0);
+    chain(k_classify, q.ntiles, kClassifyThreads, st, p, q, in, rp, ts.counter, boundary ? 1 : 0);
     const int blocks = std::min((int)((p.n + 255) / 256), num_sms * kNewPathsBlocks);
     chain(k_new_paths, blocks, 256, st, p, q, in, rp);
 }
