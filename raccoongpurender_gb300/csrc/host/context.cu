@@ -275,11 +275,10 @@ struct rgr_context {
     cudaStream_t tstream[kTraceSlots] = {};  // [0] unused: slot 0 runs on `stream`
     int trace_host_mode = RGR_TRACE_HOST_AUTO;  // rgr_trace_closest: zero copy where it can, or staged copies
     int trace_grid = 0;      // persistent traversal grid (SMs x resident blocks)
-    int trace_refill = 24;   // refill a warp when this many lanes are idle (measured best of 1..32)
+    // 24 and 8 the best of 1..32 and 1..24 for camera rays (3702 Mrays/s; 3319 with every lane waiting for
+    // the last), 12 and 12 for rays in all directions (k_trace_rays)
+    CastTuning trace_tuning{24, 8, 12, 12};
     int trace_blocks = 0;    // resident blocks per SM asked for (0: as many as fit)
-    // node steps while this many lanes of a warp search for a leaf: 8 measured best of
-    // 1..24 with refill 24 (3702 Mrays/s, 3319 with every lane waiting for the last)
-    int trace_search = 8;
     // extension rays of a bounce: persistent refilling kernel, then logic (or fused)
     // refill 12: the mixed 1080p render at 2^24 paths runs 1047.7 / 1066.6 / 1067.6 / 1066.5 /
     // 1059.5 Mpaths/s with a warp refilled at 24 / 8 / 12 / 16 / 20 idle lanes
@@ -990,13 +989,13 @@ int rgr_trace_closest_device(rgr_context* c, const rgr_ray_soa* rays, uint64_t n
                            c->tbins.as<uint32_t>(), c->trank.as<uint32_t>(), c->tpacked.as<float4>(),
                            c->num_sms * 64, st);
         launch_trace_packed(c->scene.sv, c->tpacked.as<float4>(), n, prim, t, ng_xyz, c->err.as<uint32_t>(),
-                            c->tcounter.as<unsigned long long>(), c->trace_refill, c->trace_search, c->packed_grid,
+                            c->tcounter.as<unsigned long long>(), c->trace_tuning, c->packed_grid,
                             st);
         RGR_CUDA(cudaGetLastError());
         return RGR_OK;
     }
     launch_trace_rays(c->scene.sv, rays->ox, rays->oy, rays->oz, rays->dx, rays->dy, rays->dz, rays->tmax, n, prim, t, ng_xyz,
-                      c->err.as<uint32_t>(), c->tcounter.as<unsigned long long>(), c->trace_refill, c->trace_search,
+                      c->err.as<uint32_t>(), c->tcounter.as<unsigned long long>(), c->trace_tuning,
                       c->trace_grid, c->trace_stage, st);
     RGR_CUDA(cudaGetLastError());
     return RGR_OK;
@@ -1026,7 +1025,7 @@ int rgr_set_trace_tuning(rgr_context* c, int32_t refill, int32_t blocks_per_sm) 
     RGR_CUDA(cudaSetDevice(c->device));
     int maxb = std::max(1, trace_rays_max_blocks_per_sm(c->trace_stage));
     if (blocks_per_sm > maxb) return RGR_E_INVALID;
-    c->trace_refill = refill;
+    c->trace_tuning.refill = c->trace_tuning.mixed_refill = refill;
     c->trace_blocks = blocks_per_sm;
     c->trace_grid = c->num_sms * (blocks_per_sm ? blocks_per_sm : maxb);
     const int maxb0 = std::max(1, trace_rays_max_blocks_per_sm(0));
@@ -1045,7 +1044,7 @@ int rgr_set_render_trace(rgr_context* c, int32_t persistent, int32_t refill) {
 
 int rgr_set_trace_search(rgr_context* c, int32_t closest, int32_t render) {
     if (!c || closest < 0 || closest > 32 || render < 0 || render > 32) return RGR_E_INVALID;
-    if (closest > 0) c->trace_search = closest;
+    if (closest > 0) c->trace_tuning.search = c->trace_tuning.mixed_search = closest;
     if (render > 0 && render != c->render_trace.search) {
         c->render_trace.search = render;
         c->begun = false;  // takes effect at the next render begin
@@ -1141,7 +1140,7 @@ int rgr_trace_closest(rgr_context* c, const rgr_ray_soa* rays, uint64_t n, int32
             c->mail->link_err = 0u;
             cudaStream_t st = c->stream;
             launch_trace_rays_link(c->scene.sv, dsrc, n, dprim, dt, &c->mail->link_err, ts.counter.as<unsigned long long>(),
-                                   c->trace_refill, c->trace_search, c->trace_grid, st);
+                                   c->trace_tuning, c->trace_grid, st);
             RGR_CUDA(cudaGetLastError());
             populate({prim, t}, 4 * n);
             RGR_CUDA(cudaStreamSynchronize(st));
@@ -1178,8 +1177,7 @@ int rgr_trace_closest(rgr_context* c, const rgr_ray_soa* rays, uint64_t n, int32
         launch_trace_rays(c->scene.sv, ts.rays[0].as<float>(), ts.rays[1].as<float>(), ts.rays[2].as<float>(),
                           ts.rays[3].as<float>(), ts.rays[4].as<float>(), ts.rays[5].as<float>(),
                           ts.rays[6].as<float>(), m, ts.prim.as<int32_t>(), ts.t.as<float>(), nullptr,
-                          ts.err.as<uint32_t>(), ts.counter.as<unsigned long long>(), c->trace_refill,
-                          c->trace_search, c->trace_grid, c->trace_stage, st);
+                          ts.err.as<uint32_t>(), ts.counter.as<unsigned long long>(), c->trace_tuning, c->trace_grid, c->trace_stage, st);
         RGR_CUDA(cudaGetLastError());
         RGR_CUDA(cudaMemcpyAsync(prim + off, ts.prim.p, 4 * m, cudaMemcpyDeviceToHost, st));
         RGR_CUDA(cudaMemcpyAsync(t + off, ts.t.p, 4 * m, cudaMemcpyDeviceToHost, st));

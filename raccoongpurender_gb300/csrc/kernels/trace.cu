@@ -27,6 +27,7 @@
 // order and writes each hit at the ray's own index.  Within a bucket the
 // order is that of the atomic cursor, which changes nothing but the schedule.
 #include <algorithm>
+#include <type_traits>
 
 #include "wavefront.cuh"
 #include "traverse.cuh"
@@ -51,8 +52,7 @@ struct RayBatch {
     uint32_t* err;
     unsigned long long* next;    // work counter, zero at launch (share = 0)
     uint32_t share;              // rays of a warp in a call of few, without the counter; 0 otherwise
-    int refill;                  // refill when at least this many lanes are idle
-    int search;                  // node steps while at least this many lanes search
+    CastTuning tune;
     uint32_t stage;              // inner nodes copied to shared memory (kStaged)
 };
 
@@ -77,6 +77,10 @@ struct LinkRuns {
     int32_t prim[kRuns][32];
     float t[kRuns][32];
 };
+
+// From this many rays on a warp's octants choose its thresholds (CastTuning): a warp of a call
+// of fewer takes rays a few times only (300,000 random rays in 20 K triangles 112 us, 116 so).
+constexpr uint64_t kMixedMinRays = 1ull << 19;
 
 // kFew: each lane takes one ray of its warp's share, without the rounds
 template <bool kCount, bool kStaged, bool kPacked, bool kFew, bool kLink>
@@ -157,51 +161,76 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
         if ((uint32_t)lane < b.share && r < b.n) take(r);
     }
     bool exhausted = false;
-    while (!kFew) {
-        const unsigned idle = __ballot_sync(full, ray == ~0ull);
-        if (!exhausted && (int)__popc(idle) >= b.refill) {
-            const uint32_t need = __popc(idle);
-            unsigned long long base = 0;
-            if (lane == 0) base = atomicAdd(b.next, (unsigned long long)need);
-            base = __shfl_sync(full, base, 0);
-            if (base + need >= b.n) exhausted = true;
-            if (kLink && base < b.n) {  // a run of the new rays
-                const int k = oldest;
-                oldest = (oldest + 1) % kRuns;
-                if (__shfl_sync(full, run_rays, k)) {
-                    flush(k);
-                    if (run == k) run = -1;
-                }
-                if (lane == k) {
-                    run_base = base;
-                    run_rays = b.n - base >= need ? (need < 32u ? (1u << need) - 1u : full) : (1u << (b.n - base)) - 1u;
+    // kMixed: a compile-time constant, so that each loop's thresholds are operands and not registers
+    auto rounds = [&](auto which) {
+        constexpr bool kMixed = decltype(which)::value;
+        for (;;) {
+            const unsigned idle = __ballot_sync(full, ray == ~0ull);
+            if (!exhausted && (int)__popc(idle) >= (kMixed ? b.tune.mixed_refill : b.tune.refill)) {
+                const uint32_t need = __popc(idle);
+                unsigned long long base = 0;
+                if (lane == 0) base = atomicAdd(b.next, (unsigned long long)need);
+                base = __shfl_sync(full, base, 0);
+                if (base + need >= b.n) exhausted = true;
+                if (kLink && base < b.n) {  // a run of the new rays
+                    const int k = oldest;
+                    oldest = (oldest + 1) % kRuns;
+                    if (__shfl_sync(full, run_rays, k)) {
+                        flush(k);
+                        if (run == k) run = -1;
+                    }
+                    if (lane == k) {
+                        run_base = base;
+                        run_rays = b.n - base >= need ? (need < 32u ? (1u << need) - 1u : full) : (1u << (b.n - base)) - 1u;
+                    }
+                    if (ray == ~0ull) {
+                        run = k;
+                        place = __popc(idle & lt);
+                    }
                 }
                 if (ray == ~0ull) {
-                    run = k;
-                    place = __popc(idle & lt);
+                    const uint64_t r = base + __popc(idle & lt);
+                    if (r < b.n) take(r);
                 }
             }
-            if (ray == ~0ull) {
-                const uint64_t r = base + __popc(idle & lt);
-                if (r < b.n) take(r);
+            const unsigned held = __ballot_sync(full, ray != ~0ull);
+            if (exhausted && __popc(held) <= kTailLanes) break;
+            if (held == 0u) continue;
+            trace_warp_round<kCount, kStaged, kSmemStack>(sc, s, ray != ~0ull && s.link != kDone,
+                                                          kMixed ? b.tune.mixed_search : b.tune.search, &cnt, err, pol, stn);
+            const bool ended = ray != ~0ull && s.link == kDone;
+            if (ended) put();
+            if (kLink) {
+                __syncwarp();
+    #pragma unroll
+                for (int k = 0; k < kRuns; ++k) {
+                    const unsigned places = __reduce_or_sync(full, ended && run == k ? 1u << place : 0u);
+                    if (lane == k) run_done |= places;
+                    if (places && __shfl_sync(full, run_done == run_rays, k)) flush(k);
+                }
             }
         }
-        const unsigned held = __ballot_sync(full, ray != ~0ull);
-        if (exhausted && __popc(held) <= kTailLanes) break;
-        if (held == 0u) continue;
-        trace_warp_round<kCount, kStaged, kSmemStack>(sc, s, ray != ~0ull && s.link != kDone, b.search, &cnt, err, pol,
-                                                      stn);
-        const bool ended = ray != ~0ull && s.link == kDone;
-        if (ended) put();
-        if (kLink) {
-            __syncwarp();
-#pragma unroll
-            for (int k = 0; k < kRuns; ++k) {
-                const unsigned places = __reduce_or_sync(full, ended && run == k ? 1u << place : 0u);
-                if (lane == k) run_done |= places;
-                if (places && __shfl_sync(full, run_done == run_rays, k)) flush(k);
-            }
+    };
+    if (!kFew) {
+        // Rays of one octant keep together in large batches (camera rays, ms: refill / search 24 / 8
+        // 0.81, 12 / 12 0.87); others part at once, and full lanes count for more (random
+        // rays 1.18 and 1.13; in a scene of 1280 triangles 0.199 and 0.185).  The warp looks at rays
+        // about where its first will be; chosen anew at each refill it cost registers, and 0.09 ms.
+        // Sorted rays: 1.13 with 24 / 8, 1.16 where a warp's own octants decide.
+        bool mixed = false;
+        if (!kCount && !kStaged && !kLink && !kPacked && b.n >= kMixedMinRays) {
+            const uint64_t r = (uint64_t)blockIdx.x * kStackThreads + threadIdx.x;
+            const bool has = r < b.n;
+            f3 d = mk(0.0f, 0.0f, 0.0f);
+            if (has) d = mk(__ldg(b.dx + r), __ldg(b.dy + r), __ldg(b.dz + r));
+            const unsigned rays = __ballot_sync(full, has), x = __ballot_sync(full, d.x < 0.0f),
+                           y = __ballot_sync(full, d.y < 0.0f), z = __ballot_sync(full, d.z < 0.0f);
+            mixed = (x != 0u && x != rays) || (y != 0u && y != rays) || (z != 0u && z != rays);
         }
+        if (mixed)
+            rounds(std::true_type());
+        else
+            rounds(std::false_type());
     }
     if (kLink) {  // the last rays write their own
 #pragma unroll
@@ -421,13 +450,13 @@ uint32_t spread(uint64_t n, int grid, int* blocks, unsigned long long* counter, 
 
 void launch_trace_rays(const SceneView& sc, const float* ox, const float* oy, const float* oz, const float* dx,
                        const float* dy, const float* dz, const float* tmax, uint64_t n, int32_t* prim, float* t,
-                       float* ng, uint32_t* err, unsigned long long* counter, int refill, int search, int grid,
+                       float* ng, uint32_t* err, unsigned long long* counter, const CastTuning& tune, int grid,
                        uint32_t stage, cudaStream_t st) {
     if (n == 0) return;
     int blocks;
     const uint32_t share = spread(n, grid, &blocks, counter, st);
-    RayBatch b{ox, oy, oz, dx, dy, dz, tmax, nullptr, n, prim, t, ng, nullptr, nullptr, err, counter, share, refill,
-               search, stage};
+    RayBatch b{ox, oy, oz, dx, dy, dz, tmax, nullptr, n, prim, t, ng, nullptr, nullptr, err, counter, share, tune,
+               stage};
     if (share)
         k_trace_rays<false, false, false, true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
     else if (stage > 0)
@@ -438,13 +467,13 @@ void launch_trace_rays(const SceneView& sc, const float* ox, const float* oy, co
 
 // rays and results in host memory
 void launch_trace_rays_link(const SceneView& sc, const float* const* rays, uint64_t n, int32_t* prim, float* t,
-                            uint32_t* err, unsigned long long* counter, int refill, int search, int grid,
+                            uint32_t* err, unsigned long long* counter, const CastTuning& tune, int grid,
                             cudaStream_t st) {
     if (n == 0) return;
     int blocks;
     const uint32_t share = spread(n, grid, &blocks, counter, st);
     RayBatch b{rays[0], rays[1], rays[2], rays[3], rays[4], rays[5], rays[6], nullptr, n, prim, t, nullptr,
-               nullptr, nullptr, err, counter, share, refill, search, 0u};
+               nullptr, nullptr, err, counter, share, tune, 0u};
     if (share)
         k_trace_rays<false, false, false, true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
     else
@@ -458,7 +487,8 @@ void launch_trace_rays_counts(const SceneView& sc, const float* ox, const float*
     if (n == 0) return;
     int blocks;
     const uint32_t share = spread(n, grid, &blocks, counter, st);
-    RayBatch b{ox, oy, oz, dx, dy, dz, tmax, nullptr, n, prim, t, nullptr, nodes, prims, err, counter, share, 16, 1, 0u};
+    RayBatch b{ox, oy, oz, dx, dy, dz, tmax, nullptr, n, prim, t, nullptr, nodes, prims, err, counter, share, CastTuning{16, 1, 16, 1},
+               0u};
     if (share)
         k_trace_rays<true, false, false, true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
     else
@@ -496,13 +526,13 @@ void launch_ray_reorder(const float* ox, const float* oy, const float* oz, const
 }
 
 void launch_trace_packed(const SceneView& sc, const float4* packed, uint64_t n, int32_t* prim, float* t, float* ng,
-                         uint32_t* err, unsigned long long* counter, int refill, int search, int grid,
+                         uint32_t* err, unsigned long long* counter, const CastTuning& tune, int grid,
                          cudaStream_t st) {
     if (n == 0) return;
     int blocks;
     const uint32_t share = spread(n, grid, &blocks, counter, st);
     RayBatch b{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, packed, n, prim, t, ng, nullptr,
-               nullptr, err, counter, share, refill, search, 0u};
+               nullptr, err, counter, share, tune, 0u};
     if (share)
         k_trace_rays<false, false, true, true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
     else

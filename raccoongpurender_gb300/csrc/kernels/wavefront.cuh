@@ -324,13 +324,20 @@ void launch_merge_intermediate(void* a, const void* b, uint32_t n, cudaStream_t 
 // stage: inner nodes (the breadth-first top of the tree) each CTA copies to
 // shared memory, 0..kMaxStagedNodes
 constexpr uint32_t kMaxStagedNodes = 1024;
+// A warp of the closest-hit kernels takes new rays when `refill` of its lanes are idle, and its
+// lanes take node steps while `search` of them still search for their leaf; in large calls
+// (not sorted, staged or across the link) a warp whose rays head into several octants goes by
+// the mixed pair.
+struct CastTuning {
+    int refill, search, mixed_refill, mixed_search;
+};
 void launch_trace_rays(const SceneView& sc, const float* ox, const float* oy, const float* oz, const float* dx,
                        const float* dy, const float* dz, const float* tmax, uint64_t n, int32_t* prim, float* t,
-                       float* ng, uint32_t* err, unsigned long long* counter, int refill, int search, int grid,
+                       float* ng, uint32_t* err, unsigned long long* counter, const CastTuning& tune, int grid,
                        uint32_t stage, cudaStream_t st);
 // the same for rays and results in host memory that the GPU reads and writes across a coherent link
 void launch_trace_rays_link(const SceneView& sc, const float* const* rays, uint64_t n, int32_t* prim, float* t,
-                            uint32_t* err, unsigned long long* counter, int refill, int search, int grid,
+                            uint32_t* err, unsigned long long* counter, const CastTuning& tune, int grid,
                             cudaStream_t st);
 void launch_trace_rays_counts(const SceneView& sc, const float* ox, const float* oy, const float* oz, const float* dx,
                               const float* dy, const float* dz, const float* tmax, uint64_t n, int32_t* prim,
@@ -356,7 +363,7 @@ void launch_ray_reorder(const float* ox, const float* oy, const float* oz, const
                         uint32_t* rank, float4* packed, int grid, cudaStream_t st);
 // closest hit of reordered records; hits written at each record's ray index
 void launch_trace_packed(const SceneView& sc, const float4* packed, uint64_t n, int32_t* prim, float* t, float* ng,
-                         uint32_t* err, unsigned long long* counter, int refill, int search, int grid,
+                         uint32_t* err, unsigned long long* counter, const CastTuning& tune, int grid,
                          cudaStream_t st);
 
 }  // namespace dev

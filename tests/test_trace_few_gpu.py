@@ -109,3 +109,20 @@ def test_host_runs(rg, po, refill, n):
     oprim, ot, _ = osc.trace(rays.packed8(), threads=16)
     prim, t = lane.trace_closest(rays)
     assert (prim == oprim).all() and (bits(t) == bits(ot)).all()
+
+
+@pytest.mark.parametrize("n", [(1 << 19) - 1, 1 << 19, (1 << 19) + 33])
+@pytest.mark.parametrize("order", ["one octant", "every octant", "by turns"])
+def test_octants(rg, po, n, order):
+    """Warps that choose their thresholds by their rays' octants, from 2^19 rays on."""
+    mesh = scenes.displaced_icosphere(4, seed=7)
+    sm, osc = build(mesh)
+    lane = rg.WavefrontLane(0, 1024)
+    lane.setup(sm)
+    rays = scenes.random_rays(n, (-1.3, -1.3, -1.3), (1.3, 1.3, 1.3), seed=n)
+    if order != "every octant":
+        turn = np.arange(n) % 256 < 128 if order == "by turns" else np.ones(n, bool)
+        rays.d[turn] = np.abs(rays.d[turn])
+    oprim, ot, _ = osc.trace(rays.packed8(), threads=16)
+    prim, t, _ = _hits(lane, rays)
+    assert (prim == oprim).all() and (bits(t) == bits(ot)).all()
