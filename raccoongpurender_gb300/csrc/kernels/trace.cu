@@ -67,15 +67,19 @@ RGR_DEV void ld_record(const float4* ptr, float4& a, float4& b) {
 // consecutive, and their hits wait in shared memory until the last of them is known.
 // Single 4-byte stores keep the link busy: 1M random rays in 330 K triangles took 400 us with
 // only the results across it, 342 with only the rays (320 with neither), the whole call
-// 502 and now 400 us; 2M rays in 1.31M triangles 957 and 787.  (The rays' reads hide behind the
+// 502 and now 400 us; 2M rays in 1.31M triangles 957 and 762.  (The rays' reads hide behind the
 // traversal: copying them to shared memory a batch ahead was slower, 549, as every
 // warp's first rays then share the link with the others' second.)  A warp keeps up to
-// kRuns runs open; to begin another it writes what the oldest has, and that one's missing
+// kRuns runs open (all of a run in shared memory: its words in registers spilled, 407 and 787);
+// to begin another it writes what the oldest has, and that one's missing
 // rays write their own.
 constexpr int kRuns = 4;
 struct LinkRuns {
     int32_t prim[kRuns][32];
     float t[kRuns][32];
+    uint64_t base[kRuns];  // the run's first ray
+    uint32_t rays[kRuns];  // a bit per ray of it (0: free)
+    uint32_t done[kRuns];  // the finished ones
 };
 
 // From this many rays on a warp's octants choose its thresholds (CastTuning): a warp of a call
@@ -103,20 +107,20 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
     uint64_t ray = ~0ull;  // ~0: idle
     __shared__ LinkRuns s_runs[kLink ? kStackThreads / 32 : 1];
     LinkRuns& runs = s_runs[kLink ? threadIdx.x >> 5 : 0];
-    uint64_t run_base = 0;                // lane k < kRuns: run k's first ray,
-    unsigned run_rays = 0, run_done = 0;  // its rays and the finished ones of them (none: free)
-    int run = -1, place = 0;              // this lane's ray's run, and its place there
+    if (kLink && lane < kRuns) runs.rays[lane] = runs.done[lane] = 0u;
+    __syncwarp();
+    int place = -1;  // this lane's ray's run << 5 | its place there, or it writes its own hit
     int oldest = 0;
     // writes the finished rays of run k, which is free then
     auto flush = [&](int k) {
-        const uint64_t base = __shfl_sync(full, run_base, k);
-        const unsigned done = __shfl_sync(full, run_done, k);
-        if ((done >> lane) & 1u) {
-            __stcs(b.prim + base + lane, runs.prim[k][lane]);
-            __stcs(b.t + base + lane, runs.t[k][lane]);
+        if ((runs.done[k] >> lane) & 1u) {
+            const uint64_t r = runs.base[k] + lane;
+            __stcs(b.prim + r, runs.prim[k][lane]);
+            __stcs(b.t + r, runs.t[k][lane]);
         }
         __syncwarp();
-        if (lane == k) run_rays = run_done = 0u;
+        if (lane == 0) runs.rays[k] = runs.done[k] = 0u;
+        __syncwarp();
     };
     auto take = [&](uint64_t r) {
         if (kPacked) {
@@ -136,9 +140,10 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
     };
     auto put = [&]() {
         const int32_t prim = hit_id(s.prim);
-        if (kLink && run >= 0) {
-            runs.prim[run][place] = prim;
-            runs.t[run][place] = s.tmin;
+        if (kLink && place >= 0) {
+            runs.prim[place >> 5][place & 31] = prim;
+            runs.t[place >> 5][place & 31] = s.tmin;
+            atomicOr(&runs.done[place >> 5], 1u << (place & 31));
         } else {
             __stcs(b.prim + ray, prim);
             __stcs(b.t + ray, s.tmin);
@@ -175,18 +180,16 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
                 if (kLink && base < b.n) {  // a run of the new rays
                     const int k = oldest;
                     oldest = (oldest + 1) % kRuns;
-                    if (__shfl_sync(full, run_rays, k)) {
+                    if (runs.rays[k]) {
                         flush(k);
-                        if (run == k) run = -1;
+                        if ((place >> 5) == k) place = -1;
                     }
-                    if (lane == k) {
-                        run_base = base;
-                        run_rays = b.n - base >= need ? (need < 32u ? (1u << need) - 1u : full) : (1u << (b.n - base)) - 1u;
+                    if (lane == 0) {
+                        runs.base[k] = base;
+                        runs.rays[k] =
+                            b.n - base >= need ? (need < 32u ? (1u << need) - 1u : full) : (1u << (b.n - base)) - 1u;
                     }
-                    if (ray == ~0ull) {
-                        run = k;
-                        place = __popc(idle & lt);
-                    }
+                    if (ray == ~0ull) place = k << 5 | __popc(idle & lt);
                 }
                 if (ray == ~0ull) {
                     const uint64_t r = base + __popc(idle & lt);
@@ -198,16 +201,11 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
             if (held == 0u) continue;
             trace_warp_round<kCount, kStaged, kSmemStack>(sc, s, ray != ~0ull && s.link != kDone,
                                                           kMixed ? b.tune.mixed_search : b.tune.search, &cnt, err, pol, stn);
-            const bool ended = ray != ~0ull && s.link == kDone;
-            if (ended) put();
+            if (ray != ~0ull && s.link == kDone) put();
             if (kLink) {
                 __syncwarp();
-    #pragma unroll
-                for (int k = 0; k < kRuns; ++k) {
-                    const unsigned places = __reduce_or_sync(full, ended && run == k ? 1u << place : 0u);
-                    if (lane == k) run_done |= places;
-                    if (places && __shfl_sync(full, run_done == run_rays, k)) flush(k);
-                }
+                const bool whole = lane < kRuns && runs.rays[lane] != 0u && runs.done[lane] == runs.rays[lane];
+                for (unsigned m = __ballot_sync(full, whole); m != 0u; m &= m - 1u) flush(__ffs(m) - 1);
             }
         }
     };
@@ -233,9 +231,10 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
             rounds(std::false_type());
     }
     if (kLink) {  // the last rays write their own
+        __syncwarp();
 #pragma unroll
         for (int k = 0; k < kRuns; ++k) flush(k);
-        run = -1;
+        place = -1;
     }
     if (ray != ~0ull) {
         while (s.link != kDone) trace_round<kCount, kStaged, kSmemStack, true>(sc, s, &cnt, err, pol, stn);
