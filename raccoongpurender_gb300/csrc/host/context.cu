@@ -274,6 +274,7 @@ struct rgr_context {
     } tslot[kTraceSlots];
     cudaStream_t tstream[kTraceSlots] = {};  // [0] unused: slot 0 runs on `stream`
     int trace_host_mode = RGR_TRACE_HOST_AUTO;  // rgr_trace_closest: zero copy where it can, or staged copies
+    int cast_blocks[2] = {1, 1};  // resident blocks an SM of the bounce's cast: scenes by request, one scene
     int trace_grid = 0;      // persistent traversal grid (SMs x resident blocks)
     // 24 and 8 the best of 1..32 and 1..24 for camera rays (3702 Mrays/s; 3319 with every lane waiting for
     // the last), 12 and 12 for rays in all directions (k_trace_rays)
@@ -346,6 +347,7 @@ struct rgr_context {
     int start(const RequestD* host_reqs, int nreq, unsigned long long limit, uint32_t seed_offset) {
         cudaStream_t st = stream;
         int r;
+        render_trace.grid = num_sms * cast_blocks[render_trace.one != nullptr];
         render_trace.persistent =
             render_trace_mode < 0 ? npaths >= kPersistentTraceMinPaths : render_trace_mode != 0;
         if ((r = reqtab.alloc(sizeof(RequestD) * nreq)) != RGR_OK) return r;
@@ -690,7 +692,7 @@ int rgr_context_create(rgr_context** out, int32_t device, uint32_t path_count) {
     cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device);
     c->trace_grid = c->num_sms * std::max(1, trace_rays_max_blocks_per_sm());
     c->packed_grid = c->trace_grid;
-    c->render_trace.grid = c->num_sms * std::max(1, trace_paths_max_blocks_per_sm());
+    for (int one = 0; one < 2; ++one) c->cast_blocks[one] = trace_paths_max_blocks_per_sm(one != 0);
     c->npaths = path_count;
     c->ntiles = (path_count + kTile - 1) / kTile;
     *out = c;

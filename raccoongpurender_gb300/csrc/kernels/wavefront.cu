@@ -1036,8 +1036,9 @@ RGR_DEV float guide_write(const GuideRenderD& gd, uint32_t slot, const GuideOffe
 #ifndef RGR_TRACE_PATHS_MIN_BLOCKS  // 4 / 5 / 6 (64 / 48 / 40 registers, 6 spilling): 1428 / 1473 / 1442 Mpaths/s
 #define RGR_TRACE_PATHS_MIN_BLOCKS 5
 #endif
+// Scenes by request spill at 48 registers: eight requests 3483 us with 5 blocks, 3351 with 4.
 template <bool kInner, bool kOne>
-__global__ void __launch_bounds__(256, RGR_TRACE_PATHS_MIN_BLOCKS)
+__global__ void __launch_bounds__(256, kOne ? RGR_TRACE_PATHS_MIN_BLOCKS : 4)
     k_trace_paths(PathsView P, QueueView Q, RenderParams rp, unsigned long long* next, int refill, int search,
                   SceneView one) {
     follow();
@@ -1856,10 +1857,13 @@ void launch_stamp_done(const RenderParams& rp, cudaStream_t st) {
     if (rp.nreq > 0) chain(k_stamp_done, (rp.nreq + 127) / 128, 128, st, rp);
 }
 
-int trace_paths_max_blocks_per_sm() {
+int trace_paths_max_blocks_per_sm(bool one) {
     int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_paths<true, false>, 256, 0);
-    return nb;
+    if (one)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_paths<true, true>, 256, 0);
+    else
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_paths<true, false>, 256, 0);
+    return nb > 0 ? nb : 1;
 }
 void launch_readback(int fmt, const double* accum, uint32_t npix, void* out, cudaStream_t st) {
     k_readback<<<(npix + 255) / 256, 256, 0, st>>>(fmt, accum, npix, out);

@@ -312,7 +312,8 @@ void launch_inner_queues(const PathsView& p, const QueueView& q, const InnerView
 // 3 and 4; u: the queues with `taken` at InnerView::words
 void launch_inner_shade(const PathsView& p, const QueueView& u, const RenderParams& rp, const TraceShape& ts,
                         int shade_grid, cudaStream_t st);
-int trace_paths_max_blocks_per_sm();
+// one: of a render whose scene is an argument (TraceShape::one)
+int trace_paths_max_blocks_per_sm(bool one);
 // per-request completion stamps of a batch (after the logic kernel of a bounce)
 void launch_stamp_done(const RenderParams& rp, cudaStream_t st);
 void launch_readback(int fmt, const double* accum, uint32_t npix, void* dev_out, cudaStream_t st);
