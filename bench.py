@@ -851,9 +851,9 @@ def main() -> None:
         return (time.perf_counter() - t0) / args.e2e_steps
 
     # the default: the traversal kernel reads the pinned rays and writes the hits
-    # across the CPU-GPU link itself (its warps refill only when all lanes are idle,
-    # so the shapes tuned for rays in device memory do not apply: the library's
-    # default leaf batching); for comparison, staged copies through device buffers
+    # across the CPU-GPU link itself (with the library's default thresholds: the shapes
+    # tuned for rays in device memory do not apply); for comparison, staged copies through
+    # device buffers
     lane.set_trace_reorder(0)
     lane.set_trace_staging(0)
     lane.set_trace_tuning(24, 0)

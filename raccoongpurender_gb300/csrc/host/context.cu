@@ -214,13 +214,13 @@ void give_mail(Mail* m) {  // its context's stream is idle
 
 }  // namespace
 
-// Pools of fewer paths run the fused trace + logic kernel by default (a bounce is then
-// bound by its launches' latency and the longest ray of each warp), larger ones the
+// Pools of fewer paths run the fused cast + logic kernel by default (a bounce is then
+// bound by its launches' latency and its longest rays), larger ones the
 // persistent refilling cast and, inside a run of bounces, no logic pass (launch_inner_queues).
-// Whole renders (4 spp, depth 6), persistent against fused, at 2^17 / 2^18 / 2^19 / 2^20 /
-// 2^22 paths: 36 triangles 0.84 / 0.98 / 1.12 / 1.24 / 1.36x, 5 K 0.80 / 1.00 / 1.17 / 1.39 /
-// 1.69x, 330 K 0.84 / 0.99 / 1.25 / 1.52 / 2.06x.  Single bounces at 2^18 / 2^20 / 2^22:
-// 36 triangles 0.87 / 1.00 / 1.07x, 5 K 0.96 / 1.22 / 1.40x.
+// Whole renders (4 spp, depth 6), persistent against fused, at 2^15 / 2^17 / 2^18 / 3 * 2^17 /
+// 2^19 / 2^20 paths: 36 triangles 0.81 / 0.86 / 1.02 / 1.14 / 1.14 / 1.24x, 5 K 0.73 / 0.84 / 0.94 /
+// 1.09 / 1.12 / 1.30x, 80 K 0.78 / 0.86 / 0.92 / 1.10 / 1.17 / 1.34x.  Single bounces at 2^17 / 2^18 /
+// 3 * 2^17 / 2^20: 36 triangles 0.89 / 0.97 / 1.10 / 1.06x, 5 K 0.89 / 0.96 / 1.06 / 1.16x.
 constexpr uint32_t kPersistentTraceMinPaths = 3u << 17;
 // rgr_trace_closest: 2^20-ray chunks in flight on their own streams, so that
 // the copies of some overlap the traversal of another (measured end to end
