@@ -11,7 +11,6 @@
 #include <cmath>
 #include <cstring>
 #include <initializer_list>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -19,6 +18,7 @@
 #include "../rgr_internal.h"
 #include "devbuf.h"
 #include "guide_host.h"
+#include "mail.h"
 #include "nvtx.h"
 
 using namespace rgr;
@@ -171,45 +171,6 @@ void populate(std::initializer_list<void*> arrays, size_t bytes) {
             madvise((void*)from, to - from, MADV_POPULATE_WRITE);  // where it cannot, the pages still fault
         }
 #endif
-}
-
-// Pinned host memory for the words that a context's calls wait for: copied to in its stream's
-// order, read after one wait for the stream.
-struct Mail {
-    unsigned long long next_pixel;
-    uint32_t counts[8], stop, err;
-    uint32_t link_err;  // the zero-copy path's error word, written by its kernel
-    uint32_t pad;
-};
-// Pinning a page takes some 120 us and a context 15 to create, so the first 64 contexts of
-// the process share one allocation; a further one has its own.
-constexpr int kSharedMails = 64;
-std::mutex mail_mutex;
-Mail* shared_mails = nullptr;
-uint64_t shared_taken = 0;  // a bit each
-
-Mail* take_mail() {
-    std::lock_guard<std::mutex> lock(mail_mutex);
-    Mail* m = nullptr;
-    if (!shared_mails && !cuda_ok(cudaHostAlloc(&shared_mails, sizeof(Mail) * kSharedMails, cudaHostAllocPortable),
-                                  "cudaHostAlloc")) {
-        shared_mails = nullptr;
-        return nullptr;
-    }
-    for (int k = 0; k < kSharedMails; ++k)
-        if (!((shared_taken >> k) & 1u)) {
-            shared_taken |= 1ull << k;
-            return shared_mails + k;
-        }
-    return cuda_ok(cudaHostAlloc(&m, sizeof(Mail), cudaHostAllocPortable), "cudaHostAlloc") ? m : nullptr;
-}
-void give_mail(Mail* m) {  // its context's stream is idle
-    if (!m) return;
-    std::lock_guard<std::mutex> lock(mail_mutex);
-    if (m >= shared_mails && m < shared_mails + kSharedMails)
-        shared_taken &= ~(1ull << (m - shared_mails));
-    else
-        cudaFreeHost(m);
 }
 
 }  // namespace

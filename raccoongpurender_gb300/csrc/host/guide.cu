@@ -163,15 +163,15 @@ GuideAdam rgr_guide::adam() const { return GuideAdam{cfg.learning_rate, cfg.beta
 
 void rgr_guide::iteration_launches(const float* smp, const uint32_t* count, uint32_t n, const GuideTrainD& t,
                                    const float* wsum, float weight_scale, int grid, bool step, float* grads,
-                                   cudaStream_t st) {
+                                   float* host_loss, cudaStream_t st) {
     launch_guide_train_tc(view, smp, count, n, t.min_count, wsum, weight_scale, grid, gpart.as<float>(), error_word(),
                           st);
-    launch_guide_update_tc(view, gpart.as<float>(), (uint32_t)grid, count, n, grads, step, adam(), t, st);
+    launch_guide_update_tc(view, gpart.as<float>(), (uint32_t)grid, count, n, grads, step, adam(), t, host_loss, st);
 }
 
 int rgr_guide::train_launches(cudaStream_t st) {
     if (cfg.train && cfg.training_kernel == RGR_GUIDE_TCGEN05) {
-        iteration_launches(train.samples, train.count, train.cap, train, train.wsum, 1.0f, num_sms, true, nullptr, st);
+        iteration_launches(train.samples, train.count, train.cap, train, train.wsum, 1.0f, num_sms, true, nullptr, nullptr, st);
     } else {
         if (cfg.train) {
             launch_guide_train(view, train.samples, train.count, train.cap, train.min_count, train.wsum, 1.0f, num_sms,
@@ -239,7 +239,7 @@ int rgr_guide_create(rgr_guide** out, int32_t device, const rgr_guide_config* cf
         delete g;
         return RGR_E_CUDA;
     }
-    int r = g->init(c);
+    int r = (g->mail = take_mail()) ? g->init(c) : (int)RGR_E_CUDA;
     if (r != RGR_OK) {
         delete g;
         return r;
@@ -352,11 +352,10 @@ int rgr_guide_train_device(rgr_guide* g, const float* samples, uint32_t n, float
     float hl = 0.0f;
     if (n > 0 && g->cfg.training_kernel == RGR_GUIDE_TCGEN05) {
         g->iteration_launches(samples, nullptr, n, g->test, nullptr, weight_scale, train_grid(*g, n), apply_adam != 0,
-                              grads, st);
+                              grads, &g->mail->loss, st);
         RGR_CUDA(cudaGetLastError());
-        RGR_CUDA(cudaMemcpyAsync(&hl, g->loss.as<float>() + 1, 4, cudaMemcpyDeviceToHost, st));
         RGR_CUDA(cudaStreamSynchronize(st));
-        if (loss) *loss = hl;
+        if (loss) *loss = g->mail->loss;
         return RGR_OK;
     }
     RGR_CUDA(cudaMemcpyAsync(g->test.count, &n, 4, cudaMemcpyHostToDevice, st));
@@ -390,7 +389,8 @@ int rgr_guide_train_device_async(rgr_guide* g, const float* samples, uint32_t n,
     RGR_CUDA(cudaSetDevice(g->device));
     cudaStream_t st = (cudaStream_t)stream;
     if (g->cfg.training_kernel == RGR_GUIDE_TCGEN05) {
-        g->iteration_launches(samples, nullptr, n, g->test, nullptr, weight_scale, train_grid(*g, n), true, nullptr, st);
+        g->iteration_launches(samples, nullptr, n, g->test, nullptr, weight_scale, train_grid(*g, n), true, nullptr, nullptr,
+                              st);
         RGR_CUDA(cudaGetLastError());
         return RGR_OK;
     }

@@ -4,6 +4,7 @@
 #pragma once
 #include "../kernels/guide.cuh"
 #include "devbuf.h"
+#include "mail.h"
 
 struct rgr_guide {
     int device = 0;
@@ -18,6 +19,8 @@ struct rgr_guide {
     rgr::dev::GuideTrainD train{};  // the render's stream (counter bytes 0..27)
     rgr::dev::GuideTrainD test{};   // rgr_guide_train_device's (bytes 32..59; shares iter)
     bool bounds_set = false;
+    rgr::Mail* mail = nullptr;  // the last training step's loss
+    ~rgr_guide() { rgr::give_mail(mail); }
 
     int init(const rgr_guide_config& c);
     int set_bounds(const float lo[3], const float hi[3]);
@@ -35,5 +38,6 @@ struct rgr_guide {
     // one iteration with the tcgen05 kernels over min(*count, n) samples (n with count null):
     // gradients to `grads` if given; with `step`, Adam and the bookkeeping of t; `grid` CTAs
     void iteration_launches(const float* samples, const uint32_t* count, uint32_t n, const rgr::dev::GuideTrainD& t,
-                            const float* wsum, float weight_scale, int grid, bool step, float* grads, cudaStream_t st);
+                            const float* wsum, float weight_scale, int grid, bool step, float* grads, float* host_loss,
+                            cudaStream_t st);
 };

@@ -347,10 +347,11 @@ void launch_guide_train_tc(const GuideView& g, const float* samples, const uint3
                            uint32_t* err, cudaStream_t st);
 // What follows it: the sum of the grid's slots, in a fixed order, as the gradients (to
 // `grads`, kGuideParams floats, if given) and the loss (g.loss[1]); with `step` also Adam
-// (iteration number *t.iter + 1) and the iteration's bookkeeping in t.
+// (iteration number *t.iter + 1) and the iteration's bookkeeping in t.  host_loss: also gets
+// the loss (pinned host memory), if given.
 void launch_guide_update_tc(const GuideView& g, const float* part, uint32_t nparts, const uint32_t* count,
                             uint32_t cap, float* grads, bool step, const GuideAdam& adam, const GuideTrainD& t,
-                            cudaStream_t st);
+                            float* host_loss, cudaStream_t st);
 
 // tcgen05 / TMEM inference (guide_tc.cu): same results as the mma.sync kernels up
 // to FP32 accumulation order; a timed-out tensor-core wait sets bit 0 of *err
