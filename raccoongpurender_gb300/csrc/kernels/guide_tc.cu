@@ -371,7 +371,7 @@ __device__ __forceinline__ RowIn load_row(const PathsView& P, const float* rows,
     }
     if (kPaths) return RowIn{P.ro[slot], P.rd[slot], P.ng[slot]};
     const float4* p = reinterpret_cast<const float4*>(rows + 16 * (size_t)r);
-    return RowIn{p[0], p[1], p[2]};
+    return RowIn{__ldcs(p), __ldcs(p + 1), __ldcs(p + 2)};
 }
 // the network's input: hit point, normal facing the outgoing direction (zero
 // inside a volume), outgoing direction; or the row's first 9 floats
@@ -422,10 +422,11 @@ __device__ __forceinline__ void issue_layer(uint32_t l, uint32_t tm, uint32_t ta
 // Tile k of group g is tile (blockIdx.x + k gridDim.x) kTcGroups + g of the rows.
 template <bool kPaths, bool kInner>
 __global__ void __launch_bounds__(kTcThreads, 1)
-    k_guide_infer_tc(GuideView gv, const float* __restrict__ rows, uint32_t nrows, float* __restrict__ out,
+    k_guide_infer_tc(GuideView gv, const float* rows, uint32_t nrows, float* out,
                      PathsView P, QueueView Q, GuideRenderD gd, const RequestD* inner, uint32_t* err) {
     extern __shared__ unsigned char smem_raw[];
     SmemTc& S = *reinterpret_cast<SmemTc*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    if (kPaths) follow();
     const uint32_t n = kPaths ? guide_rows(Q, gd) : nrows;
     if (blockIdx.x * kCtaRows >= n) return;
     const uint32_t t = threadIdx.x, lt = t & 127u;
@@ -443,6 +444,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&S.d_full[i])) : "memory");
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&S.tmem_base)),
+                     "r"(kTcCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    if (!kPaths) follow();  // the barriers and the tensor memory are this kernel's own
+    if (t == 32u * kMmaWarp) {
         // the weights and bias chunks, already in the staged layout (wt_sw), by
         // one bulk copy completing on wbar's first phase
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(&S.wbar)),
@@ -453,12 +463,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 smem_u32(S.wt)),
             "l"(gv.wt_sw), "r"(kGuideWtBytes), "r"(smem_u32(&S.wbar))
             : "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&S.tmem_base)),
-                     "r"(kTcCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     const uint32_t ntiles = (n + 127u) / 128u, stride = gridDim.x * kTcGroups;
     // tiles of group gg: tile k is base + k stride while below ntiles
@@ -659,18 +663,16 @@ void launch_guide_infer_tc(const GuideView& g, const float* rows, uint32_t n, fl
     if (n == 0) return;
     const uint32_t need = (n + kCtaRows - 1u) / kCtaRows;
     if ((uint32_t)grid > need) grid = (int)need;
-    k_guide_infer_tc<false, false>
-        <<<grid, kTcThreads, guide_tc_smem(), st>>>(g, rows, n, out, PathsView{}, QueueView{}, GuideRenderD{}, nullptr, err);
+    chain(k_guide_infer_tc<false, false>, grid, kTcThreads, guide_tc_smem(), st, g, rows, n, out, PathsView{}, QueueView{},
+          GuideRenderD{}, nullptr, err);
 }
 
 void launch_guide_infer_paths_tc(const GuideView& g, const PathsView& p, const QueueView& q, const GuideRenderD& gd,
                                  const RequestD* inner, int grid, uint32_t* err, cudaStream_t st) {
     if (inner)
-        k_guide_infer_tc<true, true>
-            <<<grid, kTcThreads, guide_tc_smem(), st>>>(g, nullptr, 0, nullptr, p, q, gd, inner, err);
+        chain(k_guide_infer_tc<true, true>, grid, kTcThreads, guide_tc_smem(), st, g, nullptr, 0u, nullptr, p, q, gd, inner, err);
     else
-        k_guide_infer_tc<true, false>
-            <<<grid, kTcThreads, guide_tc_smem(), st>>>(g, nullptr, 0, nullptr, p, q, gd, nullptr, err);
+        chain(k_guide_infer_tc<true, false>, grid, kTcThreads, guide_tc_smem(), st, g, nullptr, 0u, nullptr, p, q, gd, nullptr, err);
 }
 
 }  // namespace dev

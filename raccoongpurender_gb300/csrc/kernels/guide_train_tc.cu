@@ -785,7 +785,7 @@ __global__ void __launch_bounds__(32 * kReduceWarps)
     k_guide_update_tc(GuideView g, const float* part, uint32_t nparts, const uint32_t* count, uint32_t cap,
                       float* __restrict__ grads, int step, GuideAdam adam, GuideTrainD t, float* host_loss) {
     // the training kernel's slots are written from here on (and so not read through the read-only path)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    follow();
     const uint32_t n = count ? *count : cap;
     if (n == 0u || (step && n < t.min_count)) {  // no iteration
         if (step && blockIdx.x == 0 && threadIdx.x == 0) finish_iteration(g, t, n);
@@ -843,16 +843,8 @@ void launch_guide_train_tc(const GuideView& g, const float* samples, const uint3
 void launch_guide_update_tc(const GuideView& g, const float* part, uint32_t nparts, const uint32_t* count,
                             uint32_t cap, float* grads, bool step, const GuideAdam& adam, const GuideTrainD& t,
                             float* host_loss, cudaStream_t st) {
-    cudaLaunchConfig_t cfg{};  // its blocks come up while the training kernel's last still run
-    cfg.gridDim = dim3((kGuideParams + kReduceParams) / kReduceParams);
-    cfg.blockDim = dim3(32 * kReduceWarps);
-    cfg.stream = st;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_guide_update_tc, g, part, nparts, count, cap, grads, step ? 1 : 0, adam, t, host_loss);
+    chain(k_guide_update_tc, (kGuideParams + kReduceParams) / kReduceParams, 32 * kReduceWarps, 0, st, g, part, nparts,
+          count, cap, grads, step ? 1 : 0, adam, t, host_loss);
 }
 
 }  // namespace dev

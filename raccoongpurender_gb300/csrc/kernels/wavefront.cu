@@ -717,16 +717,6 @@ __global__ void k_init(PathsView P, QueueView Q, uint32_t seed_offset, InitView 
     P.req[i] = 0;
 }
 
-// The kernels of a bounce follow one another as programmatic dependent launches: the next
-// kernel's blocks are brought up as the last of this one's end, and wait, here, until it
-// has finished and its stores are visible.  Every thread of each kernel calls it first,
-// so that a kernel's end is also that of all before it.  Only the scene's tables are read
-// through the read-only path.  Whole renders at 2^15 / 2^18 paths 884 / 1705 us without,
-// 866 / 1680 with (36 triangles), eight requests 3654 and 3590; with griddepcontrol.launch_dependents
-// right after the wait 1068 / 1741 and 3610 (the waiting blocks crowd onto the SMs that happen to have
-// room).
-RGR_DEV void follow() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // Ordered compaction of new-path slots: block t owns slots [t*4096, (t+1)*4096).  The last
 // block starts the bounce: it takes the queues' counts for the kernels up to the cast, and
 // clears them for the logic, and the cast's counter; the shading kernel clears the tile
@@ -1751,28 +1741,13 @@ __global__ void k_debug_slots(PathsView P, uint32_t* out) {
 
 }  // namespace
 
-// launches a kernel that begins with follow()
-template <class... P, class... A>
-static void chain(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, const A&... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.stream = st;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
-}
-
 void launch_init(const PathsView& p, const QueueView& q, uint32_t seed_offset, const InitView& w, const RequestD& one,
                  cudaStream_t st) {
     uint32_t n = q.ntiles * kTile;
     k_init<<<(n + 255) / 256, 256, 0, st>>>(p, q, seed_offset, w, one);
 }
 void launch_compact_new(const PathsView& p, const QueueView& q, unsigned long long* cast_counter, cudaStream_t st) {
-    chain(k_compact_new, q.ntiles, 256, st, p, q, cast_counter);
+    chain(k_compact_new, q.ntiles, 256, 0, st, p, q, cast_counter);
 }
 void launch_guide_select(const PathsView& p, const QueueView& q, const GuideRenderD& gd, bool inner, int grid,
                          cudaStream_t st) {
@@ -1782,18 +1757,18 @@ void launch_guide_select(const PathsView& p, const QueueView& q, const GuideRend
 
 void launch_shade(const PathsView& p, const QueueView& q, const RenderParams& rp, int grid, cudaStream_t st) {
     if (rp.gd.lobes)
-        chain(k_shade_guided, grid, 256, st, p, q, rp);
+        chain(k_shade_guided, grid, 256, 0, st, p, q, rp);
     else
-        chain(k_shade, grid, 256, st, p, q, rp);
+        chain(k_shade, grid, 256, 0, st, p, q, rp);
 }
 template <bool kInner>
 static void cast_paths(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
                        cudaStream_t st) {
     if (ts.one && rp.nreq == 1)
-        chain(k_trace_paths<kInner, true>, ts.grid, kStackThreads, st, p, q, rp, ts.counter, ts.refill, ts.search,
+        chain(k_trace_paths<kInner, true>, ts.grid, kStackThreads, 0, st, p, q, rp, ts.counter, ts.refill, ts.search,
               *ts.one);
     else
-        chain(k_trace_paths<kInner, false>, ts.grid, kStackThreads, st, p, q, rp, ts.counter, ts.refill, ts.search,
+        chain(k_trace_paths<kInner, false>, ts.grid, kStackThreads, 0, st, p, q, rp, ts.counter, ts.refill, ts.search,
               SceneView{});
 }
 
@@ -1806,15 +1781,15 @@ template <bool kGuided>
 static void trace_logic(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
                         int num_sms, cudaStream_t st) {
     if (ts.persistent) {
-        chain(k_logic<kGuided>, (p.n + kLogicThreads - 1) / kLogicThreads, kLogicThreads, st, p, q, rp);
+        chain(k_logic<kGuided>, (p.n + kLogicThreads - 1) / kLogicThreads, kLogicThreads, 0, st, p, q, rp);
         return;
     }
     const uint32_t span = p.n <= kCastSpan / 2 * (uint32_t)(num_sms * kCastLogicBlocks) ? kCastSpan / 2 : kCastSpan;
     const unsigned nb = (p.n + span - 1) / span;
     if (ts.one && rp.nreq == 1)
-        chain(k_cast_logic<kGuided, true>, nb, kLogicThreads, st, p, q, rp, span, ts.refill, ts.search, *ts.one);
+        chain(k_cast_logic<kGuided, true>, nb, kLogicThreads, 0, st, p, q, rp, span, ts.refill, ts.search, *ts.one);
     else
-        chain(k_cast_logic<kGuided, false>, nb, kLogicThreads, st, p, q, rp, span, ts.refill, ts.search, SceneView{});
+        chain(k_cast_logic<kGuided, false>, nb, kLogicThreads, 0, st, p, q, rp, span, ts.refill, ts.search, SceneView{});
 }
 
 void launch_trace_logic(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
@@ -1839,22 +1814,22 @@ void launch_inner_cast(const PathsView& p, const QueueView& q, const RenderParam
 
 void launch_inner_queues(const PathsView& p, const QueueView& q, const InnerView& in, const RenderParams& rp,
                          const TraceShape& ts, bool boundary, int num_sms, cudaStream_t st) {
-    chain(k_classify, q.ntiles, kClassifyThreads, st, p, q, in, rp, ts.counter, boundary ? 1 : 0);
+    chain(k_classify, q.ntiles, kClassifyThreads, 0, st, p, q, in, rp, ts.counter, boundary ? 1 : 0);
     const int blocks = std::min((int)((p.n + 255) / 256), num_sms * kNewPathsBlocks);
-    chain(k_new_paths, blocks, 256, st, p, q, in, rp);
+    chain(k_new_paths, blocks, 256, 0, st, p, q, in, rp);
 }
 
 void launch_inner_shade(const PathsView& p, const QueueView& u, const RenderParams& rp, const TraceShape& ts,
                         int shade_grid, cudaStream_t st) {
     if (rp.gd.lobes)
-        chain(k_shade_inner<true>, shade_grid, 256, st, p, u, rp);
+        chain(k_shade_inner<true>, shade_grid, 256, 0, st, p, u, rp);
     else
-        chain(k_shade_inner<false>, shade_grid, 256, st, p, u, rp);
+        chain(k_shade_inner<false>, shade_grid, 256, 0, st, p, u, rp);
     cast_paths<true>(p, u, rp, ts, st);
 }
 
 void launch_stamp_done(const RenderParams& rp, cudaStream_t st) {
-    if (rp.nreq > 0) chain(k_stamp_done, (rp.nreq + 127) / 128, 128, st, rp);
+    if (rp.nreq > 0) chain(k_stamp_done, (rp.nreq + 127) / 128, 128, 0, st, rp);
 }
 
 int trace_paths_max_blocks_per_sm(bool one) {
