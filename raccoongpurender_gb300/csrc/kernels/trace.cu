@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
+    if (kFew) follow();  // calls of few, one after another: the next one's blocks are there already
     const uint64_t pol = l2_evict_last_policy();
     extern __shared__ float4 s_nodes[];
     StagedNodes stn{s_nodes, 0u};
@@ -430,7 +431,8 @@ namespace {
 // longest ray's steps, so its rays are spread over the warps, ceil(n / warps) each,
 // without the counter and its reset, and go on lane by lane: 1000 / 6000 / 20000 random
 // rays in a 20 K-triangle scene, calls in a row, 57.5 / 69.2 / 70.7 us in whole warps,
-// 35.1 / 43.3 / 60.0 spread, 24.9 / 34.9 / 53.7 with the next links brought into L1 (touch).
+// 35.1 / 43.3 / 60.0 spread, 24.9 / 34.9 / 53.7 with the next links brought into L1 (touch),
+// 21.7 / 31.3 / 49.4 as dependent launches.
 // From there on whole warps win (60,000: 79 us, 91 spread ten a warp).  Returns the rays
 // a warp, 0 for the counter, which it resets; *blocks: at most `grid`.
 constexpr uint64_t kFewRays = 4;
@@ -457,7 +459,7 @@ void launch_trace_rays(const SceneView& sc, const float* ox, const float* oy, co
     RayBatch b{ox, oy, oz, dx, dy, dz, tmax, nullptr, n, prim, t, ng, nullptr, nullptr, err, counter, share, tune,
                stage};
     if (share)
-        k_trace_rays<false, false, false, true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
+        chain(k_trace_rays<false, false, false, true, false>, blocks, kStackThreads, 0, st, sc, b);
     else if (stage > 0)
         k_trace_rays<false, true, false, false, false><<<blocks, kStackThreads, 64 * (size_t)stage, st>>>(sc, b);
     else
@@ -474,7 +476,7 @@ void launch_trace_rays_link(const SceneView& sc, const float* const* rays, uint6
     RayBatch b{rays[0], rays[1], rays[2], rays[3], rays[4], rays[5], rays[6], nullptr, n, prim, t, nullptr,
                nullptr, nullptr, err, counter, share, tune, 0u};
     if (share)
-        k_trace_rays<false, false, false, true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
+        chain(k_trace_rays<false, false, false, true, false>, blocks, kStackThreads, 0, st, sc, b);
     else
         k_trace_rays<false, false, false, false, true><<<blocks, kStackThreads, 0, st>>>(sc, b);
 }
@@ -489,7 +491,7 @@ void launch_trace_rays_counts(const SceneView& sc, const float* ox, const float*
     RayBatch b{ox, oy, oz, dx, dy, dz, tmax, nullptr, n, prim, t, nullptr, nodes, prims, err, counter, share, CastTuning{16, 1, 16, 1},
                0u};
     if (share)
-        k_trace_rays<true, false, false, true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
+        chain(k_trace_rays<true, false, false, true, false>, blocks, kStackThreads, 0, st, sc, b);
     else
         k_trace_rays<true, false, false, false, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
 }
@@ -528,14 +530,10 @@ void launch_trace_packed(const SceneView& sc, const float4* packed, uint64_t n, 
                          uint32_t* err, unsigned long long* counter, const CastTuning& tune, int grid,
                          cudaStream_t st) {
     if (n == 0) return;
-    int blocks;
-    const uint32_t share = spread(n, grid, &blocks, counter, st);
+    cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);  // sorted calls are not few
     RayBatch b{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, packed, n, prim, t, ng, nullptr,
-               nullptr, err, counter, share, tune, 0u};
-    if (share)
-        k_trace_rays<false, false, true, true, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
-    else
-        k_trace_rays<false, false, true, false, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
+               nullptr, err, counter, 0u, tune, 0u};
+    k_trace_rays<false, false, true, false, false><<<grid, kStackThreads, 0, st>>>(sc, b);
 }
 
 int trace_rays_max_blocks_per_sm(uint32_t stage) {

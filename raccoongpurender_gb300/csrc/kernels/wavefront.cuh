@@ -169,11 +169,11 @@ constexpr uint32_t kFlagFixBacksideEnvPdf = 1u;
 // reflect a BSDF sample).  Always on in guided renders.
 constexpr uint32_t kFlagTwoSidedLambertian = 2u;
 
-// The kernels of a bounce follow one another as programmatic dependent launches: the next
-// kernel's blocks are brought up as the last of this one's end, and wait, here, until it
-// has finished and its stores are visible.  Every thread of each kernel calls it before it
-// touches memory, so that a kernel's end is also that of all before it.  Only the scene's tables are read
-// through the read-only path.  Whole renders at 2^15 / 2^18 paths 884 / 1705 us without,
+// The kernels of a bounce, the guide's and calls of few rays follow one another as programmatic
+// dependent launches: the next kernel's blocks are brought up as the last of this one's end,
+// and wait, here, until it has finished and its stores are visible.  Every thread of each kernel
+// calls it before it touches memory, so that a kernel's end is also that of all before it.  Only
+// the scene's tables, which an upload waits for, are read through the read-only path.  Whole renders at 2^15 / 2^18 paths 884 / 1705 us without,
 // 866 / 1680 with (36 triangles), eight requests 3654 and 3590; with griddepcontrol.launch_dependents
 // right after the wait 1068 / 1741 and 3610 (the waiting blocks crowd onto the SMs that happen to have
 // room).
