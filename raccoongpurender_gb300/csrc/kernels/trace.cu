@@ -433,9 +433,10 @@ namespace {
 // rays in a 20 K-triangle scene, calls in a row, 57.5 / 69.2 / 70.7 us in whole warps,
 // 35.1 / 43.3 / 60.0 spread, 24.9 / 34.9 / 53.7 with the next links brought into L1 (touch),
 // 21.7 / 31.3 / 49.4 as dependent launches.
-// From there on whole warps win (60,000: 79 us, 91 spread ten a warp).  Returns the rays
-// a warp, 0 for the counter, which it resets; *blocks: at most `grid`.
-constexpr uint64_t kFewRays = 4;
+// 30,000 / 40,000: 58.5 / 60.5 us in whole warps, 52.0 / 57.9 so (1.31M triangles 99.7 / 100.3 and
+// 89.2 / 92.4); from there on whole warps win (55,000: 64 us, 71.5 spread ten a warp; 156 and 165).
+// Returns the rays a warp, 0 for the counter, which it resets; *blocks: at most `grid`.
+constexpr uint64_t kFewRays = 8;
 uint32_t spread(uint64_t n, int grid, int* blocks, unsigned long long* counter, cudaStream_t st) {
     const uint64_t per = kStackThreads / 32, warps = (uint64_t)grid * per;
     *blocks = grid;

@@ -26,7 +26,8 @@ def _hits(lane, rays):
     return prim[:n].cpu().numpy(), t[:n].cpu().numpy(), ng[:n].cpu().numpy()
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 33, WARPS - 1, WARPS, WARPS + 1, 4 * WARPS, 4 * WARPS + 1, 65535, 65536, 65537,
+@pytest.mark.parametrize("n", [1, 2, 31, 33, WARPS - 1, WARPS, WARPS + 1, 4 * WARPS, 4 * WARPS + 1,
+                               8 * WARPS, 8 * WARPS + 1, 65535, 65536, 65537,
                                131071])
 def test_counts(rg, po, n):
     mesh = scenes.displaced_icosphere(5, seed=7)
@@ -66,7 +67,7 @@ def test_far_clip(rg, po, tmax, n):
 
 
 @pytest.mark.parametrize("leaf", [1, 4, 8])
-@pytest.mark.parametrize("n", [5, 4 * WARPS, 5 * WARPS])
+@pytest.mark.parametrize("n", [5, 8 * WARPS, 9 * WARPS])
 def test_deep_tree(rg, po, n, leaf):
     """Triangles at distances that double from one to the next, whose boxes the rays pass
     from the smallest on: more pending links than the stack's entries in shared memory, in
@@ -95,7 +96,7 @@ def test_deep_tree(rg, po, n, leaf):
 
 
 @pytest.mark.parametrize("refill", [1, 7, 16, 32])
-@pytest.mark.parametrize("n", [4 * 152 * 8 + 1, 100001])
+@pytest.mark.parametrize("n", [8 * 152 * 8 + 1, 100001])
 def test_host_runs(rg, po, refill, n):
     """Hits written across the link in runs: short runs and whole ones, more open than a warp
     keeps, a last run cut by the end."""
