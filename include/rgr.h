@@ -357,8 +357,8 @@ int rgr_set_trace_search(rgr_context* c, int32_t closest, int32_t render);
 /* Shared-memory staging of the closest-hit kernel: each CTA copies the first
    staged_nodes (0..1024) inner nodes — the top levels of the tree, which the
    builder stores first in breadth-first order — into shared memory and reads
-   them from there (64 bytes each; more staging means fewer resident CTAs).
-   0 = off.  Chosen by the autotuner. */
+   them from there (64 bytes each; more staging means fewer resident CTAs).  Calls of
+   few rays, sorted calls and calls across the link do not stage.  0 = off.  Chosen by the autotuner. */
 int rgr_set_trace_staging(rgr_context* c, uint32_t staged_nodes);
 
 /* Ray reordering of rgr_trace_closest_device (no counterpart in the
