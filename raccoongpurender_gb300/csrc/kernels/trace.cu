@@ -9,11 +9,11 @@
 // rounds, hands finished lanes new rays from a global counter (one atomic per
 // refill per warp).  Within a round the lanes take node steps while at least
 // `search` of them still search for their next leaf; the others wait at
-// theirs.  A warp left with a few rays, and a call of few rays, which is spread over
-// the warps instead, go on lane by lane (kTailLanes, spread).  Rays are read and results written with streaming (evict-first)
-// cache hints; the tree is read with an L2 evict-last policy.
-// Each ray's traversal is unchanged, so results do not depend on the
-// schedule.
+// theirs.  A warp left with a few rays, and a call of few rays, which is spread
+// over the warps instead, go on lane by lane (kTailLanes, spread).  Rays are read
+// and results written with streaming (evict-first) cache hints; the tree is
+// read with an L2 evict-last policy.  Each ray's traversal is unchanged, so results
+// do not depend on the schedule.
 //
 // Ray reordering (optional, for incoherent rays): a counting sort by a 16-bit
 // key puts rays that start close together and head the same way next to each

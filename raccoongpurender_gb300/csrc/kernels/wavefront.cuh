@@ -173,10 +173,10 @@ constexpr uint32_t kFlagTwoSidedLambertian = 2u;
 // dependent launches: the next kernel's blocks are brought up as the last of this one's end,
 // and wait, here, until it has finished and its stores are visible.  Every thread of each kernel
 // calls it before it touches memory, so that a kernel's end is also that of all before it.  Only
-// the scene's tables, which an upload waits for, are read through the read-only path.  Whole renders at 2^15 / 2^18 paths 884 / 1705 us without,
-// 866 / 1680 with (36 triangles), eight requests 3654 and 3590; with griddepcontrol.launch_dependents
-// right after the wait 1068 / 1741 and 3610 (the waiting blocks crowd onto the SMs that happen to have
-// room).
+// the scene's tables, which an upload waits for, are read through the read-only path.  Whole
+// renders at 2^15 / 2^18 paths 884 / 1705 us without, 866 / 1680 with (36 triangles), eight
+// requests 3654 and 3590; with griddepcontrol.launch_dependents right after the wait 1068 /
+// 1741 and 3610 (the waiting blocks crowd onto the SMs that happen to have room).
 __device__ __forceinline__ void follow() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // launches a kernel that calls follow()
@@ -293,7 +293,8 @@ void launch_guide_select(const PathsView& p, const QueueView& q, const GuideRend
 // lanes are idle, node steps while `search` lanes still search for a leaf,
 // `grid` CTAs, `counter` a device word it may use; launch_trace_paths, between
 // the shading kernel and the queue resets), then the logic kernel; otherwise
-// one kernel casts and runs the logic (launch_trace_paths does nothing).  `one`: the scene of a render of a single request, or null.
+// one kernel casts and runs the logic (launch_trace_paths does nothing).
+// `one`: the scene of a render of a single request, or null.
 struct TraceShape {
     bool persistent;
     int refill;
