@@ -598,7 +598,7 @@ class WavefrontLane:
 
     def set_render_trace(self, persistent=-1, refill: int = 12) -> None:
         """Extension rays of a bounce: persistent refilling kernel + logic (True),
-        fused (False), or by the pool's size (-1, the default)."""
+        fused (False), or by how many paths can be in flight (-1, the default)."""
         mode = persistent if isinstance(persistent, int) and not isinstance(persistent, bool) else int(bool(persistent))
         _check(self._lib.rgr_set_render_trace(self._h, mode, refill), "rgr_set_render_trace")
 
@@ -822,7 +822,7 @@ class Batch:
 
     def set_render_trace(self, refill: int = 12) -> None:
         """Refill threshold of the bounce's persistent closest-hit kernel (the
-        kernel is chosen by the pool's size, as for a single render)."""
+        kernel is chosen by the paths in flight, as for a single render)."""
         _check(self._lib.rgr_set_render_trace(self._lib.rgr_batch_context(self._h), -1, refill),
                "rgr_set_render_trace")
 

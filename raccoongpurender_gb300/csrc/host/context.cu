@@ -16,6 +16,7 @@
 
 #include "../kernels/wavefront.cuh"
 #include "../rgr_internal.h"
+#include "choices.h"
 #include "devbuf.h"
 #include "guide_host.h"
 #include "mail.h"
@@ -175,14 +176,6 @@ void populate(std::initializer_list<void*> arrays, size_t bytes) {
 
 }  // namespace
 
-// Pools of fewer paths run the fused cast + logic kernel by default (a bounce is then
-// bound by its launches' latency and its longest rays), larger ones the
-// persistent refilling cast and, inside a run of bounces, no logic pass (launch_inner_queues).
-// Whole renders (4 spp, depth 6), persistent against fused, at 2^15 / 2^17 / 2^18 / 3 * 2^17 /
-// 2^19 / 2^20 paths: 36 triangles 0.81 / 0.86 / 1.02 / 1.14 / 1.14 / 1.24x, 5 K 0.73 / 0.84 / 0.94 /
-// 1.09 / 1.12 / 1.30x, 80 K 0.78 / 0.86 / 0.92 / 1.10 / 1.17 / 1.34x.  Single bounces at 2^17 / 2^18 /
-// 3 * 2^17 / 2^20: 36 triangles 0.89 / 0.97 / 1.10 / 1.06x, 5 K 0.89 / 0.96 / 1.06 / 1.16x.
-constexpr uint32_t kPersistentTraceMinPaths = 3u << 17;
 // rgr_trace_closest: 2^20-ray chunks in flight on their own streams, so that
 // the copies of some overlap the traversal of another (measured end to end
 // on the closest-hit workload: 2 slots 2500 Mrays/s, 3: 2647, 4: 2705-2728,
@@ -247,7 +240,7 @@ struct rgr_context {
     // 1059.5 Mpaths/s with a warp refilled at 24 / 8 / 12 / 16 / 20 idle lanes
     // search 8: 1114.8 Mpaths/s against 1032.8 with every lane waiting for the last
     TraceShape render_trace{true, 12, 8, 0, nullptr, nullptr};
-    int render_trace_mode = -1;  // 1 persistent, 0 fused, -1 by the pool's size at render begin
+    int render_trace_mode = -1;  // 1 persistent, 0 fused, -1 by the paths in flight, at render begin
     uint32_t trace_stage = 0;  // top BVH nodes staged in shared memory per CTA
     int trace_reorder = 0;     // rgr_trace_closest_device sorts the rays first
     int packed_grid = 0;       // its traversal grid (no staged nodes)
@@ -310,8 +303,7 @@ struct rgr_context {
         cudaStream_t st = stream;
         int r;
         render_trace.grid = num_sms * cast_blocks[render_trace.one != nullptr];
-        render_trace.persistent =
-            render_trace_mode < 0 ? npaths >= kPersistentTraceMinPaths : render_trace_mode != 0;
+        render_trace.persistent = persistent_cast(render_trace_mode, npaths, limit);
         if ((r = reqtab.alloc(sizeof(RequestD) * nreq)) != RGR_OK) return r;
         rp.reqs = reqtab.as<RequestD>();
         rp.nreq = nreq;

@@ -28,6 +28,7 @@
 
 #include <algorithm>
 
+#include "../host/choices.h"
 #include "wavefront.cuh"
 #include "traverse.cuh"
 #include "guide.cuh"
@@ -1310,14 +1311,11 @@ __global__ void __launch_bounds__(kLogicThreads, kGuided ? 5 : RGR_LOGIC_MIN_BLO
 // and now: 5 K triangles 2028 / 2643 / 3794 us and 1963 / 2596 / 3400, 80 K triangles
 // 1536 / 1954 / 2699 and 1414 / 1775 / 2243; 36 triangles 883 / 1264 / 1808 and
 // 939 / 1283 / 1783 (a ray is over before the list pays).
-// 4 blocks an SM: 5 the same to 2 % slower.  `span`: 256 while the blocks are one wave,
-// else 512 (256 against 512 at 2^17: 2596 / 2646 us in 5 K triangles, 1775 / 1851 in
-// 80 K; at 2^18 3807 / 3400 and 2538 / 2243).
+// 4 blocks an SM: 5 the same to 2 % slower.  half_end: the slots below it go half a span a block.
 constexpr int kCastLogicBlocks = 4;
-constexpr uint32_t kCastSpan = 512;
 template <bool kGuided, bool kOne>
 __global__ void __launch_bounds__(kLogicThreads, kCastLogicBlocks)
-    k_cast_logic(PathsView P, QueueView Q, RenderParams rp, uint32_t span, int refill, int search, SceneView one) {
+    k_cast_logic(PathsView P, QueueView Q, RenderParams rp, uint32_t half_end, int refill, int search, SceneView one) {
     follow();
     const unsigned full = 0xffffffffu;
     __shared__ uint32_t s_stack[(kSmemStack + 1) * kStackThreads];  // the last row: see touch
@@ -1327,7 +1325,10 @@ __global__ void __launch_bounds__(kLogicThreads, kCastLogicBlocks)
     __shared__ uint32_t s_n, s_next;
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
-    const uint32_t first = blockIdx.x * span;
+    const uint32_t half_blocks = half_end / (kCastSpan / 2);
+    const bool half = blockIdx.x < half_blocks;
+    const uint32_t span = half ? kCastSpan / 2 : kCastSpan;
+    const uint32_t first = half ? blockIdx.x * (kCastSpan / 2) : half_end + (blockIdx.x - half_blocks) * kCastSpan;
     if (threadIdx.x == 0) s_n = s_next = 0u;
     __syncthreads();
     for (uint32_t o = threadIdx.x; o < span; o += kLogicThreads) {
@@ -1784,12 +1785,13 @@ static void trace_logic(const PathsView& p, const QueueView& q, const RenderPara
         chain(k_logic<kGuided>, (p.n + kLogicThreads - 1) / kLogicThreads, kLogicThreads, 0, st, p, q, rp);
         return;
     }
-    const uint32_t span = p.n <= kCastSpan / 2 * (uint32_t)(num_sms * kCastLogicBlocks) ? kCastSpan / 2 : kCastSpan;
-    const unsigned nb = (p.n + span - 1) / span;
+    const uint32_t half_end = cast_half_end(p.n, rp.sample_limit, (uint32_t)(num_sms * kCastLogicBlocks), kTile);
+    const unsigned nb = cast_blocks(p.n, half_end);
     if (ts.one && rp.nreq == 1)
-        chain(k_cast_logic<kGuided, true>, nb, kLogicThreads, 0, st, p, q, rp, span, ts.refill, ts.search, *ts.one);
+        chain(k_cast_logic<kGuided, true>, nb, kLogicThreads, 0, st, p, q, rp, half_end, ts.refill, ts.search, *ts.one);
     else
-        chain(k_cast_logic<kGuided, false>, nb, kLogicThreads, 0, st, p, q, rp, span, ts.refill, ts.search, SceneView{});
+        chain(k_cast_logic<kGuided, false>, nb, kLogicThreads, 0, st, p, q, rp, half_end, ts.refill, ts.search,
+              SceneView{});
 }
 
 void launch_trace_logic(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,

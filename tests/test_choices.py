@@ -1,0 +1,61 @@
+"""The rules by which calls choose their kernels (csrc/host/choices.h, plain C++),
+compiled and called on the host."""
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parents[1] / "raccoongpurender_gb300" / "csrc"
+WRAP = """
+#include "host/choices.h"
+extern "C" int persistent(int mode, uint64_t pool, uint64_t samples) {
+    return rgr::persistent_cast(mode, pool, samples);
+}
+extern "C" uint32_t half_end(uint64_t pool, uint64_t samples, uint32_t resident, uint32_t tile) {
+    return rgr::cast_half_end(pool, samples, resident, tile);
+}
+extern "C" uint32_t blocks(uint64_t pool, uint32_t half_end) { return rgr::cast_blocks(pool, half_end); }
+"""
+
+
+@pytest.fixture(scope="module")
+def choices(tmp_path_factory):
+    d = tmp_path_factory.mktemp("choices")
+    (d / "wrap.cpp").write_text(WRAP)
+    r = subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-shared", "-fPIC", f"-I{CSRC}", str(d / "wrap.cpp"),
+                        "-o", str(d / "choices.so")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    return C.CDLL(str(d / "choices.so"))
+
+
+@pytest.mark.parametrize("pool,samples,persistent", [
+    (3 << 17, 0, 1), ((3 << 17) - 1, 0, 0), (1 << 24, 0, 1),  # no budget: the pool counts
+    (649316, 20440, 0),                                       # a small image in a large pool
+    (1 << 24, (3 << 17) - 1, 0), (1 << 24, 3 << 17, 1),
+    (1 << 18, 1 << 30, 0), (1 << 20, 1 << 40, 1),
+])
+def test_cast_by_paths_in_flight(choices, pool, samples, persistent):
+    f = choices.persistent
+    assert f(-1, C.c_uint64(pool), C.c_uint64(samples)) == persistent
+    assert f(1, C.c_uint64(pool), C.c_uint64(samples)) == 1
+    assert f(0, C.c_uint64(pool), C.c_uint64(samples)) == 0
+
+
+@pytest.mark.parametrize("pool", [1, 255, 256, 257, 4096, 4097, 20000, 155648, 155649, 160000, 649316])
+@pytest.mark.parametrize("samples", [0, 1, 2880, 4096, 4097, 20440, 155648, 155649, 1 << 40])
+def test_fused_blocks_cover_the_pool(choices, pool, samples):
+    """Every slot in one block, each block's slots in one tile; halves only while the paths in
+    flight fill no more than a wave of 608 blocks."""
+    span, tile = 512, 4096
+    half_end = choices.half_end(C.c_uint64(pool), C.c_uint64(samples), 608, tile)
+    inflight = min(pool, samples) if samples else pool
+    assert half_end == (-(-inflight // tile) * tile if inflight <= 256 * 608 else 0)
+    at = 0
+    for b in range(choices.blocks(C.c_uint64(pool), half_end)):  # as k_cast_logic finds its slots
+        half_blocks = half_end // (span // 2)
+        n = span // 2 if b < half_blocks else span
+        first = b * (span // 2) if b < half_blocks else half_end + (b - half_blocks) * span
+        assert first == at and first // tile == (first + n - 1) // tile
+        at += n
+    assert pool <= at < pool + span
