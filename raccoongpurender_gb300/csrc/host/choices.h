@@ -27,6 +27,15 @@ inline bool persistent_cast(int mode, uint64_t pool, uint64_t samples) {
     return paths_in_flight(pool, samples) >= kPersistentMinPaths;
 }
 
+// Scenes of at most so many primitives take the fused kernel with one thread a slot: a ray is
+// over before a list of the live slots pays.  Time with the list (k_cast_logic) over time with
+// one thread a slot, whole renders (8 spp, depth 6) in pools of 2^12 / 2^14 / 2^16 / 2^17 / 2^18
+// paths: 36 triangles 1.13 / 1.12 / 1.08 / 1.05 / 1.04, 600 spheres 1.12 / 1.11 / 1.07 / 1.05 / 1.07, 320
+// triangles 1.09 / 1.09 / 1.08 / 1.05 / 0.99; 1280 triangles in 2^14 / 2^16 / 2^17 / 2^18 1.05 / 1.04 /
+// 1.02 / 0.95, 5 K 1.00 / 0.99 / 0.99 / 0.91.
+constexpr uint32_t kPerSlotMaxPrims = 1024;
+inline bool per_slot_cast(uint32_t prims) { return prims <= kPerSlotMaxPrims; }
+
 // The blocks of the fused kernel (k_cast_logic) take kCastSpan slots each, those below
 // cast_half_end half as many: while the blocks of the paths in flight are one wave then (half
 // against all at 2^17 paths: 2596 / 2646 us in 5 K triangles, 1775 / 1851 in 80 K; at 2^18

@@ -304,6 +304,9 @@ struct rgr_context {
         int r;
         render_trace.grid = num_sms * cast_blocks[render_trace.one != nullptr];
         render_trace.persistent = persistent_cast(render_trace_mode, npaths, limit);
+        uint32_t prims = 0;
+        for (int k = 0; k < nreq; ++k) prims = std::max(prims, host_reqs[k].sc.num_prims);
+        render_trace.per_slot = per_slot_cast(prims);
         if ((r = reqtab.alloc(sizeof(RequestD) * nreq)) != RGR_OK) return r;
         rp.reqs = reqtab.as<RequestD>();
         rp.nreq = nreq;
@@ -574,7 +577,7 @@ struct rgr_context {
         add(&in, sizeof(in));
         add(&rp, sizeof(rp));
         add(&shade_grid, sizeof(shade_grid));
-        add(&render_trace.persistent, sizeof(render_trace.persistent));
+        for (const bool v : {render_trace.persistent, render_trace.per_slot}) add(&v, sizeof(v));
         for (const int v : {render_trace.refill, render_trace.search, render_trace.grid}) add(&v, sizeof(v));
         if (render_trace.one) add(render_trace.one, sizeof(SceneView));  // the cast's kernel argument
         add(&graph_steps, sizeof(graph_steps));

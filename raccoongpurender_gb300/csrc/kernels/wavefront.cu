@@ -1301,16 +1301,14 @@ __global__ void __launch_bounds__(kLogicThreads, kGuided ? 5 : RGR_LOGIC_MIN_BLO
     });
 }
 
-// Cast and logic of a bounce in one launch, for small pools.  A block takes the live ones
+// Cast and logic of a bounce in one launch, for few paths.  A block takes the live ones
 // of `span` consecutive slots of one tile: it lists them in shared memory, its warps cast
 // their rays (a warp takes the next rays of the list as its lanes fall idle, and
 // ends lane by lane, as in k_trace_paths), the hits stay in shared memory, and the logic
 // goes over the list.  Bound by instruction issue at few lanes and by the longest rays: with
-// one thread a slot, from its ray to its queue, 6 to 8 of a warp's lanes were in use,
-// now 12 to 15.  Whole renders (4 spp, depth 6) at 2^15 / 2^17 / 2^18 paths, one thread a slot
-// and now: 5 K triangles 2028 / 2643 / 3794 us and 1963 / 2596 / 3400, 80 K triangles
-// 1536 / 1954 / 2699 and 1414 / 1775 / 2243; 36 triangles 883 / 1264 / 1808 and
-// 939 / 1283 / 1783 (a ray is over before the list pays).
+// one thread a slot (k_slot_logic), 6 to 8 of a warp's lanes are in use, here 12 to 15.  Whole
+// renders (8 spp, depth 6) at 2^14 / 2^16 / 2^17 / 2^18 paths, time of one thread a slot over this:
+// 5 K triangles 1.00 / 1.01 / 1.01 / 1.10, 80 K 1.09 / 1.08 / 1.08 / 1.16.
 // 4 blocks an SM: 5 the same to 2 % slower.  half_end: the slots below it go half a span a block.
 constexpr int kCastLogicBlocks = 4;
 template <bool kGuided, bool kOne>
@@ -1393,6 +1391,32 @@ __global__ void __launch_bounds__(kLogicThreads, kCastLogicBlocks)
         });
         __syncthreads();  // before the counts are cleared again
     }
+}
+
+// The same for scenes whose rays are over before a list pays (per_slot_cast): one thread a
+// slot, from its ray to its queue.  Bound by latency: the longest ray of a warp, and the launches.
+template <bool kGuided, bool kOne>
+__global__ void __launch_bounds__(kLogicThreads, kCastLogicBlocks)
+    k_slot_logic(PathsView P, QueueView Q, RenderParams rp, SceneView one) {
+    follow();
+    __shared__ uint32_t s_stack[kSmemStack * kStackThreads];
+    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = slot < P.n && P.qid[slot] != kQueueIdle;
+    uint32_t err = 0;
+    TraceState s;
+    s.sstk = s_stack + threadIdx.x;
+    if (live) {
+        const SceneView& sc = kOne ? one : rp.reqs[P.req[slot]].sc;
+        float4 ro4, rd4;
+        ld_sector<0>(P, slot, ro4, rd4);
+        const uint64_t pol = l2_evict_last_policy();
+        trace_begin(sc, s, xyz(ro4), xyz(rd4), ro4.w);
+        while (s.link != kDone) trace_round<false, false, kSmemStack>(sc, s, nullptr, err, pol);
+    }
+    if (err) atomicOr(rp.err, err);
+    logic_block<kGuided>(Q, rp, slot, slot / kTile, live, [&](unsigned active, GuideOffer& go) {
+        return logic_slot<kGuided, false>(P, Q, rp, slot, active, go, hit_id(s.prim), s.tmin);
+    });
 }
 
 // The queues of a bounce inside a run, from the queue ids that the cast left: block t
@@ -1783,6 +1807,14 @@ static void trace_logic(const PathsView& p, const QueueView& q, const RenderPara
                         int num_sms, cudaStream_t st) {
     if (ts.persistent) {
         chain(k_logic<kGuided>, (p.n + kLogicThreads - 1) / kLogicThreads, kLogicThreads, 0, st, p, q, rp);
+        return;
+    }
+    if (ts.per_slot) {
+        const unsigned nb = (p.n + kLogicThreads - 1) / kLogicThreads;
+        if (ts.one && rp.nreq == 1)
+            chain(k_slot_logic<kGuided, true>, nb, kLogicThreads, 0, st, p, q, rp, *ts.one);
+        else
+            chain(k_slot_logic<kGuided, false>, nb, kLogicThreads, 0, st, p, q, rp, SceneView{});
         return;
     }
     const uint32_t half_end = cast_half_end(p.n, rp.sample_limit, (uint32_t)(num_sms * kCastLogicBlocks), kTile);

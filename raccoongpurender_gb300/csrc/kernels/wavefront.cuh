@@ -291,9 +291,9 @@ void launch_guide_select(const PathsView& p, const QueueView& q, const GuideRend
 // How a bounce casts its extension rays: persistent = a separate persistent
 // closest-hit kernel over the slots just shaded (warps refilled when `refill`
 // lanes are idle, node steps while `search` lanes still search for a leaf,
-// `grid` CTAs, `counter` a device word it may use; launch_trace_paths, between
-// the shading kernel and the queue resets), then the logic kernel; otherwise
-// one kernel casts and runs the logic (launch_trace_paths does nothing).
+// `grid` CTAs, `counter` a device word it may use; launch_trace_paths, after the
+// shading kernel), then the logic kernel; otherwise one kernel casts and runs the
+// logic (launch_trace_paths does nothing), with `per_slot` one thread a slot.
 // `one`: the scene of a render of a single request, or null.
 struct TraceShape {
     bool persistent;
@@ -302,6 +302,7 @@ struct TraceShape {
     int grid;
     unsigned long long* counter;
     const SceneView* one = nullptr;
+    bool per_slot = false;
 };
 void launch_trace_paths(const PathsView& p, const QueueView& q, const RenderParams& rp, const TraceShape& ts,
                                cudaStream_t st);

@@ -15,6 +15,7 @@ extern "C" int persistent(int mode, uint64_t pool, uint64_t samples) {
 extern "C" uint32_t half_end(uint64_t pool, uint64_t samples, uint32_t resident, uint32_t tile) {
     return rgr::cast_half_end(pool, samples, resident, tile);
 }
+extern "C" int per_slot(uint32_t prims) { return rgr::per_slot_cast(prims); }
 extern "C" uint32_t blocks(uint64_t pool, uint32_t half_end) { return rgr::cast_blocks(pool, half_end); }
 """
 
@@ -59,3 +60,7 @@ def test_fused_blocks_cover_the_pool(choices, pool, samples):
         assert first == at and first // tile == (first + n - 1) // tile
         at += n
     assert pool <= at < pool + span
+
+
+def test_small_scenes_cast_per_slot(choices):
+    assert [choices.per_slot(n) for n in (0, 36, 1024, 1025, 1 << 27)] == [1, 1, 1, 0, 0]
