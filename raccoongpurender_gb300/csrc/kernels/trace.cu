@@ -181,7 +181,9 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
                 if (kLink && base < b.n) {  // a run of the new rays
                     const int k = oldest;
                     oldest = (oldest + 1) % kRuns;
-                    if (runs.rays[k]) {
+                    const bool open = runs.rays[k] != 0u;
+                    __syncwarp();  // every lane has read it before lane 0 writes it
+                    if (open) {
                         flush(k);
                         if ((place >> 5) == k) place = -1;
                     }
