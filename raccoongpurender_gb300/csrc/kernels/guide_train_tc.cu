@@ -33,7 +33,7 @@
 //         writes dY_l-1)
 //   9     dW_0 += act_0^T . dY_0
 // Buffers per group: B1..B3 hold act_1..act_3; B0 holds act_0, then act_4
-// once layer 0 has run, then act_0 again (re-encoded) once dW_4 is done; BY
+// once layer 0 has run, then act_0 again (re-encoded) a turn after dW_4; BY
 // holds the output gradient of the current layer.  The two groups alternate on
 // the tensor core: while one waits for its MMAs the other runs its epilogue.
 //
@@ -723,7 +723,10 @@ __global__ void __launch_bounds__(kTrThreads, 1)
 #pragma unroll
                 for (uint32_t c = 0; c < 4u; ++c)
                     store_chunk(BY, lt, 4u * half + c, y[4 * c], y[4 * c + 1], y[4 * c + 2], y[4 * c + 3]);
-                if (l == 4) encode_half(v, half, B0, lt);  // act_0 back into B0 for dW_0
+                // act_0 back into B0 for dW_0.  It writes chunks whose act_4 the other half's
+                // thread reads above, at l = 4: that read comes before its warp's arrival at the
+                // next turn, and so before this turn's D
+                if (l == 3) encode_half(v, half, B0, lt);
             }
             if (timed_out) break;
             // turn 9: dW_0; its end frees B0 and BY for the next tile
