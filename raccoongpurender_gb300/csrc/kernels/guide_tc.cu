@@ -445,13 +445,16 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
+    // The barriers are this kernel's own; the tensor memory is not taken before a caller's kernel on
+    // the stream has ended: one that lets dependents start early and allocates its own after that
+    // could wait for ours, and we for its end.
+    if (!kPaths) follow();
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&S.tmem_base)),
                      "r"(kTcCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
-    if (!kPaths) follow();  // the barriers and the tensor memory are this kernel's own
     if (t == 32u * kMmaWarp) {
         // the weights and bias chunks, already in the staged layout (wt_sw), by
         // one bulk copy completing on wbar's first phase
