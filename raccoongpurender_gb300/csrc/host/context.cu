@@ -106,7 +106,7 @@ struct DeviceScene {
         v.env_h = e.present ? e.h : 0;
         v.has_env = e.present ? 1 : 0;
         bool small = true;
-        for (int k = 0; k < 6; ++k) small = small && std::fabs(b.bounds[k]) <= 1.0e30f;
+        for (int k = 0; k < 6; ++k) small = small && std::fabs(b.bounds[k]) <= kSmallCoord;
         v.small_coords = small ? 1 : 0;
         v.num_nodes = (uint32_t)b.nodes.size();
         // the hit normals, computed once here by the kernels' own function

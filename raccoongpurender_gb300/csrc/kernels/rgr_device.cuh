@@ -33,10 +33,6 @@ RGR_DEV f3 normalize(f3 v) {
     return mk(v.x / l, v.y / l, v.z / l);
 }
 RGR_DEV f3 xyz(float4 v) { return mk(v.x, v.y, v.z); }
-RGR_DEV bool is_finite_nonzero(float x) {
-    const uint32_t e = __float_as_uint(x) & 0x7fffffffu;
-    return e != 0u && e < 0x7f800000u;
-}
 RGR_DEV float4 f4(f3 v, float w) { return make_float4(v.x, v.y, v.z, w); }
 
 // ------------------------------------------------------------ RNG
@@ -71,6 +67,8 @@ template <class P>
 RGR_DEV void rng_store(const P& p, uint32_t i, const Rng& r) { p[i] = make_uint4(r.s0, r.s1, r.s2, r.s3); }
 
 // ------------------------------------------------------------ scene view
+// coordinates up to here, of scene, ray origin and direction, keep the traversal free of NaNs
+constexpr float kSmallCoord = 1.0e9f;
 struct SceneView {
     const float4* nodes;      // 4 float4 per inner node (NodeD)
     const float4* prims;      // 3 float4 per primitive record (PrimD)
@@ -94,7 +92,7 @@ struct SceneView {
     const float4* env_frag;     // w*h
     int32_t env_w, env_h;
     int32_t has_env;
-    int32_t small_coords;       // every scene coordinate within +-1e30 (no NaN in slab products)
+    int32_t small_coords;       // every scene coordinate within +-kSmallCoord (see ray_is_nan_free)
     uint32_t num_nodes;         // inner nodes
 };
 

@@ -25,6 +25,8 @@
 // BVH loads carry an L2 evict-last policy so that streaming ray data does not
 // push the tree out of L2.
 #pragma once
+#include <cfloat>
+
 #include "rgr_device.cuh"
 
 namespace rgr {
@@ -101,14 +103,17 @@ RGR_DEV bool slab(float lox, float loy, float loz, float hix, float hiy, float h
     return rmin <= rmax && 0.0f <= rmax && rmin <= farclip;
 }
 
-// (lo - ro) * inv is never NaN when ro is finite and small, every inv
-// component is finite and non-zero, and the scene box is small (checked on
-// the host): the difference is finite and the product of two finite non-zero
-// numbers is a number or an infinity.
+// Rays for which slab needs no NaN checks, in a scene whose coordinates are within +-kSmallCoord
+// (scene_small): neither (lo - ro) * inv nor a hit's distance, the far clip of the boxes after
+// it, is ever NaN.  The first: the difference is finite, inv neither 0 nor infinite.  The
+// second, with every |ro|, |rd| and |coordinate| <= S = 1e9 (|inv| >= 1 / S): in tri_test
+// |pvec| <= 4 S^2 = 4e18, |det| <= 2.4e28, so invDet, of a |det| >= 1e-8, is finite and not 0;
+// |tvec| <= 2 S, |qvec| <= 8 S^2, and u, v, t are sums of finite products below 4.8e28 times at most 1e8.
 RGR_DEV bool ray_is_nan_free(f3 ro, f3 inv, float tmax, bool scene_small) {
-    const float kBig = 1.0e30f;
-    return scene_small && tmax >= 0.0f && fabsf(ro.x) <= kBig && fabsf(ro.y) <= kBig && fabsf(ro.z) <= kBig &&
-           is_finite_nonzero(inv.x) && is_finite_nonzero(inv.y) && is_finite_nonzero(inv.z);
+    auto fits = [](float r, float i) {
+        return fabsf(r) <= kSmallCoord && fabsf(i) >= 1.0f / kSmallCoord && fabsf(i) <= FLT_MAX;
+    };
+    return scene_small && tmax >= 0.0f && fits(ro.x, inv.x) && fits(ro.y, inv.y) && fits(ro.z, inv.z);
 }
 
 // intersect_ray_triangle (intersect_triangle.cl:7-44) with precomputed edges
