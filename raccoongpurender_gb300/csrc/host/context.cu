@@ -426,12 +426,14 @@ struct rgr_context {
     // single ones
     int run_steps(int n) {
         if (n > 1 && inner()) {
+            const uint64_t before = steps;
             int r = run_first();
-            if (r == RGR_OK) r = run_inner(n - 1);
-            if (r == RGR_OK) r = run_last();
-            if (r == RGR_OK) r = run_trained(n);
-            if (r == RGR_OK) steps += n;
-            return r;
+            if (r == RGR_OK) {
+                r = run_inner(n - 1);
+                const int q = run_last();  // after an error too: the state is again one that a bounce leaves
+                if (r == RGR_OK) r = q;
+            }
+            return r == RGR_OK ? run_trained(before) : r;
         }
         while (n > 0) {
             if (graphs() && (n >= graph_steps || graph_steps == 1)) {
@@ -483,36 +485,47 @@ struct rgr_context {
         RGR_CUDA(cudaGetLastError());
         return RGR_OK;
     }
-    // `n` bounces inside the run
+    // `n` bounces inside the run; `steps` counts them
     int run_inner(int n) {
         auto one = [&] { return run_bounce(false); };
         int r = RGR_OK;
-        for (; graphs() && n >= graph_steps && r == RGR_OK; n -= graph_steps)
+        for (; graphs() && n >= graph_steps && r == RGR_OK; n -= graph_steps) {
             r = replay(inner_graph, [&] {
                 int q = RGR_OK;
                 for (int i = 0; i < graph_steps && q == RGR_OK; ++i) q = one();
                 return q;
             });
-        for (; n > 0 && r == RGR_OK; --n) r = one();
+            if (r == RGR_OK) steps += graph_steps;
+        }
+        for (; n > 0 && r == RGR_OK; --n)
+            if ((r = one()) == RGR_OK) ++steps;
         return r;
     }
-    // the logic of the run's last bounce
+    // the logic of the run's last bounce, which is then one more
     int run_last() {
+        ++steps;
         RGR_CUDA(cudaMemsetAsync(qv.tile_new, 0, sizeof(uint32_t) * ntiles, stream));
         launch_trace_logic(pv, qv, rp, render_trace, num_sms, stream);
         if (!single_render) launch_stamp_done(rp, stream);  // batches: per-request completion times
         RGR_CUDA(cudaGetLastError());
         return RGR_OK;
     }
-    // `b` bounces with a frozen guide: the end of their training intervals is bookkeeping that nothing
-    // between them reads and that leaves the same however often it is done
-    int run_trained(int b) {
+    // the bounces since `before` with a frozen guide: the end of their training intervals is bookkeeping
+    // that nothing between them reads and that leaves the same however often it is done
+    int run_trained(uint64_t before) {
         const uint64_t ti = (uint64_t)train_interval();
-        return guided && (steps + b) / ti > steps / ti ? guide->train_launches(stream) : RGR_OK;
+        return guided && steps / ti > before / ti ? guide->train_launches(stream) : RGR_OK;
     }
     // Bounces until the render is over (every path ended and the sample budget handed
     // out), looked at after every `group` bounces, at most max_steps; `*ran`: how many.
+    // The error word is there after it (check), and does not end the render early.
     int run_until_done(int group, int max_steps, int* ran, bool* over) {
+        bool open = false;  // a bounce's rays are cast and its logic is not done (run_first, run_bounce)
+        const int r = run_groups(group, max_steps, ran, over, &open);
+        if (r != RGR_OK && open) run_last();  // the state is again one that a bounce leaves
+        return r;
+    }
+    int run_groups(int group, int max_steps, int* ran, bool* over, bool* open) {
         *ran = 0;
         *over = false;
         while (*ran < max_steps && !*over) {
@@ -522,36 +535,48 @@ struct rgr_context {
             if (!inner()) {
                 if ((r = run_steps(b)) != RGR_OK) return r;
             } else {
+                const uint64_t before = steps;
                 if (*ran == 0 && (r = run_first()) != RGR_OK) return r;
+                *open = true;
                 if ((r = run_inner(b - 1)) != RGR_OK) return r;
                 if (last) {
+                    *open = false;
                     if ((r = run_last()) != RGR_OK) return r;
                 } else {
                     if ((r = run_bounce(true)) != RGR_OK) return r;
+                    ++steps;
                 }
-                if ((r = run_trained(b)) != RGR_OK) return r;
-                steps += b;
+                if ((r = run_trained(before)) != RGR_OK) return r;
             }
             *ran += b;
             if (!inner() || last) {
                 RGR_CUDA(cudaMemcpyAsync(mail->counts, counts.p, 32, cudaMemcpyDeviceToHost, stream));
                 RGR_CUDA(cudaMemcpyAsync(&mail->next_pixel, scalars.p, 8, cudaMemcpyDeviceToHost, stream));
-                if ((r = wait()) != RGR_OK) return r;
+                if ((r = settle()) != RGR_OK) return r;
                 uint64_t live = 0;
                 for (int k = 1; k < kNumQueues; ++k) live += mail->counts[k];
                 *over = mail->next_pixel >= rp.sample_limit && live == 0;
             } else {
                 RGR_CUDA(cudaMemcpyAsync(&mail->stop, in.words + InnerView::kStop, 4, cudaMemcpyDeviceToHost, stream));
-                if ((r = wait()) != RGR_OK) return r;
+                if ((r = settle()) != RGR_OK) return r;
                 *over = mail->stop != 0u;
+                *open = !*over;
             }
         }
         return RGR_OK;
     }
-    // waits for the stream; reports what the render's capacity checks found
-    int wait() {
+    // waits for the stream, and for the render's error word
+    int settle() {
         if (begun) RGR_CUDA(cudaMemcpyAsync(&mail->err, err.p, 4, cudaMemcpyDeviceToHost, stream));
         RGR_CUDA(cudaStreamSynchronize(stream));
+        return RGR_OK;
+    }
+    int wait() {
+        const int r = settle();
+        return r == RGR_OK ? check() : r;
+    }
+    // what the render's capacity checks had found when the stream was last waited for
+    int check() const {
         if (begun && mail->err) {
             set_error("device capacity check fired (flags " + std::to_string(mail->err) + ")");
             return RGR_E_OVERFLOW;
@@ -752,7 +777,7 @@ int rgr_render_until_done(rgr_context* c, int32_t max_steps, int32_t* steps_done
     int r = c->run_until_done(8, max_steps, &done, &over);
     if (r != RGR_OK) return r;
     if (steps_done) *steps_done = done;
-    return done ? RGR_OK : c->wait();  // each group of bounces ends with a wait
+    return done ? c->check() : c->wait();  // each group of bounces ends with a wait
 }
 
 namespace {
