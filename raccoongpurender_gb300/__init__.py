@@ -820,10 +820,10 @@ class Batch:
         _check(self._lib.rgr_set_render_tuning(self._lib.rgr_batch_context(self._h), shade_blocks_per_sm,
                                                graph_steps), "rgr_set_render_tuning")
 
-    def set_render_trace(self, refill: int = 12) -> None:
-        """Refill threshold of the bounce's persistent closest-hit kernel (the
-        kernel is chosen by the paths in flight, as for a single render)."""
-        _check(self._lib.rgr_set_render_trace(self._lib.rgr_batch_context(self._h), -1, refill),
+    def set_render_trace(self, refill: int = 12, persistent=-1) -> None:
+        """Refill threshold of the bounce's closest hits, and how they are cast: as
+        WavefrontLane.set_render_trace's `persistent`."""
+        _check(self._lib.rgr_set_render_trace(self._lib.rgr_batch_context(self._h), int(persistent), refill),
                "rgr_set_render_trace")
 
     def set_trace_search(self, render: int = 8) -> None:
