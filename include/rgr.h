@@ -329,9 +329,9 @@ int rgr_set_render_tuning(rgr_context* c, int32_t shade_blocks_per_sm, int32_t g
 
 /* Launch shape of the closest-hit kernel: refill a warp with new rays when at
    least `refill` of its 32 lanes are idle (1..32); `blocks_per_sm` resident
-   256-thread blocks per SM (0 = as many as fit).  Until set, 24 lanes, and in
-   large calls 12 for a warp whose rays head into several octants.  Chosen by the
-   autotuner. */
+   256-thread blocks per SM (0 = as many as fit).  The default, 24, is the library's
+   own choice: 24 lanes, and in large calls 12 for a warp whose rays head into several
+   octants; any other value holds for every warp.  Chosen by the autotuner. */
 int rgr_set_trace_tuning(rgr_context* c, int32_t refill, int32_t blocks_per_sm);
 
 /* How a bounce casts its extension rays: persistent = 1 runs a persistent
@@ -351,8 +351,9 @@ int rgr_set_render_trace(rgr_context* c, int32_t persistent, int32_t refill);
    one).  `closest` sets the closest-hit kernel (rgr_trace_closest*),
    `render` the extension rays of a render's bounces (takes effect at the
    next rgr_render_begin); 0 leaves that one unchanged.  Results are
-   identical for every value.  Default 8 (in large closest-hit calls 12 for a warp
-   whose rays head into several octants) and 8; chosen by the autotuner. */
+   identical for every value.  Default 8 (closest hits: the library's own choice, 8
+   and in large calls 12 for a warp whose rays head into several octants) and 8;
+   chosen by the autotuner. */
 int rgr_set_trace_search(rgr_context* c, int32_t closest, int32_t render);
 
 /* Shared-memory staging of the closest-hit kernel: each CTA copies the first

@@ -54,4 +54,24 @@ inline uint32_t cast_blocks(uint64_t pool, uint32_t half_end) {
     return (uint32_t)((half + kCastSpan / 2 - 1) / (kCastSpan / 2) + (rest + kCastSpan - 1) / kCastSpan);
 }
 
+// A warp of the closest-hit kernels takes new rays when `refill` of its lanes are idle, and its
+// lanes take node steps while `search` of them still search for their leaf; in large calls
+// (not sorted, staged or across the link) a warp whose rays head into several octants goes by
+// the mixed pair.  The defaults: 24 and 8 the best of 1..32 and 1..24 for camera rays (3702 Mrays/s;
+// 3319 with every lane waiting for the last), 12 and 12 for rays in all directions (k_trace_rays).
+struct CastTuning {
+    int refill = 24, search = 8, mixed_refill = 12, mixed_search = 12;
+};
+// A caller's value holds for every warp; the default value gives both pairs theirs back.
+inline void set_refill(CastTuning& t, int refill) {
+    const CastTuning d;
+    t.refill = refill;
+    t.mixed_refill = refill == d.refill ? d.mixed_refill : refill;
+}
+inline void set_search(CastTuning& t, int search) {
+    const CastTuning d;
+    t.search = search;
+    t.mixed_search = search == d.search ? d.mixed_search : search;
+}
+
 }  // namespace rgr

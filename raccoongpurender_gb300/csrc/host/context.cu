@@ -231,9 +231,7 @@ struct rgr_context {
     int trace_host_mode = RGR_TRACE_HOST_AUTO;  // rgr_trace_closest: zero copy where it can, or staged copies
     int cast_blocks[2] = {1, 1};  // resident blocks an SM of the bounce's cast: scenes by request, one scene
     int trace_grid = 0;      // persistent traversal grid (SMs x resident blocks)
-    // 24 and 8 the best of 1..32 and 1..24 for camera rays (3702 Mrays/s; 3319 with every lane waiting for
-    // the last), 12 and 12 for rays in all directions (k_trace_rays)
-    CastTuning trace_tuning{24, 8, 12, 12};
+    CastTuning trace_tuning;
     int trace_blocks = 0;    // resident blocks per SM asked for (0: as many as fit)
     // extension rays of a bounce: persistent refilling kernel, then logic (or fused)
     // refill 12: the mixed 1080p render at 2^24 paths runs 1047.7 / 1066.6 / 1067.6 / 1066.5 /
@@ -1009,7 +1007,7 @@ int rgr_set_trace_tuning(rgr_context* c, int32_t refill, int32_t blocks_per_sm) 
     RGR_CUDA(cudaSetDevice(c->device));
     int maxb = std::max(1, trace_rays_max_blocks_per_sm(c->trace_stage));
     if (blocks_per_sm > maxb) return RGR_E_INVALID;
-    c->trace_tuning.refill = c->trace_tuning.mixed_refill = refill;
+    set_refill(c->trace_tuning, refill);
     c->trace_blocks = blocks_per_sm;
     c->trace_grid = c->num_sms * (blocks_per_sm ? blocks_per_sm : maxb);
     const int maxb0 = std::max(1, trace_rays_max_blocks_per_sm(0));
@@ -1028,7 +1026,7 @@ int rgr_set_render_trace(rgr_context* c, int32_t persistent, int32_t refill) {
 
 int rgr_set_trace_search(rgr_context* c, int32_t closest, int32_t render) {
     if (!c || closest < 0 || closest > 32 || render < 0 || render > 32) return RGR_E_INVALID;
-    if (closest > 0) c->trace_tuning.search = c->trace_tuning.mixed_search = closest;
+    if (closest > 0) set_search(c->trace_tuning, closest);
     if (render > 0 && render != c->render_trace.search) {
         c->render_trace.search = render;
         c->begun = false;  // takes effect at the next render begin

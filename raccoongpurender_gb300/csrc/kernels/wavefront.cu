@@ -28,7 +28,6 @@
 
 #include <algorithm>
 
-#include "../host/choices.h"
 #include "wavefront.cuh"
 #include "traverse.cuh"
 #include "guide.cuh"

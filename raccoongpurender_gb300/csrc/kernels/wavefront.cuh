@@ -1,6 +1,7 @@
 // wavefront.cuh — device data of the wavefront renderer and the launchers
 // that the host orchestration (context.cu) calls.
 #pragma once
+#include "../host/choices.h"
 #include "rgr_device.cuh"
 
 namespace rgr {
@@ -353,13 +354,6 @@ void launch_merge_intermediate(void* a, const void* b, uint32_t n, cudaStream_t 
 // stage: inner nodes (the breadth-first top of the tree) each CTA copies to
 // shared memory, 0..kMaxStagedNodes
 constexpr uint32_t kMaxStagedNodes = 1024;
-// A warp of the closest-hit kernels takes new rays when `refill` of its lanes are idle, and its
-// lanes take node steps while `search` of them still search for their leaf; in large calls
-// (not sorted, staged or across the link) a warp whose rays head into several octants goes by
-// the mixed pair.
-struct CastTuning {
-    int refill, search, mixed_refill, mixed_search;
-};
 void launch_trace_rays(const SceneView& sc, const float* ox, const float* oy, const float* oz, const float* dx,
                        const float* dy, const float* dz, const float* tmax, uint64_t n, int32_t* prim, float* t,
                        float* ng, uint32_t* err, unsigned long long* counter, const CastTuning& tune, int grid,

@@ -16,6 +16,12 @@ extern "C" uint32_t half_end(uint64_t pool, uint64_t samples, uint32_t resident,
     return rgr::cast_half_end(pool, samples, resident, tile);
 }
 extern "C" int per_slot(uint32_t prims) { return rgr::per_slot_cast(prims); }
+extern "C" void tuning(int refill, int search, int* out) {  // 0: not set
+    rgr::CastTuning t;
+    if (refill) rgr::set_refill(t, 31), rgr::set_refill(t, refill);
+    if (search) rgr::set_search(t, 31), rgr::set_search(t, search);
+    out[0] = t.refill, out[1] = t.search, out[2] = t.mixed_refill, out[3] = t.mixed_search;
+}
 extern "C" uint32_t blocks(uint64_t pool, uint32_t half_end) { return rgr::cast_blocks(pool, half_end); }
 """
 
@@ -64,3 +70,21 @@ def test_fused_blocks_cover_the_pool(choices, pool, samples):
 
 def test_small_scenes_cast_per_slot(choices):
     assert [choices.per_slot(n) for n in (0, 36, 1024, 1025, 1 << 27)] == [1, 1, 1, 0, 0]
+
+
+def test_tuned_thresholds(choices):
+    """A caller who sets the defaults has the library's own thresholds, for warps of one octant and
+    of several; so has the autotuner's first trial."""
+    from raccoongpurender_gb300 import autotune
+
+    def tuning(refill, search):
+        out = (C.c_int * 4)()
+        choices.tuning(refill, search, out)
+        return tuple(out)
+
+    untouched = tuning(0, 0)
+    assert untouched == (24, 8, 12, 12)
+    d = autotune.TRACE_DEFAULTS
+    assert tuning(d["trace_refill"], d["trace_search"]) == untouched
+    assert tuning(16, 0) == (16, 8, 16, 12) and tuning(0, 4) == (24, 4, 12, 4)
+    assert tuning(12, 12) == (12, 12, 12, 12) and tuning(32, 1) == (32, 1, 32, 1)
