@@ -584,7 +584,7 @@ class WavefrontLane:
         _check(self._lib.rgr_trace_closest(self._h, C.byref(r), n, _ptr(prim), _ptr(t)), "rgr_trace_closest")
         return prim, t
 
-    def set_render_tuning(self, shade_blocks_per_sm: int = 8, graph_steps: int = 1) -> None:
+    def set_render_tuning(self, shade_blocks_per_sm: int = 4, graph_steps: int = 1) -> None:
         _check(self._lib.rgr_set_render_tuning(self._h, shade_blocks_per_sm, graph_steps), "rgr_set_render_tuning")
 
     def set_guide(self, guide: "Guide | None") -> None:
@@ -593,7 +593,7 @@ class WavefrontLane:
         _check(self._lib.rgr_context_set_guide(self._h, guide.handle if guide is not None else None),
                "rgr_context_set_guide")
 
-    def set_trace_tuning(self, refill: int = 16, blocks_per_sm: int = 0) -> None:
+    def set_trace_tuning(self, refill: int = 24, blocks_per_sm: int = 0) -> None:
         _check(self._lib.rgr_set_trace_tuning(self._h, refill, blocks_per_sm), "rgr_set_trace_tuning")
 
     def set_render_trace(self, persistent=-1, refill: int = 12) -> None:
@@ -816,7 +816,7 @@ class Batch:
         _check(self._lib.rgr_batch_readback(self._h, rid, RGR_FMT_RGBA8, _ptr(out), out.nbytes), "rgr_batch_readback")
         return out
 
-    def set_render_tuning(self, shade_blocks_per_sm: int = 8, graph_steps: int = 8) -> None:
+    def set_render_tuning(self, shade_blocks_per_sm: int = 4, graph_steps: int = 1) -> None:
         _check(self._lib.rgr_set_render_tuning(self._lib.rgr_batch_context(self._h), shade_blocks_per_sm,
                                                graph_steps), "rgr_set_render_tuning")
 

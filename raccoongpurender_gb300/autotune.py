@@ -2,7 +2,8 @@
 
 Knobs (all results are bit-identical across knob values; only speed changes):
   * path_count     — resident paths in the pool (queue capacities follow it);
-  * graph_steps    — bounces per replayed CUDA graph;
+  * graph_steps    — bounces between two looks at whether a batch is over
+                     (and per CUDA graph, where one is replayed);
   * shade_blocks   — resident 256-thread blocks per SM of the shade kernel;
   * render_refill  — refill a warp of the bounce's persistent trace kernel
                      when this many lanes are idle;
@@ -30,7 +31,7 @@ import os
 import time
 from pathlib import Path
 
-DEFAULTS = dict(path_count=1 << 22, graph_steps=8, shade_blocks=8, render_refill=12, render_search=8)
+DEFAULTS = dict(path_count=1 << 22, graph_steps=8, shade_blocks=4, render_refill=12, render_search=8)
 CANDIDATES = dict(path_count=[1 << 20, 1 << 21, 1 << 22, 1 << 23, 1 << 24], graph_steps=[4, 8, 16], shade_blocks=[4, 8, 16],
                   render_refill=[8, 16, 24], render_search=[4, 12, 16])
 TRACE_DEFAULTS = dict(trace_reorder=0, trace_refill=24, trace_search=8, trace_stage=0)

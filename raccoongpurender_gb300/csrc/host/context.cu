@@ -210,8 +210,7 @@ struct rgr_context {
     uint64_t steps = 0;
     uint32_t npix = 0;
     int shade_grid = 0;
-    // what is resident: a preview frame 2604 us with 8, 2566 with 4, the mixed render 69.45 and 69.07 ms
-    int shade_blocks_per_sm = 4;
+    int shade_blocks_per_sm = kShadeBlocksPerSm;
     // CUDA graph of `graph_steps` bounces
     int graph_mode = -1;  // replay captured bounces: 0 no, 1 yes, -1 where that is the faster (graphs)
     int graph_steps = 1;

@@ -22,6 +22,7 @@ extern "C" void tuning(int refill, int search, int* out) {  // 0: not set
     if (search) rgr::set_search(t, 31), rgr::set_search(t, search);
     out[0] = t.refill, out[1] = t.search, out[2] = t.mixed_refill, out[3] = t.mixed_search;
 }
+extern "C" int shade_blocks() { return rgr::kShadeBlocksPerSm; }
 extern "C" uint32_t blocks(uint64_t pool, uint32_t half_end) { return rgr::cast_blocks(pool, half_end); }
 """
 
@@ -88,3 +89,29 @@ def test_tuned_thresholds(choices):
     assert tuning(d["trace_refill"], d["trace_search"]) == untouched
     assert tuning(16, 0) == (16, 8, 16, 12) and tuning(0, 4) == (24, 4, 12, 4)
     assert tuning(12, 12) == (12, 12, 12, 12) and tuning(32, 1) == (32, 1, 32, 1)
+
+
+def test_defaults_agree(choices):
+    """The Python setters called without arguments, and the autotuner's starting points, are what
+    the library does untouched."""
+    import inspect
+
+    import raccoongpurender_gb300 as rg
+    from raccoongpurender_gb300 import autotune
+
+    def default(f, name):
+        return inspect.signature(f).parameters[name].default
+
+    out = (C.c_int * 4)()
+    choices.tuning(0, 0, out)
+    refill, search = out[0], out[1]
+    blocks = choices.shade_blocks()
+    for cls in (rg.WavefrontLane, rg.Batch):
+        assert default(cls.set_render_tuning, "shade_blocks_per_sm") == blocks
+        assert default(cls.set_render_tuning, "graph_steps") == 1  # rgr_context's graph_steps_default
+        assert default(cls.set_render_trace, "refill") == autotune.DEFAULTS["render_refill"] == 12
+        assert default(cls.set_render_trace, "persistent") == -1
+        assert default(cls.set_trace_search, "render") == autotune.DEFAULTS["render_search"] == 8
+    assert autotune.DEFAULTS["shade_blocks"] == blocks
+    assert default(rg.WavefrontLane.set_trace_tuning, "refill") == refill
+    assert default(rg.WavefrontLane.set_trace_search, "closest") == search
