@@ -74,6 +74,17 @@ inline void set_search(CastTuning& t, int search) {
     t.mixed_search = search == d.search ? d.mixed_search : search;
 }
 
+// Blocks of the closest-hit kernels: with staged nodes, and without (calls of few rays, sorted
+// ones and those across the link stage none, whatever is set).  blocks: resident ones an SM
+// asked for, 0 for as many as fit.
+struct TraceGrids {
+    int staged, plain;
+};
+inline TraceGrids trace_grids(int sms, int blocks, int fit_staged, int fit_plain) {
+    auto grid = [&](int fit) { return sms * (blocks ? std::min(blocks, fit) : fit); };
+    return TraceGrids{grid(fit_staged), grid(fit_plain)};
+}
+
 // Resident blocks an SM of the shading kernels until rgr_set_render_tuning: what is resident.  A
 // preview frame 2604 us with 8, 2566 with 4, the mixed render 69.45 and 69.07 ms.
 constexpr int kShadeBlocksPerSm = 4;

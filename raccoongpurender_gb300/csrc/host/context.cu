@@ -229,7 +229,7 @@ struct rgr_context {
     cudaStream_t tstream[kTraceSlots] = {};  // [0] unused: slot 0 runs on `stream`
     int trace_host_mode = RGR_TRACE_HOST_AUTO;  // rgr_trace_closest: zero copy where it can, or staged copies
     int cast_blocks[2] = {1, 1};  // resident blocks an SM of the bounce's cast: scenes by request, one scene
-    int trace_grid = 0;      // persistent traversal grid (SMs x resident blocks)
+    TraceGrids grids{0, 0};  // of the closest-hit kernels
     CastTuning trace_tuning;
     int trace_blocks = 0;    // resident blocks per SM asked for (0: as many as fit)
     // extension rays of a bounce: persistent refilling kernel, then logic (or fused)
@@ -240,7 +240,6 @@ struct rgr_context {
     int render_trace_mode = -1;  // 1 persistent, 0 fused, -1 by the paths in flight, at render begin
     uint32_t trace_stage = 0;  // top BVH nodes staged in shared memory per CTA
     int trace_reorder = 0;     // rgr_trace_closest_device sorts the rays first
-    int packed_grid = 0;       // its traversal grid (no staged nodes)
     DevBuf tbins, trank, tpacked;  // its bucket counts, the rays' ranks, the reordered 32-byte records
     // learned path guiding: the attached network and this render's per-slot buffers
     rgr_guide* guide = nullptr;
@@ -254,6 +253,10 @@ struct rgr_context {
             if (s) cudaStreamDestroy(s);
         if (stream) cudaStreamDestroy(stream);
         give_mail(mail);
+    }
+    void set_grids() {
+        grids = trace_grids(num_sms, trace_blocks, std::max(1, trace_rays_max_blocks_per_sm(trace_stage)),
+                            std::max(1, trace_rays_max_blocks_per_sm(0)));
     }
     // the resident path pool: state, queues, counters (WavefrontLane::setup, :451-522)
     int alloc_pool() {
@@ -669,8 +672,7 @@ int rgr_context_create(rgr_context** out, int32_t device, uint32_t path_count) {
         return RGR_E_CUDA;
     }
     cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device);
-    c->trace_grid = c->num_sms * std::max(1, trace_rays_max_blocks_per_sm());
-    c->packed_grid = c->trace_grid;
+    c->set_grids();
     for (int one = 0; one < 2; ++one) c->cast_blocks[one] = trace_paths_max_blocks_per_sm(one != 0);
     c->npaths = path_count;
     c->ntiles = (path_count + kTile - 1) / kTile;
@@ -970,14 +972,13 @@ int rgr_trace_closest_device(rgr_context* c, const rgr_ray_soa* rays, uint64_t n
                            c->tbins.as<uint32_t>(), c->trank.as<uint32_t>(), c->tpacked.as<float4>(),
                            c->num_sms * 64, st);
         launch_trace_packed(c->scene.sv, c->tpacked.as<float4>(), n, prim, t, ng_xyz, c->err.as<uint32_t>(),
-                            c->tcounter.as<unsigned long long>(), c->trace_tuning, c->packed_grid,
-                            st);
+                            c->tcounter.as<unsigned long long>(), c->trace_tuning, c->grids.plain, st);
         RGR_CUDA(cudaGetLastError());
         return RGR_OK;
     }
     launch_trace_rays(c->scene.sv, rays->ox, rays->oy, rays->oz, rays->dx, rays->dy, rays->dz, rays->tmax, n, prim, t, ng_xyz,
-                      c->err.as<uint32_t>(), c->tcounter.as<unsigned long long>(), c->trace_tuning,
-                      c->trace_grid, c->trace_stage, st);
+                      c->err.as<uint32_t>(), c->tcounter.as<unsigned long long>(), c->trace_tuning, c->grids,
+                      c->trace_stage, st);
     RGR_CUDA(cudaGetLastError());
     return RGR_OK;
 }
@@ -1008,9 +1009,7 @@ int rgr_set_trace_tuning(rgr_context* c, int32_t refill, int32_t blocks_per_sm) 
     if (blocks_per_sm > maxb) return RGR_E_INVALID;
     set_refill(c->trace_tuning, refill);
     c->trace_blocks = blocks_per_sm;
-    c->trace_grid = c->num_sms * (blocks_per_sm ? blocks_per_sm : maxb);
-    const int maxb0 = std::max(1, trace_rays_max_blocks_per_sm(0));
-    c->packed_grid = c->num_sms * (blocks_per_sm ? std::min(blocks_per_sm, maxb0) : maxb0);
+    c->set_grids();
     return RGR_OK;
 }
 
@@ -1049,9 +1048,8 @@ int rgr_set_trace_reorder(rgr_context* c, int32_t reorder) {
 int rgr_set_trace_staging(rgr_context* c, uint32_t staged_nodes) {
     if (!c || staged_nodes > kMaxStagedNodes) return RGR_E_INVALID;
     RGR_CUDA(cudaSetDevice(c->device));
-    int maxb = std::max(1, trace_rays_max_blocks_per_sm(staged_nodes));
     c->trace_stage = staged_nodes;
-    c->trace_grid = c->num_sms * (c->trace_blocks ? std::min(c->trace_blocks, maxb) : maxb);
+    c->set_grids();
     return RGR_OK;
 }
 
@@ -1067,7 +1065,7 @@ int rgr_trace_closest_counts_device(rgr_context* c, const rgr_ray_soa* rays, uin
     if ((r = c->tcounter.alloc(8)) != RGR_OK) return r;
     launch_trace_rays_counts(c->scene.sv, rays->ox, rays->oy, rays->oz, rays->dx, rays->dy, rays->dz, rays->tmax, n, prim, t,
                              node_visits, prim_tests, c->err.as<uint32_t>(), c->tcounter.as<unsigned long long>(),
-                             c->trace_grid, st);
+                             c->grids.plain, st);
     RGR_CUDA(cudaGetLastError());
     return RGR_OK;
 }
@@ -1121,7 +1119,7 @@ int rgr_trace_closest(rgr_context* c, const rgr_ray_soa* rays, uint64_t n, int32
             c->mail->link_err = 0u;
             cudaStream_t st = c->stream;
             launch_trace_rays_link(c->scene.sv, dsrc, n, dprim, dt, &c->mail->link_err, ts.counter.as<unsigned long long>(),
-                                   c->trace_tuning, c->trace_grid, st);
+                                   c->trace_tuning, c->grids.plain, st);
             RGR_CUDA(cudaGetLastError());
             populate({prim, t}, 4 * n);
             RGR_CUDA(cudaStreamSynchronize(st));
@@ -1158,7 +1156,8 @@ int rgr_trace_closest(rgr_context* c, const rgr_ray_soa* rays, uint64_t n, int32
         launch_trace_rays(c->scene.sv, ts.rays[0].as<float>(), ts.rays[1].as<float>(), ts.rays[2].as<float>(),
                           ts.rays[3].as<float>(), ts.rays[4].as<float>(), ts.rays[5].as<float>(),
                           ts.rays[6].as<float>(), m, ts.prim.as<int32_t>(), ts.t.as<float>(), nullptr,
-                          ts.err.as<uint32_t>(), ts.counter.as<unsigned long long>(), c->trace_tuning, c->trace_grid, c->trace_stage, st);
+                          ts.err.as<uint32_t>(), ts.counter.as<unsigned long long>(), c->trace_tuning, c->grids,
+                          c->trace_stage, st);
         RGR_CUDA(cudaGetLastError());
         RGR_CUDA(cudaMemcpyAsync(prim + off, ts.prim.p, 4 * m, cudaMemcpyDeviceToHost, st));
         RGR_CUDA(cudaMemcpyAsync(t + off, ts.t.p, 4 * m, cudaMemcpyDeviceToHost, st));

@@ -454,17 +454,17 @@ uint32_t spread(uint64_t n, int grid, int* blocks, unsigned long long* counter, 
 
 void launch_trace_rays(const SceneView& sc, const float* ox, const float* oy, const float* oz, const float* dx,
                        const float* dy, const float* dz, const float* tmax, uint64_t n, int32_t* prim, float* t,
-                       float* ng, uint32_t* err, unsigned long long* counter, const CastTuning& tune, int grid,
-                       uint32_t stage, cudaStream_t st) {
+                       float* ng, uint32_t* err, unsigned long long* counter, const CastTuning& tune,
+                       const TraceGrids& grids, uint32_t stage, cudaStream_t st) {
     if (n == 0) return;
     int blocks;
-    const uint32_t share = spread(n, grid, &blocks, counter, st);
+    const uint32_t share = spread(n, grids.plain, &blocks, counter, st);
     RayBatch b{ox, oy, oz, dx, dy, dz, tmax, nullptr, n, prim, t, ng, nullptr, nullptr, err, counter, share, tune,
                stage};
     if (share)
         chain(k_trace_rays<false, false, false, true, false>, blocks, kStackThreads, 0, st, sc, b);
     else if (stage > 0)
-        k_trace_rays<false, true, false, false, false><<<blocks, kStackThreads, 64 * (size_t)stage, st>>>(sc, b);
+        k_trace_rays<false, true, false, false, false><<<grids.staged, kStackThreads, 64 * (size_t)stage, st>>>(sc, b);
     else
         k_trace_rays<false, false, false, false, false><<<blocks, kStackThreads, 0, st>>>(sc, b);
 }

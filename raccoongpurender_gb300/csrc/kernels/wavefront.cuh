@@ -356,8 +356,8 @@ void launch_merge_intermediate(void* a, const void* b, uint32_t n, cudaStream_t 
 constexpr uint32_t kMaxStagedNodes = 1024;
 void launch_trace_rays(const SceneView& sc, const float* ox, const float* oy, const float* oz, const float* dx,
                        const float* dy, const float* dz, const float* tmax, uint64_t n, int32_t* prim, float* t,
-                       float* ng, uint32_t* err, unsigned long long* counter, const CastTuning& tune, int grid,
-                       uint32_t stage, cudaStream_t st);
+                       float* ng, uint32_t* err, unsigned long long* counter, const CastTuning& tune,
+                       const TraceGrids& grids, uint32_t stage, cudaStream_t st);
 // the same for rays and results in host memory that the GPU reads and writes across a coherent link
 void launch_trace_rays_link(const SceneView& sc, const float* const* rays, uint64_t n, int32_t* prim, float* t,
                             uint32_t* err, unsigned long long* counter, const CastTuning& tune, int grid,

@@ -23,6 +23,10 @@ extern "C" void tuning(int refill, int search, int* out) {  // 0: not set
     out[0] = t.refill, out[1] = t.search, out[2] = t.mixed_refill, out[3] = t.mixed_search;
 }
 extern "C" int shade_blocks() { return rgr::kShadeBlocksPerSm; }
+extern "C" void grids(int sms, int blocks, int staged, int plain, int* out) {
+    const rgr::TraceGrids g = rgr::trace_grids(sms, blocks, staged, plain);
+    out[0] = g.staged, out[1] = g.plain;
+}
 extern "C" uint32_t blocks(uint64_t pool, uint32_t half_end) { return rgr::cast_blocks(pool, half_end); }
 """
 
@@ -115,3 +119,14 @@ def test_defaults_agree(choices):
     assert autotune.DEFAULTS["shade_blocks"] == blocks
     assert default(rg.WavefrontLane.set_trace_tuning, "refill") == refill
     assert default(rg.WavefrontLane.set_trace_search, "closest") == search
+
+
+@pytest.mark.parametrize("blocks,staged,plain,want", [
+    (0, 5, 5, (760, 760)),
+    (0, 2, 5, (304, 760)),  # staged nodes leave room for fewer blocks; calls that stage none keep theirs
+    (3, 2, 5, (304, 456)), (2, 3, 5, (304, 304)),
+])
+def test_grids(choices, blocks, staged, plain, want):
+    out = (C.c_int * 2)()
+    choices.grids(152, blocks, staged, plain, out)
+    assert tuple(out) == want
