@@ -161,13 +161,15 @@ RequestD request_d(const SceneView& sv, const rgr_camera& cam, const rgr_render_
 // take a 64 KB page at a time far slower than the CPU does, or under the copy's.  It runs
 // beside the GPU's work, all arrays from the front, as closest hits arrive: 1M hits into
 // new arrays 2950 us without, 670 with it before the launch, 426 beside the kernel (256 KB
-// at a time; 1 MB: 495); into old ones 400 / 413 / 400.
+// at a time; 1 MB: 495); into old ones 400 / 413 / 400.  Only ordinary memory: managed pages would
+// move to the host from under the kernel (1M hits 2061 us, left alone 388).  Null: none.
 void populate(std::initializer_list<void*> arrays, size_t bytes) {
 #ifdef MADV_POPULATE_WRITE
     const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
     const size_t chunk = 256u << 10;
     for (size_t o = 0; o < bytes; o += chunk)
         for (void* p : arrays) {
+            if (!p) continue;
             const uintptr_t from = ((uintptr_t)p + o) / page * page, to = (uintptr_t)p + std::min(o + chunk, bytes);
             madvise((void*)from, to - from, MADV_POPULATE_WRITE);  // where it cannot, the pages still fault
         }
@@ -1079,14 +1081,17 @@ namespace {
 // page-locked (or registered) host memory has a device address; on a system
 // whose GPU walks the host's page tables (NVLink-C2C with address
 // translation) any host address is one.
-void* device_view(const void* p, bool pageable_ok) {
+// `plain`: whether it is ordinary memory, neither page-locked nor the runtime's.
+void* device_view(const void* p, bool pageable_ok, bool* plain = nullptr) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
-    if (a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged || a.type == cudaMemoryTypeDevice)
-        return a.devicePointer;
+    const bool known =
+        a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged || a.type == cudaMemoryTypeDevice;
+    if (plain) *plain = !known;
+    if (known) return a.devicePointer;
     return pageable_ok ? const_cast<void*>(p) : nullptr;
 }
 
@@ -1111,8 +1116,9 @@ int rgr_trace_closest(rgr_context* c, const rgr_ray_soa* rays, uint64_t n, int32
         const float* dsrc[7];
         bool direct = true;
         for (int k = 0; k < 7 && direct; ++k) direct = (dsrc[k] = (const float*)device_view(src[k], pageable)) != nullptr;
-        int32_t* dprim = direct ? (int32_t*)device_view(prim, pageable) : nullptr;
-        float* dt = direct ? (float*)device_view(t, pageable) : nullptr;
+        bool prim_plain = false, t_plain = false;
+        int32_t* dprim = direct ? (int32_t*)device_view(prim, pageable, &prim_plain) : nullptr;
+        float* dt = direct ? (float*)device_view(t, pageable, &t_plain) : nullptr;
         if (direct && dprim && dt) {
             rgr_context::TraceSlot& ts = c->tslot[0];
             if ((r = ts.counter.alloc(8)) != RGR_OK) return r;
@@ -1121,7 +1127,7 @@ int rgr_trace_closest(rgr_context* c, const rgr_ray_soa* rays, uint64_t n, int32
             launch_trace_rays_link(c->scene.sv, dsrc, n, dprim, dt, &c->mail->link_err, ts.counter.as<unsigned long long>(),
                                    c->trace_tuning, c->grids.plain, st);
             RGR_CUDA(cudaGetLastError());
-            populate({prim, t}, 4 * n);
+            populate({prim_plain ? prim : nullptr, t_plain ? t : nullptr}, 4 * n);
             RGR_CUDA(cudaStreamSynchronize(st));
             if (c->mail->link_err) {
                 set_error("traversal stack overflow");
