@@ -201,23 +201,35 @@ def render_bench(dev_index: int, which: str, repeats: int = 2, pools=(1 << 22,))
             "config": f"{camd['w']}x{camd['h']}, {spp} spp, max depth {depth}, {mesh.ntris} triangles"}
 
 
-# Algorithmic bytes per extension segment of the wavefront render (the state
-# each stage uses, in 16-byte vectors of the slot records), traversal
-# excluded.  Per shaded queue item: the item (4), request id (2), material
-# reference (8), ro, rd, T, L, ng and RNG in (6 x 16) and out (6 x 16), the
-# volume list in (32); the persistent trace: the item (4), ro and rd in (32),
-# ng, t and the volume hit out (24); the logic: queue id (1), request id (2),
-# rd, ng, T, L and RNG in (5 x 16), T, L and RNG out (3 x 16), queue id and
-# queue item out (5); the new-path compaction: the queue id of a slot (1).
-RENDER_STATE_BYTES = (4 + 2 + 8 + 96 + 96 + 32) + (4 + 32 + 24) + (1 + 2 + 80 + 48 + 5) + 1
+def render_state_bytes(ended: float, listed: float, entered: float) -> float:
+    """Path-state bytes per extension segment of the wavefront render inside a
+    run of bounces, as its kernels use the slot records (32-byte sectors: the
+    ray, (T, L), (ng, RNG), the volume list), traversal excluded.  `ended`: the
+    share of segments that end their path; of the others, `listed` are in a
+    volume or meet one (the list is read), `entered` meet one (it is written).
+
+    The cast: the queue item, the ray and (T, L), the hit's sector out, the
+    next queue's id.  Classification: the id, then a 2-byte entry of an ended
+    path or a 4-byte queue item.  New paths, per ended one: the entry, the
+    request id, three sectors in and out, the queue item, the request id out.
+    Shading, per path that goes on: the queue item, request id, material
+    reference, three sectors in and out, the volume list.  (The roulette's look
+    at the RNG in the cast, the hit normals' table and the first and last
+    bounce of a run are left out.)"""
+    cast = 4 + 64 + 32 + 1
+    classify = 1 + 2 * ended + 4 * (1 - ended)
+    new_paths = 2 + 2 + 96 + 96 + 4 + 2
+    shade = 4 + 2 + 8 + 96 + 96 + 32 * listed + 32 * entered
+    return cast + classify + ended * new_paths + (1 - ended) * shade
 
 
 def render_roofline(dev_index: int, mrays_s: float, mpaths_s: float, l2_gbs: float, hbm_gbs: float) -> dict:
     """Roofline of the mixed 1080p render: bytes per extension segment = the
-    path-state traffic the stages use (RENDER_STATE_BYTES) + 64 per BVH
-    node visited + 48 per primitive tested, the counts measured by the
-    instrumented closest-hit kernel on the extension rays of the render's
-    third bounce (2^22 resident paths).  The state streams from HBM, the tree
+    path-state traffic the kernels use (render_state_bytes, with the share of
+    ended paths measured over the whole render and that of volume lists on
+    the third bounce) + 64 per BVH node visited + 48 per primitive tested, the
+    counts measured by the instrumented closest-hit kernel on the extension
+    rays of the render's third bounce (2^22 resident paths).  The state streams from HBM, the tree
     from L2; both fractions are stated, against the HBM copy rate and the L2
     read rate measured in this run.  The FP64 accumulation (32 bytes per
     finished path) is counted per path."""
@@ -255,10 +267,15 @@ def render_roofline(dev_index: int, mrays_s: float, mpaths_s: float, l2_gbs: flo
     nv, pt = float(nodes.double().mean()), float(prims.double().mean())
     trav = 64.0 * nv + 48.0 * pt
     seg = mrays_s * 1e6
-    state_gbs = (seg * RENDER_STATE_BYTES + mpaths_s * 1e6 * 32) / 1e9
+    queue = np.asarray(sl["queue"])
+    material = queue > 0
+    entered = queue[material] == 5  # a volume's surface (kMatVolume)
+    listed = entered | (np.asarray(sl["vol_count"])[material] > 0)
+    state = render_state_bytes(mpaths_s / mrays_s, float(listed.mean()), float(entered.mean()))
+    state_gbs = (seg * state + mpaths_s * 1e6 * 32) / 1e9
     trav_gbs = seg * trav / 1e9
     return {"rays_sampled": n, "nodes_per_ray": round(nv, 2), "prims_per_ray": round(pt, 2),
-            "state_bytes_per_segment": RENDER_STATE_BYTES, "traversal_bytes_per_segment": round(trav, 1),
+            "state_bytes_per_segment": round(state, 1), "traversal_bytes_per_segment": round(trav, 1),
             "state_gbs": round(state_gbs, 1), "state_frac_of_hbm": round(state_gbs / hbm_gbs, 4),
             "traversal_gbs": round(trav_gbs, 1), "traversal_frac_of_l2": round(trav_gbs / l2_gbs, 4),
             "time_frac_of_bound": round((state_gbs / hbm_gbs + trav_gbs / l2_gbs), 4),
@@ -270,8 +287,8 @@ def batch_bench(dev_index: int, n: int = 32) -> dict:
     """Batched uneven requests: n requests (square side log-uniform 64..1024,
     spp log-uniform 1..256, 1k..2M triangles, full-render material mix and
     envmap, half with a volume box) rendered to completion in one shared path
-    pool, shortest request first, bounce loop replayed from a CUDA graph;
-    pool size, graph length, shade grid and trace refill from the autotuner."""
+    pool, shortest request first; pool size, bounces between two looks at the
+    outcome, shade grid and trace refill from the autotuner."""
     import numpy as np
     import raccoongpurender_gb300 as rg
     from raccoongpurender_gb300 import autotune, scenes
