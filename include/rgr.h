@@ -338,10 +338,10 @@ int rgr_set_trace_tuning(rgr_context* c, int32_t refill, int32_t blocks_per_sm);
    closest-hit kernel over the slots just shaded whose warps take new slots
    when at least `refill` (1..32, default 12) lanes are idle, then the logic
    kernel; persistent = 0 casts and runs the logic in one kernel (a block per
-   256 or 512 slots, in scenes of at most 1024 primitives a thread per slot); persistent = -1 (default) picks 1 where at least 3 * 2^17 paths can
-   be in flight (the pool's, or the sample budget where that is less).  Results are
-   identical.  Takes effect at the next
-   rgr_render_begin. */
+   256 or 512 slots, in scenes of at most 1024 primitives a thread per slot);
+   persistent = -1 (default) picks 1 where at least 3 * 2^17 paths can be in
+   flight (the pool's, or the sample budget where that is less).  Results are
+   identical.  Takes effect at the next rgr_render_begin. */
 int rgr_set_render_trace(rgr_context* c, int32_t persistent, int32_t refill);
 
 /* Leaf batching of the persistent traversal kernels: within a round a warp's

@@ -1,8 +1,8 @@
 // context.cu — the device half of the C ABI: upload, render loop, readback,
 // ray-cast service.  Replaces rt::WavefrontLane
-// (common/wavefront_path_tracing.hpp:339-1153) on one GPU.  The per-bounce
-// launch sequence is captured once into a CUDA graph and replayed, instead of
-// the reference's ~24 enqueued NDRange launches per bounce.
+// (common/wavefront_path_tracing.hpp:339-1153) on one GPU.  A bounce is three
+// to five dependent launches instead of the reference's ~24 enqueued NDRange
+// launches; renders that train a guide replay theirs from a CUDA graph (graphs).
 #include <cuda_runtime.h>
 #include <sys/mman.h>
 #include <unistd.h>
@@ -182,12 +182,12 @@ void populate(std::initializer_list<void*> arrays, size_t bytes) {
 // the copies of some overlap the traversal of another (measured end to end
 // on the closest-hit workload: 2 slots 2500 Mrays/s, 3: 2647, 4: 2705-2728,
 // 6: 2682, 8: 2627; 8 slots of 2^19 rays: 2749)
+constexpr int kTraceSlots = 4;
 // rgr_trace_closest_device sorts the rays, where asked to, from this many on: the
 // sort's launches cost 21 us, and a call of fewer is bound by its longest rays.  Random rays
 // in 1.31M triangles, sorted / unsorted: 1 K 104 / 60 us, 20 K 160 / 123, 60 K 241 / 222,
 // 400 K 332 / 309, 1M 467 / 464, 4M 1178 / 1241 (from 2^16 to 1M the caller's choice stands).
 constexpr uint64_t kReorderMinRays = 1ull << 16;
-constexpr int kTraceSlots = 4;
 
 struct rgr_context {
     int device = 0;
@@ -423,9 +423,8 @@ struct rgr_context {
         RGR_CUDA(cudaGraphLaunch(g.exec, st));
         return RGR_OK;
     }
-    // run `n` bounces.  A render that records nothing takes the bounces inside the run by
-    // run_bounce; otherwise replays of a graph of graph_steps bounces, then
-    // single ones
+    // run `n` bounces: without logic passes between them where that is the choice (inner);
+    // otherwise replays of a graph of graph_steps bounces (graphs), then single ones
     int run_steps(int n) {
         if (n > 1 && inner()) {
             const uint64_t before = steps;
@@ -463,10 +462,11 @@ struct rgr_context {
     // and 2613), a guided one with a frozen guide 6299 and 6314 (its first 8752 and 7199); where the
     // guide trains, with more launches a bounce, a replay is the faster.
     bool graphs() const { return graph_mode < 0 ? guided && !inner() : graph_mode != 0; }
-    // the first bounce of a run up to its rays' cast
+    // whether a run's bounces go without a logic pass (launch_inner_queues)
     bool inner() const {
         return render_trace.persistent && (!guided || (!rp.gd.record && guide->frozen()));
     }
+    // the first bounce of a run up to its rays' cast
     int run_first() {
         cudaStream_t st = stream;
         launch_compact_new(pv, qv, render_trace.counter, st);
@@ -1203,9 +1203,9 @@ int rgr_debug_read_slots(rgr_context* c, uint32_t* out, uint64_t nslots) {
 // Batched requests: many renders of uneven size share one path pool.  Each
 // request owns a range of the global sample index (in run order), so the
 // new-path compaction hands free slots to the requests in that order and a
-// slot renders its request's scene with its camera and constants.  The
-// bounce loop is replayed from a CUDA graph; every request's last finished
-// path stamps %globaltimer, giving per-request completion latency.
+// slot renders its request's scene with its camera and constants.  Every
+// request's last finished path stamps %globaltimer, giving per-request
+// completion latency.
 struct rgr_batch {
     rgr_context* ctx = nullptr;
     struct Req {

@@ -83,7 +83,8 @@ struct LinkRuns {
 };
 
 // From this many rays on a warp's octants choose its thresholds (CastTuning): a warp of a call
-// of fewer takes rays a few times only (300,000 random rays in 20 K triangles 112 us, 116 so).
+// of fewer takes rays a few times only (300,000 random rays in 20 K triangles 112 us, 116 with
+// thresholds of its own).
 constexpr uint64_t kMixedMinRays = 1ull << 19;
 
 // kFew: each lane takes one ray of its warp's share, without the rounds
@@ -213,11 +214,11 @@ __global__ void __launch_bounds__(256, RGR_TRACE_MIN_BLOCKS) k_trace_rays(SceneV
         }
     };
     if (!kFew) {
-        // Rays of one octant keep together in large batches (camera rays, ms: refill / search 24 / 8
-        // 0.81, 12 / 12 0.87); others part at once, and full lanes count for more (random
-        // rays 1.18 and 1.13; in a scene of 1280 triangles 0.199 and 0.185).  The warp looks at rays
-        // about where its first will be; chosen anew at each refill it cost registers, and 0.09 ms.
-        // Sorted rays: 1.13 with 24 / 8, 1.16 where a warp's own octants decide.
+        // Rays of one octant keep together in large batches (4M camera rays in 1.31M triangles, calls in
+        // a row: refill / search 24 / 8 658 us, 12 / 12 721); others part at once, and full lanes
+        // count for more (random rays 1098 and 1036; in a scene of 1280 triangles 700 and 633).  The
+        // warp looks at rays about where its first will be; chosen anew at each refill it cost
+        // registers, and a tenth of the camera rays' time.  Sorted rays: 999 with 24 / 8, 1040 with 12 / 12.
         bool mixed = false;
         if (!kCount && !kStaged && !kLink && !kPacked && b.n >= kMixedMinRays) {
             const uint64_t r = (uint64_t)blockIdx.x * kStackThreads + threadIdx.x;

@@ -44,8 +44,9 @@ constexpr int kSmemStack = RGR_SMEM_STACK;
 constexpr int kStackThreads = 256;  // block size of the kernels that use it
 // A persistent warp that finds no more work and holds at most this many rays leaves the
 // rounds, and each of its lanes goes through its ray alone with the next links in L1
-// (kFew).  A cast ends in 200 to 270 us of few long rays; random rays at 4 / 8 / 12 lanes
-// 1226 / 1221 / 1223 us (1238 without), the mixed render's casts likewise.
+// (kFew).  A cast ends in 200 to 270 us of few long rays; 4M random rays in 1.31M triangles, calls in a
+// row, at 4 / 8 / 12 lanes 1039 / 1036 / 1034 us (1045 without), each waited for 1152 / 1144 / 1147
+// (1216), the mixed render's casts likewise.
 constexpr int kTailLanes = 8;
 constexpr uint32_t kDone = 0xffffffffu;
 constexpr uint32_t kErrStackOverflow = 1u;
@@ -336,8 +337,8 @@ RGR_DEV void trace_round_t(const SceneView& sc, TraceState& s, TraceCounters* cn
     s.link = link;
 }
 
-// kSm: stack entries in shared memory (s.sstk set), 0 for a local-memory stack; kFew: see touch
-template <bool kCount, bool kStaged = false, int kSm = 0, bool kFew = false>
+// kSm: stack entries in shared memory (s.sstk set; with RGR_SMEM_STACK=0 none); kFew: see touch
+template <bool kCount, bool kStaged, int kSm, bool kFew = false>
 RGR_DEV void trace_round(const SceneView& sc, TraceState& s, TraceCounters* cnt, uint32_t& err, uint64_t pol,
                          StagedNodes st = StagedNodes{nullptr, 0u}) {
     if (s.nan_free) {

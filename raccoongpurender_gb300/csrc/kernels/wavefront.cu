@@ -1011,8 +1011,7 @@ RGR_DEV float guide_write(const GuideRenderD& gd, uint32_t slot, const GuideOffe
 // shading kernel reads them, less the new-path slots it retired — by
 // persistent warps that hand finished lanes the next items (one atomic per
 // refill per warp), as the closest-hit service kernel does with rays.  Runs
-// between the shading kernel and the queue resets.  A hit writes the ray's
-// sector once: t into P.ro.w and the primitive, as -2 - prim, into the volume-hit
+// after the shading kernel.  A hit writes the ray's sector once: t into P.ro.w and the primitive, as -2 - prim, into the volume-hit
 // field P.rd.w (its readers take a negative id as none); the logic kernel computes
 // Ng into P.ng.  A miss leaves P.ng.w at the -1 the shading stage wrote.  Each slot may belong
 // to another request (scene).
@@ -1398,7 +1397,7 @@ template <bool kGuided, bool kOne>
 __global__ void __launch_bounds__(kLogicThreads, kCastLogicBlocks)
     k_slot_logic(PathsView P, QueueView Q, RenderParams rp, SceneView one) {
     follow();
-    __shared__ uint32_t s_stack[kSmemStack * kStackThreads];
+    __shared__ uint32_t s_stack[(kSmemStack > 0 ? kSmemStack : 1) * kStackThreads];
     const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = slot < P.n && P.qid[slot] != kQueueIdle;
     uint32_t err = 0;

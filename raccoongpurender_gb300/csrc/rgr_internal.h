@@ -57,7 +57,6 @@ inline uint32_t make_leaf_link(uint32_t first, uint32_t count) {
 //   sphere:   (center.xyz, word) (radius, 0, 0, flag 1) (0)
 // word: the primitive id (below 2^28), and in bits 28..30 its material type (1..5),
 // so that a render's cast knows the queue of a hit without another gather
-constexpr uint32_t kPrimIdMask = 0x0fffffffu;
 inline uint32_t prim_word(uint32_t id, int32_t type) { return id | (uint32_t)type << 28; }
 struct alignas(16) PrimD {
     float a[4];
