@@ -199,7 +199,7 @@ struct rgr_context {
     DevBuf slots, qid, req, queues[kNumQueues], counts, tile_new, scalars, accum, err;
     DevBuf inner_words, inner_tiles, inner_ended;  // the bounces inside a run (launch_inner_queues)
     InnerView in{};
-    Mail* mail = nullptr;
+    MailSlot mail;
     DevBuf reqtab, done;  // request table and its per-request (done, done_ns) counters
     PathsView pv{};
     QueueView qv{};
@@ -254,7 +254,6 @@ struct rgr_context {
         for (cudaStream_t s : tstream)
             if (s) cudaStreamDestroy(s);
         if (stream) cudaStreamDestroy(stream);
-        give_mail(mail);
     }
     void set_grids() {
         grids = trace_grids(num_sms, trace_blocks, std::max(1, trace_rays_max_blocks_per_sm(trace_stage)),
@@ -669,7 +668,7 @@ int rgr_context_create(rgr_context** out, int32_t device, uint32_t path_count) {
     c->device = device;
     if (!cuda_ok(cudaSetDevice(device), "cudaSetDevice") ||
         !cuda_ok(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "cudaStreamCreate") ||
-        !(c->mail = take_mail())) {
+        !c->mail.take()) {
         delete c;
         return RGR_E_CUDA;
     }

@@ -239,7 +239,7 @@ int rgr_guide_create(rgr_guide** out, int32_t device, const rgr_guide_config* cf
         delete g;
         return RGR_E_CUDA;
     }
-    int r = (g->mail = take_mail()) ? g->init(c) : (int)RGR_E_CUDA;
+    int r = g->mail.take() ? g->init(c) : (int)RGR_E_CUDA;
     if (r != RGR_OK) {
         delete g;
         return r;

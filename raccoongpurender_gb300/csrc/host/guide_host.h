@@ -19,8 +19,7 @@ struct rgr_guide {
     rgr::dev::GuideTrainD train{};  // the render's stream (counter bytes 0..27)
     rgr::dev::GuideTrainD test{};   // rgr_guide_train_device's (bytes 32..59; shares iter)
     bool bounds_set = false;
-    rgr::Mail* mail = nullptr;  // the last training step's loss
-    ~rgr_guide() { rgr::give_mail(mail); }
+    rgr::MailSlot mail;  // the last training step's loss
 
     int init(const rgr_guide_config& c);
     int set_bounds(const float lo[3], const float hi[3]);

@@ -17,34 +17,71 @@ struct Mail {
     float loss;         // a guide's training step's, written by its kernel
 };
 // Pinning a page takes some 120 us and a context 15 to create, so the first 64 contexts and
-// guides of the process share one allocation; a further one has its own.
+// guides that live at a time share one allocation, which the process keeps; a further one has its
+// own.  cudaDeviceReset frees the page with everything else of the process: the next slot is then
+// of a new page, and slots of the old one are forgotten.
 constexpr int kSharedMails = 64;
-inline std::mutex mail_mutex;
-inline Mail* shared_mails = nullptr;
-inline uint64_t shared_taken = 0;  // a bit each
+struct MailPage {
+    std::mutex mutex;
+    Mail* mails = nullptr;
+    uint64_t taken = 0;  // a bit each
+    uint64_t age = 0;    // pages before this one
+};
+inline MailPage mail_page;
 
-inline Mail* take_mail() {
-    std::lock_guard<std::mutex> lock(mail_mutex);
-    Mail* m = nullptr;
-    if (!shared_mails && !cuda_ok(cudaHostAlloc(&shared_mails, sizeof(Mail) * kSharedMails, cudaHostAllocPortable),
-                                  "cudaHostAlloc")) {
-        shared_mails = nullptr;
-        return nullptr;
-    }
-    for (int k = 0; k < kSharedMails; ++k)
-        if (!((shared_taken >> k) & 1u)) {
-            shared_taken |= 1ull << k;
-            return shared_mails + k;
+inline bool is_pinned(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    return false;
+}
+
+class MailSlot {
+public:
+    MailSlot() = default;
+    MailSlot(const MailSlot&) = delete;
+    MailSlot& operator=(const MailSlot&) = delete;
+    ~MailSlot() { give(); }  // nothing in flight writes to it
+    bool take() {
+        MailPage& page = mail_page;
+        std::lock_guard<std::mutex> lock(page.mutex);
+        if (page.mails && !is_pinned(page.mails)) {
+            page.mails = nullptr;
+            page.taken = 0;
+            ++page.age;
         }
-    return cuda_ok(cudaHostAlloc(&m, sizeof(Mail), cudaHostAllocPortable), "cudaHostAlloc") ? m : nullptr;
-}
-inline void give_mail(Mail* m) {  // nothing in flight writes to it
-    if (!m) return;
-    std::lock_guard<std::mutex> lock(mail_mutex);
-    if (m >= shared_mails && m < shared_mails + kSharedMails)
-        shared_taken &= ~(1ull << (m - shared_mails));
-    else
-        cudaFreeHost(m);
-}
+        if (!page.mails &&
+            !cuda_ok(cudaHostAlloc(&page.mails, sizeof(Mail) * kSharedMails, cudaHostAllocPortable), "cudaHostAlloc")) {
+            page.mails = nullptr;
+            return false;
+        }
+        age_ = page.age;
+        for (index_ = 0; index_ < kSharedMails; ++index_)
+            if (!((page.taken >> index_) & 1u)) {
+                page.taken |= 1ull << index_;
+                mail_ = page.mails + index_;
+                return true;
+            }
+        if (!cuda_ok(cudaHostAlloc(&mail_, sizeof(Mail), cudaHostAllocPortable), "cudaHostAlloc")) mail_ = nullptr;
+        return mail_ != nullptr;
+    }
+    Mail* operator->() const { return mail_; }
+
+private:
+    void give() {
+        if (!mail_) return;
+        MailPage& page = mail_page;
+        std::lock_guard<std::mutex> lock(page.mutex);
+        if (index_ == kSharedMails) {
+            if (is_pinned(mail_)) cudaFreeHost(mail_);
+        } else if (age_ == page.age) {
+            page.taken &= ~(1ull << index_);
+        }
+        mail_ = nullptr;
+    }
+    Mail* mail_ = nullptr;
+    int index_ = 0;  // in the page; kSharedMails: an allocation of its own
+    uint64_t age_ = 0;
+};
 
 }  // namespace rgr
